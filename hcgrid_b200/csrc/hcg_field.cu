@@ -38,7 +38,7 @@ __global__ void k_sample_keys(HpxParams h, uint64_t n, const double *__restrict_
         double theta = dsub(kHalfPi, dmul(kDeg2Rad, la));
         double phi = dmul(kDeg2Rad, lo);
         int hard;
-        uint64_t k = ang2pix(h, theta, phi, hard);
+        uint64_t k = ang2pix_quick(h, theta, phi, hard);
         if (hard) atomicAdd(&stats->hard_roundings, 1ULL);
         keys[i] = k;
         idx[i] = (uint32_t)i;

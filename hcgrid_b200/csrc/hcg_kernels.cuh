@@ -59,10 +59,10 @@ __device__ __forceinline__ void prep_item(HpxParams h, uint64_t firstring, uint6
     double utheta = dsub(disc_theta, disc);
     if (dmul(utheta, kRad2Deg) < 0) utheta = 0;
     int hard1, hard2;
-    uint64_t uring = pix2ring(h, ang2pix(h, utheta, disc_phi, hard1));
+    uint64_t uring = pix2ring(h, ang2pix_quick(h, utheta, disc_phi, hard1));
     if (uring < firstring) uring = firstring;
     utheta = dadd(disc_theta, disc);
-    uint64_t dring = pix2ring(h, ang2pix(h, utheta, disc_phi, hard2));
+    uint64_t dring = pix2ring(h, ang2pix_quick(h, utheta, disc_phi, hard2));
     if (dring >= firstring + usedrings) dring = firstring + usedrings - 1;
     if (hard1 | hard2) atomicAdd(&stats->hard_roundings, 1ULL);
     P.ur = (int)(uring - firstring);

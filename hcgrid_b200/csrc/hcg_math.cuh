@@ -258,6 +258,49 @@ HCG_HD uint64_t ang2pix(const HpxParams &h, double theta, double phi, int &hard)
     return loc2pix(h, c, phi, 0., false);
 }
 
+// The same pixel without the double-double cosine, for nearly every input.
+// A pixel index depends on cos(theta) only through two truncations (jp, jm)
+// and the cap / equator choice. cos() is within 3e-16 of the correctly
+// rounded value, which moves jp's and jm's arguments by less than 4e-15 nside
+// (equator) or 4e-14 nside (caps, |z| < 0.99, where 1 - |z| keeps 14 digits);
+// where both lie further than that from an integer, and z away from 2/3, the
+// truncations are the same and so is the index. Everything else takes
+// ang2pix. What bounds it: FP64 issue; the double-double series costs about
+// 500 FP64 operations an angle, this about 60.
+HCG_HD uint64_t ang2pix_quick(const HpxParams &h, double theta, double phi, int &hard) {
+    hard = 0;
+    if (theta > 0.02 && theta < 3.12 && h.order > 0 && h.order <= 26) {
+        const double z = cos(theta), za = fabs(z), ns = u2d(h.nside);
+        const bool eq = za < 0.6666666;
+        if (eq || (za > 0.6666667 && za < 0.99)) {
+            const double tt = fmodulo(dmul(phi, kInvHalfPi), 4.0);
+            double a, b;
+            if (eq) {
+                const double temp1 = dmul(ns, dadd(0.5, tt)), temp2 = dmul(dmul(ns, z), 0.75);
+                a = dsub(temp1, temp2);
+                b = dadd(temp1, temp2);
+            } else {
+                const double tp = dsub(tt, floor(tt)), tmp = dmul(ns, dsqrt(dmul(3., dsub(1., za))));
+                a = dmul(tp, tmp);
+                b = dmul(dsub(1.0, tp), tmp);
+            }
+            const double fa = floor(a), fb = floor(b), eps = dmul(ns, eq ? 4e-15 : 4e-14);
+            const double ra = dsub(a, fa), rb = dsub(b, fb), top = dsub(1.0, eps);
+            if (ra > eps && ra < top && rb > eps && rb < top && fa >= 0.0) {
+                const uint64_t jp = d2u(fa), jm = d2u(fb);
+                if (eq) {
+                    const uint64_t nl4 = 4 * h.nside, ir = h.nside + 1 + jp - jm, kshift = 1 - (ir & 1);
+                    const uint64_t t1 = jp + jm + kshift + 1 + nl4 + nl4 - h.nside;
+                    return h.ncap + (ir - 1) * nl4 + ((t1 >> 1) & (nl4 - 1));
+                }
+                const uint64_t ir = jp + jm + 1, ip = d2u(dmul(tt, u2d(ir)));
+                return z > 0 ? 2 * ir * (ir - 1) + ip : h.npix - 2 * ir * (ir + 1) + ip;
+            }
+        }
+    }
+    return ang2pix(h, theta, phi, hard);
+}
+
 // healpix.cu:227-273: location of a pixel centre (z, phi, sin theta).
 HCG_HD void pix2loc(const HpxParams &h, uint64_t pix, double &z, double &phi, double &sth, bool &have_sth) {
     have_sth = false;
