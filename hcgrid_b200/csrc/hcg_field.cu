@@ -12,6 +12,8 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "hcg_internal.h"
@@ -20,141 +22,339 @@ namespace hcg {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;
 
+// Range of the keys as two maxima that start at zero: of ~key and of key.
 struct KeyRange {
-    unsigned long long kmin, kmax;
+    unsigned long long nmin, kmax;
 };
 
-__global__ void k_sample_keys(HpxParams h, uint64_t n, const double *__restrict__ lon, const double *__restrict__ lat,
-                              uint64_t *__restrict__ keys, uint32_t *__restrict__ idx, KeyRange *range,
-                              DevStats *stats) {
-    uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    unsigned long long kmin = ~0ULL, kmax = 0;
-    if (i < n) {
-        double lo = lon[i], la = lat[i];
+// A resident grid of blocks sweeps the samples, so that the range costs two
+// atomics a block: one pair per warp (125,000 on one address for 4,000,000
+// samples) held the kernel at 175 us.
+__global__ void __launch_bounds__(256) k_sample_keys(HpxParams h, uint64_t n, const double *__restrict__ lon,
+                                                     const double *__restrict__ lat, uint64_t *__restrict__ keys,
+                                                     KeyRange *range, DevStats *stats) {
+    __shared__ unsigned long long s_nmin[8], s_kmax[8];
+    unsigned long long nmin = 0, kmax = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const double lo = lon[i], la = lat[i];
         if (!isfinite(lo) || !isfinite(la) || fabs(la) > 90.0) atomicAdd(&stats->invalid_input, 1ULL);
-        double theta = dsub(kHalfPi, dmul(kDeg2Rad, la));
-        double phi = dmul(kDeg2Rad, lo);
+        const double theta = dsub(kHalfPi, dmul(kDeg2Rad, la));
+        const double phi = dmul(kDeg2Rad, lo);
         int hard;
-        uint64_t k = ang2pix_quick(h, theta, phi, hard);
+        const uint64_t k = ang2pix_quick(h, theta, phi, hard);
         if (hard) atomicAdd(&stats->hard_roundings, 1ULL);
         keys[i] = k;
-        idx[i] = (uint32_t)i;
-        kmin = kmax = k;
+        nmin = max(nmin, ~(unsigned long long)k);
+        kmax = max(kmax, (unsigned long long)k);
     }
-    // warp then block min/max
     for (int o = 16; o; o >>= 1) {
-        kmin = min(kmin, __shfl_xor_sync(0xffffffffu, kmin, o));
+        nmin = max(nmin, __shfl_xor_sync(0xffffffffu, nmin, o));
         kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicMin(&range->kmin, kmin);
+        s_nmin[threadIdx.x >> 5] = nmin;
+        s_kmax[threadIdx.x >> 5] = kmax;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            nmin = max(nmin, s_nmin[w]);
+            kmax = max(kmax, s_kmax[w]);
+        }
+        atomicMax(&range->nmin, nmin);
         atomicMax(&range->kmax, kmax);
     }
 }
 
-__global__ void k_init_range(KeyRange *r) {
-    r->kmin = ~0ULL;
-    r->kmax = 0;
+// ---------------------------------------------------------------------------
+// Stable LSD radix sort of (key, input index), 8 bits a pass over the bits in
+// which the keys differ (key - kmin; 32-bit words whenever they fit, which they
+// do for every field smaller than about a quarter of the sky at nside 8192).
+// Per pass: k_rs_hist (digit counts of each tile), k_rs_scan (a block per digit
+// scans the tiles' counts) and k_rs_scatter. What bounds a pass is the
+// scattered writes; sorting a tile by digit in shared memory first makes them
+// runs of consecutive positions. 4,000,000 keys in four passes: 0.23 ms
+// (1.17 ms with a one-block scan of the 250,000 counts and four block barriers
+// per 256 keys).
+//
+// One tile: each warp ranks kItems x 32 consecutive items with
+// ballots against its own digit counters (no block barrier inside),
+// then the warps' counts are scanned per digit. Item order is (warp, round,
+// lane) = input order, so equal digits keep it.
+constexpr int kSortWarps = kSortThreads / 32;
+
+// rank of this lane's digit among the warp's items so far; `cnt` is the warp's
+// counter row. Inactive lanes have no counter.
+template <typename CNT>
+__device__ __forceinline__ uint32_t warp_rank(CNT *cnt, uint32_t d, bool valid) {
+    const int lane = threadIdx.x & 31;
+    // lanes with the same digit, by its bits: eight votes that overlap (a
+    // match instruction takes a turn per distinct digit)
+    unsigned peers = __ballot_sync(0xffffffffu, valid);
+    if (!valid) peers = ~peers;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+        const unsigned bal = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+        peers &= (d >> b) & 1u ? bal : ~bal;
+    }
+    const int leader = __ffs(peers) - 1;
+    uint32_t old = 0;
+    if (valid && lane == leader) {
+        old = cnt[d];
+        cnt[d] = (CNT)(old + __popc(peers));
+    }
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, old, leader) + __popc(peers & ((1u << lane) - 1u));
 }
 
-// Per-tile digit histogram, stored digit-major: hist[d * nblocks + b].
-__global__ void __launch_bounds__(kSortThreads) k_rs_hist(const uint64_t *__restrict__ keys, uint64_t n, int shift,
-                                                         uint64_t kmin, uint32_t *__restrict__ hist,
-                                                         uint32_t nblocks) {
-    __shared__ uint32_t h[8][256];
-    int warp = threadIdx.x >> 5;
-    for (int d = threadIdx.x; d < 256 * 8; d += kSortThreads) (&h[0][0])[d] = 0;
-    __syncthreads();
-    uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-#pragma unroll 4
-    for (int j = 0; j < kSortItems; ++j) {
-        uint64_t i = base + (uint64_t)j * kSortThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[warp][((keys[i] - kmin) >> shift) & 255], 1u);
+// exclusive scan of one value per thread over the first 256 threads of a
+// block; every thread of the block calls it
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t *s_w) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
     }
+    if (lane == 31 && w < 8) s_w[w] = incl;
     __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += kSortThreads) {
-        uint32_t s = 0;
-        for (int w = 0; w < 8; ++w) s += h[w][d];
-        hist[(uint64_t)d * nblocks + blockIdx.x] = s;
-    }
+    uint32_t before = 0;
+    for (int i = 0; i < w && i < 8; ++i) before += s_w[i];
+    __syncthreads();  // s_w may be written again
+    return before + incl - v;
 }
 
-// In-place exclusive scan of n uint32 values by one block of 1024 threads.
-__global__ void __launch_bounds__(1024) k_scan_u32_1block(uint32_t *data, uint64_t n) {
-    __shared__ uint32_t part[1024];
-    uint64_t per = (n + 1023) / 1024;
-    uint64_t b = threadIdx.x * per, e = min(n, b + per);
+// Digit counts of each tile, digit-major (hist[d * nblocks + b]), and of all
+// tiles (total[d]).
+template <typename KIn, int kItems>
+__global__ void __launch_bounds__(kSortThreads) k_rs_hist(const KIn *__restrict__ keys, uint64_t n, int shift,
+                                                         uint64_t kmin, uint32_t *__restrict__ hist, uint32_t nblocks,
+                                                         unsigned long long *__restrict__ total) {
+    __shared__ uint32_t h[kSortWarps][256];
+    const int warp = threadIdx.x >> 5;
+    for (int d = threadIdx.x; d < 256 * kSortWarps; d += kSortThreads) (&h[0][0])[d] = 0;
+    __syncthreads();
+    const uint64_t base = (uint64_t)blockIdx.x * (kSortThreads * kItems);
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        const uint64_t i = base + (uint64_t)j * kSortThreads + threadIdx.x;
+        if (i < n) atomicAdd(&h[warp][(uint32_t)(((uint64_t)keys[i] - kmin) >> shift) & 255u], 1u);
+    }
+    __syncthreads();
+    const int d = threadIdx.x;
     uint32_t s = 0;
-    for (uint64_t i = b; i < e; ++i) s += data[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        uint32_t v = (threadIdx.x >= o) ? part[threadIdx.x - o] : 0;
+    for (int w = 0; w < kSortWarps; ++w) s += h[w][d];
+    hist[(uint64_t)d * nblocks + blockIdx.x] = s;
+    if (s) atomicAdd(total + d, (unsigned long long)s);
+}
+
+// Block d: the tiles' counts of digit d -> their first output positions.
+__global__ void __launch_bounds__(256) k_rs_scan(uint32_t *__restrict__ hist, uint32_t nblocks,
+                                                 const unsigned long long *__restrict__ total) {
+    __shared__ uint32_t s_w[8];
+    __shared__ uint32_t s_tot;
+    const int tid = threadIdx.x;
+    const uint32_t d = blockIdx.x;
+    uint32_t run = 0;
+    {
+        const uint32_t ex = scan256((uint32_t)total[tid], s_w);
+        if (tid == (int)d) s_tot = ex;
         __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
+        run = s_tot;
     }
-    uint32_t run = part[threadIdx.x] - s;
-    for (uint64_t i = b; i < e; ++i) {
-        uint32_t v = data[i];
-        data[i] = run;
-        run += v;
+    uint32_t *row = hist + (uint64_t)d * nblocks;
+    for (uint32_t c = 0; c < nblocks; c += 256) {
+        const uint32_t i = c + tid;
+        const uint32_t v = i < nblocks ? row[i] : 0u;
+        const uint32_t ex = scan256(v, s_w);
+        if (i < nblocks) row[i] = run + ex;
+        if (tid == 255) s_tot = ex + v;
+        __syncthreads();
+        run += s_tot;
+        __syncthreads();
     }
 }
 
-// Stable scatter: items are ranked in index order (round, warp, lane), the
-// rank among equal digits coming from __match_any_sync within a warp and a
-// per-digit running count across warps and rounds.
-__global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const uint64_t *__restrict__ kin,
+// Input keys are kin[i] - kmin (the first pass reads the samples' keys, and
+// their indices are i: vin null); output keys are kout = that + kadd (the last
+// pass writes the samples' keys).
+template <typename KIn, typename KOut, int kItems>
+__global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const KIn *__restrict__ kin,
                                                             const uint32_t *__restrict__ vin,
-                                                            uint64_t *__restrict__ kout, uint32_t *__restrict__ vout,
-                                                            uint64_t n, int shift, uint64_t kmin,
+                                                            KOut *__restrict__ kout, uint32_t *__restrict__ vout,
+                                                            uint64_t n, int shift, uint64_t kmin, uint64_t kadd,
                                                             const uint32_t *__restrict__ offs, uint32_t nblocks) {
-    __shared__ uint32_t s_off[256];
-    __shared__ uint32_t s_run[256];
-    __shared__ uint32_t s_cnt[8][256];
-    int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int d = tid; d < 256; d += kSortThreads) {
-        s_off[d] = offs[(uint64_t)d * nblocks + blockIdx.x];
-        s_run[d] = 0;
+    using K = typename std::conditional<sizeof(KIn) == 4 || sizeof(KOut) == 4, uint32_t, uint64_t>::type;
+    constexpr int kTile = kSortThreads * kItems;
+    __shared__ uint32_t s_cnt[kSortWarps][256];
+    __shared__ uint32_t s_base[256], s_w[8];
+    __shared__ K s_key[kTile];
+    __shared__ uint32_t s_val[kTile];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    for (int d = tid; d < kSortWarps * 256; d += kSortThreads) (&s_cnt[0][0])[d] = 0;
+    const uint64_t base = (uint64_t)blockIdx.x * kTile, first = base + (uint64_t)warp * (32 * kItems) + lane;
+    K key[kItems];
+    uint32_t val[kItems], rank[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        const uint64_t i = first + 32 * j;
+        key[j] = i < n ? (K)((uint64_t)kin[i] - kmin) : 0;
+        val[j] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0;
     }
-    for (int d = tid; d < 8 * 256; d += kSortThreads) (&s_cnt[0][0])[d] = 0;
     __syncthreads();
-    uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-    unsigned lt = (1u << lane) - 1u;
-    for (int r = 0; r < kSortItems; ++r) {
-        uint64_t i = base + (uint64_t)r * kSortThreads + tid;
-        bool valid = i < n;
-        uint64_t k = valid ? kin[i] : 0;
-        uint32_t v = valid ? vin[i] : 0;
-        uint32_t d = valid ? (uint32_t)(((k - kmin) >> shift) & 255) : 0x1000u;
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        uint32_t rank = __popc(peers & lt);
-        if (valid && rank == 0) s_cnt[warp][d] = __popc(peers);
-        __syncthreads();
-        if (tid < 256) {
-            uint32_t run = s_run[tid];
-            for (int w = 0; w < 8; ++w) {
-                uint32_t c = s_cnt[w][tid];
-                s_cnt[w][tid] = run;
-                run += c;
-            }
-            s_run[tid] = run;
-        }
-        __syncthreads();
-        if (valid) {
-            uint32_t pos = s_off[d] + s_cnt[warp][d] + rank;
-            kout[pos] = k;
-            vout[pos] = v;
-        }
-        __syncthreads();
-        if (tid < 256)
-            for (int w = 0; w < 8; ++w) s_cnt[w][tid] = 0;
-        __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        const bool valid = first + 32 * j < n;
+        rank[j] = warp_rank(s_cnt[warp], (uint32_t)(key[j] >> shift) & 255u, valid);
     }
+    __syncthreads();
+    uint32_t cnt = 0;
+    for (int w = 0; w < kSortWarps; ++w) {
+        const uint32_t c = s_cnt[w][tid];
+        s_cnt[w][tid] = cnt;
+        cnt += c;
+    }
+    const uint32_t start = scan256(cnt, s_w);
+    for (int w = 0; w < kSortWarps; ++w) s_cnt[w][tid] += start;
+    s_base[tid] = offs[(uint64_t)tid * nblocks + blockIdx.x] - start;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+        if (first + 32 * j < n) {
+            const uint32_t p = s_cnt[warp][(uint32_t)(key[j] >> shift) & 255u] + rank[j];
+            s_key[p] = key[j];
+            s_val[p] = val[j];
+        }
+    }
+    __syncthreads();
+    const uint32_t m = n - base < (uint64_t)kTile ? (uint32_t)(n - base) : (uint32_t)kTile;
+    for (uint32_t p = tid; p < m; p += kSortThreads) {
+        const K k = s_key[p];
+        const uint32_t dst = s_base[(uint32_t)(k >> shift) & 255u] + p;
+        kout[dst] = (KOut)((uint64_t)k + kadd);
+        vout[dst] = s_val[p];
+    }
+}
+
+// The whole sort of at most kSmallSort keys in one block: the items stay in
+// registers between passes and cross shared memory once a pass. Latency is all
+// there is at this size: 10,000 keys in three passes take 35 us here against
+// 84 us in nine launches of three blocks each.
+constexpr int kSmallThreads = 1024, kSmallItems = 16;
+constexpr uint64_t kSmallSort = (uint64_t)kSmallThreads * kSmallItems;
+constexpr size_t kSmallSmem = kSmallSort * 8 + (kSmallThreads / 32) * 256 * sizeof(uint16_t);
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const uint64_t *__restrict__ kin,
+                                                              uint64_t *__restrict__ kout,
+                                                              uint32_t *__restrict__ vout, uint32_t n, int passes,
+                                                              uint64_t kmin) {
+    extern __shared__ uint32_t s_small[];
+    uint32_t *s_key = s_small, *s_val = s_key + kSmallSort;
+    uint16_t(*s_cnt)[256] = reinterpret_cast<uint16_t(*)[256]>(s_val + kSmallSort);
+    __shared__ uint32_t s_w[8], s_start[256], s_part[4][256];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // rounds a warp takes: its items are consecutive, so unused rounds are skipped for every warp
+    const uint32_t rounds = (n + kSmallThreads - 1) / kSmallThreads, first = warp * 32 * rounds + lane;
+    uint32_t key[kSmallItems], val[kSmallItems], rank[kSmallItems];
+#pragma unroll
+    for (int j = 0; j < kSmallItems; ++j) {
+        const uint32_t i = first + 32 * j;
+        key[j] = j < (int)rounds && i < n ? (uint32_t)(kin[i] - kmin) : 0;
+        val[j] = i;
+    }
+    for (int p = 0; p < passes; ++p) {
+        const int shift = 8 * p;
+        for (int d = tid; d < (kSmallThreads / 32) * 256; d += kSmallThreads) (&s_cnt[0][0])[d] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kSmallItems; ++j) {
+            if (j >= (int)rounds) break;
+            const bool valid = first + 32 * j < n;
+            rank[j] = warp_rank(s_cnt[warp], (key[j] >> shift) & 255u, valid);
+        }
+        __syncthreads();
+        // per digit, the warps' counts in four quarters of eight warps
+        const uint32_t d = tid & 255, w0 = (tid >> 8) * 8;
+        uint32_t cnt = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) cnt += s_cnt[w0 + w][d];
+        s_part[tid >> 8][d] = cnt;
+        __syncthreads();
+        uint32_t start = scan256(tid < 256 ? s_part[0][d] + s_part[1][d] + s_part[2][d] + s_part[3][d] : 0u, s_w);
+        if (tid < 256) s_start[d] = start;
+        __syncthreads();
+        start = s_start[d];
+        for (int q = 0; q < (tid >> 8); ++q) start += s_part[q][d];
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t c = s_cnt[w0 + w][d];
+            s_cnt[w0 + w][d] = (uint16_t)start;
+            start += c;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kSmallItems; ++j) {
+            if (j < (int)rounds && first + 32 * j < n) {
+                const uint32_t q = s_cnt[warp][(key[j] >> shift) & 255u] + rank[j];
+                s_key[q] = key[j];
+                s_val[q] = val[j];
+            }
+        }
+        __syncthreads();
+        if (p + 1 < passes) {
+#pragma unroll
+            for (int j = 0; j < kSmallItems; ++j) {
+                const uint32_t i = first + 32 * j;
+                if (j < (int)rounds && i < n) {
+                    key[j] = s_key[i];
+                    val[j] = s_val[i];
+                }
+            }
+        }
+    }
+    for (uint32_t i = tid; i < n; i += kSmallThreads) {
+        kout[i] = kmin + s_key[i];
+        vout[i] = s_val[i];
+    }
+}
+
+// One pass on the host side: counts, scan, scatter.
+template <typename KIn, typename KOut, int kItems>
+cudaError_t sort_pass(const KIn *kin, const uint32_t *vin, KOut *kout, uint32_t *vout, uint64_t n, int shift,
+                      uint64_t kmin, uint64_t kadd, uint32_t *hist, unsigned long long *total, cudaStream_t s) {
+    const uint32_t nblocks = (uint32_t)((n + kSortThreads * kItems - 1) / (kSortThreads * kItems));
+    k_rs_hist<KIn, kItems><<<nblocks, kSortThreads, 0, s>>>(kin, n, shift, kmin, hist, nblocks, total);
+    k_rs_scan<<<256, 256, 0, s>>>(hist, nblocks, total);
+    k_rs_scatter<KIn, KOut, kItems>
+        <<<nblocks, kSortThreads, 0, s>>>(kin, vin, kout, vout, n, shift, kmin, kadd, hist, nblocks);
+    return cudaGetLastError();
+}
+
+// All passes with keys of type K between them; `keys` (the samples' keys) is
+// read by the first pass, out_k / out_v written by the last one.
+template <typename K, int kItems>
+cudaError_t sort_passes(const uint64_t *keys, uint64_t n, int passes, uint64_t kmin, K *t0, K *t1, uint32_t *v0,
+                        uint32_t *v1, uint64_t *out_k, uint32_t *out_v, uint32_t *hist, unsigned long long *total,
+                        cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    K *a = t0, *b = t1;
+    uint32_t *va = v0, *vb = v1;
+    for (int p = 0; p < passes && e == cudaSuccess; ++p, total += 256) {
+        const bool first = p == 0, last = p + 1 == passes;
+        if (first && last)
+            e = sort_pass<uint64_t, uint64_t, 8>(keys, nullptr, out_k, out_v, n, 8 * p, kmin, kmin, hist, total, s);
+        else if (first)
+            e = sort_pass<uint64_t, K, kItems>(keys, nullptr, a, va, n, 8 * p, kmin, 0, hist, total, s);
+        else if (last)
+            e = sort_pass<K, uint64_t, kItems>(a, va, out_k, out_v, n, 8 * p, 0, kmin, hist, total, s);
+        else {
+            e = sort_pass<K, K, kItems>(a, va, b, vb, n, 8 * p, 0, 0, hist, total, s);
+            std::swap(a, b);
+            std::swap(va, vb);
+        }
+    }
+    return e;
 }
 
 struct RingSpan {
@@ -423,11 +623,10 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     const uint64_t n = f->n;
     cudaError_t e;
     uint64_t *k0 = nullptr, *k1 = nullptr;
-    uint32_t *v0 = nullptr, *v1 = nullptr, *hist = nullptr;
+    uint32_t *v0 = nullptr, *hist = nullptr, *perm = nullptr;
     KeyRange *range = nullptr;
     RingSpan *span = nullptr;
     unsigned long long *wbits = nullptr;
-    uint32_t nblocks = (uint32_t)((n + kSortTile - 1) / kSortTile);
 #define TRY(x)                         \
     do {                               \
         e = (x);                       \
@@ -435,14 +634,12 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     } while (0)
     TRY(dalloc(&k0, (n + 1) * sizeof(uint64_t), s, ctx->pool));
     TRY(dalloc(&k1, (n + 1) * sizeof(uint64_t), s, ctx->pool));
-    TRY(dalloc(&v0, n * sizeof(uint32_t), s, ctx->pool));
-    TRY(dalloc(&v1, n * sizeof(uint32_t), s, ctx->pool));
-    TRY(dalloc(&hist, (size_t)256 * nblocks * sizeof(uint32_t), s, ctx->pool));
+    TRY(dalloc(&perm, n * sizeof(uint32_t), s, ctx->pool));
     TRY(dalloc(&range, sizeof(KeyRange) + sizeof(RingSpan), s, ctx->pool));
     span = reinterpret_cast<RingSpan *>(range + 1);
     TRY(cudaMemsetAsync(&ctx->d_stats->invalid_input, 0, sizeof(unsigned long long), s));
-    k_init_range<<<1, 1, 0, s>>>(range);
-    k_sample_keys<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(f->hpx, n, d_lon, d_lat, k0, v0, range, ctx->d_stats);
+    TRY(cudaMemsetAsync(range, 0, sizeof(KeyRange), s));
+    k_sample_keys<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(f->hpx, n, d_lon, d_lat, k0, range, ctx->d_stats);
     TRY(cudaGetLastError());
     {
         KeyRange hr;
@@ -455,18 +652,35 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
             e = cudaErrorInvalidValue;
             goto fail;
         }
-        uint64_t span_bits = 64 - (hr.kmax == hr.kmin ? 64 : __builtin_clzll(hr.kmax - hr.kmin));
-        int passes = (int)((span_bits + 7) / 8);
-        for (int p = 0; p < passes; ++p) {
-            int shift = 8 * p;
-            k_rs_hist<<<nblocks, kSortThreads, 0, s>>>(k0, n, shift, hr.kmin, hist, nblocks);
-            k_scan_u32_1block<<<1, 1024, 0, s>>>(hist, (uint64_t)256 * nblocks);
-            k_rs_scatter<<<nblocks, kSortThreads, 0, s>>>(k0, v0, k1, v1, n, shift, hr.kmin, hist, nblocks);
+        const uint64_t kmin = ~hr.nmin;
+        uint64_t span_bits = 64 - (hr.kmax == kmin ? 64 : __builtin_clzll(hr.kmax - kmin));
+        const int passes = span_bits ? (int)((span_bits + 7) / 8) : 1;
+        const bool wide = span_bits > 32;
+        if (n <= kSmallSort && !wide) {
+            TRY(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
+            k_sort_small<<<1, kSmallThreads, kSmallSmem, s>>>(k0, k1, perm, (uint32_t)n, passes, kmin);
             TRY(cudaGetLastError());
-            std::swap(k0, k1);
-            std::swap(v0, v1);
+        } else {
+            // tiles of 16 x 256 keys write the longest runs; below about two
+            // tiles an SM, and for 64-bit keys (shared memory), smaller ones
+            const bool small = n < (1u << 20);
+            const size_t word = wide ? 8 : 4, tile = kSortThreads * (wide ? 8 : small ? 4 : 16);
+            const size_t nblocks = (n + std::min<size_t>(tile, kSortThreads * 8) - 1) / std::min<size_t>(tile, kSortThreads * 8);
+            TRY(dalloc(&v0, 2 * n * (word + 4) + 16, s, ctx->pool));
+            TRY(dalloc(&hist, 256 * nblocks * sizeof(uint32_t) + 8 * 256 * sizeof(unsigned long long), s, ctx->pool));
+            unsigned long long *total = (unsigned long long *)hist;
+            uint32_t *counts = (uint32_t *)(total + 8 * 256), *va = v0 + 2 * n * (word / 4), *vb = va + n;
+            TRY(cudaMemsetAsync(total, 0, passes * 256 * sizeof(unsigned long long), s));
+            if (wide)
+                TRY((sort_passes<uint64_t, 8>(k0, n, passes, kmin, (uint64_t *)v0, (uint64_t *)v0 + n, va, vb, k1,
+                                              perm, counts, total, s)));
+            else if (small)
+                TRY((sort_passes<uint32_t, 4>(k0, n, passes, kmin, v0, v0 + n, va, vb, k1, perm, counts, total, s)));
+            else
+                TRY((sort_passes<uint32_t, 16>(k0, n, passes, kmin, v0, v0 + n, va, vb, k1, perm, counts, total, s)));
         }
     }
+    std::swap(k0, k1);
     k_ring_span<<<1, 1, 0, s>>>(f->hpx, n, k0, span);
     TRY(cudaGetLastError());
     {
@@ -477,9 +691,9 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         f->usedrings = hs.usedrings;
     }
     f->d_keys = k0;
-    f->d_perm = v0;
+    f->d_perm = perm;
     k0 = nullptr;
-    v0 = nullptr;
+    perm = nullptr;
     TRY(dalloc(&f->d_lut, (f->usedrings + 1) * sizeof(uint32_t), s, ctx->pool));
     TRY(dalloc(&f->d_rings, f->usedrings * sizeof(RingRec), s, ctx->pool));
     k_ring_lut<<<(unsigned)((f->usedrings + 1 + 255) / 256), 256, 0, s>>>(f->hpx, n, f->d_keys, f->firstring,
@@ -541,7 +755,7 @@ fail:
     if (k0) cudaFreeAsync(k0, s);
     if (k1) cudaFreeAsync(k1, s);
     if (v0) cudaFreeAsync(v0, s);
-    if (v1) cudaFreeAsync(v1, s);
+    if (perm) cudaFreeAsync(perm, s);
     if (hist) cudaFreeAsync(hist, s);
     if (range) cudaFreeAsync(range, s);
 #undef TRY
