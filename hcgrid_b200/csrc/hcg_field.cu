@@ -357,52 +357,26 @@ cudaError_t sort_passes(const uint64_t *keys, uint64_t n, int passes, uint64_t k
     return e;
 }
 
-struct RingSpan {
-    unsigned long long firstring, usedrings;
+// Bounds of a ring's samples, kept as maxima of order-preserving 32-bit codes
+// (a code of 0 is below every value): |phi| distance from the pixel centre,
+// -cos(lat), -lat and lat, each rounded so that the bound holds.
+struct RingAcc {
+    uint32_t dphi, ncb, nb, b;
 };
-
-__global__ void k_ring_span(HpxParams h, uint64_t n, uint64_t *keys, RingSpan *span) {
-    keys[n] = h.npix;  // sentinel (gridding.cu:100)
-    uint64_t first = pix2ring(h, keys[0]);
-    span->firstring = first;
-    span->usedrings = (uint32_t)(1 + pix2ring(h, keys[n - 1]) - first);
+__device__ __forceinline__ uint32_t order_code(float x) {
+    const uint32_t u = __float_as_uint(x);
+    return u >> 31 ? ~u : u | 0x80000000u;
 }
-
-__device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t *a, uint32_t lo, uint32_t hi, uint64_t key) {
-    while (lo < hi) {
-        uint32_t mid = lo + ((hi - lo) >> 1);
-        if (a[mid] < key)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-// LUT[k] = number of samples with key < startpix(firstring + k): the value
-// the reference's incremental search produces (gridding.cu:118-136).
-__global__ void k_ring_lut(HpxParams h, uint64_t n, const uint64_t *__restrict__ keys, uint64_t firstring,
-                           uint64_t usedrings, uint32_t *__restrict__ lut) {
-    uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (k > usedrings) return;
-    uint32_t v;
-    if (k == 0)
-        v = 0;
-    else if (k == usedrings)
-        v = (uint32_t)n;
-    else {
-        uint64_t sp, npr;
-        ring_info(h, firstring + k, sp, npr);
-        v = lower_bound_u64(keys, 0, (uint32_t)n, sp);
-    }
-    lut[k] = v;
+__device__ __forceinline__ float order_value(uint32_t c) {
+    return c >> 31 ? __uint_as_float(c & 0x7fffffffu) : __uint_as_float(~c);
 }
 
 // Ring half of loc2pix at each used ring's first pixel centre
 // (gridding.cu:330-334: ring info, pix2ang of startpix, then the theta used
 // by ang2pix for lpix and rpix).
 __global__ void k_ring_table(HpxParams h, uint64_t firstring, uint64_t usedrings, const uint32_t *__restrict__ lut,
-                             const uint64_t *__restrict__ keys, RingRec *__restrict__ rings, DevStats *stats) {
+                             const uint64_t *__restrict__ keys, const RingAcc *__restrict__ acc,
+                             RingRec *__restrict__ rings, DevStats *stats) {
     uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (k >= usedrings) return;
     RingRec R;
@@ -431,11 +405,18 @@ __global__ void k_ring_table(HpxParams h, uint64_t firstring, uint64_t usedrings
     R.lut_lo = lut[k];
     R.lut_hi = lut[k + 1];
     R.phi0 = phi;
-    R.dphi = 0.0;  // set by k_ring_phi
+    R.dphi = 0.0;
     R.cbmin = 1.0;
     R.bmin = 0.0;
     R.bmax = 0.0;
-    // pixel range of the ring's samples; the table offsets are set on the host
+    if (R.lut_hi > R.lut_lo) {
+        const RingAcc A = acc[k];
+        R.dphi = order_value(A.dphi);
+        R.cbmin = -order_value(A.ncb);
+        R.bmin = -order_value(A.nb);
+        R.bmax = order_value(A.b);
+    }
+    // pixel range of the ring's samples; the table offsets follow (k_ring_offsets)
     R.pmin = 0;
     R.span = 0;
     R.tbl = 0;
@@ -446,77 +427,92 @@ __global__ void k_ring_table(HpxParams h, uint64_t firstring, uint64_t usedrings
     rings[k] = R;
 }
 
-// Per ring: the largest |phi| distance of a sample from its pixel centre,
-// the smallest cos(lat) and the latitude range of its samples (block per ring).
-__global__ void __launch_bounds__(256) k_ring_phi(HpxParams h, RingRec *__restrict__ rings,
-                                                  const uint64_t *__restrict__ keys, const double *__restrict__ l2,
-                                                  const double *__restrict__ b2, const double *__restrict__ cb2) {
-    __shared__ double s_d[8], s_c[8], s_lo[8], s_hi[8];
-    const uint32_t lo = rings[blockIdx.x].lut_lo, hi = rings[blockIdx.x].lut_hi;
-    double dmax = 0.0, cmin = 1.0, bl = 1e300, bh = -1e300;
-    for (uint32_t j = lo + threadIdx.x; j < hi; j += blockDim.x) {
-        double z, phi, sth;
-        bool have;
-        pix2loc(h, keys[j], z, phi, sth, have);
-        dmax = fmax(dmax, fabs(remainder(l2[j] - phi, 2.0 * kPi)));
-        cmin = fmin(cmin, cb2[j]);
-        bl = fmin(bl, b2[j]);
-        bh = fmax(bh, b2[j]);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-        cmin = fmin(cmin, __shfl_xor_sync(0xffffffffu, cmin, o));
-        bl = fmin(bl, __shfl_xor_sync(0xffffffffu, bl, o));
-        bh = fmax(bh, __shfl_xor_sync(0xffffffffu, bh, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        s_d[threadIdx.x >> 5] = dmax;
-        s_c[threadIdx.x >> 5] = cmin;
-        s_lo[threadIdx.x >> 5] = bl;
-        s_hi[threadIdx.x >> 5] = bh;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            dmax = fmax(dmax, s_d[w]);
-            cmin = fmin(cmin, s_c[w]);
-            bl = fmin(bl, s_lo[w]);
-            bh = fmax(bh, s_hi[w]);
+// Table offset of each ring (span + 1 entries where it holds samples) and the
+// total; one block.
+__global__ void __launch_bounds__(1024) k_ring_offsets(RingRec *__restrict__ rings, uint64_t usedrings,
+                                                       unsigned long long *__restrict__ total) {
+    __shared__ unsigned long long s_w[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    unsigned long long run = 0;
+    for (uint64_t c = 0; c < usedrings; c += 1024) {
+        const uint64_t k = c + tid;
+        const uint32_t span = k < usedrings ? rings[k].span : 0;
+        const unsigned long long v = span ? span + 1ULL : 0ULL;
+        unsigned long long incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
         }
-        rings[blockIdx.x].dphi = dmax;
-        rings[blockIdx.x].cbmin = cmin;
-        rings[blockIdx.x].bmin = hi > lo ? bl : 0.0;
-        rings[blockIdx.x].bmax = hi > lo ? bh : 0.0;
+        if (lane == 31) s_w[w] = incl;
+        __syncthreads();
+        unsigned long long before = 0, all = 0;
+        for (int i = 0; i < 32; ++i) {
+            if (i == w) before = all;
+            all += s_w[i];
+        }
+        __syncthreads();
+        if (k < usedrings) rings[k].tbl = run + before + incl - v;
+        run += all;
     }
+    if (tid == 0) *total = run;
+}
+
+// A field whose tables are too large: no ring has one.
+__global__ void k_ring_no_tables(RingRec *__restrict__ rings, uint64_t usedrings) {
+    const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (k < usedrings) rings[k].span = 0, rings[k].tbl = 0;
 }
 
 // Per-ring pixel tables: entry q of ring k is the first sorted sample of the
-// ring whose pixel is >= startpix + pmin + q (one block per ring).
-__global__ void __launch_bounds__(256) k_ring_ptab(const RingRec *__restrict__ rings, const uint64_t *__restrict__ keys,
-                                                   uint32_t *__restrict__ ptab) {
-    const RingRec R = rings[blockIdx.x];
+// ring whose pixel is >= startpix + pmin + q (entry span: the end of the ring).
+// Each sample fills the entries after its predecessor's pixel up to its own,
+// so an entry costs one store instead of a binary search (4,000,000 samples:
+// 70 us with the searches).
+__global__ void __launch_bounds__(256) k_ring_ptab(HpxParams h, uint64_t n, uint64_t firstring,
+                                                   const RingRec *__restrict__ rings,
+                                                   const uint64_t *__restrict__ keys, uint32_t *__restrict__ ptab) {
+    const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const uint64_t key = keys[j];
+    const RingRec &R = rings[pix2ring(h, key) - firstring];
+    const uint32_t span = R.span;
+    if (!span) return;
     const uint64_t p0 = R.startpix + R.pmin;
-    for (uint32_t q = threadIdx.x; q < R.span; q += blockDim.x)
-        ptab[R.tbl + q] = lower_bound_u64(keys, R.lut_lo, R.lut_hi, p0 + q);
+    uint32_t *t = ptab + R.tbl;
+    uint64_t q = j > R.lut_lo ? keys[j - 1] - p0 + 1 : 0;
+    for (; q <= key - p0; ++q) t[q] = (uint32_t)j;
+    if (j + 1 == R.lut_hi) t[span] = (uint32_t)(j + 1);
 }
 
-// Also the largest |w| of the per-sample weights (when given) into *wbits as
-// the bits of a non-negative double, whose order as integers is the order of
-// the values; NaN sorts above infinity.
-__global__ void k_permute_geometry(uint64_t n, const uint32_t *__restrict__ perm, const double *__restrict__ lon,
-                                   const double *__restrict__ lat, const double *__restrict__ w,
-                                   double *__restrict__ l2, double *__restrict__ b2, double *__restrict__ cb2,
-                                   double *__restrict__ wout, double4 *__restrict__ half,
-                                   unsigned long long *__restrict__ wbits) {
-    uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+// One thread per sorted sample: the permuted geometry, the inverse
+// permutation, the ring table's entries at ring changes, and the bounds of
+// the sample's ring (one atomic per ring and warp). One pass over the samples
+// instead of five (searches per ring, inverse, geometry, a block per ring for
+// the bounds). Also the largest |w| of the per-sample weights (when given)
+// into *wbits as the bits of a non-negative double, whose order as integers is
+// the order of the values; NaN sorts above infinity.
+__global__ void __launch_bounds__(256) k_sample_geometry(
+    HpxParams h, uint64_t n, uint64_t firstring, uint64_t usedrings, uint64_t *__restrict__ keys,
+    const uint32_t *__restrict__ perm, const double *__restrict__ lon, const double *__restrict__ lat,
+    const double *__restrict__ w, double *__restrict__ l2, double *__restrict__ b2, double *__restrict__ cb2,
+    double *__restrict__ wout, double4 *__restrict__ half, uint32_t *__restrict__ inv, uint32_t *__restrict__ lut,
+    RingAcc *__restrict__ acc, unsigned long long *__restrict__ wbits) {
+    const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const bool act = j < n;
     unsigned long long wb = 0;
-    if (j < n) {
-        uint32_t i = perm[j];
-        double b = dmul(lat[i], kDeg2Rad);
-        double l = dmul(lon[i], kDeg2Rad);
+    uint32_t ring = 0xffffffffu;
+    RingAcc A{};
+    if (act) {
+        const uint32_t i = perm[j];
+        const double b = dmul(lat[i], kDeg2Rad);
+        const double l = dmul(lon[i], kDeg2Rad);
+        const double cb = cos(b);
         l2[j] = l;
         b2[j] = b;
-        cb2[j] = cos(b);
+        cb2[j] = cb;
+        inv[i] = (uint32_t)j;
         const double wi = w ? w[i] : 1.0;
         wout[j] = wi;
         wb = (unsigned long long)__double_as_longlong(fabs(wi));
@@ -524,11 +520,47 @@ __global__ void k_permute_geometry(uint64_t n, const uint32_t *__restrict__ perm
         sincos(l * 0.5, &q.x, &q.y);
         sincos(b * 0.5, &q.z, &q.w);
         half[j] = q;
+        const uint64_t key = keys[j], r = pix2ring(h, key);
+        ring = (uint32_t)(r - firstring);
+        uint64_t start, npr;
+        ring_info(h, r, start, npr);
+        const bool centred = r >= h.nside && r <= 3 * h.nside && ((r + h.nside) & 1);  // first centre at phi 0
+        double d = l - (u2d(key - start) + (centred ? 0.0 : 0.5)) * (2.0 * kPi / u2d(npr));
+        d -= 2.0 * kPi * rint(d * (0.5 / kPi));
+        A.dphi = order_code(__double2float_ru(fabs(d)));
+        A.ncb = order_code(-__double2float_rd(cb));
+        A.nb = order_code(-__double2float_rd(b));
+        A.b = order_code(__double2float_ru(b));
+    }
+    uint32_t prev = __shfl_up_sync(0xffffffffu, ring, 1);
+    if (act) {
+        if (j == 0) {
+            keys[n] = h.npix;  // sentinel (gridding.cu:100)
+            lut[0] = 0;
+        } else {
+            if (lane == 0) prev = (uint32_t)(pix2ring(h, keys[j - 1]) - firstring);
+            for (uint32_t k = prev + 1; k <= ring; ++k) lut[k] = (uint32_t)j;  // gridding.cu:118-136
+        }
+        if (j + 1 == n) lut[usedrings] = (uint32_t)n;
+    }
+    const unsigned peers = __match_any_sync(0xffffffffu, ring);
+    if (act) {
+        A.dphi = __reduce_max_sync(peers, A.dphi);
+        A.ncb = __reduce_max_sync(peers, A.ncb);
+        A.nb = __reduce_max_sync(peers, A.nb);
+        A.b = __reduce_max_sync(peers, A.b);
+        if (lane == __ffs(peers) - 1) {
+            RingAcc *p = acc + ring;
+            atomicMax(&p->dphi, A.dphi);
+            atomicMax(&p->ncb, A.ncb);
+            atomicMax(&p->nb, A.nb);
+            atomicMax(&p->b, A.b);
+        }
     }
     if (!w) return;
 #pragma unroll
     for (int o = 16; o; o >>= 1) wb = max(wb, __shfl_xor_sync(0xffffffffu, wb, o));
-    if ((threadIdx.x & 31) == 0 && wb) atomicMax(wbits, wb);
+    if (lane == 0 && wb) atomicMax(wbits, wb);
 }
 
 // out[j][0..cstride) = in[perm[j]][0..nchan), zero padded; one warp per row.
@@ -565,12 +597,6 @@ __global__ void k_permute_cols(uint64_t n, uint32_t nchan, uint32_t cstride, con
         uint32_t c = c0 + tx;
         if (j < n && c < cstride) out[j * cstride + c] = tile[tx][r];
     }
-}
-
-// inv[perm[j]] = j: the sorted position of each input sample.
-__global__ void k_inverse_perm(uint64_t n, const uint32_t *__restrict__ perm, uint32_t *__restrict__ inv) {
-    const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (j < n) inv[perm[j]] = (uint32_t)j;
 }
 
 // One uploaded chunk of sample-major spectra (input rows [r0, r0 + rows))
@@ -624,9 +650,14 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     cudaError_t e;
     uint64_t *k0 = nullptr, *k1 = nullptr;
     uint32_t *v0 = nullptr, *hist = nullptr, *perm = nullptr;
-    KeyRange *range = nullptr;
-    RingSpan *span = nullptr;
-    unsigned long long *wbits = nullptr;
+    // device words read back: the keys' range, then the pixel tables' total and the largest weight
+    struct Back {
+        KeyRange range;
+        unsigned long long total, wbits;
+    };
+    Back *back = nullptr;
+    Back hb{};
+    RingAcc *acc = nullptr;
 #define TRY(x)                         \
     do {                               \
         e = (x);                       \
@@ -635,16 +666,14 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     TRY(dalloc(&k0, (n + 1) * sizeof(uint64_t), s, ctx->pool));
     TRY(dalloc(&k1, (n + 1) * sizeof(uint64_t), s, ctx->pool));
     TRY(dalloc(&perm, n * sizeof(uint32_t), s, ctx->pool));
-    TRY(dalloc(&range, sizeof(KeyRange) + sizeof(RingSpan), s, ctx->pool));
-    span = reinterpret_cast<RingSpan *>(range + 1);
+    TRY(dalloc(&back, sizeof(Back), s, ctx->pool));
     TRY(cudaMemsetAsync(&ctx->d_stats->invalid_input, 0, sizeof(unsigned long long), s));
-    TRY(cudaMemsetAsync(range, 0, sizeof(KeyRange), s));
-    k_sample_keys<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(f->hpx, n, d_lon, d_lat, k0, range, ctx->d_stats);
+    TRY(cudaMemsetAsync(back, 0, sizeof(Back), s));
+    k_sample_keys<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(f->hpx, n, d_lon, d_lat, k0, &back->range, ctx->d_stats);
     TRY(cudaGetLastError());
     {
-        KeyRange hr;
         unsigned long long invalid = 0;
-        TRY(cudaMemcpyAsync(&hr, range, sizeof hr, cudaMemcpyDeviceToHost, s));
+        TRY(cudaMemcpyAsync(&hb, back, sizeof hb, cudaMemcpyDeviceToHost, s));
         TRY(cudaMemcpyAsync(&invalid, &ctx->d_stats->invalid_input, sizeof invalid, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
         if (invalid) {
@@ -652,8 +681,10 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
             e = cudaErrorInvalidValue;
             goto fail;
         }
-        const uint64_t kmin = ~hr.nmin;
-        uint64_t span_bits = 64 - (hr.kmax == kmin ? 64 : __builtin_clzll(hr.kmax - kmin));
+        const uint64_t kmin = ~hb.range.nmin, kmax = hb.range.kmax;
+        f->firstring = pix2ring(f->hpx, kmin);
+        f->usedrings = 1 + pix2ring(f->hpx, kmax) - f->firstring;
+        const uint64_t span_bits = 64 - (kmax == kmin ? 64 : __builtin_clzll(kmax - kmin));
         const int passes = span_bits ? (int)((span_bits + 7) / 8) : 1;
         const bool wide = span_bits > 32;
         if (n <= kSmallSort && !wide) {
@@ -681,83 +712,56 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         }
     }
     std::swap(k0, k1);
-    k_ring_span<<<1, 1, 0, s>>>(f->hpx, n, k0, span);
-    TRY(cudaGetLastError());
-    {
-        RingSpan hs;
-        TRY(cudaMemcpyAsync(&hs, span, sizeof hs, cudaMemcpyDeviceToHost, s));
-        TRY(cudaStreamSynchronize(s));
-        f->firstring = hs.firstring;
-        f->usedrings = hs.usedrings;
-    }
     f->d_keys = k0;
     f->d_perm = perm;
     k0 = nullptr;
     perm = nullptr;
     TRY(dalloc(&f->d_lut, (f->usedrings + 1) * sizeof(uint32_t), s, ctx->pool));
     TRY(dalloc(&f->d_rings, f->usedrings * sizeof(RingRec), s, ctx->pool));
-    k_ring_lut<<<(unsigned)((f->usedrings + 1 + 255) / 256), 256, 0, s>>>(f->hpx, n, f->d_keys, f->firstring,
-                                                                          f->usedrings, f->d_lut);
-    k_ring_table<<<(unsigned)((f->usedrings + 255) / 256), 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_lut,
-                                                                        f->d_keys, f->d_rings, ctx->d_stats);
-    TRY(cudaGetLastError());
-    {
-        // Pixel tables: one u32 per HEALPix pixel between the first and last
-        // sample of each ring, when they fit in max(2^24, 4n) entries
-        // (HCG_RING_TABLE_MAX overrides; 0 keeps the binary searches).
-        uint64_t cap = std::max<uint64_t>(1ull << 24, 4 * n);
-        if (const char *v = getenv("HCG_RING_TABLE_MAX")) cap = strtoull(v, nullptr, 10);
-        std::vector<RingRec> hr(f->usedrings);
-        TRY(cudaMemcpyAsync(hr.data(), f->d_rings, hr.size() * sizeof(RingRec), cudaMemcpyDeviceToHost, s));
-        TRY(cudaStreamSynchronize(s));
-        uint64_t total = 0;
-        for (RingRec &R : hr) {
-            R.tbl = total;
-            total += R.span;
-        }
-        if (total > 0 && total <= cap && dalloc(&f->d_ptab, total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess) {
-            TRY(cudaMemcpyAsync(f->d_rings, hr.data(), hr.size() * sizeof(RingRec), cudaMemcpyHostToDevice, s));
-            k_ring_ptab<<<(unsigned)f->usedrings, 256, 0, s>>>(f->d_rings, f->d_keys, f->d_ptab);
-            TRY(cudaGetLastError());
-            TRY(cudaStreamSynchronize(s));  // the host copy of the table must outlive the upload
-        } else {
-            cudaGetLastError();
-            for (RingRec &R : hr) R.span = 0, R.tbl = 0;
-            TRY(cudaMemcpyAsync(f->d_rings, hr.data(), hr.size() * sizeof(RingRec), cudaMemcpyHostToDevice, s));
-            TRY(cudaStreamSynchronize(s));
-        }
-        f->ptab_entries = f->d_ptab ? total : 0;
-    }
     TRY(dalloc(&f->d_l2, n * sizeof(double), s, ctx->pool));
     TRY(dalloc(&f->d_b2, n * sizeof(double), s, ctx->pool));
     TRY(dalloc(&f->d_cb2, n * sizeof(double), s, ctx->pool));
     TRY(dalloc(&f->d_half, n * sizeof(double4), s, ctx->pool));
     TRY(dalloc(&f->d_w, n * sizeof(double), s, ctx->pool));
-    TRY(dalloc(&wbits, sizeof(unsigned long long), s, ctx->pool));
     TRY(dalloc(&f->d_inv, n * sizeof(uint32_t), s, ctx->pool));
-    k_inverse_perm<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, f->d_perm, f->d_inv);
-    TRY(cudaGetLastError());
-    TRY(cudaMemsetAsync(wbits, 0, sizeof(unsigned long long), s));
-    k_permute_geometry<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, f->d_perm, d_lon, d_lat, d_w, f->d_l2, f->d_b2,
-                                                                   f->d_cb2, f->d_w, f->d_half, wbits);
-    TRY(cudaGetLastError());
-    k_ring_phi<<<(unsigned)f->usedrings, 256, 0, s>>>(f->hpx, f->d_rings, f->d_keys, f->d_l2, f->d_b2, f->d_cb2);
-    TRY(cudaGetLastError());
-    f->wmax = 1.0;
-    if (d_w) {
-        unsigned long long hb = 0;
-        TRY(cudaMemcpyAsync(&hb, wbits, sizeof hb, cudaMemcpyDeviceToHost, s));
+    TRY(dalloc(&acc, f->usedrings * sizeof(RingAcc), s, ctx->pool));
+    TRY(cudaMemsetAsync(acc, 0, f->usedrings * sizeof(RingAcc), s));
+    {
+        const unsigned rblocks = (unsigned)((f->usedrings + 255) / 256), nblk = (unsigned)((n + 255) / 256);
+        k_sample_geometry<<<nblk, 256, 0, s>>>(f->hpx, n, f->firstring, f->usedrings, f->d_keys, f->d_perm, d_lon,
+                                               d_lat, d_w, f->d_l2, f->d_b2, f->d_cb2, f->d_w, f->d_half, f->d_inv,
+                                               f->d_lut, acc, &back->wbits);
+        k_ring_table<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_lut, f->d_keys, acc, f->d_rings,
+                                             ctx->d_stats);
+        k_ring_offsets<<<1, 1024, 0, s>>>(f->d_rings, f->usedrings, &back->total);
+        TRY(cudaGetLastError());
+        TRY(cudaMemcpyAsync(&hb, back, sizeof hb, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
-        memcpy(&f->wmax, &hb, sizeof hb);
+        f->wmax = 1.0;
+        if (d_w) memcpy(&f->wmax, &hb.wbits, sizeof hb.wbits);
+        // Pixel tables: one u32 per HEALPix pixel between the first and last
+        // sample of each ring and one more, when they fit in max(2^24, 4n)
+        // entries (HCG_RING_TABLE_MAX overrides; 0 keeps the binary searches).
+        uint64_t cap = std::max<uint64_t>(1ull << 24, 4 * n);
+        if (const char *v = getenv("HCG_RING_TABLE_MAX")) cap = strtoull(v, nullptr, 10);
+        if (hb.total > 0 && hb.total <= cap &&
+            dalloc(&f->d_ptab, hb.total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess) {
+            k_ring_ptab<<<nblk, 256, 0, s>>>(f->hpx, n, f->firstring, f->d_rings, f->d_keys, f->d_ptab);
+        } else {
+            cudaGetLastError();
+            k_ring_no_tables<<<rblocks, 256, 0, s>>>(f->d_rings, f->usedrings);
+        }
+        TRY(cudaGetLastError());
+        f->ptab_entries = f->d_ptab ? hb.total : 0;
     }
 fail:
-    if (wbits) cudaFreeAsync(wbits, s);
+    if (acc) cudaFreeAsync(acc, s);
     if (k0) cudaFreeAsync(k0, s);
     if (k1) cudaFreeAsync(k1, s);
     if (v0) cudaFreeAsync(v0, s);
     if (perm) cudaFreeAsync(perm, s);
     if (hist) cudaFreeAsync(hist, s);
-    if (range) cudaFreeAsync(range, s);
+    if (back) cudaFreeAsync(back, s);
 #undef TRY
     return e;
 }
