@@ -55,7 +55,7 @@ struct JobDesc {
     uint32_t skip;  // routed to the single-job path: no entries, no sums here
 };
 
-enum { Q_TILE = 0, Q_COUNT, Q_GEOM, Q_ACC, Q_C1, Q_TC, Q_N = Q_TC + kKbShapes };
+enum { Q_TILE = 0, Q_GEOM, Q_ACC, Q_C1, Q_TC, Q_N = Q_TC + kKbShapes };
 
 struct BatchHdr {
     uint32_t njobs;
@@ -112,43 +112,63 @@ __device__ __forceinline__ unsigned long long warp_fetch(BatchHdr *H, int q) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
 
-__global__ void __launch_bounds__(256) kb_tile_rings(BatchHdr *H, const JobDesc *__restrict__ jobs) {
+__global__ void __launch_bounds__(128, kRingCtas) kb_tile_rings(BatchHdr *H, const JobDesc *__restrict__ jobs) {
     for (;;) {
         unsigned long long it = block_fetch(H, Q_TILE);
         if (it >= H->tot_tile) return;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.tile_base; });
         const JobDesc &J = jobs[j];
-        tile_rings_item(J.a, J.g, J.T, it - J.tile_base);
+        tile_rings_item<4>(J.a, J.g, J.T, it - J.tile_base);
     }
 }
 
-template <bool COUNT>
-__global__ void __launch_bounds__(256, 3) kb_group(BatchHdr *H, const JobDesc *__restrict__ jobs) {
-    __shared__ PixPrep s_prep[8][4];
-    __shared__ PixHalf s_half[8][4];
+// Candidate counts of the groups of jobs with tiles beyond the ring table
+// (those jobs leave the batch after it); without one the block returns.
+__global__ void __launch_bounds__(256) kb_group_count(BatchHdr *H, const JobDesc *__restrict__ jobs) {
+    __shared__ GroupShared S[8];
+    bool any = false;
+    for (uint32_t j = threadIdx.x; j < H->njobs; j += blockDim.x)
+        any = any || (jobs[j].g.ngroups && *jobs[j].T.overflow);
+    if (!__syncthreads_or(any)) return;
     const int warp = threadIdx.x >> 5;
-    for (;;) {
-        unsigned long long it = warp_fetch(H, COUNT ? Q_COUNT : Q_GEOM);
-        if (it >= H->tot_grp) return;
-        int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.grp_base; });
+    for (uint32_t j = 0; j < H->njobs; ++j) {
         const JobDesc &J = jobs[j];
-        uint64_t grp = it - J.grp_base;
-        if (!COUNT) {
-            if (J.skip) continue;
-            // the pool must hold this group's entries; otherwise skip and report
-            // (no entries recorded: the pass is replayed once the pool has grown)
-            unsigned long long end = J.off[grp] + J.cap[grp];
-            if (end > H->entry_cap) {
-                if ((threadIdx.x & 31) == 0) {
-                    J.cnt[grp] = 0;
-                    atomicAdd(&H->pool_overflow, 1ULL);
-                }
-                continue;
-            }
-        }
-        group_item<COUNT>(J.a, J.g, J.cap, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, grp, s_prep[warp],
-                          s_half[warp]);
+        if (J.g.ngroups == 0 || *J.T.overflow == 0) continue;
+        for (uint64_t grp = blockIdx.x * 8ull + warp; grp < J.g.ngroups; grp += gridDim.x * 8ull)
+            group_count_item(J.a, J.g, J.cap, grp, S[warp]);
     }
+}
+
+// The weight pass, a tile per item. The pool must hold the tile's entries;
+// otherwise its groups are skipped and reported (no entries recorded: the pass
+// is replayed once the pool has grown).
+__global__ void __launch_bounds__(kWeightThreads, 4) kb_group(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
+    __shared__ TileGroupShared S;
+    PairCounts pc;
+    for (;;) {
+        unsigned long long it = block_fetch(H, Q_GEOM);
+        if (it >= H->tot_tile) break;
+        int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.tile_base; });
+        const JobDesc &J = jobs[j];
+        if (J.skip) continue;
+        const uint64_t tile = it - J.tile_base;
+        bool over = false;
+        if (threadIdx.x < kTileGroups) {
+            const uint32_t gxi = (uint32_t)(tile % J.T.ntx) * (kTileX / 2) + threadIdx.x % (kTileX / 2);
+            const uint32_t gyi = (uint32_t)(tile / J.T.ntx) * (kTileY / 2) + threadIdx.x / (kTileX / 2);
+            const uint64_t grp = (uint64_t)gyi * J.g.gx + gxi;
+            if (gxi < J.g.gx && grp < J.g.ngroups && J.off[grp] + J.cap[grp] > H->entry_cap) over = true;
+        }
+        if (__syncthreads_or(over)) {
+            if (over) atomicAdd(&H->pool_overflow, 1ULL);
+            continue;
+        }
+        if (J.a.unit_w && J.a.series32)
+            group_tile_item<kPairUnit>(J.a, J.g, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, true, tile, 0, 1, S, pc);
+        else
+            group_tile_item<kPairGeneral>(J.a, J.g, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, true, tile, 0, 1, S, pc);
+    }
+    flush_counts(pc, stats);
 }
 
 // Exclusive scan of all jobs' group capacities: three fixed-shape passes
@@ -245,14 +265,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     tc_teardown<KbTcCfg>(S, gk, timeouts);
 }
 
-__global__ void __launch_bounds__(256) kb_1chan(BatchHdr *H, const JobDesc *__restrict__ jobs) {
+__global__ void __launch_bounds__(256, 2) kb_1chan(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
+    __shared__ GroupShared S[8];
+    if (H->tot_c1 == 0) return;
+    PairCounts pc;
+    const int warp = threadIdx.x >> 5;
     for (;;) {
         unsigned long long it = warp_fetch(H, Q_C1);
-        if (it >= H->tot_c1) return;
+        if (it >= H->tot_c1) break;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.c1_base; });
         const JobDesc &J = jobs[j];
-        grid1_item<false>(J.a, J.spec, J.cstride, J.out, J.wout, it - J.c1_base);  // GAUSS1D jobs only
+        grid1_item<false>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp],
+                          pc);  // GAUSS1D jobs only
     }
+    flush_counts(pc, stats);
 }
 
 }  // namespace
@@ -325,21 +351,21 @@ static cudaError_t capture(hcg_context *ctx, BatchState &B) {
         cudaMemsetAsync(&B.d_hdr->pool_overflow, 0, sizeof(unsigned long long), s);
         if (part == 0) {
             kb_prep<<<n * kPersistPerSM, 256, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
-            kb_tile_rings<<<n * 4, 256, 0, s>>>(B.d_hdr, B.d_jobs);
-            kb_group<true><<<n * kPersistPerSM, 256, 0, s>>>(B.d_hdr, B.d_jobs);
+            kb_tile_rings<<<n * kRingCtas, 128, 0, s>>>(B.d_hdr, B.d_jobs);
+            kb_group_count<<<n * 3, 256, 0, s>>>(B.d_hdr, B.d_jobs);
             kb_scan_sums<<<kBatchScanParts, kScanThreads, 0, s>>>(B.d_hdr);
             kb_scan_psum<<<1, kScanThreads, 0, s>>>(B.d_hdr);
             kb_scan_apply<<<kBatchScanParts, kScanThreads, 0, s>>>(B.d_hdr);
             kb_job_entries<<<1, 256, 0, s>>>(B.d_hdr, B.d_jobs, B.d_jent);
         } else {
-            kb_group<false><<<n * kPersistPerSM, 256, 0, s>>>(B.d_hdr, B.d_jobs);
+            kb_group<<<n * 4, kWeightThreads, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
             kb_accum<<<n, kBatchTileThreads, smem, s>>>(B.d_hdr, B.d_jobs, &ctx->d_stats->timeouts);
             unsigned long long *to = &ctx->d_stats->timeouts, *macs = &ctx->d_stats->tc_macs;
             kb_tc<0><<<n, kTcThreads, KbShape<0>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_tc<1><<<n, kTcThreads, KbShape<1>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_tc<2><<<n, kTcThreads, KbShape<2>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_tc<3><<<n, kTcThreads, KbShape<3>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
-            kb_1chan<<<n * kPersistPerSM, 256, 0, s>>>(B.d_hdr, B.d_jobs);
+            kb_1chan<<<n * 2, 256, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
         }
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
         if (ce != cudaSuccess) return ce;
@@ -479,7 +505,7 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
             tcs[d.tc_shape] += ntiles * d.tc.ncb;
             tcn += ntiles * d.tc.ncb;
         }
-        if (f->nchan == 1) c1 += P;
+        if (f->nchan == 1) c1 += (uint64_t)d.g.gx * ((t->ny + 1) / 2);  // 2x2 groups
     }
     // tensor-core jobs grouped by shape, in job order within a shape (their
     // bases rise along the list)

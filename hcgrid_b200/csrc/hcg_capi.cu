@@ -78,7 +78,7 @@ void release_field(hcg_field *f, cudaStream_t s) {
     free_split(f, s);
     if (f->geom_refs && --*f->geom_refs > 0) return;
     void *ps[] = {f->d_keys, f->d_perm, f->d_inv, f->d_l2,    f->d_b2,
-                  f->d_cb2,  f->d_w,    f->d_half, f->d_lut, f->d_rings, f->d_ptab};
+                  f->d_cb2,  f->d_w,    f->d_half, f->d_lut, f->d_rings, f->d_rwin, f->d_ptab};
     for (void *p : ps)
         if (p) cudaFreeAsync(p, s);
     delete f->geom_refs;

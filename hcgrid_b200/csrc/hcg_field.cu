@@ -464,6 +464,29 @@ __global__ void k_ring_no_tables(RingRec *__restrict__ rings, uint64_t usedrings
     if (k < usedrings) rings[k].span = 0, rings[k].tbl = 0;
 }
 
+// The rings' window records.
+__global__ void k_ring_windows(HpxParams h, uint64_t firstring, uint64_t usedrings, const RingRec *__restrict__ rings,
+                               RingWin *__restrict__ out) {
+    const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (k >= usedrings) return;
+    const RingRec R = rings[k];
+    const uint64_t r = firstring + k;
+    RingWin w;
+    w.t2 = R.t2;
+    w.bmin = R.bmin;
+    w.bmax = R.bmax;
+    w.inv_dp = u2d(R.npr) * (0.5 / kPi);
+    w.icb = __double2float_ru(1.0 / R.cbmin);
+    w.dphi = __double2float_ru(R.dphi + 2e-9);
+    w.lut_lo = R.lut_lo;
+    w.lut_hi = R.lut_hi;
+    w.pmin = R.pmin;
+    w.span = R.span;
+    const bool centred = r >= h.nside && r <= 3 * h.nside && ((r + h.nside) & 1);
+    w.tbl = R.tbl | (R.eq ? kRingEq : 0) | (centred ? 0 : kRingHalf);
+    out[k] = w;
+}
+
 // Per-ring pixel tables: entry q of ring k is the first sorted sample of the
 // ring whose pixel is >= startpix + pmin + q (entry span: the end of the ring).
 // Each sample fills the entries after its predecessor's pixel up to its own,
@@ -496,7 +519,7 @@ __global__ void __launch_bounds__(256) k_sample_geometry(
     HpxParams h, uint64_t n, uint64_t firstring, uint64_t usedrings, uint64_t *__restrict__ keys,
     const uint32_t *__restrict__ perm, const double *__restrict__ lon, const double *__restrict__ lat,
     const double *__restrict__ w, double *__restrict__ l2, double *__restrict__ b2, double *__restrict__ cb2,
-    double *__restrict__ wout, double4 *__restrict__ half, uint32_t *__restrict__ inv, uint32_t *__restrict__ lut,
+    double *__restrict__ wout, double2 *__restrict__ half, uint32_t *__restrict__ inv, uint32_t *__restrict__ lut,
     RingAcc *__restrict__ acc, unsigned long long *__restrict__ wbits) {
     const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -516,10 +539,11 @@ __global__ void __launch_bounds__(256) k_sample_geometry(
         const double wi = w ? w[i] : 1.0;
         wout[j] = wi;
         wb = (unsigned long long)__double_as_longlong(fabs(wi));
-        double4 q;
+        double2 q;
         sincos(l * 0.5, &q.x, &q.y);
-        sincos(b * 0.5, &q.z, &q.w);
         half[j] = q;
+        sincos(b * 0.5, &q.x, &q.y);
+        half[n + j] = q;
         const uint64_t key = keys[j], r = pix2ring(h, key);
         ring = (uint32_t)(r - firstring);
         uint64_t start, npr;
@@ -721,7 +745,7 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     TRY(dalloc(&f->d_l2, n * sizeof(double), s, ctx->pool));
     TRY(dalloc(&f->d_b2, n * sizeof(double), s, ctx->pool));
     TRY(dalloc(&f->d_cb2, n * sizeof(double), s, ctx->pool));
-    TRY(dalloc(&f->d_half, n * sizeof(double4), s, ctx->pool));
+    TRY(dalloc(&f->d_half, 2 * n * sizeof(double2), s, ctx->pool));
     TRY(dalloc(&f->d_w, n * sizeof(double), s, ctx->pool));
     TRY(dalloc(&f->d_inv, n * sizeof(uint32_t), s, ctx->pool));
     TRY(dalloc(&acc, f->usedrings * sizeof(RingAcc), s, ctx->pool));
@@ -738,6 +762,7 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         TRY(cudaMemcpyAsync(&hb, back, sizeof hb, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
         f->wmax = 1.0;
+        f->unit_w = d_w == nullptr;
         if (d_w) memcpy(&f->wmax, &hb.wbits, sizeof hb.wbits);
         // Pixel tables: one u32 per HEALPix pixel between the first and last
         // sample of each ring and one more, when they fit in max(2^24, 4n)
@@ -747,6 +772,10 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         if (hb.total > 0 && hb.total <= cap &&
             dalloc(&f->d_ptab, hb.total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess) {
             k_ring_ptab<<<nblk, 256, 0, s>>>(f->hpx, n, f->firstring, f->d_rings, f->d_keys, f->d_ptab);
+            if (f->hpx.order <= kQuickOrder) {
+                TRY(dalloc(&f->d_rwin, f->usedrings * sizeof(RingWin), s, ctx->pool));
+                k_ring_windows<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_rings, f->d_rwin);
+            }
         } else {
             cudaGetLastError();
             k_ring_no_tables<<<rblocks, 256, 0, s>>>(f->d_rings, f->usedrings);

@@ -16,9 +16,10 @@
 //
 // Kernels
 //   k_pixel_prep     per pixel: ring range and the phi half of loc2pix
-//   k_grid_1chan     one warp per pixel, candidates spread over lanes, FP64
-//   k_group<COUNT>   one warp per 2x2 pixel group: candidate count (COUNT)
-//                    or FP64 weights written as compact (sample, w[4]) entries
+//   k_grid_1chan     one warp per 2x2 pixel group, candidates spread over
+//                    lanes, FP64
+//   k_group          one warp per 2x2 pixel group: FP64 weights written as
+//                    compact (sample, w[4]) entries
 //   k_group_accum    one warp per group: FP32 channel accumulation from the
 //                    entries, 4 channels per lane, normalised on store
 #include <cuda_runtime.h>
@@ -47,27 +48,40 @@ __global__ void k_pixel_prep(HpxParams h, uint64_t firstring, uint64_t usedrings
 
 // GEN: fields whose kernel is not GAUSS1D
 template <bool GEN>
-__global__ void __launch_bounds__(256) k_grid_1chan(GridArgs a, uint64_t npixmap, const float *__restrict__ data,
-                                                    uint32_t cstride, float *__restrict__ out,
-                                                    float *__restrict__ wout) {
-    uint64_t p = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    if (p < npixmap) grid1_item<GEN>(a, data, cstride, out, wout, p);
+__global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_grid_1chan(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+                                                        const float *__restrict__ data, uint32_t cstride,
+                                                        float *__restrict__ out, float *__restrict__ wout) {
+    __shared__ GroupShared S[kGroupWarps];
+    PairCounts pc;
+    const int warp = threadIdx.x >> 5;
+    const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
+    if (grp < ngroups) grid1_item<GEN>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
+    flush_counts(pc, a.stats);
 }
 
-// GEN: fields whose kernel is not GAUSS1D; PACK: entries as 16-bit hi/lo
-// pairs for the tensor-core builders (1) or as FP32 weights (0)
-template <bool COUNT, bool GEN = false, int PACK = 0>
-__global__ void __launch_bounds__(256, 3) k_group(GridArgs a, GroupArgs g, uint32_t *__restrict__ cap,
-                                               const unsigned long long *__restrict__ off,
-                                               uint32_t *__restrict__ e_idx, float4 *__restrict__ e_w,
-                                               uint32_t *__restrict__ cnt, double *__restrict__ wsum,
-                                               TileArgs tiles) {
-    __shared__ PixPrep s_prep[8][4];
-    __shared__ PixHalf s_half[8][4];
-    int warp = threadIdx.x >> 5;
-    uint64_t grp = g.g0 + blockIdx.x * 8ull + warp;
-    if (grp < g.g1)
-        group_item<COUNT, GEN, PACK>(a, g, cap, off, e_idx, e_w, cnt, wsum, tiles, grp, s_prep[warp], s_half[warp]);
+// The weight pass, a block per 16x8-pixel tile. MODE as pair_weights; PACK:
+// entries as 16-bit hi/lo pairs for the tensor-core builders (1) or as FP32
+// weights (0)
+template <int MODE, int PACK>
+__global__ void __launch_bounds__(kWeightThreads, MODE == kPairUnit ? kWeightCtas : 4)
+    k_group(GridArgs a, GroupArgs g, const unsigned long long *__restrict__ off, uint32_t *__restrict__ e_idx,
+            float4 *__restrict__ e_w, uint32_t *__restrict__ cnt, double *__restrict__ wsum, TileArgs tiles, bool tiled) {
+    __shared__ TileGroupShared S;
+    PairCounts pc;
+    group_tile_item<MODE, PACK>(a, g, off, e_idx, e_w, cnt, wsum, tiles, tiled, tiles.t0 + blockIdx.x, blockIdx.y,
+                                gridDim.y, S, pc);
+    flush_counts(pc, a.stats);
+}
+
+// Candidate counts of the groups whose tile's ring span exceeds the tile
+// table; a few resident blocks, which return at once when no tile does.
+__global__ void __launch_bounds__(kGroupThreads) k_group_count(GridArgs a, GroupArgs g, uint32_t *__restrict__ cap,
+                                                     const unsigned long long *__restrict__ overflow) {
+    __shared__ GroupShared S[kGroupWarps];
+    if (*overflow == 0) return;
+    const int warp = threadIdx.x >> 5;
+    for (uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp; grp < g.ngroups; grp += gridDim.x * (uint64_t)kGroupWarps)
+        group_count_item(a, g, cap, grp, S[warp]);
 }
 
 __global__ void __launch_bounds__(256) k_group_accum(GroupArgs g, const unsigned long long *__restrict__ off,
@@ -82,8 +96,9 @@ __global__ void __launch_bounds__(256) k_group_accum(GroupArgs g, const unsigned
         group_accum_item(g, off, cnt, e_idx, e_w, wsum, spec, nchan, cstride, out, ostride, wout, grp);
 }
 
-__global__ void __launch_bounds__(256) k_tile_rings(GridArgs a, GroupArgs g, TileArgs T) {
-    tile_rings_item(a, g, T, T.t0 + blockIdx.x);
+template <int W>
+__global__ void __launch_bounds__(32 * W, W == 4 ? kRingCtas : 2) k_tile_rings(GridArgs a, GroupArgs g, TileArgs T) {
+    tile_rings_item<W>(a, g, T, T.t0 + blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kTileThreads, kAccumCtas) k_tile_accum(GroupArgs g, TileArgs T,
@@ -139,11 +154,7 @@ __global__ void k_coarsen(PixPrep *__restrict__ prep, uint32_t nx, uint64_t npix
     if (back == 0) return;
     const PixPrep L = prep[p - back];
     PixPrep &P = prep[p];
-    for (int e = 0; e < 2; ++e) {
-        P.tt[e] = L.tt[e];
-        P.t1[e] = L.t1[e];
-        P.tp[e] = L.tp[e];
-    }
+    for (int e = 0; e < 2; ++e) P.tt[e] = L.tt[e];
     P.ur = L.ur;
     P.nr = L.nr;
     P.polar = L.polar;
@@ -192,11 +203,12 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
     if (f->nchan == 1) {
         cudaEventRecord(ctx->evp[1], s);
         cudaEventRecord(ctx->evp[2], s);
-        const unsigned nblk = (unsigned)((P * 32 + 255) / 256);
+        const uint64_t ngroups = (uint64_t)((t->nx + 1) / 2) * ((t->ny + 1) / 2);
+        const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
         if (f->kernel_type == HCG_GAUSS1D)
-            k_grid_1chan<false><<<nblk, 256, 0, s>>>(a, P, f->d_spec, f->cstride, d_cube, d_wts);
+            k_grid_1chan<false><<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
         else
-            k_grid_1chan<true><<<nblk, 256, 0, s>>>(a, P, f->d_spec, f->cstride, d_cube, d_wts);
+            k_grid_1chan<true><<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else {
         GroupArgs g;
@@ -213,7 +225,7 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         g.g0 = 0;
         g.g1 = g.ngroups;
         g.ebase = 0;
-        unsigned gblocks = (unsigned)((g.ngroups + 7) / 8);
+        unsigned gblocks = (unsigned)((g.ngroups + kGroupWarps - 1) / kGroupWarps);
         // tile table (union of ring windows per 16x8-pixel tile)
         TileArgs T{};
         T.ntx = (t->nx + kTileX - 1) / kTileX;
@@ -248,10 +260,12 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         if (e != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(T.overflow, 0, 3 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(T.ustat, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
-        k_tile_rings<<<(unsigned)ntiles, 256, 0, s>>>(a, g, T);
-        TileArgs none{};
+        if (ntiles <= 148 * 4)
+            k_tile_rings<8><<<(unsigned)ntiles, 256, 0, s>>>(a, g, T);
+        else
+            k_tile_rings<4><<<(unsigned)ntiles, 128, 0, s>>>(a, g, T);
         // groups of tiles whose ring span exceeds the table (cap unknown) are counted here
-        k_group<true><<<gblocks, 256, 0, s>>>(a, g, cap, nullptr, nullptr, nullptr, nullptr, nullptr, none);
+        k_group_count<<<std::min(gblocks, 148u * 3), kGroupThreads, 0, s>>>(a, g, cap, T.overflow);
         k_scan_sums<<<parts, kScanThreads, 0, s>>>(cap, g.ngroups, parts, psum);
         k_scan_psum<<<1, kScanThreads, 0, s>>>(psum, parts);
         k_scan_apply<<<parts, kScanThreads, 0, s>>>(cap, g.ngroups, parts, psum, off);
@@ -321,19 +335,21 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
             gc.g1 = std::min<uint64_t>((uint64_t)ch.second * groups_per_row, g.ngroups);
             gc.ebase = ro[ch.first];
             if (gc.g1 <= gc.g0) continue;
-            unsigned cb = (unsigned)((gc.g1 - gc.g0 + 7) / 8);
-            const TileArgs &tt = tiled ? T : none;
-            if (f->kernel_type == HCG_GAUSS1D) {
-                if (gc.pack)
-                    k_group<false, false, 1><<<cb, 256, 0, s>>>(a, gc, nullptr, off, e_idx, e_w, cnt, wsum, tt);
-                else
-                    k_group<false, false, 0><<<cb, 256, 0, s>>>(a, gc, nullptr, off, e_idx, e_w, cnt, wsum, tt);
-            } else {
-                if (gc.pack)
-                    k_group<false, true, 1><<<cb, 256, 0, s>>>(a, gc, nullptr, off, e_idx, e_w, cnt, wsum, tt);
-                else
-                    k_group<false, true, 0><<<cb, 256, 0, s>>>(a, gc, nullptr, off, e_idx, e_w, cnt, wsum, tt);
-            }
+            unsigned cb = (unsigned)((gc.g1 - gc.g0 + 7) / 8), gb = (ch.second - ch.first) * T.ntx;
+            TileArgs tt = T;
+            tt.t0 = (uint64_t)ch.first * T.ntx;
+            const int mode = f->kernel_type != HCG_GAUSS1D ? kPairOther
+                             : a.unit_w && a.series32      ? kPairUnit
+                                                           : kPairGeneral;
+            auto weights = gc.pack ? (mode == kPairOther  ? k_group<kPairOther, 1>
+                                      : mode == kPairUnit ? k_group<kPairUnit, 1>
+                                                          : k_group<kPairGeneral, 1>)
+                                   : (mode == kPairOther  ? k_group<kPairOther, 0>
+                                      : mode == kPairUnit ? k_group<kPairUnit, 0>
+                                                          : k_group<kPairGeneral, 0>);
+            // two waves of blocks or more: a tile's groups are shared by up to four blocks
+            const unsigned parts = gb >= 148 * kWeightCtas * 2 ? 1 : gb >= 148 * kWeightCtas ? 2 : 4;
+            weights<<<dim3(gb, parts), kWeightThreads, 0, s>>>(a, gc, off, e_idx, e_w, cnt, wsum, tt, tiled);
             if (first) cudaEventRecord(ctx->evp[2], s);  // phase marks are exact for a single chunk
             first = false;
             if (tiled && tc) {

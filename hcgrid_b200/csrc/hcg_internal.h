@@ -39,7 +39,8 @@ struct RingRec {
     int zpos;        // z > 0
     // Pixel table of the ring (span > 0): entry q at tbl + q is the first
     // sorted sample whose pixel is >= startpix + pmin + q, for the pixels
-    // pmin .. pmin + span - 1 between the ring's first and last sample.
+    // pmin .. pmin + span - 1 between the ring's first and last sample; entry
+    // span is the end of the ring.
     uint32_t pmin;
     uint32_t span;
     uint64_t tbl;
@@ -53,17 +54,41 @@ struct RingRec {
     double bmin, bmax;
 };
 
-// One target pixel: its coordinates and the phi half of loc2pix for the two
-// window edges phi -/+ disc_size (gridding.cu:306-351).
+// What the windows of a ring with a pixel table need, in one 64-byte record
+// (RingRec, 104 bytes, serves the general form): the doubles as RingRec has
+// them, the chord bounds rounded outwards to floats, and ring-local 32-bit
+// pixel numbers. nside <= 2^26 (kQuickOrder).
+struct __align__(16) RingWin {
+    double t2;
+    double bmin, bmax;
+    double inv_dp;           // pixels per radian of phi
+    float icb;               // >= 1 / cbmin
+    float dphi;              // >= RingRec::dphi + 2e-9
+    uint32_t lut_lo, lut_hi;
+    uint32_t pmin, span;     // span 0: no window of the ring holds samples
+    uint64_t tbl;            // table offset | kRingEq | kRingHalf
+};
+constexpr uint64_t kRingEq = 1ull << 63;    // equatorial form of the window edges
+constexpr uint64_t kRingHalf = 1ull << 62;  // first pixel centre half a pixel from phi 0
+constexpr uint64_t kRingTbl = kRingHalf - 1;
+constexpr uint64_t kQuickOrder = 26;
+static_assert(sizeof(RingWin) == 64, "four 16-byte loads");
+
+// Half-angle sines and cosines of a position (the pair test's operands).
+struct PixHalf {
+    double sl, cl, sb, cb;
+};
+
+// One target pixel: its coordinates and, for the two window edges phi -/+
+// disc_size (gridding.cu:306-351), the longitude loc2pix starts from.
 struct PixPrep {
     double l1, b1, cb1;    // radians, cos(b1)
     double tt[2];          // fmodulo((phi -/+ disc) / (pi/2), 4)
-    double t1[2];          // nside * (0.5 + tt)
-    double tp[2];          // tt - trunc(tt)
+    PixHalf h;
     int ur;                // first ring, relative to firstring
     int nr;                // number of rings (0: pixel sees no samples)
     int polar;             // whole-ring windows (theta <= 20 or >= 160 deg)
-    int pad;
+    float icb1;            // >= 1 / cb1 (chord windows)
 };
 
 // Stream-ordered allocation from a context's memory pool. The pool keeps
@@ -134,6 +159,7 @@ struct hcg_field {
     uint32_t kernel_type = 0;
     bool taper_fix = false;
     double wmax = 1.0;    // max |per-sample weight| (inf or NaN when one is not finite)
+    bool unit_w = true;   // no per-sample weights were given: all 1
     double wbound = 1.0;  // bound of |weight| of an accepted pair: wmax * the kernel's bound
     uint64_t firstring = 0, usedrings = 0;
     uint64_t *d_keys = nullptr;   // n + 1, sorted, sentinel npix
@@ -143,11 +169,12 @@ struct hcg_field {
     double *d_b2 = nullptr;
     double *d_cb2 = nullptr;      // cos(b2)
     double *d_w = nullptr;        // per-sample input weight, sorted
-    double4 *d_half = nullptr;    // sorted: sin(l/2), cos(l/2), sin(b/2), cos(b/2) of each sample
+    double2 *d_half = nullptr;    // sorted: [n] sin(l/2), cos(l/2), then [n] sin(b/2), cos(b/2)
     uint32_t *d_lut = nullptr;    // usedrings + 1
     uint32_t *d_ptab = nullptr;   // per-ring pixel tables (RingRec::tbl), or none when too large
     uint64_t ptab_entries = 0;
     hcg::RingRec *d_rings = nullptr;
+    hcg::RingWin *d_rwin = nullptr;  // the rings' window records, or none (no tables, nside > 2^26)
     float *d_spec = nullptr;      // [n][cstride], sorted
     uint32_t nchan = 0, cstride = 0;
     // 16-bit hi/lo split of the sorted spectra for the tensor-core engine

@@ -46,10 +46,11 @@ __device__ __forceinline__ void prep_item(HpxParams h, uint64_t firstring, uint6
     P.l1 = dmul(x, kDeg2Rad);
     P.b1 = dmul(y, kDeg2Rad);
     P.cb1 = cos(P.b1);
-    P.pad = 0;
+    P.icb1 = __double2float_ru(1.0 / P.cb1);
     if (!isfinite(x) || !isfinite(y)) {
         P.ur = 0; P.nr = 0; P.polar = 0;
-        for (int e = 0; e < 2; ++e) P.tt[e] = P.t1[e] = P.tp[e] = 0.0;
+        for (int e = 0; e < 2; ++e) P.tt[e] = 0.0;
+        P.h = PixHalf{0.0, 1.0, 0.0, 1.0};
         out[p] = P;
         return;
     }
@@ -69,33 +70,32 @@ __device__ __forceinline__ void prep_item(HpxParams h, uint64_t firstring, uint6
     P.nr = (dring >= uring) ? (int)(dring - uring + 1) : 0;
     double dt = dmul(disc_theta, kRad2Deg);
     P.polar = (dt <= kNorthB || dt >= kSouthB);
-    double ns = u2d(h.nside);
-    double phis[2] = {dsub(disc_phi, disc), dadd(disc_phi, disc)};
-    for (int e = 0; e < 2; ++e) {
-        double tt = fmodulo(dmul(phis[e], kInvHalfPi), 4.0);
-        P.tt[e] = tt;
-        P.t1[e] = dmul(ns, dadd(0.5, tt));
-        P.tp[e] = dsub(tt, u2d(d2u(tt)));
-    }
+    P.tt[0] = fmodulo(dmul(dsub(disc_phi, disc), kInvHalfPi), 4.0);
+    P.tt[1] = fmodulo(dmul(dadd(disc_phi, disc), kInvHalfPi), 4.0);
+    sincos(P.l1 * 0.5, &P.h.sl, &P.h.cl);
+    sincos(P.b1 * 0.5, &P.h.sb, &P.h.cb);
     out[p] = P;
 }
 
 // loc2pix(z_ring, phi_edge) from its ring half and phi half.
 __device__ __forceinline__ uint64_t edge_pix(const HpxParams &h, const RingRec &R, const PixPrep &P, int e) {
+    const double tt = P.tt[e];
     if (R.eq) {
         uint64_t nl4 = 4 * h.nside;
-        uint64_t jp = d2u(dsub(P.t1[e], R.t2));
-        uint64_t jm = d2u(dadd(P.t1[e], R.t2));
+        const double temp1 = dmul(u2d(h.nside), dadd(0.5, tt));
+        uint64_t jp = d2u(dsub(temp1, R.t2));
+        uint64_t jm = d2u(dadd(temp1, R.t2));
         uint64_t ir = h.nside + 1 + jp - jm;
         uint64_t kshift = 1 - (ir & 1);
         uint64_t t1 = jp + jm + kshift + 1 + nl4 + nl4 - h.nside;
         uint64_t ip = (h.order > 0) ? ((t1 >> 1) & (nl4 - 1)) : ((t1 >> 1) % nl4);
         return h.ncap + (ir - 1) * nl4 + ip;
     }
-    uint64_t jp = d2u(dmul(P.tp[e], R.t2));
-    uint64_t jm = d2u(dmul(dsub(1.0, P.tp[e]), R.t2));
+    const double tp = dsub(tt, u2d(d2u(tt)));
+    uint64_t jp = d2u(dmul(tp, R.t2));
+    uint64_t jm = d2u(dmul(dsub(1.0, tp), R.t2));
     uint64_t ir = jp + jm + 1;
-    uint64_t ip = d2u(dmul(P.tt[e], u2d(ir)));
+    uint64_t ip = d2u(dmul(tt, u2d(ir)));
     return R.zpos ? 2 * ir * (ir - 1) + ip : h.npix - 2 * ir * (ir + 1) + ip;
 }
 
@@ -136,17 +136,6 @@ __device__ __forceinline__ double dist_deg(double l1, double b1, double cb1, dou
     double sb = sin((b1 - b2) * 0.5);
     double sl = sin((l1 - l2) * 0.5);
     return 2.0 * asin(sqrt(sb * sb + cb1 * cb2 * (sl * sl))) * kRad2Deg;
-}
-
-// Lane of the warp whose inclusive prefix `incl` first exceeds t.
-__device__ __forceinline__ int owner_lane(uint32_t incl, uint32_t t) {
-    int lo = 0;
-#pragma unroll
-    for (int step = 16; step; step >>= 1) {
-        uint32_t v = __shfl_sync(0xffffffffu, incl, lo + step - 1);
-        if (v <= t) lo += step;
-    }
-    return lo;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -190,9 +179,9 @@ struct GridArgs {
     const double *l2, *b2, *cb2, *w;
     double sphere_radius, p0;
     DevStats *stats;
-    const double4 *half;  // per sorted sample: sin(l/2), cos(l/2), sin(b/2), cos(b/2)
+    const double2 *half;  // sorted samples: [n] sin(l/2), cos(l/2), then [n] sin(b/2), cos(b/2)
     const uint32_t *ptab; // per-ring pixel tables (RingRec::tbl)
-    double hlo, hhi;      // haversine thresholds bracketing sphere_radius (see pair_weight)
+    double hlo, hhi;      // haversine thresholds bracketing sphere_radius (see grid_args)
     int series;           // d^2 from the arcsine-squared series (small sphere_radius)
     double hpolar;        // haversine bound of every accepted pair (chord windows)
     float x2scale;        // 4 R2D^2 p0 log2(e): the FP32 Gaussian's exponent per unit of the series
@@ -200,6 +189,13 @@ struct GridArgs {
     uint32_t ktype;       // HCG_GAUSS1D, HCG_GAUSS2D or HCG_TAPERED_SINC
     int ktaper;           // TAPERED_SINC with HCG_TAPER_FIX
     double kp1, kp2;      // second and third kernel parameters (p0 is the first)
+    const RingWin *rwin;  // the rings' window records (null: ring_window_mc's general form only)
+    uint64_t firstring;
+    float hpolar32;       // >= hpolar
+    int unit_w;           // every sample weight is 1
+    float hlo32, hhi32;   // <= hlo, >= hhi: the brackets an FP32 haversine decides
+    uint64_t n;           // samples
+    double spa, cpa;      // GAUSS2D: sine and cosine of the position angle
 };
 
 namespace {
@@ -224,6 +220,15 @@ inline GridArgs grid_args(const hcg_field *f, const PixPrep *prep, DevStats *sta
     a.ktaper = f->taper_fix;
     a.kp1 = f->kparams[1];
     a.kp2 = f->kparams[2];
+    a.rwin = f->d_rwin;
+    a.firstring = f->firstring;
+    a.hpolar32 = (float)(hstar * (1.0 + 2e-6));
+    a.unit_w = f->unit_w;
+    a.hlo32 = (float)(a.hlo * (1.0 - 2e-7));
+    a.hhi32 = (float)(a.hhi * (1.0 + 2e-7));
+    a.n = f->n;
+    a.spa = std::sin(f->kparams[2]);
+    a.cpa = std::cos(f->kparams[2]);
     return a;
 }
 
@@ -265,22 +270,186 @@ __device__ __forceinline__ bool ring_window_mc(const GridArgs &a, const RingRec 
     return true;
 }
 
-// 32-byte read-only load (no double4 overload of __ldg)
-__device__ __forceinline__ double4 ldg4(const double4 *p) {
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
-    const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
+// Out of line and by value, so that only a thread that comes here stores its
+// arguments.
+struct RingWindow {
+    uint32_t lo, hi, ref_len;
+    bool ok;
+};
+__device__ __noinline__ RingWindow ring_window_call(GridArgs a, PixPrep P, int k) {
+    RingWindow w;
+    w.ok = ring_window_mc(a, a.rings[k], P, w.lo, w.hi, w.ref_len);
+    return w;
+}
+__device__ __forceinline__ bool ring_window_general(const GridArgs &a, const PixPrep &P, int k, uint32_t &lo,
+                                                    uint32_t &hi, uint32_t &ref_len) {
+    const RingWindow w = ring_window_call(a, P, k);
+    lo = w.lo;
+    hi = w.hi;
+    ref_len = w.ref_len;
+    return w.ok;
 }
 
-// Pixel side of the pair test: half-angle sines and cosines.
-struct PixHalf {
-    double sl, cl, sb, cb;
+// The pixels of a 2x2 group as the window arithmetic takes them: per pixel the
+// edges' longitudes and ring range (empty for pixels outside the map or
+// without samples), and the group's extent for the chord's bound.
+struct GroupGeo {
+    double tt[4][2];
+    int ur[4], ue[4];  // rings [ur, ue)
+    unsigned polar;    // bit q: whole-ring windows
+    double lmin, lmax, bmin, bmax;  // longitudes in [0, 2 pi)
+    float icb;         // >= 1 / cos(lat) of every pixel; inf: no chord bound
+    int r0, r1;        // union of the ring ranges, [r0, r1]
 };
-__device__ __forceinline__ PixHalf pix_half(const PixPrep &P) {
-    PixHalf q;
-    sincos(P.l1 * 0.5, &q.sl, &q.cl);
-    sincos(P.b1 * 0.5, &q.sb, &q.cb);
-    return q;
+
+template <typename GET>  // get(q): the PixPrep of pixel q, or null
+__device__ __forceinline__ GroupGeo group_geo(GET get) {
+    GroupGeo G;
+    G.polar = 0;
+    G.lmin = G.bmin = 1e300;
+    G.lmax = G.bmax = -1e300;
+    G.icb = 0.f;
+    G.r0 = 1 << 30;
+    G.r1 = -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const PixPrep *P = get(q);
+        G.tt[q][0] = G.tt[q][1] = 0.0;
+        G.ur[q] = 1;
+        G.ue[q] = 0;
+        if (!P || P->nr <= 0) continue;
+        G.tt[q][0] = P->tt[0];
+        G.tt[q][1] = P->tt[1];
+        G.ur[q] = P->ur;
+        G.ue[q] = P->ur + P->nr;
+        G.r0 = min(G.r0, G.ur[q]);
+        G.r1 = max(G.r1, G.ue[q] - 1);
+        if (P->polar) G.polar |= 1u << q;
+        const double lp = P->l1 - 2.0 * kPi * floor(P->l1 * (0.5 / kPi));
+        G.lmin = fmin(G.lmin, lp);
+        G.lmax = fmax(G.lmax, lp);
+        G.bmin = fmin(G.bmin, P->b1);
+        G.bmax = fmax(G.bmax, P->b1);
+        G.icb = P->icb1 >= 0.f ? fmaxf(G.icb, P->icb1) : __int_as_float(0x7f800000);
+    }
+    if (G.lmax - G.lmin > kPi) G.icb = __int_as_float(0x7f800000);  // the group straddles phi = 0
+    return G;
+}
+
+// The windows of a group's four pixels in the field's ring k in the general
+// form, for fields without window records and stray edges.
+__device__ __forceinline__ void group_windows_general(const GridArgs &a, int k, const GroupGeo &G, uint64_t pix0,
+                                                      uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
+                                                      uint32_t &skips) {
+    for (int q = 0; q < 4; ++q) {
+        lo[q] = hi[q] = 0;
+        if (k < G.ur[q] || k >= G.ue[q]) continue;
+        uint32_t rl;
+        if (ring_window_general(a, a.prep[pix0 + (q & 1) + (uint64_t)(q >> 1) * nx], k, lo[q], hi[q], rl)) {
+            ref += rl;
+        } else {
+            lo[q] = 1;
+            hi[q] = 0;
+            ++skips;
+        }
+    }
+}
+
+// The windows of a group's four pixels in the field's ring k from its 64-byte
+// record: the reference window of each pixel (ring_window's integers, from the
+// same rounded operations on ring-local 32-bit pixel numbers; an edge that
+// rounds into another ring takes the general form), intersected with one chord
+// bound for the group. The bound is FP32 rounded outwards, from the group's
+// extent: it only leaves out candidates beyond the radius of every pixel, so it
+// needs no more, and whole pixels inside it are kept without a pixel of margin.
+// lo > hi marks a ring the reference would spin on; `ref` adds the reference
+// windows' lengths, `skips` such rings. What bounds it: instruction issue; a
+// general window takes about 600 instructions (four FP64 divisions, a root,
+// 64-bit pixel numbers, a 104-byte record), a group's four here about 300.
+__device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &R, int k, const GroupGeo &G,
+                                              uint64_t pix0, uint32_t nx, uint32_t lo[4], uint32_t hi[4],
+                                              uint32_t &ref, uint32_t &skips) {
+    const int ns = (int)a.h.nside, ring = (int)(a.firstring + (uint64_t)k);
+    const double nsd = (double)ns;
+    const bool eq = (R.tbl & kRingEq) != 0;
+    const int i4 = eq ? 4 * ns : 4 * min(ring, 4 * ns - ring);  // pixels of the ring
+    const int span = (int)R.span, pmin = (int)R.pmin;
+    const uint32_t *t = a.ptab + (R.tbl & kRingTbl);
+    auto first_of = [&](int pix) { return __ldg(t + max(0, min(pix - pmin, span))); };  // first sample at or after pix
+    uint32_t clo = 0, chi = 0xffffffffu;
+    if (span) {
+        const float y = 0.5f * (float)fmax(0.0, fmax(R.bmin - G.bmax, G.bmin - R.bmax));
+        const float hb = y < 1.f ? y * y * (1.f - y * y * (1.f / 3.f)) * (1.f - 1e-6f) : 0.f;
+        const float H = (a.hpolar32 - hb) * R.icb * G.icb * (1.f + 1e-6f);
+        if (!(hb < a.hpolar32)) {  // no sample of the ring within the radius
+            chi = 0;
+        } else if (H >= 0.f && H < 0.25f) {
+            // |dphi| <= 2 asin(sqrt(H)) <= 2 sqrt(H / (1 - H)), and a sample lies within dphi of its pixel centre
+            const float W = 2.f * sqrtf(__fdividef(H, 1.f - H)) * (1.f + 4e-6f) + R.dphi;
+            const double w = (double)W * R.inv_dp + 1e-4, s = (R.tbl & kRingHalf) ? 0.5 : 0.0;
+            const int jl = __double2int_ru(G.lmin * R.inv_dp - s - w), jh = __double2int_rd(G.lmax * R.inv_dp - s + w);
+            if (jl >= 0 && jh < i4 && jh - jl + 1 < i4) {  // else: wraps, the reference windows stay
+                clo = first_of(jl);
+                chi = first_of(jh + 1);
+            }
+        }
+    }
+    // straight-line code over the four pixels: the lookups of all of them are
+    // in flight together
+    int e0[4], e1[4];
+    bool stray = false;
+    if (eq) {
+        const int c = ((ring - ns) & 1) + 1 + 7 * ns, want = ring - 2 * ns;
+        auto edge = [&](double tt, bool &same) {
+            const double t1 = dmul(nsd, dadd(0.5, tt));
+            const int jp = (int)__double2uint_rz(dsub(t1, R.t2)), jm = (int)__double2uint_rz(dadd(t1, R.t2));
+            same = same && jp - jm == want;
+            return ((jp + jm + c) >> 1) & (i4 - 1);
+        };
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            bool same = true;
+            e0[q] = edge(G.tt[q][0], same);
+            e1[q] = edge(G.tt[q][1], same);
+            stray = stray || (!same && k >= G.ur[q] && k < G.ue[q] && !(G.polar >> q & 1u));
+        }
+    } else {
+        auto edge = [&](double tt, bool &same) {
+            const double tp = dsub(tt, floor(tt));
+            const int ir = (int)__double2uint_rz(dmul(tp, R.t2)) + (int)__double2uint_rz(dmul(dsub(1.0, tp), R.t2)) + 1;
+            const int ip = (int)__double2uint_rz(dmul(tt, (double)ir));
+            same = same && 4 * ir == i4 && ip < i4;
+            return ip;
+        };
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            bool same = true;
+            e0[q] = edge(G.tt[q][0], same);
+            e1[q] = edge(G.tt[q][1], same);
+            stray = stray || (!same && k >= G.ur[q] && k < G.ue[q] && !(G.polar >> q & 1u));
+        }
+    }
+    if (stray) {  // an edge rounded into another ring
+        group_windows_general(a, k, G, pix0, nx, lo, hi, ref, skips);
+        return;
+    }
+    uint32_t rl[4] = {0, 0, 0, 0}, rh[4] = {0, 0, 0, 0};
+    if (span) {  // else no samples, or the first used ring (the reference's search returns "none")
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool whole = G.polar >> q & 1u;
+            rl[q] = first_of(whole ? 0 : e0[q]);
+            rh[q] = first_of(whole ? i4 : e1[q] + 1);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const bool act = k >= G.ur[q] && k < G.ue[q];
+        const uint32_t h = max(rl[q], rh[q]);
+        ref += act ? h - rl[q] : 0u;
+        lo[q] = act ? max(rl[q], clo) : 0u;
+        hi[q] = act ? max(lo[q], min(h, chi)) : 0u;
+    }
 }
 
 // exp(-x) for the FP32 weights of the multi-channel path, x >= 0 from FP64:
@@ -306,132 +475,360 @@ __device__ __forceinline__ float gauss_series_f32(double h, float x2scale) {
     return r;
 }
 
+// Half-angle differences of a pair and its haversine: sin((b1 - b2) / 2),
+// sin((l1 - l2) / 2) and h = sin^2(db / 2) + cos b1 cos b2 sin^2(dl / 2),
+// expanded from the precomputed sines and cosines (`sl2` = sin, cos of l2 / 2;
+// `sb2` of b2 / 2).
+struct PairHav {
+    double sb, sl, h;
+};
+__device__ __forceinline__ PairHav pair_hav(const PixHalf &q, double cb1, const double2 &sl2, const double2 &sb2,
+                                            double cb2) {
+    PairHav v;
+    v.sb = q.sb * sb2.y - q.cb * sb2.x;
+    v.sl = q.sl * sl2.y - q.cl * sl2.x;
+    v.h = v.sb * v.sb + cb1 * cb2 * (v.sl * v.sl);
+    return v;
+}
+
+// d^2 (degrees^2) of an accepted pair from its haversine: asin^2(x) =
+// sum_n (2x)^(2n) / (2 n^2 C(2n, n)) at x = sqrt(h), five terms (used when
+// h* < 1e-3, truncation below 1e-16 relative), else asin itself.
+__device__ __forceinline__ double pair_d2(const GridArgs &a, double h) {
+    if (a.series) {
+        const double t = h * (1.0 + h * (1.0 / 3.0 + h * (8.0 / 45.0 + h * (4.0 / 35.0 + h * (128.0 / 1575.0)))));
+        return 4.0 * t * (kRad2Deg * kRad2Deg);
+    }
+    const double d = 2.0 * asin(sqrt(h)) * kRad2Deg;
+    return d * d;
+}
+
 // The grid kernels other than GAUSS1D (gridding.cu:242-256), FP64, for an
-// accepted pair at d degrees: GAUSS2D (sigma_maj, sigma_min, PA) at the
-// great-circle bearing of the sample seen from the pixel (helpers.cu:133-137),
-// TAPERED_SINC (sigma, a, b) with sinc(x) = 1 for |x| < 1e-10
-// (gridding.cu:229-235) and the taper exp(+(arg/a)^2) of the reference, or
-// exp(-(arg/a)^2) with HCG_TAPER_FIX. Kept out of line: the GAUSS1D loops
-// that inline pair_weight_s only branch to it.
-__device__ __noinline__ double kernel_other(const GridArgs &a, const PixPrep &P, double d, double cb2,
-                                            uint32_t idx) {
+// accepted pair with squared distance d2: GAUSS2D (sigma_maj, sigma_min, PA)
+// at the great-circle bearing of the sample seen from the pixel
+// (helpers.cu:133-137), TAPERED_SINC (sigma, a, b) with sinc(x) = 1 for
+// |x| < 1e-10 (gridding.cu:229-235) and the taper exp(+(arg/a)^2) of the
+// reference, or exp(-(arg/a)^2) with HCG_TAPER_FIX. The bearing's tangent
+// y / x has y = cos b2 sin dl and x = cos b1 sin b2 - sin b1 cos b2 cos dl =
+// sin(b2 - b1) + 2 sin b1 cos b2 sin^2(dl / 2); both follow from the half-angle
+// products, and only sin^2 and cos^2 of (bearing - PA) are wanted, so neither
+// the arc tangent nor any sine or cosine is evaluated (the weight pass of
+// 150,001 samples on 251 x 203 pixels took 355 us with them).
+__device__ __forceinline__ double kernel_other(const GridArgs &a, const PixHalf &q, const PairHav &v,
+                                               const double2 &sl2, const double2 &sb2, double cb2, double d2) {
     const double p0 = a.p0, p1 = a.kp1, p2 = a.kp2;
     if (a.ktype == HCG_GAUSS2D) {
-        double sdl, cdl;
-        sincos(__ldg(a.l2 + idx) - P.l1, &sdl, &cdl);
-        const double sb2 = sin(__ldg(a.b2 + idx)), sb1 = sin(P.b1);
-        const double bear = atan2(cb2 * sdl, P.cb1 * sb2 - sb1 * cb2 * cdl);
-        double sa, ca;
-        sincos(bear - p2, &sa, &ca);
-        const double ell = (p0 * p0) * (sa * sa) + (p1 * p1) * (ca * ca);
-        const double q = d / p0 / p1;
-        return exp(-((q * q) / 2. * ell));
+        const double cl = q.cl * sl2.y + q.sl * sl2.x;  // cos((l1 - l2) / 2)
+        const double cb = q.cb * sb2.y + q.sb * sb2.x;  // cos((b1 - b2) / 2)
+        const double y = -2.0 * cb2 * (v.sl * cl);
+        const double x = 2.0 * (2.0 * (q.sb * q.cb) * cb2 * (v.sl * v.sl) - v.sb * cb);
+        const double ys = y * a.cpa - x * a.spa, xc = x * a.cpa + y * a.spa;
+        const double n2 = x * x + y * y;
+        const double ell = n2 > 0.0 ? ((p0 * p0) * (ys * ys) + (p1 * p1) * (xc * xc)) / n2 : 0.0;
+        const double pp = p0 * p1;
+        return exp(-0.5 * d2 * ell / (pp * pp));
     }
-    const double arg = kPi * d / p0;
+    const double arg = kPi * sqrt(d2) / p0;
     const double x = arg / p2;
     const double s = fabs(x) < 1.e-10 ? 1. : sin(x) / x;
     const double t = (arg / p1) * (arg / p1);
     return s * exp(a.ktaper ? -t : t);
 }
 
-// Weight of sample idx for the pixel (0 outside sphere_radius): the
-// haversine h = sin^2(db/2) + cos b1 cos b2 sin^2(dl/2) with the half-angle
-// differences expanded from precomputed sines and cosines; d^2 for accepted
-// pairs from asin^2(x) = sum_n (2x)^(2n) / (2 n^2 C(2n, n)) at x = sqrt(h)
-// (five terms; used when h* < 1e-3, truncation below 1e-16 relative), else
-// from asin itself. Pairs inside the threshold band take the full formula.
-// GEN: the field's kernel may be other than GAUSS1D (kernel_other); without
-// it the code is GAUSS1D's alone.
-template <bool F32EXP = false, bool GEN = true>
-__device__ __forceinline__ double pair_weight_s(const GridArgs &a, const PixPrep &P, const PixHalf &q,
-                                                const double4 &s, double cb2, double win, uint32_t idx) {
-    const double sb = q.sb * s.w - q.cb * s.z;  // sin((b1 - b2) / 2)
-    const double sl = q.sl * s.y - q.cl * s.x;  // sin((l1 - l2) / 2)
-    const double h = sb * sb + P.cb1 * cb2 * (sl * sl);
-    if (h > a.hhi) return 0.0;
-    if (F32EXP && h < a.hlo && a.series32) return win * (double)gauss_series_f32(h, a.x2scale);
-    double d2;
-    if (h < a.hlo) {
-        if (a.series) {
-            const double t = h * (1.0 + h * (1.0 / 3.0 + h * (8.0 / 45.0 + h * (4.0 / 35.0 + h * (128.0 / 1575.0)))));
-            d2 = 4.0 * t * (kRad2Deg * kRad2Deg);
-        } else {
-            const double d = 2.0 * asin(sqrt(h)) * kRad2Deg;
-            d2 = d * d;
+// Weight of an accepted pair with squared distance d2 (degrees^2). GEN: the
+// field's kernel may be other than GAUSS1D. F32: multi-channel entries hold
+// FP32 weights, so the Gaussian is evaluated in FP32 (gauss_f32).
+template <bool F32, bool GEN>
+__device__ __forceinline__ double kernel_at(const GridArgs &a, const PixHalf &q, const PairHav &v, const double2 &sl2,
+                                            const double2 &sb2, double cb2, double win, double d2) {
+    if (GEN && a.ktype != HCG_GAUSS1D) {
+        const double k = kernel_other(a, q, v, sl2, sb2, cb2, d2);
+        return win * (F32 ? (double)(float)k : k);
+    }
+    return win * (F32 ? (double)gauss_f32(d2 * a.p0) : exp(-d2 * a.p0));
+}
+
+// A pair near the cutoff (rare): inside the band [hlo, hhi] the reference's
+// full formula decides. Out of line, by value and from memory again, so that the
+// loop around it keeps nothing for it.
+template <bool F32, bool GEN>
+__device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t idx) {
+    const PixPrep Q = *P;
+    const double2 sl2 = __ldg(a.half + idx), sb2 = __ldg(a.half + a.n + idx);
+    const double cb2 = __ldg(a.cb2 + idx), win = __ldg(a.w + idx);
+    const PairHav v = pair_hav(Q.h, Q.cb1, sl2, sb2, cb2);
+    if (v.h > a.hhi) return 0.0;
+    if (v.h < a.hlo) {
+        if (F32 && !GEN && a.series32) return win * (double)gauss_series_f32(v.h, a.x2scale);
+        return kernel_at<F32, GEN>(a, Q.h, v, sl2, sb2, cb2, win, pair_d2(a, v.h));
+    }
+    const double d = dist_deg(Q.l1, Q.b1, Q.cb1, __ldg(a.l2 + idx), __ldg(a.b2 + idx), cb2);
+    if (!(d < a.sphere_radius)) return 0.0;
+    return kernel_at<F32, GEN>(a, Q.h, v, sl2, sb2, cb2, win, d * d);
+}
+
+// Weights of sample idx for the four pixels of a group (0 outside
+// sphere_radius, decided from the haversine). `in`: the sample is in the
+// pixel's window. `wf` is the weight rounded to FP32 (F32 only). Straight-line
+// code: the four pixels' chains interleave, and a pair that is not accepted
+// costs a select, not a branch. MODE kPairUnit: FP32 Gaussians of unit-weight
+// samples, where the haversine rounded to FP32 (which the series takes anyway)
+// decides all but the pairs within 2e-7 of the cutoff, relative.
+enum { kPairGeneral = 0, kPairUnit = 1, kPairOther = 2 };  // kPairOther: kernels other than GAUSS1D
+template <bool F32, int MODE>
+__device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P, uint32_t nx, const PixHalf q[4],
+                                             const double cb1[4], const double2 &sl2, const double2 &sb2, double cb2,
+                                             double win, uint32_t idx, const bool in[4], double w[4], float wf[4]) {
+    constexpr bool GEN = MODE == kPairOther;
+    PairHav v[4];
+    bool acc[4];
+    unsigned band = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = pair_hav(q[i], cb1[i], sl2, sb2, cb2);
+    if (MODE == kPairUnit) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float hf = (float)v[i].h;
+            acc[i] = in[i] && hf < a.hlo32;
+            if (in[i] && !acc[i] && hf <= a.hhi32) band |= 1u << i;
+            wf[i] = acc[i] ? gauss_series_f32(v[i].h, a.x2scale) : 0.f;
+            w[i] = (double)wf[i];
         }
     } else {
-        const double d = dist_deg(P.l1, P.b1, P.cb1, __ldg(a.l2 + idx), __ldg(a.b2 + idx), cb2);
-        if (!(d < a.sphere_radius)) return 0.0;
-        d2 = d * d;
-    }
-    if (GEN && a.ktype != HCG_GAUSS1D) {
-        const double k = kernel_other(a, P, sqrt(d2), cb2, idx);
-        return win * (F32EXP ? (double)(float)k : k);
-    }
-    // Multi-channel entries hold FP32 weights: the Gaussian is evaluated in
-    // FP32 there (gauss_f32); distance and cutoff stay FP64.
-    if (F32EXP) return win * (double)gauss_f32(d2 * a.p0);
-    return win * exp(-d2 * a.p0);
-}
-
-template <bool GEN>
-__device__ __forceinline__ double pair_weight(const GridArgs &a, const PixPrep &P, const PixHalf &q, uint32_t idx) {
-    return pair_weight_s<false, GEN>(a, P, q, ldg4(a.half + idx), __ldg(a.cb2 + idx), __ldg(a.w + idx), idx);
-}
-
-// Single channel: one warp per pixel, FP64 throughout.
-// Warp-collective: every lane passes the same pixel p. GEN as pair_weight_s.
-template <bool GEN>
-__device__ __forceinline__ void grid1_item(const GridArgs &a, const float *__restrict__ data, uint32_t cstride,
-                                           float *__restrict__ out, float *__restrict__ wout, uint64_t p) {
-    int lane = threadIdx.x & 31;
-    const PixPrep P = a.prep[p];
-    const PixHalf ph = pix_half(P);
-    double acc = 0.0, ws = 0.0;
-    unsigned long long cand = 0, within = 0, skips = 0;
-    for (int rb = 0; rb < P.nr; rb += 32) {
-        int r = rb + lane;
-        uint32_t lo = 0, hi = 0;
-        if (r < P.nr) {
-            if (!ring_window(a.h, a.rings[P.ur + r], P, a.keys, a.ptab, lo, hi)) ++skips;
-        }
-        uint32_t len = hi > lo ? hi - lo : 0;
-        uint32_t incl = len;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
+        for (int i = 0; i < 4; ++i) {
+            acc[i] = in[i] && v[i].h < a.hlo;
+            if (in[i] && !acc[i] && v[i].h <= a.hhi) band |= 1u << i;
         }
-        uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t tb = 0; tb < total; tb += 32) {
-            uint32_t t = tb + lane;
-            int src = owner_lane(incl, t);
-            uint32_t s_lo = __shfl_sync(0xffffffffu, lo, src);
-            uint32_t s_incl = __shfl_sync(0xffffffffu, incl, src);
-            uint32_t s_len = __shfl_sync(0xffffffffu, len, src);
-            if (t < total) {
-                uint32_t idx = s_lo + (t - (s_incl - s_len));
-                const double wt = pair_weight<GEN>(a, P, ph, idx);
-                ++cand;
-                if (wt != 0.0) {
-                    acc += (double)__ldg(data + (uint64_t)idx * cstride) * wt;
-                    ws += wt;
-                    ++within;
-                }
+        if (F32 && !GEN && a.series32) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float gs = gauss_series_f32(v[i].h, a.x2scale);
+                w[i] = acc[i] ? win * (double)gs : 0.0;
+            }
+        } else {
+            double d2[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d2[i] = pair_d2(a, acc[i] ? v[i].h : 0.0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double k = kernel_at<F32, GEN>(a, q[i], v[i], sl2, sb2, cb2, win, d2[i]);
+                w[i] = acc[i] ? k : 0.0;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) wf[i] = F32 ? (float)w[i] : 0.f;
+    }
+    if (band) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (band >> i & 1u) {
+                w[i] = pair_band<F32, GEN>(a, P + (i & 1) + (uint64_t)(i >> 1) * nx, idx);
+                wf[i] = F32 ? (float)w[i] : 0.f;
             }
         }
     }
-    acc = warp_sum(acc);
-    ws = warp_sum(ws);
-    cand = warp_sum_u64(cand);
-    within = warp_sum_u64(within);
-    skips = warp_sum_u64(skips);
-    if (lane == 0) {
-        out[p] = (float)(acc / ws);
-        if (wout) wout[p] = (float)ws;
-        if (cand) atomicAdd(&a.stats->pairs_candidate, cand);
-        if (within) atomicAdd(&a.stats->pairs_within, within);
-        if (skips) atomicAdd(&a.stats->ring_skips, skips);
+}
+
+// Sums of four values over a warp's lanes: lanes 8q .. 8q + 7 return value q's
+// (six exchanges instead of twenty).
+__device__ __forceinline__ double warp_sum4(const double v[4]) {
+    const int lane = threadIdx.x & 31;
+    const bool up = lane & 16, odd = lane & 8;
+    double a0 = up ? v[2] : v[0], a1 = up ? v[3] : v[1];
+    a0 += __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+    a1 += __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+    double s = odd ? a1 : a0;
+    s += __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 8);
+#pragma unroll
+    for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// A warp's ring records: per ring with candidates (compacted, in ring order),
+// the union's first candidate as the sample index of candidate 0 of the ring
+// block, the slot shift, and the four pixels' windows as (first sample, length).
+struct GroupRecords {
+    uint4 ra[32], rb[32];
+    uint2 rc[32];
+};
+// A warp's shared memory for one 2x2 group taken by itself: pixels and records.
+constexpr int kGroupWarps = 4, kGroupThreads = 32 * kGroupWarps, kGroupCtas = 5;
+struct GroupShared {
+    PixPrep prep[4];
+    PixHalf h[4];
+    double cb1[4];
+    GroupRecords rec;
+};
+
+// Pixels of group grp into the warp's shared memory (pixels outside the map
+// hold no rings).
+__device__ __forceinline__ void group_load(GroupShared &S, const PixPrep *__restrict__ prep, uint64_t pix0,
+                                           uint32_t nx, bool xin, bool yin) {
+    static_assert(sizeof(PixPrep) == 11 * sizeof(double), "eleven words a pixel");
+    const int lane = threadIdx.x & 31, q = lane >> 3, i = lane & 7;
+    const bool valid = (!(q & 1) || xin) && (!(q >> 1) || yin);
+    const double *src = reinterpret_cast<const double *>(prep + pix0 + (q & 1) + (uint64_t)(q >> 1) * nx);
+    double *dst = reinterpret_cast<double *>(&S.prep[q]);
+    __syncwarp();
+    dst[i] = valid ? __ldg(src + i) : 0.0;
+    if (i < 3) dst[8 + i] = valid ? __ldg(src + 8 + i) : 0.0;
+    __syncwarp();
+    if (lane < 4) {
+        S.h[lane] = S.prep[lane].h;
+        S.cb1[lane] = S.prep[lane].cb1;
+    }
+    __syncwarp();
+}
+
+// One block of up to 32 rings (lane = ring) of a group: every union candidate,
+// 32 at a time, tested against the four pixels; `body(idx, slot, w, wf)` gets
+// the candidate's weights. Warp-collective. What bounds it: instruction
+// issue (about 40 a pair) with the FP64 pipe next. The ring of a candidate is
+// found from one reduction of the ring ends that fall into the round (a bit
+// each) instead of a search by shuffles, its record read from shared memory
+// instead of sixteen shuffles, and a candidate's geometry is loaded once for
+// four pixels.
+template <bool F32, int MODE, typename BODY>
+__device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s_h, const double *s_cb1,
+                                             GroupRecords &S, uint64_t pix0, uint32_t nx, const uint32_t lo[4],
+                                             const uint32_t hi[4], uint32_t shift, BODY body) {
+    const int lane = threadIdx.x & 31;
+    uint32_t glo = 0xffffffffu, ghi = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (hi[q] > lo[q]) {
+            glo = min(glo, lo[q]);
+            ghi = max(ghi, hi[q]);
+        }
+    }
+    const uint32_t len = glo < ghi ? ghi - glo : 0;
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    const int c = __popc(__ballot_sync(0xffffffffu, len > 0) & ((1u << lane) - 1u));
+    __syncwarp();  // the records of the previous ring block are no longer read
+    if (len) {
+        auto n = [&](int q) { return hi[q] > lo[q] ? hi[q] - lo[q] : 0u; };
+        S.ra[c] = make_uint4(glo - (incl - len), shift, lo[0], n(0));
+        S.rb[c] = make_uint4(lo[1], n(1), lo[2], n(2));
+        S.rc[c] = make_uint2(lo[3], n(3));
+    }
+    __syncwarp();
+    for (uint32_t tb = 0; tb < total; tb += 32) {
+        // the pixels' constants are read anew each round (the barrier keeps the
+        // compiler from holding their 40 registers, which cost a third of the warps)
+        __syncwarp();
+        PixHalf ph[4];
+        double cb1[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            ph[q] = s_h[q];
+            cb1[q] = s_cb1[q];
+        }
+        const uint32_t t = tb + lane;
+        const unsigned ends = __reduce_or_sync(0xffffffffu, len && incl > tb && incl - tb < 32 ? 1u << (incl - tb) : 0u);
+        const int c0 = __popc(__ballot_sync(0xffffffffu, len && incl <= tb));
+        const bool act = t < total;
+        const int r = act ? c0 + __popc(ends & (0xffffffffu >> (31 - lane))) : c0;
+        const uint4 ra = S.ra[r], rb = S.rb[r];
+        const uint2 rc = S.rc[r];
+        // a lane past the last candidate repeats the round's first one, outside every window
+        const uint32_t idx = ra.x + (act ? t : tb);
+        const double2 sl2 = __ldg(a.half + idx), sb2 = __ldg(a.half + a.n + idx);
+        const double cb2 = __ldg(a.cb2 + idx), win = MODE == kPairUnit || a.unit_w ? 1.0 : __ldg(a.w + idx);
+        const bool in[4] = {act && idx - ra.z < ra.w, act && idx - rb.x < rb.y, act && idx - rb.z < rb.w,
+                            act && idx - rc.x < rc.y};
+        double w[4];
+        float wf[4];
+        pair_weights<F32, MODE>(a, a.prep + pix0, nx, ph, cb1, sl2, sb2, cb2, win, idx, in, w, wf);
+        body(idx, idx + ra.y, w, wf);
+    }
+}
+
+// Windows of this lane's ring k of a group computed from the pixels in the
+// warp's shared memory.
+__device__ __forceinline__ void group_lane_windows(const GridArgs &a, const GroupGeo &G, int k, uint64_t pix0,
+                                                   uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
+                                                   uint32_t &skips) {
+    if (k > G.r1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) lo[q] = hi[q] = 0;
+    } else if (a.rwin) {
+        group_windows(a, a.rwin[k], k, G, pix0, nx, lo, hi, ref, skips);
+    } else {
+        group_windows_general(a, k, G, pix0, nx, lo, hi, ref, skips);
+    }
+}
+
+// Pair counts a warp's groups add up (flushed by its kernel).
+struct PairCounts {
+    unsigned long long cand = 0, within = 0, skips = 0;
+};
+// The block's counts to the context's statistics: one atomic per block (one
+// per pixel or group on one address was a bound of its own). Block-collective.
+__device__ __forceinline__ void flush_counts(const PairCounts &c, DevStats *stats) {
+    __shared__ unsigned long long s_c[3];
+    if (threadIdx.x < 3) s_c[threadIdx.x] = 0;
+    __syncthreads();
+    const unsigned long long v[3] = {warp_sum_u64(c.cand), warp_sum_u64(c.within), warp_sum_u64(c.skips)};
+    if ((threadIdx.x & 31) == 0)
+        for (int i = 0; i < 3; ++i)
+            if (v[i]) atomicAdd(&s_c[i], v[i]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_c[0]) atomicAdd(&stats->pairs_candidate, s_c[0]);
+        if (s_c[1]) atomicAdd(&stats->pairs_within, s_c[1]);
+        if (s_c[2]) atomicAdd(&stats->ring_skips, s_c[2]);
+    }
+}
+
+// Single channel: one warp per 2x2 group of pixels, FP64 throughout: the
+// windows (a ring per lane, four pixels each), every union candidate against
+// the four pixels, normalise. Warp-collective.
+template <bool GEN>
+__device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint32_t ny,
+                                           const float *__restrict__ data, uint32_t cstride, float *__restrict__ out,
+                                           float *__restrict__ wout, uint64_t grp, GroupShared &S, PairCounts &pc) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t gx = (nx + 1) / 2, gyi = (uint32_t)(grp / gx), gxi = (uint32_t)(grp % gx);
+    const bool xin = 2 * gxi + 1 < nx, yin = 2 * gyi + 1 < ny;
+    const uint64_t pix0 = (uint64_t)(2 * gyi) * nx + 2 * gxi;
+    group_load(S, a.prep, pix0, nx, xin, yin);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0}, ws[4] = {0.0, 0.0, 0.0, 0.0};
+    uint32_t ref = 0, within = 0, skips = 0;
+    for (int rb = 0, nr = 1; rb < nr; rb += 32) {
+        uint32_t lo[4], hi[4];
+        {  // the group's extent is not kept across the pair tests (registers)
+            const GroupGeo G = group_geo([&](int q) { return &S.prep[q]; });
+            nr = G.r1 - G.r0 + 1;
+            group_lane_windows(a, G, G.r0 + rb + lane, pix0, nx, lo, hi, ref, skips);
+        }
+        group_rounds<false, GEN ? kPairOther : kPairGeneral>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u, [&](uint32_t idx, uint32_t, const double w[4], const float[4]) {
+            const double x = (double)__ldg(data + (uint64_t)idx * cstride);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (w[q] != 0.0) {
+                    acc[q] += x * w[q];
+                    ws[q] += w[q];
+                    ++within;
+                }
+            }
+        });
+    }
+    pc.cand += ref;
+    pc.within += within;
+    pc.skips += skips;
+    const double A = warp_sum4(acc), W = warp_sum4(ws);
+    const int q = lane >> 3;
+    if ((lane & 7) == 0 && (!(q & 1) || xin) && (!(q >> 1) || yin)) {
+        const uint64_t p = pix0 + (q & 1) + (uint64_t)(q >> 1) * nx;
+        out[p] = (float)(A / W);
+        if (wout) wout[p] = (float)W;
     }
 }
 
@@ -502,9 +899,9 @@ struct TileArgs {
     int *r0, *nr;
     uint32_t *U, *ulo, *base;  // ulo: [tile][kTileMaxRings], base: [tile][kTileMaxRings + 1]
     uint16_t *ring_idx;        // [tile][kTileMaxSpan]: index c of ring r0 + j (0xffff: no candidates)
-    uint32_t *cap;             // per 2x2 group: union candidate count (kCapUnknown: left to k_group<true>)
+    uint32_t *cap;             // per 2x2 group: union candidate count (kCapUnknown: left to group_count_item)
     uint4 *win;                // [tile][kWinSpan][kTileGroups][2]: the group's 4 pixel windows per ring (or null)
-    unsigned long long *overflow;
+    unsigned long long *overflow;  // tiles beyond the ring table (their groups are counted by group_count_item)
     uint32_t pad;  // ring runs take a multiple of `pad` slots (> 1: the tensor-core engine's 8-row boxes)
     unsigned long long *ustat;  // [0]: sum, [1]: largest of the tiles' staged slots U (or null)
 };
@@ -527,179 +924,191 @@ cudaError_t tc_weights(hcg_context *ctx, const hcg_field *f, const GridArgs &a, 
 
 namespace {
 
-// One warp per 2x2 pixel group. COUNT: number of union candidates (upper
-// bound of the entries). Otherwise: FP64 weights of every union candidate
-// for the 4 pixels, compacted to entries with any non-zero weight.
-// With a tile table (`tiles.ulo` set) the entries hold the sample's slot in
-// its tile's staged list instead of the sample index.
-// Warp-collective: every lane passes the same group; s_prep is this warp's
-// 4-entry shared-memory slot.
-// PACK: 0 FP32 weights, 1 packed hi/lo pairs (GroupArgs::pack), 2 as g.pack says.
-template <bool COUNT, bool GEN = false, int PACK = 2>  // GEN as pair_weight_s
-__device__ __forceinline__ void group_item(const GridArgs &a, const GroupArgs &g, uint32_t *__restrict__ cap,
-                                           const unsigned long long *__restrict__ off,
-                                           uint32_t *__restrict__ e_idx, float4 *__restrict__ e_w,
-                                           uint32_t *__restrict__ cnt, double *__restrict__ wsum,
-                                           const TileArgs &tiles, uint64_t grp, PixPrep *s_prep, PixHalf *s_half) {
-    int lane = threadIdx.x & 31;
-    __syncwarp();
-    if (COUNT && cap[grp] != kCapUnknown) return;  // counted by the tile pass
-    uint32_t gyi = (uint32_t)(grp / g.gx), gxi = (uint32_t)(grp % g.gx);
-    uint64_t pix[4];
-    bool valid[4];
+// Union candidates of a 2x2 group (upper bound of its entries), for the groups
+// the tile pass left uncounted. Warp-collective.
+__device__ __forceinline__ void group_count_item(const GridArgs &a, const GroupArgs &g, uint32_t *__restrict__ cap,
+                                                 uint64_t grp, GroupShared &S) {
+    const int lane = threadIdx.x & 31;
+    if (cap[grp] != kCapUnknown) return;  // counted by the tile pass
+    const uint32_t gyi = (uint32_t)(grp / g.gx), gxi = (uint32_t)(grp % g.gx);
+    const uint64_t pix0 = (uint64_t)(2 * gyi) * g.nx + 2 * gxi;
+    group_load(S, a.prep, pix0, g.nx, 2 * gxi + 1 < g.nx, 2 * gyi + 1 < g.ny);
+    const GroupGeo G = group_geo([&](int q) { return &S.prep[q]; });
+    unsigned long long count = 0;
+    for (int rb = G.r0; rb <= G.r1; rb += 32) {
+        uint32_t lo[4], hi[4], ref = 0, skips = 0, glo = 0xffffffffu, ghi = 0;
+        group_lane_windows(a, G, rb + lane, pix0, g.nx, lo, hi, ref, skips);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        uint32_t xx = 2 * gxi + (q & 1), yy = 2 * gyi + (q >> 1);
-        valid[q] = xx < g.nx && yy < g.ny;
-        pix[q] = (uint64_t)yy * g.nx + xx;
-    }
-    if (lane < 4 && valid[lane]) {
-        s_prep[lane] = a.prep[pix[lane]];
-        if (!COUNT) s_half[lane] = pix_half(s_prep[lane]);
-    }
-    __syncwarp();
-    int R0 = 1 << 30, R1 = -1;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        if (valid[q] && s_prep[q].nr > 0) {
-            R0 = min(R0, s_prep[q].ur);
-            R1 = max(R1, s_prep[q].ur + s_prep[q].nr - 1);
-        }
-    }
-    unsigned lt = (1u << lane) - 1u;
-    unsigned long long count = 0, within = 0;
-    uint32_t base = 0;
-    double ws[4] = {0.0, 0.0, 0.0, 0.0};
-    const unsigned long long eoff = COUNT ? 0 : off[grp] - g.ebase;
-    bool slots = !COUNT && tiles.ulo != nullptr;
-    uint64_t tile = 0;
-    int tr0 = 0;
-    if (slots) {
-        tile = (uint64_t)(gyi / (kTileY / 2)) * tiles.ntx + gxi / (kTileX / 2);
-        tr0 = tiles.r0[tile];
-        slots = tiles.nr[tile] > 0;  // no ring table (tile without samples, or one spanning too many rings)
-    }
-    for (int rb = R0; rb <= R1; rb += 32) {
-        int k = rb + lane;
-        uint32_t lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
-        uint32_t glo = 0xffffffffu, ghi = 0;
-        long long slot_shift = 0;  // slot = idx + slot_shift for this lane's ring
-        if (slots && k <= R1) {
-            const uint32_t c = tiles.ring_idx[tile * kTileMaxSpan + (uint64_t)(k - tr0)];
-            if (c < kTileMaxRings)  // rings without tile candidates have none for the group either
-                slot_shift = (long long)tiles.base[tile * (kTileMaxRings + 1) + c] -
-                             (long long)tiles.ulo[tile * kTileMaxRings + c];
-        }
-        if (k <= R1 && !COUNT && slots && tiles.win && k - tr0 < kWinSpan) {
-            // the tile pass kept this group's windows for the ring
-            const uint4 *w = tiles.win + ((tile * kWinSpan + (uint64_t)(k - tr0)) * kTileGroups +
-                                          (uint64_t)((gyi % (kTileY / 2)) * (kTileX / 2) + gxi % (kTileX / 2))) * 2;
-            const uint4 w0 = __ldg(w), w1 = __ldg(w + 1);
-            const uint32_t kl[4] = {w0.x, w0.z, w1.x, w1.z}, kh[4] = {w0.y, w0.w, w1.y, w1.w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (kl[q] <= kh[q]) {  // lo > hi: a ring the reference would spin on
-                    lo[q] = kl[q];
-                    hi[q] = kh[q];
-                    if (hi[q] > lo[q]) {
-                        glo = min(glo, lo[q]);
-                        ghi = max(ghi, hi[q]);
-                    }
-                }
-            }
-        } else if (k <= R1) {
-            const RingRec R = a.rings[k];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const PixPrep &P = s_prep[q];
-                if (valid[q] && k >= P.ur && k < P.ur + P.nr) {
-                    uint32_t rl;
-                    if (ring_window_mc(a, R, P, lo[q], hi[q], rl) && hi[q] > lo[q]) {
-                        glo = min(glo, lo[q]);
-                        ghi = max(ghi, hi[q]);
-                    }
-                }
+        for (int q = 0; q < 4; ++q) {
+            if (hi[q] > lo[q]) {
+                glo = min(glo, lo[q]);
+                ghi = max(ghi, hi[q]);
             }
         }
-        uint32_t len = glo < ghi ? ghi - glo : 0;
-        if (COUNT) {
-            count += len;
-            continue;
-        }
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t tb = 0; tb < total; tb += 32) {
-            uint32_t t = tb + lane;
-            int src = owner_lane(incl, t);
-            uint32_t s_glo = __shfl_sync(0xffffffffu, glo, src);
-            uint32_t s_excl = __shfl_sync(0xffffffffu, incl - len, src);
-            long long s_shift = __shfl_sync(0xffffffffu, slot_shift, src);
-            uint32_t s_lo[4], s_hi[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                s_lo[q] = __shfl_sync(0xffffffffu, lo[q], src);
-                s_hi[q] = __shfl_sync(0xffffffffu, hi[q], src);
-            }
-            float wq[4] = {0.f, 0.f, 0.f, 0.f};
-            uint32_t idx = 0;
-            bool any = false;
-            if (t < total) {
-                idx = s_glo + (t - s_excl);
-                const double4 hs = ldg4(a.half + idx);
-                const double cb2 = __ldg(a.cb2 + idx), win = __ldg(a.w + idx);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (idx >= s_lo[q] && idx < s_hi[q]) {
-                        const double wt = pair_weight_s<true, GEN>(a, s_prep[q], s_half[q], hs, cb2, win, idx);
-                        if (wt != 0.0) {
-                            ws[q] += wt;
-                            wq[q] = (float)wt;
-                            any = true;
-                            ++within;
-                        }
-                    }
-                }
-                if (PACK == 1 || (PACK == 2 && g.pack)) {
-                    // the four slots carry {hi(w0, w1), lo(w0, w1), hi(w2, w3), lo(w2, w3)}
-                    uint32_t h01, l01, h23, l23;
-                    tc_split2(wq[0] * g.wscale, wq[1] * g.wscale, g.fmt, h01, l01);
-                    tc_split2(wq[2] * g.wscale, wq[3] * g.wscale, g.fmt, h23, l23);
-                    wq[0] = __uint_as_float(h01);
-                    wq[1] = __uint_as_float(l01);
-                    wq[2] = __uint_as_float(h23);
-                    wq[3] = __uint_as_float(l23);
-                }
-            }
-            unsigned ball = __ballot_sync(0xffffffffu, any);
-            if (any) {
-                unsigned long long pos = eoff + base + __popc(ball & lt);
-                e_idx[pos] = slots ? (uint32_t)((long long)idx + s_shift) : idx;
-                e_w[pos] = make_float4(wq[0], wq[1], wq[2], wq[3]);
-            }
-            base += __popc(ball);
-        }
+        if (glo < ghi) count += ghi - glo;
     }
     count = warp_sum_u64(count);
-    within = warp_sum_u64(within);
-    if constexpr (COUNT) {
-        if (lane == 0) cap[grp] = (uint32_t)count;
-        return;
-    } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) ws[q] = warp_sum(ws[q]);
-        if (lane == 0) {
-            cnt[grp] = base;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (valid[q]) wsum[pix[q]] = ws[q];
-            if (within) atomicAdd(&a.stats->pairs_within, within);
+    if (lane == 0) cap[grp] = (uint32_t)count;
+}
+
+// Shared memory of a tile's weight pass: per 2x2 group the pixel constants of
+// the pair test and the ring range, per ring of the tile's span the shift from
+// sample index to slot, and each warp's ring records.
+constexpr int kTileShifts = 128, kWeightWarps = 4, kWeightThreads = 32 * kWeightWarps, kWeightCtas = 5;
+struct TileGroupShared {
+    struct Px {
+        PixHalf h[4];
+        double cb1[4];
+    } px[kTileGroups];
+    int r0[kTileGroups], r1[kTileGroups];
+    uint32_t shift[kTileShifts];
+    GroupRecords rec[kWeightWarps];
+};
+
+// FP64 distance and cutoff of every union candidate of the tile's 2x2 groups
+// for their 4 pixels, compacted to entries with any non-zero weight, and the
+// FP64 weight sums. Block-collective (kWeightThreads, one a pixel): the tile's
+// pixels and slot shifts are loaded once, then each warp takes eight groups in
+// turn (or `parts` blocks share the tile, block `part` taking every parts-th
+// four groups). With a tile
+// table (`T.ulo` set) the entries hold the sample's slot in the tile's staged
+// list instead of the sample index, and the windows are the ones the tile pass
+// kept. What bounds it: the latency of the window and geometry loads at the
+// warps that fit, then instruction issue. 500,000 samples, 512 x 500 pixels:
+// 305 us with a warp per group, each finding its own tile, pixels and windows.
+// PACK: 0 FP32 weights, 1 packed hi/lo pairs (GroupArgs::pack), 2 as g.pack says.
+template <int MODE = kPairGeneral, int PACK = 2>
+__device__ __forceinline__ void group_tile_item(const GridArgs &a, const GroupArgs &g,
+                                                const unsigned long long *__restrict__ off,
+                                                uint32_t *__restrict__ e_idx, float4 *__restrict__ e_w,
+                                                uint32_t *__restrict__ cnt, double *__restrict__ wsum,
+                                                const TileArgs &T, bool tiled, uint64_t tile, uint32_t part,
+                                                uint32_t parts, TileGroupShared &S, PairCounts &pc) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t tx0 = (uint32_t)(tile % T.ntx) * kTileX, ty0 = (uint32_t)(tile / T.ntx) * kTileY;
+    __syncthreads();  // shared state of a previous item is no longer read
+    static_assert(kWeightThreads == kTileX * kTileY, "a thread per pixel");
+    const uint32_t px = tid % kTileX, py = tid / kTileX;
+    const int pg = (py / 2) * (kTileX / 2) + px / 2, pq = (py & 1) * 2 + (px & 1);
+    const bool pin = tx0 + px < g.nx && ty0 + py < g.ny;
+    if (tid < kTileGroups) {
+        S.r0[tid] = 1 << 30;
+        S.r1[tid] = -1;
+    }
+    __syncthreads();
+    {
+        const PixPrep *src = a.prep + (uint64_t)(ty0 + py) * g.nx + tx0 + px;
+        S.px[pg].h[pq] = pin ? src->h : PixHalf{0.0, 0.0, 0.0, 0.0};
+        S.px[pg].cb1[pq] = pin ? src->cb1 : 0.0;
+        if (pin && src->nr > 0) {
+            atomicMin(&S.r0[pg], src->ur);
+            atomicMax(&S.r1[pg], src->ur + src->nr - 1);
         }
     }
+    // no ring table: a tile without samples, or one spanning too many rings
+    const bool slots = tiled && T.nr[tile] > 0;
+    const int tr0 = slots ? T.r0[tile] : 0;
+    __syncthreads();
+    if (slots) {
+        const int span = __reduce_max_sync(0xffffffffu, S.r1[lane]) - tr0 + 1;
+        for (int j = tid; j < min(span, kTileShifts); j += kWeightThreads) {
+            const uint32_t c = T.ring_idx[tile * kTileMaxSpan + j];
+            // rings without tile candidates have none for the groups either
+            S.shift[j] = c < kTileMaxRings
+                             ? T.base[tile * (kTileMaxRings + 1) + c] - T.ulo[tile * kTileMaxRings + c]
+                             : 0u;
+        }
+    }
+    __syncthreads();
+    const unsigned lt = (1u << lane) - 1u;
+    const uint4 *win = slots && T.win ? T.win + tile * (kWinSpan * kTileGroups * 2) : nullptr;
+    // windows of ring (first ring of group gl + lane) kept by the tile pass
+    auto kept = [&](int gl, int rb, uint4 &w0, uint4 &w1) {
+        const int j = rb + lane - tr0;
+        w0 = w1 = make_uint4(0, 0, 0, 0);
+        if (win && rb + lane <= S.r1[gl] && j < kWinSpan) {
+            w0 = __ldg(win + (j * kTileGroups + gl) * 2);
+            w1 = __ldg(win + (j * kTileGroups + gl) * 2 + 1);
+        }
+    };
+    const uint32_t gx0 = tx0 / 2, gy0 = ty0 / 2, gny = (g.ny + 1) / 2;
+    uint32_t within = 0;
+    for (int gl = part * kWeightWarps + warp; gl < kTileGroups; gl += kWeightWarps * parts) {
+        const uint32_t gxi = gx0 + gl % (kTileX / 2), gyi = gy0 + gl / (kTileX / 2);
+        if (gxi >= g.gx || gyi >= gny) continue;
+        const uint64_t grp = (uint64_t)gyi * g.gx + gxi;
+        const bool xin = 2 * gxi + 1 < g.nx, yin = 2 * gyi + 1 < g.ny;
+        const uint64_t pix0 = (uint64_t)(2 * gyi) * g.nx + 2 * gxi;
+        const int R0 = S.r0[gl], R1 = S.r1[gl];
+        const unsigned long long first = off[grp] - g.ebase;
+        uint32_t *const ei = e_idx + first;
+        float4 *const ew = e_w + first;
+        uint32_t n = 0;
+        double ws[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int rb = R0; rb <= R1; rb += 32) {
+            const int k = rb + lane, j = k - tr0;
+            uint4 w0, w1;
+            kept(gl, rb, w0, w1);
+            uint32_t lo[4] = {w0.x, w0.z, w1.x, w1.z}, hi[4] = {w0.y, w0.w, w1.y, w1.w};
+            uint32_t shift = 0;  // slot = idx + shift (mod 2^32) for this lane's ring
+            if (k <= R1) {
+                if (slots) {
+                    if (j < kTileShifts) {
+                        shift = S.shift[j];
+                    } else {
+                        const uint32_t c = T.ring_idx[tile * kTileMaxSpan + j];
+                        if (c < kTileMaxRings)
+                            shift = T.base[tile * (kTileMaxRings + 1) + c] - T.ulo[tile * kTileMaxRings + c];
+                    }
+                }
+                if (!win || j >= kWinSpan) {
+                    uint32_t ref = 0, skips = 0;
+                    const GroupGeo G = group_geo([&](int q) -> const PixPrep * {
+                        return (!(q & 1) || xin) && (!(q >> 1) || yin) ? a.prep + pix0 + (q & 1) + (uint64_t)(q >> 1) * g.nx
+                                                                       : nullptr;
+                    });
+                    group_lane_windows(a, G, k, pix0, g.nx, lo, hi, ref, skips);
+                }
+            }
+            group_rounds<true, MODE>(
+                a, S.px[gl].h, S.px[gl].cb1, S.rec[warp], pix0, g.nx, lo, hi, shift,
+                [&](uint32_t, uint32_t slot, const double w[4], const float wf[4]) {
+                    bool any = false;
+                    float e[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        e[q] = wf[q];
+                        const bool nz = MODE == kPairUnit ? wf[q] != 0.f : w[q] != 0.0;
+                        ws[q] += w[q];
+                        any = any || nz;
+                        within += nz;
+                    }
+                    if (PACK == 1 || (PACK == 2 && g.pack)) {
+                        // the four slots carry {hi(w0, w1), lo(w0, w1), hi(w2, w3), lo(w2, w3)}
+                        uint32_t h01, l01, h23, l23;
+                        tc_split2(e[0] * g.wscale, e[1] * g.wscale, g.fmt, h01, l01);
+                        tc_split2(e[2] * g.wscale, e[3] * g.wscale, g.fmt, h23, l23);
+                        e[0] = __uint_as_float(h01);
+                        e[1] = __uint_as_float(l01);
+                        e[2] = __uint_as_float(h23);
+                        e[3] = __uint_as_float(l23);
+                    }
+                    const unsigned ball = __ballot_sync(0xffffffffu, any);
+                    if (any) {
+                        const uint32_t at = n + __popc(ball & lt);
+                        ei[at] = slot;
+                        ew[at] = make_float4(e[0], e[1], e[2], e[3]);
+                    }
+                    n += __popc(ball);
+                });
+        }
+        const double W = warp_sum4(ws);
+        const int q = lane >> 3;
+        if (lane == 0) cnt[grp] = n;
+        if ((lane & 7) == 0 && (!(q & 1) || xin) && (!(q >> 1) || yin))
+            wsum[pix0 + (q & 1) + (uint64_t)(q >> 1) * g.nx] = W;
+    }
+    pc.within += within;
 }
 
 // Exclusive scan of n u32 counts into u64 offsets (out[n] = the total), in
@@ -867,37 +1276,45 @@ __device__ __forceinline__ void group_accum_item(const GroupArgs &g, const unsig
 
 // Union of the ring windows of all pixels of one tile, per ring, and the
 // slot each ring's union starts at in the tile's staged list.
-// Block-collective (call with every thread of a 256-thread block).
+// Block-collective (W warps): a warp
+// takes every W-th ring of the tile's span and each lane one 2x2 group, so a
+// ring's record is one broadcast load, the chord's bound is formed once for
+// four pixels, and the tile's union of a ring is one warp reduction. What bounds
+// it: issue of the windows' arithmetic, then the latency of their table
+// lookups. 4M samples, 1200 x 1200 pixels: 1034 us with a general window per
+// thread and shared-memory atomics per group.
+// W: four warps a tile where the tiles fill the GPU (96 registers, 20 warps an
+// SM), eight where they do not and the latency of one tile is what counts.
+constexpr int kRingCtas = 5;
+template <int W>
 __device__ __forceinline__ void tile_rings_item(const GridArgs &a, const GroupArgs &g, const TileArgs &T,
                                                 uint64_t tile) {
-    __shared__ PixPrep s_prep[kTileX * kTileY];
     __shared__ uint32_t s_lo[kTileMaxSpan], s_hi[kTileMaxSpan];
     __shared__ uint32_t s_cnt[kTileGroups];
+    __shared__ unsigned long long s_cand, s_skips;
     __shared__ int s_r0, s_r1;
     const uint32_t tx0 = (uint32_t)(tile % T.ntx) * kTileX, ty0 = (uint32_t)(tile / T.ntx) * kTileY;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t xx = tx0 + 2 * (lane % (kTileX / 2)), yy = ty0 + 2 * (lane / (kTileX / 2));
+    const uint64_t pix0 = (uint64_t)yy * g.nx + xx;
+    static_assert(kTileGroups == 32, "a lane per group");
+    const GroupGeo G = group_geo([&](int q) -> const PixPrep * {
+        return xx + (q & 1) < g.nx && yy + (q >> 1) < g.ny ? a.prep + pix0 + (q & 1) + (uint64_t)(q >> 1) * g.nx
+                                                            : nullptr;
+    });
     __syncthreads();  // shared state of a previous item is no longer read
-    if (tid == 0) { s_r0 = 1 << 30; s_r1 = -1; }
     if (tid < kTileGroups) s_cnt[tid] = 0;
-    __syncthreads();
-    if (tid < kTileX * kTileY) {
-        uint32_t xx = tx0 + tid % kTileX, yy = ty0 + tid / kTileX;
-        PixPrep P;
-        if (xx < g.nx && yy < g.ny) {
-            P = a.prep[(uint64_t)yy * g.nx + xx];
-        } else {
-            P.nr = 0;
-            P.ur = 0;
-        }
-        s_prep[tid] = P;
-        if (P.nr > 0) {
-            atomicMin(&s_r0, P.ur);
-            atomicMax(&s_r1, P.ur + P.nr - 1);
+    if (warp == 0) {
+        const int lo = __reduce_min_sync(0xffffffffu, G.r0), hi = __reduce_max_sync(0xffffffffu, G.r1);
+        if (lane == 0) {
+            s_r0 = lo;
+            s_r1 = hi;
+            s_cand = s_skips = 0;
         }
     }
     __syncthreads();
     const int r0 = s_r0, nrt = s_r1 - s_r0 + 1;
-    // candidate counts of the tile's 2x2 groups (the entries k_group<false> may emit)
+    // candidate counts of the tile's 2x2 groups (the entries k_group may emit)
     auto write_caps = [&](bool known) {
         if (!T.cap || tid >= kTileGroups) return;
         const uint32_t gxi = (uint32_t)(tile % T.ntx) * (kTileX / 2) + tid % (kTileX / 2);
@@ -905,84 +1322,62 @@ __device__ __forceinline__ void tile_rings_item(const GridArgs &a, const GroupAr
         const uint64_t grp = (uint64_t)gyi * g.gx + gxi;
         if (gxi < g.gx && grp < g.ngroups) T.cap[grp] = known ? s_cnt[tid] : kCapUnknown;
     };
+    // a span beyond the table keeps no windows and no unions; its groups are
+    // counted later, its candidate statistic is taken here all the same
+    const bool known = nrt <= kTileMaxSpan;
+    unsigned long long cand = 0;
+    uint32_t skips = 0, mine = 0;  // mine: the group's union candidates
+    for (int j = warp; j < nrt; j += W) {
+        const int k = r0 + j;
+        uint32_t lo[4], hi[4], ref = 0;
+        if (a.rwin)
+            group_windows(a, a.rwin[k], k, G, pix0, g.nx, lo, hi, ref, skips);
+        else
+            group_windows_general(a, k, G, pix0, g.nx, lo, hi, ref, skips);
+        cand += ref;
+        if (!known) continue;
+        if (T.win && j < kWinSpan) {
+            uint4 *w = T.win + ((tile * kWinSpan + j) * kTileGroups + lane) * 2;
+            w[0] = make_uint4(lo[0], hi[0], lo[1], hi[1]);
+            w[1] = make_uint4(lo[2], hi[2], lo[3], hi[3]);
+        }
+        uint32_t glo = 0xffffffffu, ghi = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (hi[q] > lo[q]) {
+                glo = min(glo, lo[q]);
+                ghi = max(ghi, hi[q]);
+            }
+        }
+        if (glo < ghi) mine += ghi - glo;
+        glo = __reduce_min_sync(0xffffffffu, glo);
+        ghi = __reduce_max_sync(0xffffffffu, ghi);
+        if (lane == 0) {
+            s_lo[j] = glo;
+            s_hi[j] = ghi;
+        }
+    }
     // the candidate statistic: the reference windows' lengths (the pairs the
     // reference visits) of every (pixel, ring) of the tile, and the rings the
     // reference would spin on
-    unsigned long long cand = 0, skips = 0;
-    auto add_cand = [&]() {
-        cand = warp_sum_u64(cand);
-        skips = warp_sum_u64(skips);
-        if ((tid & 31) == 0 && cand) atomicAdd(&a.stats->pairs_candidate, cand);
-        if ((tid & 31) == 0 && skips) atomicAdd(&a.stats->ring_skips, skips);
-    };
-    if (nrt <= 0 || nrt > kTileMaxSpan) {
+    if (mine) atomicAdd(&s_cnt[lane], mine);
+    cand = warp_sum_u64(cand);
+    skips = __reduce_add_sync(0xffffffffu, skips);
+    if (lane == 0 && cand) atomicAdd(&s_cand, cand);
+    if (lane == 0 && skips) atomicAdd(&s_skips, (unsigned long long)skips);
+    __syncthreads();
+    if (tid == 0 && s_cand) atomicAdd(&a.stats->pairs_candidate, s_cand);
+    if (tid == 0 && s_skips) atomicAdd(&a.stats->ring_skips, s_skips);
+    write_caps(nrt <= 0 || known);  // no samples: nothing to count
+    if (nrt <= 0 || !known) {
         if (tid == 0) {
             T.r0[tile] = 0;
             T.nr[tile] = 0;
             T.U[tile] = 0;
-            if (nrt > kTileMaxSpan) atomicAdd(T.overflow, 1ULL);
+            if (!known) atomicAdd(T.overflow, 1ULL);
         }
-        write_caps(nrt <= 0);  // no samples: nothing to count
-        if (nrt > 0 && tid < kTileX * kTileY) {
-            const PixPrep &P = s_prep[tid];
-            for (int k = P.ur; k < P.ur + P.nr; ++k) {
-                uint32_t lo, hi, rl;
-                if (ring_window_mc(a, a.rings[k], P, lo, hi, rl))
-                    cand += rl;
-                else
-                    ++skips;
-            }
-        }
-        add_cand();
         return;
     }
-    for (int j = tid; j < nrt; j += blockDim.x) { s_lo[j] = 0xffffffffu; s_hi[j] = 0; }
-    __syncthreads();
-    // one (group, ring, pixel) triple per thread, the four pixels of a group in
-    // consecutive lanes: each thread forms one window (its dependent loads run
-    // beside the other lanes'), the quad's shuffles give the group's union
-    // (group_item's count) and the tile union takes min / max over groups. The
-    // loop runs whole warps (inactive lanes hold empty windows).
-    const int total = 4 * kTileGroups * nrt;
-    for (int ib = 0; ib < total; ib += blockDim.x) {
-        const int i = ib + tid;
-        const bool act = i < total;
-        const int q = i & 3, quad = i >> 2;
-        const int gq = quad % kTileGroups, j = quad / kTileGroups;
-        const int k = r0 + j;
-        uint32_t lo = 0, hi = 0;
-        if (act) {
-            const int p = (2 * (gq / (kTileX / 2)) + (q >> 1)) * kTileX + 2 * (gq % (kTileX / 2)) + (q & 1);
-            const PixPrep &P = s_prep[p];
-            if (P.nr > 0 && k >= P.ur && k < P.ur + P.nr) {
-                uint32_t rl;
-                if (!ring_window_mc(a, a.rings[k], P, lo, hi, rl)) {
-                    lo = 1;  // lo > hi: the reference would spin on this ring
-                    hi = 0;
-                    ++skips;
-                } else {
-                    cand += rl;
-                }
-            }
-        }
-        uint32_t glo = hi > lo ? lo : 0xffffffffu, ghi = hi > lo ? hi : 0;
-#pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-            glo = min(glo, __shfl_xor_sync(0xffffffffu, glo, o));
-            ghi = max(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
-        }
-        if (!act) continue;
-        if (T.win && j < kWinSpan)
-            reinterpret_cast<uint2 *>(T.win + ((tile * kWinSpan + j) * kTileGroups + gq) * 2)[q] = make_uint2(lo, hi);
-        if (q == 0 && glo < ghi) {
-            atomicAdd(&s_cnt[gq], ghi - glo);
-            atomicMin(&s_lo[j], glo);
-            atomicMax(&s_hi[j], ghi);
-        }
-    }
-    add_cand();
-    __syncthreads();
-    write_caps(true);
     if (tid < 32) {  // one warp: compaction of the occupied rings and prefix sums of their lengths
         uint32_t run = 0, count = 0;
         for (int jb = 0; jb < nrt; jb += 32) {

@@ -11,7 +11,7 @@
 // the library instead.
 //
 // The scratch is the per-pixel setup (ring range and the phi half of the
-// window arithmetic, 96 bytes a pixel) in a file-scope __device__ array of
+// window arithmetic, 88 bytes a pixel) in a file-scope __device__ array of
 // kNoAllocMaxPixels entries: 131072 pixels, 12 MiB, held by every GPU that
 // loads the library until the process exits. Host code may not pass the
 // array's name to a kernel (on the host it names a stand-in, not device
@@ -45,11 +45,15 @@ __global__ void k_noalloc_prep(HpxParams h, uint64_t firstring, uint64_t usedrin
 }
 
 template <bool GEN>  // fields whose kernel is not GAUSS1D
-__global__ void __launch_bounds__(256) k_noalloc_grid(GridArgs a, uint64_t npix, const float *__restrict__ data,
-                                                      uint32_t cstride, float *__restrict__ out,
-                                                      float *__restrict__ wout) {
-    uint64_t p = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    if (p < npix) grid1_item<GEN>(a, data, cstride, out, wout, p);
+__global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_noalloc_grid(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+                                                          const float *__restrict__ data, uint32_t cstride,
+                                                          float *__restrict__ out, float *__restrict__ wout) {
+    __shared__ GroupShared S[kGroupWarps];
+    PairCounts pc;
+    const int warp = threadIdx.x >> 5;
+    const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
+    if (grp < ngroups) grid1_item<GEN>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
+    flush_counts(pc, a.stats);
 }
 
 constexpr int kMaxDevices = 64;
@@ -128,11 +132,14 @@ extern "C" hcg_status hcg_grid_noalloc(hcg_context *ctx, const hcg_field *field,
         e = coarsen_prep(prep, target->nx, P, ctx->factor, s);
         for (auto &ev : ctx->evp) cudaEventRecord(ev, s);
         const GridArgs a = grid_args(field, prep, ctx->d_stats);
-        const unsigned nblk = (unsigned)((P * 32 + 255) / 256);
+        const uint64_t ngroups = (uint64_t)((target->nx + 1) / 2) * ((target->ny + 1) / 2);
+        const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
         if (field->kernel_type == HCG_GAUSS1D)
-            k_noalloc_grid<false><<<nblk, 256, 0, s>>>(a, P, field->d_spec, field->cstride, cube, weights_out);
+            k_noalloc_grid<false><<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride,
+                                                       cube, weights_out);
         else
-            k_noalloc_grid<true><<<nblk, 256, 0, s>>>(a, P, field->d_spec, field->cstride, cube, weights_out);
+            k_noalloc_grid<true><<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride,
+                                                      cube, weights_out);
         cudaEventRecord(ctx->ev1, s);
         if (e == cudaSuccess) e = cudaGetLastError();
     }

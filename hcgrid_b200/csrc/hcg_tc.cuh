@@ -861,7 +861,7 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, uint64_
 // (cp.async, one chunk ahead); then, for each slot whose sample lies in its
 // pixel's window of the slot's ring (ring_window_mc, the windows the tile pass
 // unioned), a builder evaluates the FP64 distance, cutoff and FP32 Gaussian
-// (pair_weight_s's arithmetic), accumulates the FP64 weight sum and writes its
+// (pair_weights' arithmetic), accumulates the FP64 weight sum and writes its
 // hi/lo pieces of the K-major operand row (16-byte stores). The epilogue adds
 // the three partial weight sums of a row from shared memory.
 constexpr int kTcGeo = 64;          // slots per chunk of the direct builders
@@ -909,7 +909,7 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
     const bool valid = xx < J.g.nx && yy < J.g.ny;
     PixPrep P{};
     if (valid) P = a.prep[(uint64_t)yy * J.g.nx + xx];
-    const PixHalf ph = pix_half(P);
+    const PixHalf ph = P.h;
     const int r0 = T.r0[tile];
     const uint32_t nrows = J.nrows;
     // kernel-parameter scalars held in registers for the slot loop
@@ -933,8 +933,7 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
             }
             const uint32_t b = kk % kTcGeoBufs;
             cp_async16(&S.g_half[b][bt], a.half + idx, true);
-            cp_async16(reinterpret_cast<uint8_t *>(&S.g_half[b][bt]) + 16,
-                       reinterpret_cast<const uint8_t *>(a.half + idx) + 16, true);
+            cp_async16(reinterpret_cast<uint8_t *>(&S.g_half[b][bt]) + 16, a.half + a.n + idx, true);
             cp_async8(&S.g_cb[b][bt], a.cb2 + idx);
             cp_async8(&S.g_w[b][bt], a.w + idx);
         }
@@ -988,7 +987,7 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
                     }
                 } else if (P.nr > 0 && kr >= P.ur && kr < P.ur + P.nr) {
                     uint32_t lo, hi, rl;
-                    if (ring_window_mc(a, a.rings[kr], P, lo, hi, rl)) {
+                    if (ring_window_general(a, P, kr, lo, hi, rl)) {
                         wlo = lo;
                         whi = hi;
                     }
@@ -997,8 +996,8 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
             // The piece's pair tests in two halves of 4 slots as straight-line
             // code (independent FP64 chains the scheduler can interleave):
             // haversines, then the weights of the pairs below the threshold
-            // band, the same arithmetic as pair_weight_s; pairs inside the band
-            // take pair_weight_s itself.
+            // band, the same arithmetic as pair_weights; pairs inside the band
+            // take pair_band.
             uint32_t hv[4], lv[4];
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
@@ -1019,7 +1018,7 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const double h = hh[e];
-                    // the Gaussian of an accepted pair, as pair_weight_s evaluates it
+                    // the Gaussian of an accepted pair, as pair_weights evaluates it
                     float ex;
                     if (series) {
                         ex = gauss_series_f32(h, x2scale);
@@ -1041,10 +1040,8 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         if (!(inw[e] && hh[e] >= hlo && hh[e] <= hhi)) continue;
-                        const uint32_t q = s8 * 8 + half * 4 + e;
                         const double wt =
-                            pair_weight_s<true, false>(a, P, ph, S.g_half[b][q], S.g_cb[b][q], S.g_w[b][q],
-                                                       culo + (slot0 + half * 4 + e - cbase));
+                            pair_band<true, false>(a, a.prep + (uint64_t)yy * J.g.nx + xx, culo + (slot0 + half * 4 + e - cbase));
                         if (wt != 0.0) {
                             wsum += wt;
                             ++within;
