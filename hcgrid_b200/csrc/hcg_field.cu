@@ -587,20 +587,41 @@ __global__ void __launch_bounds__(256) k_sample_geometry(
     if (lane == 0 && wb) atomicMax(wbits, wb);
 }
 
-// out[j][0..cstride) = in[perm[j]][0..nchan), zero padded; one warp per row.
-__global__ void k_permute_rows(uint64_t n, uint32_t nchan, uint32_t cstride, const uint32_t *__restrict__ perm,
-                               const float *__restrict__ in, float *__restrict__ out) {
-    uint64_t j = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (j >= n) return;
-    const float *src = in + (uint64_t)perm[j] * nchan;
-    float *dst = out + j * cstride;
-    if ((nchan & 3) == 0 && ((uintptr_t)in & 15) == 0) {
-        for (uint32_t c = lane * 4; c < nchan; c += 128)
+// One row of nchan values to a row of cstride (a multiple of 4, zero padded),
+// by the `tpr` threads that share it (a power of two up to 32; `t` is the
+// thread's place): 16 bytes a thread and step.
+__device__ __forceinline__ void copy_row(const float *__restrict__ src, float *__restrict__ dst, uint32_t nchan,
+                                         uint32_t cstride, uint32_t t, uint32_t tpr) {
+    if ((nchan & 3) == 0 && ((uintptr_t)src & 15) == 0) {
+        for (uint32_t c = t * 4; c < nchan; c += tpr * 4)
             *reinterpret_cast<float4 *>(dst + c) = __ldg(reinterpret_cast<const float4 *>(src + c));
     } else {
-        for (uint32_t c = lane; c < cstride; c += 32) dst[c] = c < nchan ? src[c] : 0.f;
+        for (uint32_t c = t * 4; c < cstride; c += tpr * 4) {
+            float4 v;
+            v.x = __ldg(src + c);
+            v.y = c + 1 < nchan ? __ldg(src + c + 1) : 0.f;
+            v.z = c + 2 < nchan ? __ldg(src + c + 2) : 0.f;
+            v.w = c + 3 < nchan ? __ldg(src + c + 3) : 0.f;
+            *reinterpret_cast<float4 *>(dst + c) = v;
+        }
     }
+}
+// threads that share a row: one per 16 bytes, so that short rows (a single
+// channel above all: 470 us for 4,000,000 with a warp each) do not leave most
+// of a warp idle
+inline uint32_t row_threads(uint32_t cstride) {
+    uint32_t t = 1;
+    while (t < 32 && 4 * t < cstride) t *= 2;
+    return t;
+}
+
+// out[j][0..cstride) = in[perm[j]][0..nchan), zero padded.
+__global__ void __launch_bounds__(256) k_permute_rows(uint64_t n, uint32_t nchan, uint32_t cstride, uint32_t tpr,
+                                                      const uint32_t *__restrict__ perm, const float *__restrict__ in,
+                                                      float *__restrict__ out) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, j = i / tpr;
+    if (j >= n) return;
+    copy_row(in + (uint64_t)__ldg(perm + j) * nchan, out + j * cstride, nchan, cstride, (uint32_t)(i % tpr), tpr);
 }
 
 // out[j][c] = in[c][perm[j]]: 32x32 tiles through shared memory.
@@ -624,21 +645,13 @@ __global__ void k_permute_cols(uint64_t n, uint32_t nchan, uint32_t cstride, con
 }
 
 // One uploaded chunk of sample-major spectra (input rows [r0, r0 + rows))
-// scattered to its sorted rows: one warp per row, zero padding to cstride.
-__global__ void k_scatter_rows(uint64_t r0, uint64_t rows, uint32_t nchan, uint32_t cstride,
-                               const uint32_t *__restrict__ inv, const float *__restrict__ in,
-                               float *__restrict__ out) {
-    const uint64_t r = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+// scattered to its sorted rows, zero padding to cstride.
+__global__ void __launch_bounds__(256) k_scatter_rows(uint64_t r0, uint64_t rows, uint32_t nchan, uint32_t cstride,
+                                                      uint32_t tpr, const uint32_t *__restrict__ inv,
+                                                      const float *__restrict__ in, float *__restrict__ out) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, r = i / tpr;
     if (r >= rows) return;
-    const float *src = in + r * nchan;
-    float *dst = out + (uint64_t)__ldg(inv + r0 + r) * cstride;
-    if ((nchan & 3) == 0 && ((uintptr_t)in & 15) == 0) {
-        for (uint32_t c = lane * 4; c < nchan; c += 128)
-            *reinterpret_cast<float4 *>(dst + c) = __ldg(reinterpret_cast<const float4 *>(src + c));
-    } else {
-        for (uint32_t c = lane; c < cstride; c += 32) dst[c] = c < nchan ? src[c] : 0.f;
-    }
+    copy_row(in + r * nchan, out + (uint64_t)__ldg(inv + r0 + r) * cstride, nchan, cstride, (uint32_t)(i % tpr), tpr);
 }
 
 // One uploaded chunk of channel-major spectra (planes [c0, c1) of n samples)
@@ -835,9 +848,9 @@ cudaError_t upload_spectra(hcg_context *ctx, hcg_field *f, const float *h_in, ui
         if ((e = cudaEventRecord(ctx->evu[b], cs)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(s, ctx->evu[b], 0)) != cudaSuccess) return e;
         if (layout == HCG_LAYOUT_SAMPLE_MAJOR) {
-            const uint64_t threads = cnt * 32;
-            k_scatter_rows<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(u0, cnt, nchan, cstride, f->d_inv,
-                                                                             stage[b], f->d_spec);
+            const uint32_t tpr = row_threads(cstride);
+            k_scatter_rows<<<(unsigned)((cnt * tpr + 255) / 256), 256, 0, s>>>(u0, cnt, nchan, cstride, tpr, f->d_inv,
+                                                                               stage[b], f->d_spec);
         } else {
             const uint32_t c0 = (uint32_t)u0, c1 = (uint32_t)(u0 + cnt);
             const uint32_t cend = c1 == nchan ? cstride : c1;  // the last chunk writes the padding
@@ -901,9 +914,9 @@ cudaError_t permute_spectra(hcg_context *ctx, hcg_field *f, const float *d_in, u
     f->nchan = nchan;
     f->cstride = cstride;
     if (layout == HCG_LAYOUT_SAMPLE_MAJOR) {
-        uint64_t threads = f->n * 32;
-        k_permute_rows<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(f->n, nchan, cstride, f->d_perm, d_in,
-                                                                         f->d_spec);
+        const uint32_t tpr = row_threads(cstride);
+        k_permute_rows<<<(unsigned)((f->n * tpr + 255) / 256), 256, 0, s>>>(f->n, nchan, cstride, tpr, f->d_perm, d_in,
+                                                                            f->d_spec);
     } else {
         dim3 grid((unsigned)((f->n + 31) / 32), (cstride + 31) / 32);
         k_permute_cols<<<grid, dim3(32, 8), 0, s>>>(f->n, nchan, cstride, f->d_perm, d_in, f->d_spec);
