@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) kb_job_entries(const BatchHdr *__restrict
         jent[j] = H->off_all[jobs[j].grp_base + jobs[j].g.ngroups] - H->off_all[jobs[j].grp_base];
 }
 
-__global__ void __launch_bounds__(kBatchTileThreads) kb_accum(BatchHdr *H, const JobDesc *__restrict__ jobs,
+__global__ void __launch_bounds__(kTileThreads) kb_accum(BatchHdr *H, const JobDesc *__restrict__ jobs,
                                                              unsigned long long *timeouts) {
     if (H->pool_overflow) return;  // entries incomplete: this pass is replayed after the pool grows
     for (;;) {
@@ -204,10 +204,9 @@ __global__ void __launch_bounds__(kBatchTileThreads) kb_accum(BatchHdr *H, const
         if (J.skip) continue;
         unsigned long long local = it - J.acc_base;
         uint64_t tile = local / J.nslices;
-        uint32_t c0 = (uint32_t)(local % J.nslices) * kBatchSlice;
-        tile_accum_item<kBatchAccumBufs, kBatchAccumRows, kBatchAccumCpt, kBatchSlice>(
-            J.g, J.T, J.off, J.cnt, H->e_idx, H->e_w, J.wsum, J.spec, J.nchan, J.cstride, J.out, J.ostride, J.wout,
-            tile, c0, timeouts);
+        uint32_t c0 = (uint32_t)(local % J.nslices) * kAccumSlice;
+        tile_accum_item(J.g, J.T, J.off, J.cnt, H->e_idx, H->e_w, J.wsum, J.spec, J.nchan, J.cstride, J.out, J.ostride,
+                        J.wout, tile, c0, timeouts);
     }
 }
 
@@ -335,7 +334,7 @@ static cudaError_t grow(BatchState &B, int slot, size_t bytes, cudaStream_t s, v
 
 static cudaError_t capture(hcg_context *ctx, BatchState &B) {
     cudaStream_t s = ctx->stream;
-    const int smem = kBatchAccumBufs * kBatchAccumRows * kBatchSlice * (int)sizeof(float);
+    const int smem = kAccumSmem;
     cudaError_t e = cudaFuncSetAttribute(kb_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     if ((e = tc_set_smem((const void *)kb_tc<0>, KbShape<0>::Cfg::kSmem)) != cudaSuccess ||
@@ -359,7 +358,7 @@ static cudaError_t capture(hcg_context *ctx, BatchState &B) {
             kb_job_entries<<<1, 256, 0, s>>>(B.d_hdr, B.d_jobs, B.d_jent);
         } else {
             kb_group<<<n * 4, kWeightThreads, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
-            kb_accum<<<n, kBatchTileThreads, smem, s>>>(B.d_hdr, B.d_jobs, &ctx->d_stats->timeouts);
+            kb_accum<<<n, kTileThreads, smem, s>>>(B.d_hdr, B.d_jobs, &ctx->d_stats->timeouts);
             unsigned long long *to = &ctx->d_stats->timeouts, *macs = &ctx->d_stats->tc_macs;
             kb_tc<0><<<n, kTcThreads, KbShape<0>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_tc<1><<<n, kTcThreads, KbShape<1>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
@@ -479,7 +478,7 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
         d.T.nty = (t->ny + kTileY - 1) / kTileY;
         uint64_t ntiles = (f->nchan > 1) ? (uint64_t)d.T.ntx * d.T.nty : 0;
         const bool tc = batch_uses_tc(f);
-        d.nslices = tc ? 0 : (f->cstride + kBatchSlice - 1) / kBatchSlice;
+        d.nslices = tc ? 0 : (f->cstride + kAccumSlice - 1) / kAccumSlice;
         if (tc) {
             d.T.pad = 8;  // ring runs as boxes of 8 samples
             d.tc_shape = (uint32_t)kb_shape_of(ctx, f);

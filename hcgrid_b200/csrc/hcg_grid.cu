@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(32 * W, W == 4 ? kRingCtas : 2) k_tile_rings(G
     tile_rings_item<W>(a, g, T, T.t0 + blockIdx.x);
 }
 
-__global__ void __launch_bounds__(kTileThreads, kAccumCtas) k_tile_accum(GroupArgs g, TileArgs T,
+__global__ void __launch_bounds__(kTileThreads, 1) k_tile_accum(GroupArgs g, TileArgs T,
                                                             const unsigned long long *__restrict__ off,
                                                             const uint32_t *__restrict__ cnt,
                                                             const uint32_t *__restrict__ e_slot,
@@ -113,9 +113,8 @@ __global__ void __launch_bounds__(kTileThreads, kAccumCtas) k_tile_accum(GroupAr
                                                             unsigned long long *timeouts) {
     // slices of a tile are adjacent blocks: they run together and share the
     // tile's entries through L2
-    tile_accum_item<kAccumBufs, kAccumRows, kAccumCpt, kAccumSlice>(g, T, off, cnt, e_slot, e_w, wsum, spec, nchan,
-                                                                    cstride, out, ostride, wout, T.t0 + blockIdx.y,
-                                                                    blockIdx.x * kAccumSlice, timeouts);
+    tile_accum_item(g, T, off, cnt, e_slot, e_w, wsum, spec, nchan, cstride, out, ostride, wout, T.t0 + blockIdx.y,
+                    blockIdx.x * kAccumSlice, timeouts);
 }
 
 // Exclusive scan of n uint32 counts into uint64 offsets (out[n] = total),
@@ -316,7 +315,7 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
             return e;
         }
         float *dst = d_cube;
-        const int smem = kAccumBufs * kAccumRows * kAccumSlice * (int)sizeof(float);
+        const int smem = kAccumSmem;
         static bool attr_set = false;
         if (tiled && !attr_set) {
             if ((e = cudaFuncSetAttribute(k_tile_accum, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) !=

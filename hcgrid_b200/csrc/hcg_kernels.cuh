@@ -1420,25 +1420,22 @@ __device__ __forceinline__ void tile_rings_item(const GridArgs &a, const GroupAr
     }
 }
 
-// Channel sums of one tile for one slice of SL channels: the tile's union
-// of candidate spectra (slots) is staged in shared memory chunk by chunk;
-// SL / CPT threads per 2x2 group each own CPT channels of the slice, so a
-// staged value is used for 4 pixels. A CTA has one thread per (group,
-// channel part): tile_threads(CPT, SL).
-constexpr int tile_threads(int cpt, int sl) { return (kTileX / 2) * (kTileY / 2) * (sl / cpt); }
-// FP32 staging rings (buffers x rows of a slice), channels per thread and
-// slice width, the same for k_tile_accum and the batch engine's kb_accum:
-// 16 threads per 2x2 group, 8 channels each, over 128 channels (one
-// 512-thread CTA per SM), so a group's entries are loaded once per 128
-// channels; the ring is three 144-row buffers (216 KB): long chunks leave
-// the warps a chunk of slack between barrier waits (measured on 4M x 1,024
-// -> 1200^2: 96-row chunks x 4 buffers 34.3 ms, 128 x 3 31.8 ms, 144 x 3
-// 30.5 ms).
-constexpr int kAccumBufs = 3, kAccumRows = 144, kAccumCpt = 8, kAccumSlice = 128, kAccumCtas = 1;
-constexpr int kBatchAccumBufs = kAccumBufs, kBatchAccumRows = kAccumRows, kBatchAccumCpt = kAccumCpt,
-              kBatchSlice = kAccumSlice;
-constexpr int kTileThreads = tile_threads(kAccumCpt, kAccumSlice);
-constexpr int kBatchTileThreads = tile_threads(kBatchAccumCpt, kBatchSlice);
+// Shared-memory reads by 32-bit address.
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint4 lds4u(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds1(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
 
 // 16-byte asynchronous global -> shared copy (zero-filled when !valid).
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid) {
@@ -1465,21 +1462,39 @@ constexpr uint64_t kTileWaitNs = 1000000000ull;  // bound of the FP32 staging ri
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Channel sums of one tile for one slice of SL channels. The tile's
-// union of candidate spectra (its slots) is staged in shared memory in
-// chunks of CH rows through a ring of NB buffers: every thread copies its
-// share of a chunk with cp.async and arrives on the chunk's `full` barrier
-// when its copies land; each warp arrives on the buffer's `empty` barrier
-// when it has summed the chunk, and the chunk NB - 2 ahead is staged into a
-// buffer only once every warp is done with that buffer's previous chunk. So a
-// warp whose groups have many entries in one chunk holds the others back only
-// two chunks later, not at every chunk. SL / CPT threads per 2x2 group
-// each own CPT channels of the slice (float4 q, q + SL / CPT, ... of a
-// row, so the group's loads of one row are contiguous), and a staged value
-// feeds 4 pixels. Block-collective (every thread of a tile_threads(CPT, SL)
-// block; NB * CH * SL floats of dynamic shared memory). A barrier wait
-// that runs out (1 s) is counted in `timeouts` and the item winds down.
-template <int NB, int CH, int CPT, int SL>
+// Channel sums of one tile for one slice of kAccumSlice channels. The tile's
+// union of candidate spectra (its slots) is staged in shared memory in chunks
+// of kAccumRows rows through a ring of kAccumBufs buffers: every thread copies
+// its share of a chunk with cp.async and arrives on the chunk's `full` barrier
+// when its copies land; each warp arrives on the buffer's `empty` barrier when
+// it has summed the chunk, and the chunk kAccumBufs - 2 ahead is staged into a
+// buffer only once every warp is done with that buffer's previous chunk.
+//
+// A warp sums two 2x2 groups, one after the other within a chunk, a lane owning
+// four channels: an entry is the same for the whole warp, so nothing diverges.
+// A chunk is a band of declination, and a group has entries in about half of
+// the chunks; its warp's second group lies two group rows below the first, so
+// that most warps have work in most chunks (a warp with two groups of one row
+// waited through the other half). Each group's entries come in batches of 32,
+// one a lane: the next batch is loaded into registers while the present one is
+// summed from shared memory. Channel planes leave through a shared-memory
+// transpose, as 64-byte runs (stores from the sums' layout write 4 bytes of
+// every 32-byte sector). What bounds it: issue and shared-memory latency at 16
+// warps an SM; an entry is six shared-memory wavefronts for 128 channels (four of
+// spectra, two of entry) and 26 instructions, 16 of them multiply-adds. Packed
+// FP32 pairs (fma.rn.f32x2) gained nothing: they take one of the two FMA pipes.
+// 1M samples x 512 channels, 600 x 600 pixels: 3.09 ms (3.70 ms with half a warp
+// a group, each thread reading every entry from L2).
+//
+// Block-collective (kTileThreads; kAccumBufs * kAccumRows * kAccumSlice floats
+// of dynamic shared memory). A barrier wait that runs out (1 s) is counted in
+// `timeouts` and the item winds down.
+constexpr int kAccumBufs = 3, kAccumRows = 128, kAccumSlice = 128, kAccumWarps = 16;
+constexpr int kTileThreads = 32 * kAccumWarps;
+constexpr int kAccumSmem = kAccumBufs * kAccumRows * kAccumSlice * (int)sizeof(float);
+constexpr int kAccumPitch = kTileX * kTileY + 1;  // the transpose's rows (channels) of pixels
+static_assert(kTileGroups == 2 * kAccumWarps && kAccumSlice == 128, "two groups a warp, four channels a lane");
+static_assert(kAccumSlice * kAccumPitch * (int)sizeof(float) <= kAccumSmem, "the transpose fits the staging ring");
 __device__ __forceinline__ void tile_accum_item(const GroupArgs &g, const TileArgs &T,
                                                 const unsigned long long *__restrict__ off,
                                                 const uint32_t *__restrict__ cnt,
@@ -1489,52 +1504,85 @@ __device__ __forceinline__ void tile_accum_item(const GroupArgs &g, const TileAr
                                                 float *__restrict__ out, uint32_t ostride,
                                                 float *__restrict__ wout, uint64_t tile, uint32_t c0,
                                                 unsigned long long *timeouts) {
+    constexpr int NB = kAccumBufs, CH = kAccumRows;
     static_assert(NB >= 3, "the chunk NB - 2 ahead is staged while one is summed");
-    static_assert(CPT % 4 == 0 && SL % CPT == 0, "whole float4 channel quads per thread");
-    constexpr int kThreads = tile_threads(CPT, SL), kWarps = kThreads / 32, kTpg = SL / CPT, kQ = CPT / 4;
-    extern __shared__ float4 s_spec[];  // [NB][CH][SL / 4]
+    extern __shared__ float4 s_spec[];  // [NB][CH][kAccumSlice / 4]
     __shared__ uint32_t s_ulo[kTileMaxRings], s_base[kTileMaxRings + 1];
+    __shared__ float4 s_ew[kTileGroups][32];    // the groups' current batches of entries: weights
+    __shared__ __align__(16) uint32_t s_er[kTileGroups][32];  // and slot * row bytes (mod 2^32)
     __shared__ uint64_t s_full[NB], s_empty[NB];
     __shared__ volatile int s_abort;
     __syncthreads();  // shared state of a previous item is no longer read
-    const int tid = threadIdx.x, q = tid % kTpg, gl = tid / kTpg;
+    const int tid = threadIdx.x;
+    const uint32_t lane = tid & 31, warp = tid >> 5;
     const int nrt = T.nr[tile];
     const uint32_t U = T.U[tile];
-    for (int j = tid; j < nrt; j += kThreads) s_ulo[j] = T.ulo[tile * kTileMaxRings + j];
-    for (int j = tid; j <= nrt; j += kThreads) s_base[j] = T.base[tile * (kTileMaxRings + 1) + j];
+    for (int j = tid; j < nrt; j += kTileThreads) s_ulo[j] = T.ulo[tile * kTileMaxRings + j];
+    for (int j = tid; j <= nrt; j += kTileThreads) s_base[j] = T.base[tile * (kTileMaxRings + 1) + j];
     if (tid == 0) {
         for (int b = 0; b < NB; ++b) {
-            sm100::mbar_init(&s_full[b], kThreads);
-            sm100::mbar_init(&s_empty[b], kWarps);
+            sm100::mbar_init(&s_full[b], kTileThreads);
+            sm100::mbar_init(&s_empty[b], kAccumWarps);
         }
         s_abort = 0;
         sm100::mbar_fence_init();
     }
-    const uint32_t gxi = (uint32_t)(tile % T.ntx) * (kTileX / 2) + gl % (kTileX / 2);
-    const uint32_t gyi = (uint32_t)(tile / T.ntx) * (kTileY / 2) + gl / (kTileX / 2);
-    const bool gvalid = gxi < g.gx && (uint64_t)gyi * g.gx + gxi < g.ngroups;
-    const uint64_t grp = (uint64_t)gyi * g.gx + gxi;
-    uint64_t e = 0, e_end = 0;
-    if (gvalid) {
-        e = off[grp] - g.ebase;
-        e_end = e + cnt[grp];
+    // the warp's groups: rows (0, 2) or (1, 3) of the tile's four group rows
+    const uint32_t gxl = warp & 7, gyl = warp >> 3;
+    const uint32_t gxi = (uint32_t)(tile % T.ntx) * (kTileX / 2) + gxl;
+    const uint32_t gy0 = (uint32_t)(tile / T.ntx) * (kTileY / 2) + gyl;
+    constexpr uint32_t kRowBytes = kAccumSlice * 4;
+    struct Batch {
+        uint64_t e, end;   // next entry to load
+        float4 w;          // the next batch's entry of this lane
+        uint32_t next;     // and its slot (0xffffffff: none)
+        uint32_t slot;     // the present batch's slot of this lane
+        uint32_t pos;      // entries of it summed
+    } B[2];
+    auto load_batch = [&](Batch &b) {
+        const bool in = b.e + lane < b.end;
+        b.next = in ? __ldg(e_slot + b.e + lane) : 0xffffffffu;
+        if (in) b.w = __ldg(e_w + b.e + lane);
+        b.e += 32;
+    };
+    auto next_batch = [&](Batch &b, uint32_t gl) {  // false: the group's entries are all summed
+        b.slot = b.next;
+        b.pos = 0;
+        if (__shfl_sync(0xffffffffu, b.next, 0) == 0xffffffffu) return false;
+        __syncwarp();  // the previous batch is no longer read
+        s_ew[gl][lane] = b.w;
+        s_er[gl][lane] = b.next * kRowBytes;
+        load_batch(b);
+        __syncwarp();
+        return true;
+    };
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint64_t grp = (uint64_t)(gy0 + 2 * i) * g.gx + gxi;
+        const bool in = gxi < g.gx && grp < g.ngroups;
+        B[i].e = in ? off[grp] - g.ebase : 0;
+        B[i].end = in ? B[i].e + cnt[grp] : 0;
+        B[i].w = make_float4(0.f, 0.f, 0.f, 0.f);
+        load_batch(B[i]);
     }
-    float4 acc[4][kQ];  // [pixel of the group][channel quad of the thread]
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
+    for (int i = 0; i < 2; ++i) next_batch(B[i], 2 * warp + i);
+    float4 acc[2][4];  // [group][pixel of the group]
 #pragma unroll
-        for (int j = 0; j < kQ; ++j) acc[k][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[i][k] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncthreads();
     // stage rows [cs, min(U, cs + CH)) into buffer b: each warp takes kRows
     // consecutive rows, its lane r finds row r's sample (the ring j with
     // base[j] <= slot < base[j+1]) once, and the warp's 16-byte copies take
     // their row's sample from that lane; the thread's arrival on full[b]
     // completes when its copies have landed
-    constexpr uint32_t kRows = (CH + kWarps - 1) / kWarps, kParts = SL / 4;
-    static_assert(kRows <= 32 && 32 % kParts == 0, "one lane per staged row of a warp, whole rows per pass");
-    const uint32_t lane = tid & 31, warp = tid >> 5;
-    const uint32_t pc = c0 + 4 * (lane % kParts);  // the channels of this lane's copies (32 % kParts == 0)
+    constexpr uint32_t kRows = CH / kAccumWarps, kParts = kAccumSlice / 4;
+    static_assert(CH % kAccumWarps == 0 && kRows <= 32 && kParts == 32, "a row per copy of a warp");
+    const uint32_t pc = c0 + 4 * lane;  // this lane's channels
     const bool pok = pc < cstride;
+    const float *src0 = spec + (pok ? pc : 0);
     auto stage = [&](uint32_t cs, int b) {
         const uint32_t ce = min(U, cs + CH), r0 = cs + warp * kRows;
         const uint32_t nr = r0 < ce ? min(kRows, ce - r0) : 0;
@@ -1548,12 +1596,10 @@ __device__ __forceinline__ void tile_accum_item(const GroupArgs &g, const TileAr
             }
             idx = s_ulo[lo] + (slot - s_base[lo]);
         }
-        float4 *dst = s_spec + ((size_t)b * CH + (r0 - cs)) * kParts + lane % kParts;
-        const float *src0 = spec + (pok ? pc : 0);
-        for (uint32_t i0 = 0; i0 < nr * kParts; i0 += 32) {  // warp-uniform trip count
-            const uint32_t row = (i0 + lane) / kParts;
-            const uint32_t ri = __shfl_sync(0xffffffffu, idx, row & 31);
-            if (i0 + lane < nr * kParts) cp_async16(dst + row * kParts, src0 + (uint64_t)ri * cstride, pok);
+        float4 *dst = s_spec + ((size_t)b * CH + (r0 - cs)) * kParts + lane;
+        for (uint32_t r = 0; r < nr; ++r) {
+            const uint32_t ri = __shfl_sync(0xffffffffu, idx, r);
+            cp_async16(dst + r * kParts, src0 + (uint64_t)ri * cstride, pok);
         }
         cp_async_arrive(&s_full[b]);
     };
@@ -1577,85 +1623,93 @@ __device__ __forceinline__ void tile_accum_item(const GroupArgs &g, const TileAr
             atomicAdd(timeouts, 1ULL);
             s_abort = 1;
         }
-        if (s_abort) break;
-        const float4 *buf = s_spec + (size_t)b * CH * (SL / 4) + q;
-        auto fma_entry = [&](uint32_t sl, const float4 &w) {
-            const float wv[4] = {w.x, w.y, w.z, w.w};
+        if (__any_sync(0xffffffffu, s_abort)) break;
+        // shared address of this lane's channels of slot 0 (mod 2^32)
+        const uint32_t at0 = sm100::smem_u32(s_spec + (size_t)b * CH * kParts + lane) - cs * kRowBytes;
 #pragma unroll
-            for (int j = 0; j < kQ; ++j) {
-                const float4 sv = buf[(sl - cs) * (SL / 4) + j * kTpg];
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t gl = 2 * warp + i;
+            Batch &t = B[i];
+            const uint32_t ew = sm100::smem_u32(&s_ew[gl][0]), er = sm100::smem_u32(&s_er[gl][0]);
+            auto fma_entry = [&](const float4 &w, const float4 &x) {
+                const float wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
-                    acc[kk][j].x = fmaf(wv[kk], sv.x, acc[kk][j].x);
-                    acc[kk][j].y = fmaf(wv[kk], sv.y, acc[kk][j].y);
-                    acc[kk][j].z = fmaf(wv[kk], sv.z, acc[kk][j].z);
-                    acc[kk][j].w = fmaf(wv[kk], sv.w, acc[kk][j].w);
+                    acc[i][kk].x = fmaf(wv[kk], x.x, acc[i][kk].x);
+                    acc[i][kk].y = fmaf(wv[kk], x.y, acc[i][kk].y);
+                    acc[i][kk].z = fmaf(wv[kk], x.z, acc[i][kk].z);
+                    acc[i][kk].w = fmaf(wv[kk], x.w, acc[i][kk].w);
                 }
+            };
+            for (;;) {
+                // entries [pos, lim) of the batch belong to this chunk: slots rise
+                // along a group's entries, so they are the lanes below its end
+                const uint32_t lim = __popc(__ballot_sync(0xffffffffu, t.slot < ce));
+                uint32_t pos = t.pos;
+                for (; pos < lim && (pos & 3); ++pos) fma_entry(lds4(ew + 16 * pos), lds4(at0 + lds1(er + 4 * pos)));
+                for (; pos + 4 <= lim; pos += 4) {  // four rows' offsets in one read
+                    const uint4 r = lds4u(er + 4 * pos);
+                    const float4 x0 = lds4(at0 + r.x), x1 = lds4(at0 + r.y), x2 = lds4(at0 + r.z), x3 = lds4(at0 + r.w);
+                    fma_entry(lds4(ew + 16 * pos), x0);
+                    fma_entry(lds4(ew + 16 * pos + 16), x1);
+                    fma_entry(lds4(ew + 16 * pos + 32), x2);
+                    fma_entry(lds4(ew + 16 * pos + 48), x3);
+                }
+                for (; pos < lim; ++pos) fma_entry(lds4(ew + 16 * pos), lds4(at0 + lds1(er + 4 * pos)));
+                t.pos = pos;
+                if (lim < 32 || !next_batch(t, gl)) break;
             }
-        };
-        // entries kSet at a time from two register sets in turn: the next set
-        // is loaded while one is summed, and no set is copied
-        // (one lane of the group also asks L1 for the entries kPrefetch ahead,
-        // which the registers cannot hold: measured 29.1 against 30.5 ms of
-        // channel sums on 4M x 1,024 -> 1200^2)
-        constexpr int kSet = 3, kPrefetch = 24;
-        auto load = [&](uint32_t *sl, float4 *w, uint64_t at) {
-#pragma unroll
-            for (int u = 0; u < kSet; ++u) {
-                sl[u] = __ldg(e_slot + at + u);
-                w[u] = __ldg(e_w + at + u);
-            }
-            if (q == 0) {  // the group's last entry at most
-                const uint64_t pa = min(at + kPrefetch, e_end - 1);
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(e_w + pa));
-                asm volatile("prefetch.global.L1 [%0];" ::"l"(e_slot + pa));
-            }
-        };
-        auto sum = [&](const uint32_t *sl, const float4 *w) {
-#pragma unroll
-            for (int u = 0; u < kSet; ++u) fma_entry(sl[u], w[u]);
-        };
-        if (e + kSet <= e_end) {
-            uint32_t sa[kSet], sb[kSet];
-            float4 wa[kSet], wb[kSet];
-            load(sa, wa, e);
-            for (;;) {  // sa holds entries [e, e + kSet)
-                const bool nb = e + 2 * kSet <= e_end;
-                if (nb) load(sb, wb, e + kSet);
-                if (sa[kSet - 1] >= ce) break;
-                sum(sa, wa);
-                e += kSet;
-                if (!nb) break;
-                const bool na = e + 2 * kSet <= e_end;  // sb holds entries [e, e + kSet)
-                if (na) load(sa, wa, e + kSet);
-                if (sb[kSet - 1] >= ce) break;
-                sum(sb, wb);
-                e += kSet;
-                if (!na) break;
-            }
-        }
-        for (; e < e_end; ++e) {
-            uint32_t sl = __ldg(e_slot + e);
-            if (sl >= ce) break;
-            fma_entry(sl, __ldg(e_w + e));
         }
         __syncwarp();
-        if ((tid & 31) == 0) sm100::mbar_arrive(&s_empty[b]);  // this warp is done with buffer b
+        if (lane == 0) sm100::mbar_arrive(&s_empty[b]);  // this warp is done with buffer b
     }
     cp_async_wait_all();  // no copy into the ring outlives the item
-    if (!gvalid) return;
+    const uint64_t npix = (uint64_t)g.nx * g.ny;
+    float *s_t = reinterpret_cast<float *>(s_spec);  // [channel (4 * lane + j at j * 32 + lane)][pixel of the tile]
+    // lane 4 i + k has pixel k of group i: weight sum and reciprocal
+    float inv_l = 0.f;
+    {
+        const uint32_t i = (lane >> 2) & 1, k = lane & 3;
+        const uint32_t xx = 2 * gxi + (k & 1), yy = 2 * (gy0 + 2 * i) + (k >> 1);
+        if (lane < 8 && xx < g.nx && yy < g.ny) {
+            const uint64_t p = (uint64_t)yy * g.nx + xx;
+            const double ws = wsum[p];
+            inv_l = (float)(1.0 / ws);
+            if (wout && c0 == 0) wout[p] = (float)ws;
+        }
+    }
+    if (!ostride) __syncthreads();                   // every warp is done with the ring
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        uint32_t xx = 2 * gxi + (k & 1), yy = 2 * gyi + (k >> 1);
-        if (xx >= g.nx || yy >= g.ny) continue;
-        uint64_t p = (uint64_t)yy * g.nx + xx;
-        double ws = wsum[p];
-        float inv = (float)(1.0 / ws);
-        if (wout && c0 == 0 && q == 0) wout[p] = (float)ws;
+    for (int i = 0; i < 2; ++i) {
 #pragma unroll
-        for (int j = 0; j < kQ; ++j) {
-            const float v[4] = {acc[k][j].x * inv, acc[k][j].y * inv, acc[k][j].z * inv, acc[k][j].w * inv};
-            store_cube4(out, ostride, (uint64_t)g.nx * g.ny, p, c0 + 4 * (q + j * kTpg), nchan, v);
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t xx = 2 * gxi + (k & 1), yy = 2 * (gy0 + 2 * i) + (k >> 1);
+            if (xx >= g.nx || yy >= g.ny) continue;
+            const uint64_t p = (uint64_t)yy * g.nx + xx;
+            const float inv = __shfl_sync(0xffffffffu, inv_l, 4 * i + k);  // the branch is the warp's
+            const float4 A = acc[i][k];
+            const float v[4] = {A.x * inv, A.y * inv, A.z * inv, A.w * inv};
+            if (ostride) {
+                store_cube4(out, ostride, npix, p, pc, nchan, v);
+            } else {
+                const uint32_t tp = (2 * (gyl + 2 * i) + (k >> 1)) * kTileX + 2 * gxl + (k & 1);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s_t[(j * 32 + lane) * kAccumPitch + tp] = v[j];
+            }
+        }
+    }
+    if (!ostride) {
+        __syncthreads();
+        const uint32_t tx0 = (uint32_t)(tile % T.ntx) * kTileX, ty0 = (uint32_t)(tile / T.ntx) * kTileY;
+        const uint32_t xx = tx0 + lane % kTileX;
+        for (uint32_t c = warp; c < kAccumSlice && c0 + c < nchan; c += kAccumWarps) {
+            const float *row = s_t + ((c & 3) * 32 + (c >> 2)) * kAccumPitch;
+            float *plane = out + (uint64_t)(c0 + c) * npix;
+#pragma unroll
+            for (uint32_t h = 0; h < kTileY / 2; ++h) {
+                const uint32_t yy = ty0 + 2 * h + lane / kTileX;
+                if (xx < g.nx && yy < g.ny) plane[(uint64_t)yy * g.nx + xx] = row[h * 32 + lane];
+            }
         }
     }
 }
