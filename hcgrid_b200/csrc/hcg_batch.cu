@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const uint64_t tile = local % ntiles;  // tiles fastest: neighbours share staged samples in L2
         tc_load_rings(S, J.T, tile);
         __syncthreads();
-        tc_item<KbTcCfg>(S, J, tile, (uint32_t)(local / ntiles), gk, itn, timeouts, macs);
+        tc_item<KbTcCfg>(S, J, J.map, J.out_map, tile, (uint32_t)(local / ntiles), gk, itn, timeouts, macs);
         ++itn;
         __syncthreads();  // every role is done with the item's ring table and accumulator
     }

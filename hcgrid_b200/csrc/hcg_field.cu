@@ -541,6 +541,9 @@ __global__ void __launch_bounds__(256) k_sample_geometry(
         wb = (unsigned long long)__double_as_longlong(fabs(wi));
         double2 q;
         sincos(l * 0.5, &q.x, &q.y);
+        const double rc = sqrt(fmax(cb, 0.0));
+        q.x *= rc;
+        q.y *= rc;
         half[j] = q;
         sincos(b * 0.5, &q.x, &q.y);
         half[n + j] = q;

@@ -74,7 +74,9 @@ constexpr uint64_t kRingTbl = kRingHalf - 1;
 constexpr uint64_t kQuickOrder = 26;
 static_assert(sizeof(RingWin) == 64, "four 16-byte loads");
 
-// Half-angle sines and cosines of a position (the pair test's operands).
+// The pair test's operands of a position: sine and cosine of half the
+// longitude, both times sqrt(cos(lat)), and of half the latitude. With the
+// factor in them the haversine of a pair is a sum of two squares.
 struct PixHalf {
     double sl, cl, sb, cb;
 };
@@ -169,7 +171,7 @@ struct hcg_field {
     double *d_b2 = nullptr;
     double *d_cb2 = nullptr;      // cos(b2)
     double *d_w = nullptr;        // per-sample input weight, sorted
-    double2 *d_half = nullptr;    // sorted: [n] sin(l/2), cos(l/2), then [n] sin(b/2), cos(b/2)
+    double2 *d_half = nullptr;    // sorted: [n] sin(l/2), cos(l/2) times sqrt(cos b), then [n] sin(b/2), cos(b/2)
     uint32_t *d_lut = nullptr;    // usedrings + 1
     uint32_t *d_ptab = nullptr;   // per-ring pixel tables (RingRec::tbl), or none when too large
     uint64_t ptab_entries = 0;

@@ -73,6 +73,9 @@ __device__ __forceinline__ void prep_item(HpxParams h, uint64_t firstring, uint6
     P.tt[0] = fmodulo(dmul(dsub(disc_phi, disc), kInvHalfPi), 4.0);
     P.tt[1] = fmodulo(dmul(dadd(disc_phi, disc), kInvHalfPi), 4.0);
     sincos(P.l1 * 0.5, &P.h.sl, &P.h.cl);
+    const double rc = sqrt(fmax(P.cb1, 0.0));
+    P.h.sl *= rc;
+    P.h.cl *= rc;
     sincos(P.b1 * 0.5, &P.h.sb, &P.h.cb);
     out[p] = P;
 }
@@ -179,7 +182,7 @@ struct GridArgs {
     const double *l2, *b2, *cb2, *w;
     double sphere_radius, p0;
     DevStats *stats;
-    const double2 *half;  // sorted samples: [n] sin(l/2), cos(l/2), then [n] sin(b/2), cos(b/2)
+    const double2 *half;  // sorted samples' pair operands (hcg_field::d_half)
     const uint32_t *ptab; // per-ring pixel tables (RingRec::tbl)
     double hlo, hhi;      // haversine thresholds bracketing sphere_radius (see grid_args)
     int series;           // d^2 from the arcsine-squared series (small sphere_radius)
@@ -475,19 +478,17 @@ __device__ __forceinline__ float gauss_series_f32(double h, float x2scale) {
     return r;
 }
 
-// Half-angle differences of a pair and its haversine: sin((b1 - b2) / 2),
-// sin((l1 - l2) / 2) and h = sin^2(db / 2) + cos b1 cos b2 sin^2(dl / 2),
-// expanded from the precomputed sines and cosines (`sl2` = sin, cos of l2 / 2;
-// `sb2` of b2 / 2).
+// Half-angle differences of a pair and its haversine: sb = sin((b1 - b2) / 2),
+// sl = sin((l1 - l2) / 2) sqrt(cos b1 cos b2) and h = sb^2 + sl^2, expanded from
+// the positions' operands (PixHalf; `sl2`, `sb2` are the sample's).
 struct PairHav {
     double sb, sl, h;
 };
-__device__ __forceinline__ PairHav pair_hav(const PixHalf &q, double cb1, const double2 &sl2, const double2 &sb2,
-                                            double cb2) {
+__device__ __forceinline__ PairHav pair_hav(const PixHalf &q, const double2 &sl2, const double2 &sb2) {
     PairHav v;
     v.sb = q.sb * sb2.y - q.cb * sb2.x;
     v.sl = q.sl * sl2.y - q.cl * sl2.x;
-    v.h = v.sb * v.sb + cb1 * cb2 * (v.sl * v.sl);
+    v.h = v.sb * v.sb + v.sl * v.sl;
     return v;
 }
 
@@ -510,18 +511,18 @@ __device__ __forceinline__ double pair_d2(const GridArgs &a, double h) {
 // |x| < 1e-10 (gridding.cu:229-235) and the taper exp(+(arg/a)^2) of the
 // reference, or exp(-(arg/a)^2) with HCG_TAPER_FIX. The bearing's tangent
 // y / x has y = cos b2 sin dl and x = cos b1 sin b2 - sin b1 cos b2 cos dl =
-// sin(b2 - b1) + 2 sin b1 cos b2 sin^2(dl / 2); both follow from the half-angle
-// products, and only sin^2 and cos^2 of (bearing - PA) are wanted, so neither
-// the arc tangent nor any sine or cosine is evaluated (the weight pass of
-// 150,001 samples on 251 x 203 pixels took 355 us with them).
-__device__ __forceinline__ double kernel_other(const GridArgs &a, const PixHalf &q, const PairHav &v,
-                                               const double2 &sl2, const double2 &sb2, double cb2, double d2) {
+// sin(b2 - b1) + 2 sin b1 cos b2 sin^2(dl / 2); both, times cos b1, follow from
+// the half-angle products, and only sin^2 and cos^2 of (bearing - PA) are
+// wanted, so neither the arc tangent nor any sine or cosine is evaluated (the
+// weight pass of 150,001 samples on 251 x 203 pixels took 355 us with them).
+__device__ __forceinline__ double kernel_other(const GridArgs &a, const PixHalf &q, double cb1, const PairHav &v,
+                                               const double2 &sl2, const double2 &sb2, double d2) {
     const double p0 = a.p0, p1 = a.kp1, p2 = a.kp2;
     if (a.ktype == HCG_GAUSS2D) {
-        const double cl = q.cl * sl2.y + q.sl * sl2.x;  // cos((l1 - l2) / 2)
+        const double cl = q.cl * sl2.y + q.sl * sl2.x;  // cos((l1 - l2) / 2) sqrt(cos b1 cos b2)
         const double cb = q.cb * sb2.y + q.sb * sb2.x;  // cos((b1 - b2) / 2)
-        const double y = -2.0 * cb2 * (v.sl * cl);
-        const double x = 2.0 * (2.0 * (q.sb * q.cb) * cb2 * (v.sl * v.sl) - v.sb * cb);
+        const double y = -2.0 * (v.sl * cl);
+        const double x = 2.0 * (2.0 * (q.sb * q.cb) * (v.sl * v.sl) - cb1 * v.sb * cb);
         const double ys = y * a.cpa - x * a.spa, xc = x * a.cpa + y * a.spa;
         const double n2 = x * x + y * y;
         const double ell = n2 > 0.0 ? ((p0 * p0) * (ys * ys) + (p1 * p1) * (xc * xc)) / n2 : 0.0;
@@ -539,10 +540,10 @@ __device__ __forceinline__ double kernel_other(const GridArgs &a, const PixHalf 
 // field's kernel may be other than GAUSS1D. F32: multi-channel entries hold
 // FP32 weights, so the Gaussian is evaluated in FP32 (gauss_f32).
 template <bool F32, bool GEN>
-__device__ __forceinline__ double kernel_at(const GridArgs &a, const PixHalf &q, const PairHav &v, const double2 &sl2,
-                                            const double2 &sb2, double cb2, double win, double d2) {
+__device__ __forceinline__ double kernel_at(const GridArgs &a, const PixHalf &q, double cb1, const PairHav &v,
+                                            const double2 &sl2, const double2 &sb2, double win, double d2) {
     if (GEN && a.ktype != HCG_GAUSS1D) {
-        const double k = kernel_other(a, q, v, sl2, sb2, cb2, d2);
+        const double k = kernel_other(a, q, cb1, v, sl2, sb2, d2);
         return win * (F32 ? (double)(float)k : k);
     }
     return win * (F32 ? (double)gauss_f32(d2 * a.p0) : exp(-d2 * a.p0));
@@ -555,16 +556,17 @@ template <bool F32, bool GEN>
 __device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t idx) {
     const PixPrep Q = *P;
     const double2 sl2 = __ldg(a.half + idx), sb2 = __ldg(a.half + a.n + idx);
-    const double cb2 = __ldg(a.cb2 + idx), win = __ldg(a.w + idx);
-    const PairHav v = pair_hav(Q.h, Q.cb1, sl2, sb2, cb2);
+    const double win = __ldg(a.w + idx);
+    const PairHav v = pair_hav(Q.h, sl2, sb2);
     if (v.h > a.hhi) return 0.0;
     if (v.h < a.hlo) {
         if (F32 && !GEN && a.series32) return win * (double)gauss_series_f32(v.h, a.x2scale);
-        return kernel_at<F32, GEN>(a, Q.h, v, sl2, sb2, cb2, win, pair_d2(a, v.h));
+        return kernel_at<F32, GEN>(a, Q.h, Q.cb1, v, sl2, sb2, win, pair_d2(a, v.h));
     }
-    const double d = dist_deg(Q.l1, Q.b1, Q.cb1, __ldg(a.l2 + idx), __ldg(a.b2 + idx), cb2);
+    const double d = dist_deg(Q.l1, Q.b1, Q.cb1, __ldg(a.l2 + idx), __ldg(a.b2 + idx),
+                              __ldg(a.cb2 + idx));
     if (!(d < a.sphere_radius)) return 0.0;
-    return kernel_at<F32, GEN>(a, Q.h, v, sl2, sb2, cb2, win, d * d);
+    return kernel_at<F32, GEN>(a, Q.h, Q.cb1, v, sl2, sb2, win, d * d);
 }
 
 // Weights of sample idx for the four pixels of a group (0 outside
@@ -577,14 +579,14 @@ __device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t 
 enum { kPairGeneral = 0, kPairUnit = 1, kPairOther = 2 };  // kPairOther: kernels other than GAUSS1D
 template <bool F32, int MODE>
 __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P, uint32_t nx, const PixHalf q[4],
-                                             const double cb1[4], const double2 &sl2, const double2 &sb2, double cb2,
-                                             double win, uint32_t idx, const bool in[4], double w[4], float wf[4]) {
+                                             const double cb1[4], const double2 &sl2, const double2 &sb2, double win,
+                                              uint32_t idx, const bool in[4], double w[4], float wf[4]) {
     constexpr bool GEN = MODE == kPairOther;
     PairHav v[4];
     bool acc[4];
     unsigned band = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = pair_hav(q[i], cb1[i], sl2, sb2, cb2);
+    for (int i = 0; i < 4; ++i) v[i] = pair_hav(q[i], sl2, sb2);
     if (MODE == kPairUnit) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -612,7 +614,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
             for (int i = 0; i < 4; ++i) d2[i] = pair_d2(a, acc[i] ? v[i].h : 0.0);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const double k = kernel_at<F32, GEN>(a, q[i], v[i], sl2, sb2, cb2, win, d2[i]);
+                const double k = kernel_at<F32, GEN>(a, q[i], GEN ? cb1[i] : 0.0, v[i], sl2, sb2, win, d2[i]);
                 w[i] = acc[i] ? k : 0.0;
             }
         }
@@ -728,7 +730,7 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             ph[q] = s_h[q];
-            cb1[q] = s_cb1[q];
+            cb1[q] = MODE == kPairOther ? s_cb1[q] : 0.0;  // only the other kernels take it
         }
         const uint32_t t = tb + lane;
         const unsigned ends = __reduce_or_sync(0xffffffffu, len && incl > tb && incl - tb < 32 ? 1u << (incl - tb) : 0u);
@@ -740,12 +742,12 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
         // a lane past the last candidate repeats the round's first one, outside every window
         const uint32_t idx = ra.x + (act ? t : tb);
         const double2 sl2 = __ldg(a.half + idx), sb2 = __ldg(a.half + a.n + idx);
-        const double cb2 = __ldg(a.cb2 + idx), win = MODE == kPairUnit || a.unit_w ? 1.0 : __ldg(a.w + idx);
+        const double win = MODE == kPairUnit || a.unit_w ? 1.0 : __ldg(a.w + idx);
         const bool in[4] = {act && idx - ra.z < ra.w, act && idx - rb.x < rb.y, act && idx - rb.z < rb.w,
                             act && idx - rc.x < rc.y};
         double w[4];
         float wf[4];
-        pair_weights<F32, MODE>(a, a.prep + pix0, nx, ph, cb1, sl2, sb2, cb2, win, idx, in, w, wf);
+        pair_weights<F32, MODE>(a, a.prep + pix0, nx, ph, cb1, sl2, sb2, win, idx, in, w, wf);
         body(idx, idx + ra.y, w, wf);
     }
 }

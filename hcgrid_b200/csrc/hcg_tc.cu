@@ -21,40 +21,35 @@ namespace {
 
 template <class Cfg>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    k_tile_tc(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_out, int has_out, TcJob J,
+    k_tile_tc(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tm_out, int has_out,
+              const __grid_constant__ TcJob J,
               unsigned long long *timeouts, unsigned long long *macs) {
     __shared__ TcShared S;
-    J.map = &tm;
-    J.out_map = has_out ? &tm_out : nullptr;
     const uint64_t tile = J.T.t0 + blockIdx.x;
     tc_load_rings(S, J.T, tile);
     tc_setup<Cfg>(S);  // ends with a CTA barrier
     if (threadIdx.x == 0) sm100::prefetch_tensormap(&tm);
     uint32_t gk = 0;
-    tc_item<Cfg>(S, J, tile, blockIdx.y, gk, 0, timeouts, macs);
+    tc_item<Cfg>(S, J, &tm, has_out ? &tm_out : nullptr, tile, blockIdx.y, gk, 0, timeouts, macs);
     tc_teardown<Cfg>(S, gk, timeouts);
 }
 
 template <class Cfg>
 __global__ void __launch_bounds__(kTcPersistThreads, 1)
-    k_tile_tc_persist(const __grid_constant__ CUtensorMap tm, TcJob J, uint64_t nitems, uint64_t ntiles,
+    k_tile_tc_persist(const __grid_constant__ CUtensorMap tm, const __grid_constant__ TcJob J, uint64_t nitems, uint64_t ntiles,
                       unsigned long long *timeouts, unsigned long long *macs) {
     __shared__ TcPShared S;
-    J.map = &tm;
-    J.out_map = nullptr;
     if (threadIdx.x == 0) sm100::prefetch_tensormap(&tm);
-    tc_persist<Cfg>(S, J, nitems, ntiles, timeouts, macs);
+    tc_persist<Cfg>(S, J, &tm, nitems, ntiles, timeouts, macs);
 }
 
-template <class Cfg>
+template <class Cfg, bool UNIT>  // UNIT: unit sample weights, FP32 series Gaussian (pair_weights' kPairUnit)
 __global__ void __launch_bounds__(kTcDThreads, 1)
-    k_tile_tc_weights(const __grid_constant__ CUtensorMap tm, TcJob J, uint64_t nitems, uint64_t ntiles,
+    k_tile_tc_weights(const __grid_constant__ CUtensorMap tm, const __grid_constant__ TcJob J, uint64_t nitems, uint64_t ntiles,
                       unsigned long long *timeouts, unsigned long long *macs) {
     __shared__ TcDShared S;
-    J.map = &tm;
-    J.out_map = nullptr;
     if (threadIdx.x == 0) sm100::prefetch_tensormap(&tm);
-    tc_persist_weights<Cfg>(S, J, nitems, ntiles, timeouts, macs);
+    tc_persist_weights<Cfg, UNIT>(S, J, &tm, nitems, ntiles, timeouts, macs);
 }
 
 // ------------------------------------------------------------ spectra split
@@ -403,7 +398,7 @@ cudaError_t launch_tc(hcg_context *ctx, const hcg_field *f, TcJob &J, const Tile
 }  // namespace
 
 namespace {
-template <class Cfg>
+template <class Cfg, bool UNIT>
 cudaError_t launch_tc_weights(hcg_context *ctx, const hcg_field *f, TcJob &J, const TileArgs &T, uint64_t ntiles,
                               std::string &why) {
     cudaStream_t s = ctx->stream;
@@ -414,7 +409,7 @@ cudaError_t launch_tc_weights(hcg_context *ctx, const hcg_field *f, TcJob &J, co
     }
     static bool attr_set = false;  // per instantiation
     if (!attr_set) {
-        cudaError_t e = tc_set_smem((const void *)k_tile_tc_weights<Cfg>, Cfg::kSmem);
+        cudaError_t e = tc_set_smem((const void *)k_tile_tc_weights<Cfg, UNIT>, Cfg::kSmem);
         if (e != cudaSuccess) return e;
         attr_set = true;
     }
@@ -424,7 +419,7 @@ cudaError_t launch_tc_weights(hcg_context *ctx, const hcg_field *f, TcJob &J, co
     const uint64_t nitems = ntiles * J.ncb;
     const unsigned grid = (unsigned)std::min<uint64_t>(nitems, (uint64_t)(nsm > 0 ? nsm : 148));
     if (grid == 0) return cudaSuccess;
-    k_tile_tc_weights<Cfg><<<grid, kTcDThreads, Cfg::kSmem, s>>>(tm, J, nitems, ntiles,
+    k_tile_tc_weights<Cfg, UNIT><<<grid, kTcDThreads, Cfg::kSmem, s>>>(tm, J, nitems, ntiles,
                                                                       &ctx->d_stats->timeouts, &ctx->d_stats->tc_macs);
     return cudaGetLastError();
 }
@@ -441,9 +436,15 @@ cudaError_t tc_weights(hcg_context *ctx, const hcg_field *f, const GridArgs &a, 
     J.wout = wout;
     tc_pipeline(ctx, f, J);
     const uint32_t b = f->xcpad / 64;
-    if (b >= 4) return launch_tc_weights<TcCfgN4S2>(ctx, f, J, T, ntiles, why);
-    if (b >= 2) return launch_tc_weights<TcCfgN2S3>(ctx, f, J, T, ntiles, why);
-    return launch_tc_weights<TcCfgN1S4>(ctx, f, J, T, ntiles, why);
+    const bool unit = a.unit_w && a.series32;
+    if (b >= 4)
+        return unit ? launch_tc_weights<TcCfgN4S2, true>(ctx, f, J, T, ntiles, why)
+                    : launch_tc_weights<TcCfgN4S2, false>(ctx, f, J, T, ntiles, why);
+    if (b >= 2)
+        return unit ? launch_tc_weights<TcCfgN2S3, true>(ctx, f, J, T, ntiles, why)
+                    : launch_tc_weights<TcCfgN2S3, false>(ctx, f, J, T, ntiles, why);
+    return unit ? launch_tc_weights<TcCfgN1S4, true>(ctx, f, J, T, ntiles, why)
+                : launch_tc_weights<TcCfgN1S4, false>(ctx, f, J, T, ntiles, why);
 }
 
 cudaError_t tc_accum(hcg_context *ctx, const hcg_field *f, const GroupArgs &g, const TileArgs &T, uint64_t ntiles,

@@ -96,9 +96,11 @@ using TcCfgN4K32 = TcCfg<4, 4, 32>;  // 256 channels, 32-slot chunks, 4 stages
 // overlapped with the next item)
 static_assert(kTcConfigCount == 6, "hcg_tc_set_config numbers the shapes 0-3 above and 4-5 persistent");
 
-// One job's tensor-core arguments.
+// One job's tensor-core arguments. The single-job kernels take it as a grid
+// constant and the tensor maps beside it: a kernel that writes into its
+// parameter works on a copy in local memory.
 struct TcJob {
-    const CUtensorMap *map;  // [2][ncb64][n][64] 16-bit hi/lo arrays, boxes 64 x 8 x nb x 2
+    const CUtensorMap *map;  // batch kernel: [2][ncb64][n][64] 16-bit hi/lo arrays, boxes 64 x 8 x nb x 2
     GroupArgs g;
     TileArgs T;
     const unsigned long long *off;  // entry offset of each group (minus g.ebase)
@@ -254,7 +256,7 @@ struct TcStage {
 // S.base hold the item's ring table (nrt rings); `gk` is the CTA's chunk count
 // before the item.
 template <class Cfg, class SH>
-__device__ __forceinline__ void tc_produce(SH &S, const TcJob &J, uint32_t cblk, uint32_t U, uint32_t nchunks,
+__device__ __forceinline__ void tc_produce(SH &S, const TcJob &J, const CUtensorMap *map, uint32_t cblk, uint32_t U, uint32_t nchunks,
                                            uint32_t gk, int nrt, unsigned long long *timeouts) {
     using namespace sm100;
     constexpr uint32_t ST = Cfg::kStages, KC = Cfg::kK;
@@ -277,7 +279,7 @@ __device__ __forceinline__ void tc_produce(SH &S, const TcJob &J, uint32_t cblk,
     // the item's chunks [ST, pf) are prefetched at its start; chunk k + pf with chunk k
     for (uint32_t i = lane; J.pf && i < (pf - ST) * (uint32_t)NB8; i += 32) {
         const uint32_t c = ST + i / NB8;
-        if (c < nchunks) tma_prefetch_4d(J.map, 0, row_of(c * KC + 8 * (i % NB8)), (int)(cblk * J.nb), 0);
+        if (c < nchunks) tma_prefetch_4d(map, 0, row_of(c * KC + 8 * (i % NB8)), (int)(cblk * J.nb), 0);
     }
     for (uint32_t k = 0; k < nchunks; ++k) {
         const uint32_t g = gk + k, s = g % ST;
@@ -298,9 +300,9 @@ __device__ __forceinline__ void tc_produce(SH &S, const TcJob &J, uint32_t cblk,
         if (lane < nlanes && kk < nchunks) {
             const int row = row_of(kk * KC + 8 * b);
             if (lane < NB8)
-                tma_load_4d(st.B(s) + b * Cfg::kBGroup, J.map, &S.full_b[s], 0, row, (int)(cblk * J.nb), 0);
+                tma_load_4d(st.B(s) + b * Cfg::kBGroup, map, &S.full_b[s], 0, row, (int)(cblk * J.nb), 0);
             else
-                tma_prefetch_4d(J.map, 0, row, (int)(cblk * J.nb), 0);
+                tma_prefetch_4d(map, 0, row, (int)(cblk * J.nb), 0);
         }
     }
 }
@@ -529,7 +531,8 @@ __device__ __forceinline__ void tc_build(SH &S, const TcJob &J, uint64_t tile, u
 // Whole CTA: one item. `gk` counts the K chunks this CTA has run (all items),
 // `itn` its items; both advance identically in every thread.
 template <class Cfg>
-__device__ __forceinline__ void tc_item(TcShared &S, const TcJob &J, uint64_t tile, uint32_t cblk, uint32_t &gk,
+__device__ __forceinline__ void tc_item(TcShared &S, const TcJob &J, const CUtensorMap *map,
+                                        const CUtensorMap *out_map, uint64_t tile, uint32_t cblk, uint32_t &gk,
                                         uint32_t itn, unsigned long long *timeouts,
                                         unsigned long long *macs) {
     using namespace sm100;
@@ -539,7 +542,7 @@ __device__ __forceinline__ void tc_item(TcShared &S, const TcJob &J, uint64_t ti
     const uint32_t nchunks = (U + Cfg::kK - 1) / Cfg::kK;
     const uint32_t taddr = S.tmem;
     if (warp == 0) {
-        tc_produce<Cfg>(S, J, cblk, U, nchunks, gk, T.nr[tile], timeouts);
+        tc_produce<Cfg>(S, J, map, cblk, U, nchunks, gk, T.nr[tile], timeouts);
     } else if (warp == 1) {
         if (lane == 0) {
             tc_mma<Cfg>(S, J, nchunks, gk, taddr, timeouts, macs);
@@ -588,7 +591,7 @@ __device__ __forceinline__ void tc_item(TcShared &S, const TcJob &J, uint64_t ti
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = (__uint_as_float(r[i]) * S.inv_scale[cb * 32 + i]) * inv;
             if (!store) continue;
-            if (J.out_map) {
+            if (out_map) {
                 if (J.ostride) {
                     // box [y][x][channel]: this pixel's 32 values, 16-byte pieces in a
                     // lane-rotated order (fewer bank conflicts)
@@ -621,14 +624,14 @@ __device__ __forceinline__ void tc_item(TcShared &S, const TcJob &J, uint64_t ti
                 }
             }
         }
-        if (store && J.out_map) {
+        if (store && out_map) {
             fence_proxy_async_smem();
             named_barrier(2, kTcBuilders);  // the staging tile is complete
             if (bt == 0) {
                 if (J.ostride)
-                    tma_store_3d(J.out_map, stage, (int)c_item, (int)tx0, (int)ty0);
+                    tma_store_3d(out_map, stage, (int)c_item, (int)tx0, (int)ty0);
                 else
-                    tma_store_3d(J.out_map, stage, (int)tx0, (int)ty0, (int)c_item);
+                    tma_store_3d(out_map, stage, (int)tx0, (int)ty0, (int)c_item);
                 bulk_commit_group();
                 bulk_wait_group_read0();  // the staging tile may be overwritten after this
             }
@@ -782,7 +785,7 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
 }
 
 template <class Cfg>
-__device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, uint64_t nitems, uint64_t ntiles,
+__device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const CUtensorMap *map, uint64_t nitems, uint64_t ntiles,
                                            unsigned long long *timeouts, unsigned long long *macs) {
     using namespace sm100;
     constexpr uint32_t ST = Cfg::kStages, KC = Cfg::kK;
@@ -821,7 +824,7 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, uint64_
             for (int j = lane; j < nrt; j += 32) S.ulo[j] = J.T.ulo[tile * kTileMaxRings + j];
             for (int j = lane; j <= nrt; j += 32) S.base[j] = J.T.base[tile * (kTileMaxRings + 1) + j];
             __syncwarp();
-            tc_produce<Cfg>(S, J, cblk, U, nchunks, gk, nrt, timeouts);
+            tc_produce<Cfg>(S, J, map, cblk, U, nchunks, gk, nrt, timeouts);
         } else if (warp == 1) {
             if (lane == 0) tc_mma_seg<Cfg, true>(S, J, nchunks, gk, gs, timeouts, macs);
         } else if (warp < 6) {
@@ -861,8 +864,15 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, uint64_
 // (cp.async, one chunk ahead); then, for each slot whose sample lies in its
 // pixel's window of the slot's ring (ring_window_mc, the windows the tile pass
 // unioned), a builder evaluates the FP64 distance, cutoff and FP32 Gaussian
-// (pair_weights' arithmetic), accumulates the FP64 weight sum and writes its
-// hi/lo pieces of the K-major operand row (16-byte stores). The epilogue adds
+// (pair_weights' arithmetic; UNIT: its kPairUnit form), accumulates the FP64
+// weight sum and writes its hi/lo pieces of the K-major operand row (16-byte
+// stores). The next ring's window is loaded when a ring begins. What bounds it:
+// issue, about 45 instructions a (pixel, slot) pair at three builder warps a
+// scheduler (eight builder warps with more registers, or samples read through
+// L1 without the chunk barriers, were slower: 10.5 and 12.4 against 9.3 ms on
+// 150,000 samples x 64 channels, 768 x 768 pixels, beam 54 pixels wide; 13.5 ms
+// with FP64 cutoff tests, weights converted to and from FP64, and the window
+// fetched at each ring). The epilogue adds
 // the three partial weight sums of a row from shared memory.
 constexpr int kTcGeo = 64;          // slots per chunk of the direct builders
 constexpr int kTcGeoBufs = 2;       // geometry buffers: loads run one chunk ahead
@@ -879,11 +889,13 @@ struct TcDShared {
     uint32_t bulo[kTileMaxRings], bbase[kTileMaxRings + 1];  // the builders' current item
     float inv_scale[2][kTcMaxN];
     double wsum[2][kTcDRow][kTcM];  // by item parity: the builders' partial sums of each row
+    uint16_t ring_j[kTileMaxRings];      // the item's occupied rings: place in the tile's ring span
+    int span;                            // rings of that span
     double4 g_half[kTcGeoBufs][kTcGeo];  // sample geometry of the chunks in flight
-    double g_cb[kTcGeoBufs][kTcGeo], g_w[kTcGeoBufs][kTcGeo];
+    double g_w[kTcGeoBufs][kTcGeo];
 };
 
-template <class Cfg>
+template <class Cfg, bool UNIT>
 __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, uint64_t tile, uint32_t cblk,
                                                  uint32_t U, uint32_t nchunks, uint32_t gk, uint32_t il, int bt,
                                                  unsigned long long *timeouts) {
@@ -907,13 +919,30 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
     const uint32_t xx = (uint32_t)(tile % T.ntx) * kTileX + (m & (kTileX - 1));
     const uint32_t yy = (uint32_t)(tile / T.ntx) * kTileY + m / kTileX;
     const bool valid = xx < J.g.nx && yy < J.g.ny;
-    PixPrep P{};
-    if (valid) P = a.prep[(uint64_t)yy * J.g.nx + xx];
-    const PixHalf ph = P.h;
+    const PixPrep *prep = a.prep + (uint64_t)yy * J.g.nx + xx;  // read only where valid
+    PixHalf ph{};
+    int rend = 0;  // end of the pixel's rings
     const int r0 = T.r0[tile];
     const uint32_t nrows = J.nrows;
+    if (valid) {
+        ph = prep->h;
+        if (prep->nr > 0) rend = prep->ur + prep->nr;
+    }
+    // the rings' places in the tile's span
+    if (bt == 0) S.span = 0;
+    named_barrier(4, kTcDBuilders);
+    if (qb == 0 && rend > 0) atomicMax(&S.span, rend - r0);
+    named_barrier(4, kTcDBuilders);
+    for (int jj = bt; jj < S.span; jj += kTcDBuilders) {
+        const uint32_t cc = T.ring_idx[tile * kTileMaxSpan + jj];
+        if (cc < kTileMaxRings) S.ring_j[cc] = (uint16_t)jj;
+    }
+    named_barrier(4, kTcDBuilders);
+    const uint2 *win = T.win ? reinterpret_cast<const uint2 *>(T.win + (tile * kWinSpan * kTileGroups + wgq) * 2) + wq
+                             : nullptr;
     // kernel-parameter scalars held in registers for the slot loop
-    const double hlo = a.hlo, hhi = a.hhi, p0 = a.p0, cb1 = P.cb1;
+    const double hlo = a.hlo, hhi = a.hhi, p0 = a.p0;
+    const float hlo32 = a.hlo32, hhi32 = a.hhi32;
     const bool series = a.series != 0;
     const float x2scale = a.x2scale;
     const float wscale = J.wscale;
@@ -934,15 +963,29 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
             const uint32_t b = kk % kTcGeoBufs;
             cp_async16(&S.g_half[b][bt], a.half + idx, true);
             cp_async16(reinterpret_cast<uint8_t *>(&S.g_half[b][bt]) + 16, a.half + a.n + idx, true);
-            cp_async8(&S.g_cb[b][bt], a.cb2 + idx);
-            cp_async8(&S.g_w[b][bt], a.w + idx);
+            if (!UNIT) cp_async8(&S.g_w[b][bt], a.w + idx);
         }
         cp_async_commit();
     };
     load(0);
-    // ring cursor: compacted ring c of the current slot, its span index j and this pixel's window there
-    int c = -1, j = -1;
+    // ring cursor: compacted ring c of the current slot and this pixel's window
+    // there; the next ring's window is loaded when a ring begins, so that no
+    // piece waits for it
+    int c = -1, cpre = -1;
     uint32_t cbase = 0, cnext = 0, culo = 0, wlo = 0, whi = 0;
+    uint2 pre = make_uint2(0u, 0u);
+    auto window = [&](int cc) {
+        // the window the tile pass kept for this pixel and ring (lo > hi: none)
+        const int jj = S.ring_j[cc];
+        uint2 w = make_uint2(0u, 0u);
+        if (win && jj < kWinSpan) {
+            w = __ldg(win + jj * (kTileGroups * 4));
+        } else if (valid && prep->nr > 0 && r0 + jj >= prep->ur && r0 + jj < rend) {
+            uint32_t lo, hi, rl;
+            if (ring_window_general(a, *prep, r0 + jj, lo, hi, rl)) w = make_uint2(lo, hi);
+        }
+        return w;
+    };
     double wsum = 0.0;
     uint32_t within = 0;
     bool failed = false;
@@ -971,27 +1014,24 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
                 cbase = S.bbase[c];
                 cnext = S.bbase[c + 1];
                 culo = S.bulo[c];
-                do {
-                    ++j;
-                } while (j < kTileMaxSpan && T.ring_idx[tile * kTileMaxSpan + j] != (uint16_t)c);
-                wlo = whi = 0;
-                const int kr = r0 + j;
-                if (T.win && j < kWinSpan) {
-                    // the window the tile pass kept for this pixel and ring (lo > hi: none)
-                    const uint32_t *w = reinterpret_cast<const uint32_t *>(
-                        T.win + ((tile * kWinSpan + (uint64_t)j) * kTileGroups + wgq) * 2);
-                    const uint32_t lo = __ldg(w + 2 * wq), hi = __ldg(w + 2 * wq + 1);
-                    if (lo <= hi) {
-                        wlo = lo;
-                        whi = hi;
-                    }
-                } else if (P.nr > 0 && kr >= P.ur && kr < P.ur + P.nr) {
-                    uint32_t lo, hi, rl;
-                    if (ring_window_general(a, P, kr, lo, hi, rl)) {
-                        wlo = lo;
-                        whi = hi;
-                    }
-                }
+                const uint2 w = c == cpre ? pre : window(c);
+                wlo = w.x;
+                whi = w.y;
+                cpre = c + 1;
+                if (cpre < nrt) pre = window(cpre);
+            }
+            // the piece's slots inside the window, a bit each
+            const uint32_t idx0 = culo + (slot0 - cbase);
+            uint32_t in = 0;
+            if (slot0 < U) {
+                const uint32_t lo = wlo > idx0 ? min(wlo - idx0, 8u) : 0u, hi = whi > idx0 ? min(whi - idx0, 8u) : 0u;
+                in = hi > lo ? ((1u << hi) - 1u) & ~((1u << lo) - 1u) & ((1u << min(U - slot0, 8u)) - 1u) : 0u;
+            }
+            const uint32_t o = tc_a_offset<KC>(m, s8 * 8);
+            if (__ballot_sync(0xffffffffu, in != 0) == 0) {  // none for any pixel of the warp
+                *reinterpret_cast<uint4 *>(ah + o) = make_uint4(0, 0, 0, 0);
+                *reinterpret_cast<uint4 *>(al + o) = make_uint4(0, 0, 0, 0);
+                continue;
             }
             // The piece's pair tests in two halves of 4 slots as straight-line
             // code (independent FP64 chains the scheduler can interleave):
@@ -1002,58 +1042,58 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 double hh[4];
-                bool inw[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const uint32_t q = s8 * 8 + half * 4 + e;
-                    const uint32_t idx = culo + (slot0 + half * 4 + e - cbase);
-                    inw[e] = slot0 + half * 4 + e < U && idx >= wlo && idx < whi;
                     const double4 gq = S.g_half[b][q];
-                    const double sb = ph.sb * gq.w - ph.cb * gq.z;  // sin((b1 - b2) / 2)
-                    const double sl = ph.sl * gq.y - ph.cl * gq.x;  // sin((l1 - l2) / 2)
-                    hh[e] = sb * sb + cb1 * S.g_cb[b][q] * (sl * sl);
+                    hh[e] = pair_hav(ph, make_double2(gq.x, gq.y), make_double2(gq.z, gq.w)).h;
                 }
                 float wv[4];
-                bool band = false;
+                uint32_t band = 0;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const double h = hh[e];
-                    // the Gaussian of an accepted pair, as pair_weights evaluates it
-                    float ex;
-                    if (series) {
-                        ex = gauss_series_f32(h, x2scale);
+                    const bool inw = in >> (half * 4 + e) & 1u;
+                    if (UNIT) {
+                        // as pair_weights with kPairUnit
+                        const float hf = (float)h;
+                        const bool acc = inw && hf < hlo32;
+                        if (inw && !acc && hf <= hhi32) band |= 1u << e;
+                        wv[e] = acc ? gauss_series_f32(h, x2scale) : 0.f;
+                        wsum += (double)wv[e];
+                        within += wv[e] != 0.f;
                     } else {
-                        const double d = 2.0 * asin(sqrt(h)) * kRad2Deg;
-                        ex = gauss_f32(d * d * p0);
-                    }
-                    const bool acc = inw[e] && h < hlo;
-                    band |= inw[e] && h >= hlo && h <= hhi;
-                    const double wt = acc ? S.g_w[b][s8 * 8 + half * 4 + e] * (double)ex : 0.0;
-                    wv[e] = 0.f;
-                    if (wt != 0.0) {
-                        wsum += wt;
-                        ++within;
+                        // the Gaussian of an accepted pair, as pair_weights evaluates it
+                        float ex;
+                        if (series) {
+                            ex = gauss_series_f32(h, x2scale);
+                        } else {
+                            const double d = 2.0 * asin(sqrt(h)) * kRad2Deg;
+                            ex = gauss_f32(d * d * p0);
+                        }
+                        const bool acc = inw && h < hlo;
+                        if (inw && h >= hlo && h <= hhi) band |= 1u << e;
+                        const double wt = acc ? S.g_w[b][s8 * 8 + half * 4 + e] * (double)ex : 0.0;
                         wv[e] = (float)wt;
+                        wsum += wt;
+                        within += wt != 0.0;
                     }
                 }
                 if (band) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        if (!(inw[e] && hh[e] >= hlo && hh[e] <= hhi)) continue;
+                        if (!(band >> e & 1u)) continue;
                         const double wt =
-                            pair_band<true, false>(a, a.prep + (uint64_t)yy * J.g.nx + xx, culo + (slot0 + half * 4 + e - cbase));
-                        if (wt != 0.0) {
-                            wsum += wt;
-                            ++within;
-                            wv[e] = (float)wt;
-                        }
+                            pair_band<true, false>(a, prep, idx0 + half * 4 + e);
+                        wsum += wt;
+                        within += wt != 0.0;
+                        wv[e] = (float)wt;
                     }
                 }
 #pragma unroll
                 for (int e = 0; e < 4; e += 2)
                     tc_split2(wv[e] * wscale, wv[e + 1] * wscale, fmt, hv[half * 2 + e / 2], lv[half * 2 + e / 2]);
             }
-            const uint32_t o = tc_a_offset<KC>(m, s8 * 8);
             *reinterpret_cast<uint4 *>(ah + o) = make_uint4(hv[0], hv[1], hv[2], hv[3]);
             *reinterpret_cast<uint4 *>(al + o) = make_uint4(lv[0], lv[1], lv[2], lv[3]);
         }
@@ -1072,8 +1112,8 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
 
 // Persistent direct-weight kernel body: roles as in tc_persist, the builders
 // being tc_build_weights and the epilogue reading their weight sums.
-template <class Cfg>
-__device__ __forceinline__ void tc_persist_weights(TcDShared &S, const TcJob &J, uint64_t nitems, uint64_t ntiles,
+template <class Cfg, bool UNIT>
+__device__ __forceinline__ void tc_persist_weights(TcDShared &S, const TcJob &J, const CUtensorMap *map, uint64_t nitems, uint64_t ntiles,
                                                    unsigned long long *timeouts, unsigned long long *macs) {
     using namespace sm100;
     constexpr uint32_t ST = Cfg::kStages, KC = Cfg::kK;
@@ -1113,11 +1153,11 @@ __device__ __forceinline__ void tc_persist_weights(TcDShared &S, const TcJob &J,
             for (int j = lane; j < nrt; j += 32) S.ulo[j] = J.T.ulo[tile * kTileMaxRings + j];
             for (int j = lane; j <= nrt; j += 32) S.base[j] = J.T.base[tile * (kTileMaxRings + 1) + j];
             __syncwarp();
-            tc_produce<Cfg>(S, J, cblk, U, nchunks, gk, nrt, timeouts);
+            tc_produce<Cfg>(S, J, map, cblk, U, nchunks, gk, nrt, timeouts);
         } else if (warp == 1) {
             if (lane == 0) tc_mma_seg<Cfg, false>(S, J, nchunks, gk, gs, timeouts, macs);
         } else if (tid < 64 + kTcDBuilders) {
-            tc_build_weights<Cfg>(S, J, tile, cblk, U, nchunks, gk, il, tid - 64, timeouts);
+            tc_build_weights<Cfg, UNIT>(S, J, tile, cblk, U, nchunks, gk, il, tid - 64, timeouts);
         } else {
             tc_epilogue_direct<KC, TcDShared, true>(S, J, tile, cblk, nchunks, il, gse, tid - (64 + kTcDBuilders),
                                                 timeouts);
