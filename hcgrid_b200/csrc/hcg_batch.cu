@@ -264,8 +264,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     tc_teardown<KbTcCfg>(S, gk, timeouts);
 }
 
-__global__ void __launch_bounds__(256, 2) kb_1chan(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
-    __shared__ GroupShared S[8];
+__global__ void __launch_bounds__(kGroupThreads, 4) kb_1chan(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
+    __shared__ GroupShared S[kGroupWarps];
     if (H->tot_c1 == 0) return;
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
@@ -274,8 +274,10 @@ __global__ void __launch_bounds__(256, 2) kb_1chan(BatchHdr *H, const JobDesc *_
         if (it >= H->tot_c1) break;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.c1_base; });
         const JobDesc &J = jobs[j];
-        grid1_item<false>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp],
-                          pc);  // GAUSS1D jobs only
+        if (J.a.unit_w && J.a.exp2ok)  // GAUSS1D jobs only
+            grid1_item<kPairUnit>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp], pc);
+        else
+            grid1_item<kPairGeneral>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp], pc);
     }
     flush_counts(pc, stats);
 }
@@ -364,7 +366,7 @@ static cudaError_t capture(hcg_context *ctx, BatchState &B) {
             kb_tc<1><<<n, kTcThreads, KbShape<1>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_tc<2><<<n, kTcThreads, KbShape<2>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_tc<3><<<n, kTcThreads, KbShape<3>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
-            kb_1chan<<<n * 2, 256, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
+            kb_1chan<<<n * 4, kGroupThreads, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
         }
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
         if (ce != cudaSuccess) return ce;

@@ -46,16 +46,15 @@ __global__ void k_pixel_prep(HpxParams h, uint64_t firstring, uint64_t usedrings
     if (p < npixmap) prep_item(h, firstring, usedrings, disc, X, Y, out, stats, p);
 }
 
-// GEN: fields whose kernel is not GAUSS1D
-template <bool GEN>
-__global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_grid_1chan(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+template <int MODE>  // as pair_weights
+__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_grid_1chan(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
                                                         const float *__restrict__ data, uint32_t cstride,
                                                         float *__restrict__ out, float *__restrict__ wout) {
     __shared__ GroupShared S[kGroupWarps];
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
     const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
-    if (grp < ngroups) grid1_item<GEN>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
+    if (grp < ngroups) grid1_item<MODE>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
     flush_counts(pc, a.stats);
 }
 
@@ -204,10 +203,11 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         cudaEventRecord(ctx->evp[2], s);
         const uint64_t ngroups = (uint64_t)((t->nx + 1) / 2) * ((t->ny + 1) / 2);
         const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
-        if (f->kernel_type == HCG_GAUSS1D)
-            k_grid_1chan<false><<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
-        else
-            k_grid_1chan<true><<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
+        const int mode = pair_mode1(f, a);
+        auto grid1 = mode == kPairOther ? k_grid_1chan<kPairOther>
+                     : mode == kPairUnit ? k_grid_1chan<kPairUnit>
+                                         : k_grid_1chan<kPairGeneral>;
+        grid1<<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else {
         GroupArgs g;
@@ -337,9 +337,7 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
             unsigned cb = (unsigned)((gc.g1 - gc.g0 + 7) / 8), gb = (ch.second - ch.first) * T.ntx;
             TileArgs tt = T;
             tt.t0 = (uint64_t)ch.first * T.ntx;
-            const int mode = f->kernel_type != HCG_GAUSS1D ? kPairOther
-                             : a.unit_w && a.series32      ? kPairUnit
-                                                           : kPairGeneral;
+            const int mode = pair_mode(f, a);
             auto weights = gc.pack ? (mode == kPairOther  ? k_group<kPairOther, 1>
                                       : mode == kPairUnit ? k_group<kPairUnit, 1>
                                                           : k_group<kPairGeneral, 1>)

@@ -197,6 +197,8 @@ struct GridArgs {
     float hpolar32;       // >= hpolar
     int unit_w;           // every sample weight is 1
     float hlo32, hhi32;   // <= hlo, >= hhi: the brackets an FP32 haversine decides
+    double e2scale;       // -4 R2D^2 p0 log2(e): GAUSS1D's base-2 exponent per unit of the series
+    int exp2ok;           // series, GAUSS1D, and no accepted pair's weight is below 2^-1000 (exp2_small)
     uint64_t n;           // samples
     double spa, cpa;      // GAUSS2D: sine and cosine of the position angle
 };
@@ -227,6 +229,8 @@ inline GridArgs grid_args(const hcg_field *f, const PixPrep *prep, DevStats *sta
     a.firstring = f->firstring;
     a.hpolar32 = (float)(hstar * (1.0 + 2e-6));
     a.unit_w = f->unit_w;
+    a.e2scale = -4.0 * kRad2Deg * kRad2Deg * f->kparam0 * 1.4426950408889634;
+    a.exp2ok = a.series32 && a.e2scale <= 0.0 && a.e2scale * hstar * 1.01 > -1000.0;
     a.hlo32 = (float)(a.hlo * (1.0 - 2e-7));
     a.hhi32 = (float)(a.hhi * (1.0 + 2e-7));
     a.n = f->n;
@@ -504,6 +508,29 @@ __device__ __forceinline__ double pair_d2(const GridArgs &a, double h) {
     return d * d;
 }
 
+// 2^t for -1000 < t <= 0: the nearest integer by adding and subtracting
+// 1.5 * 2^52, the Taylor series of 2^f = exp(f ln 2) on |f| <= 1/2 (degree 13,
+// remainder below 5e-18), and the integer into the exponent. The range is known,
+// so nothing is tested; within 2 ulp.
+__device__ __forceinline__ double exp2_small(double t) {
+    const double big = 6755399441055744.0, k = t + big, f = t - (k - big), x = f * 0.6931471805599453;
+    double p = 1.0 / 6227020800.0;
+    p = fma(p, x, 1.0 / 479001600.0);
+    p = fma(p, x, 1.0 / 39916800.0);
+    p = fma(p, x, 1.0 / 3628800.0);
+    p = fma(p, x, 1.0 / 362880.0);
+    p = fma(p, x, 1.0 / 40320.0);
+    p = fma(p, x, 1.0 / 5040.0);
+    p = fma(p, x, 1.0 / 720.0);
+    p = fma(p, x, 1.0 / 120.0);
+    p = fma(p, x, 1.0 / 24.0);
+    p = fma(p, x, 1.0 / 6.0);
+    p = fma(p, x, 0.5);
+    p = fma(p, x, 1.0);
+    p = fma(p, x, 1.0);
+    return __hiloint2double(__double2hiint(p) + (__double2loint(k) << 20), __double2loint(p));
+}
+
 // The grid kernels other than GAUSS1D (gridding.cu:242-256), FP64, for an
 // accepted pair with squared distance d2: GAUSS2D (sigma_maj, sigma_min, PA)
 // at the great-circle bearing of the sample seen from the pixel
@@ -571,16 +598,17 @@ __device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t 
 
 // Weights of sample idx for the four pixels of a group (0 outside
 // sphere_radius, decided from the haversine). `in`: the sample is in the
-// pixel's window. `wf` is the weight rounded to FP32 (F32 only). Straight-line
-// code: the four pixels' chains interleave, and a pair that is not accepted
-// costs a select, not a branch. MODE kPairUnit: FP32 Gaussians of unit-weight
-// samples, where the haversine rounded to FP32 (which the series takes anyway)
-// decides all but the pairs within 2e-7 of the cutoff, relative.
+// pixel's window. `wf` is the weight rounded to FP32 (F32 only), `nz`: it is
+// not zero. Straight-line code: the four pixels' chains interleave, and a pair
+// that is not accepted costs a select, not a branch. MODE kPairUnit: GAUSS1D
+// with unit-weight samples (F32: the FP32 Gaussian of the series; else
+// exp2_small), where the haversine rounded to FP32 decides all but the pairs
+// within 2e-7 of the cutoff, relative.
 enum { kPairGeneral = 0, kPairUnit = 1, kPairOther = 2 };  // kPairOther: kernels other than GAUSS1D
 template <bool F32, int MODE>
 __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P, uint32_t nx, const PixHalf q[4],
                                              const double cb1[4], const double2 &sl2, const double2 &sb2, double win,
-                                              uint32_t idx, const bool in[4], double w[4], float wf[4]) {
+                                             uint32_t idx, const bool in[4], double w[4], float wf[4], bool nz[4]) {
     constexpr bool GEN = MODE == kPairOther;
     PairHav v[4];
     bool acc[4];
@@ -593,8 +621,27 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
             const float hf = (float)v[i].h;
             acc[i] = in[i] && hf < a.hlo32;
             if (in[i] && !acc[i] && hf <= a.hhi32) band |= 1u << i;
-            wf[i] = acc[i] ? gauss_series_f32(v[i].h, a.x2scale) : 0.f;
-            w[i] = (double)wf[i];
+        }
+        if (F32) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                wf[i] = acc[i] ? gauss_series_f32(v[i].h, a.x2scale) : 0.f;
+                w[i] = (double)wf[i];
+                nz[i] = wf[i] != 0.f;
+            }
+        } else {
+            double t[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double h = v[i].h;
+                t[i] = (h * a.e2scale) *
+                       (1.0 + h * (1.0 / 3.0 + h * (8.0 / 45.0 + h * (4.0 / 35.0 + h * (128.0 / 1575.0)))));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                w[i] = exp2_small(t[i]);  // of a pair beyond the cutoff: not used
+                nz[i] = acc[i];
+            }
         }
     } else {
 #pragma unroll
@@ -619,7 +666,10 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) wf[i] = F32 ? (float)w[i] : 0.f;
+        for (int i = 0; i < 4; ++i) {
+            wf[i] = F32 ? (float)w[i] : 0.f;
+            nz[i] = w[i] != 0.0;
+        }
     }
     if (band) {
 #pragma unroll
@@ -627,9 +677,18 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
             if (band >> i & 1u) {
                 w[i] = pair_band<F32, GEN>(a, P + (i & 1) + (uint64_t)(i >> 1) * nx, idx);
                 wf[i] = F32 ? (float)w[i] : 0.f;
+                nz[i] = MODE == kPairUnit && F32 ? wf[i] != 0.f : w[i] != 0.0;
             }
         }
     }
+}
+
+// The single-channel and the multi-channel pair mode of a field.
+inline int pair_mode1(const hcg_field *f, const GridArgs &a) {
+    return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.exp2ok ? kPairUnit : kPairGeneral;
+}
+inline int pair_mode(const hcg_field *f, const GridArgs &a) {
+    return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.series32 ? kPairUnit : kPairGeneral;
 }
 
 // Sums of four values over a warp's lanes: lanes 8q .. 8q + 7 return value q's
@@ -684,8 +743,8 @@ __device__ __forceinline__ void group_load(GroupShared &S, const PixPrep *__rest
 }
 
 // One block of up to 32 rings (lane = ring) of a group: every union candidate,
-// 32 at a time, tested against the four pixels; `body(idx, slot, w, wf)` gets
-// the candidate's weights. Warp-collective. What bounds it: instruction
+// 32 at a time, tested against the four pixels; `body(idx, slot, w, wf, nz)`
+// gets the candidate's weights. Warp-collective. What bounds it: instruction
 // issue (about 40 a pair) with the FP64 pipe next. The ring of a candidate is
 // found from one reduction of the ring ends that fall into the round (a bit
 // each) instead of a search by shuffles, its record read from shared memory
@@ -747,8 +806,9 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
                             act && idx - rc.x < rc.y};
         double w[4];
         float wf[4];
-        pair_weights<F32, MODE>(a, a.prep + pix0, nx, ph, cb1, sl2, sb2, win, idx, in, w, wf);
-        body(idx, idx + ra.y, w, wf);
+        bool nz[4];
+        pair_weights<F32, MODE>(a, a.prep + pix0, nx, ph, cb1, sl2, sb2, win, idx, in, w, wf, nz);
+        body(idx, idx + ra.y, w, wf, nz);
     }
 }
 
@@ -767,9 +827,16 @@ __device__ __forceinline__ void group_lane_windows(const GridArgs &a, const Grou
     }
 }
 
-// Pair counts a warp's groups add up (flushed by its kernel).
+// Pair counts a warp's groups add up (the same in every lane; flushed by its
+// kernel).
 struct PairCounts {
     unsigned long long cand = 0, within = 0, skips = 0;
+    // warp-collective: the lanes' counts of one item
+    __device__ __forceinline__ void add(uint32_t c, uint32_t w, uint32_t s) {
+        cand += __reduce_add_sync(0xffffffffu, c);
+        within += __reduce_add_sync(0xffffffffu, w);
+        skips += __reduce_add_sync(0xffffffffu, s);
+    }
 };
 // The block's counts to the context's statistics: one atomic per block (one
 // per pixel or group on one address was a bound of its own). Block-collective.
@@ -777,10 +844,11 @@ __device__ __forceinline__ void flush_counts(const PairCounts &c, DevStats *stat
     __shared__ unsigned long long s_c[3];
     if (threadIdx.x < 3) s_c[threadIdx.x] = 0;
     __syncthreads();
-    const unsigned long long v[3] = {warp_sum_u64(c.cand), warp_sum_u64(c.within), warp_sum_u64(c.skips)};
-    if ((threadIdx.x & 31) == 0)
-        for (int i = 0; i < 3; ++i)
-            if (v[i]) atomicAdd(&s_c[i], v[i]);
+    if ((threadIdx.x & 31) == 0) {
+        if (c.cand) atomicAdd(&s_c[0], c.cand);
+        if (c.within) atomicAdd(&s_c[1], c.within);
+        if (c.skips) atomicAdd(&s_c[2], c.skips);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         if (s_c[0]) atomicAdd(&stats->pairs_candidate, s_c[0]);
@@ -792,7 +860,7 @@ __device__ __forceinline__ void flush_counts(const PairCounts &c, DevStats *stat
 // Single channel: one warp per 2x2 group of pixels, FP64 throughout: the
 // windows (a ring per lane, four pixels each), every union candidate against
 // the four pixels, normalise. Warp-collective.
-template <bool GEN>
+template <int MODE>
 __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint32_t ny,
                                            const float *__restrict__ data, uint32_t cstride, float *__restrict__ out,
                                            float *__restrict__ wout, uint64_t grp, GroupShared &S, PairCounts &pc) {
@@ -810,11 +878,12 @@ __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint3
             nr = G.r1 - G.r0 + 1;
             group_lane_windows(a, G, G.r0 + rb + lane, pix0, nx, lo, hi, ref, skips);
         }
-        group_rounds<false, GEN ? kPairOther : kPairGeneral>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u, [&](uint32_t idx, uint32_t, const double w[4], const float[4]) {
+        group_rounds<false, MODE>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u,
+                                  [&](uint32_t idx, uint32_t, const double w[4], const float[4], const bool nz[4]) {
             const double x = (double)__ldg(data + (uint64_t)idx * cstride);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                if (w[q] != 0.0) {
+                if (nz[q]) {
                     acc[q] += x * w[q];
                     ws[q] += w[q];
                     ++within;
@@ -822,9 +891,7 @@ __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint3
             }
         });
     }
-    pc.cand += ref;
-    pc.within += within;
-    pc.skips += skips;
+    pc.add(ref, within, skips);
     const double A = warp_sum4(acc), W = warp_sum4(ws);
     const int q = lane >> 3;
     if ((lane & 7) == 0 && (!(q & 1) || xin) && (!(q >> 1) || yin)) {
@@ -1074,16 +1141,15 @@ __device__ __forceinline__ void group_tile_item(const GridArgs &a, const GroupAr
             }
             group_rounds<true, MODE>(
                 a, S.px[gl].h, S.px[gl].cb1, S.rec[warp], pix0, g.nx, lo, hi, shift,
-                [&](uint32_t, uint32_t slot, const double w[4], const float wf[4]) {
+                [&](uint32_t, uint32_t slot, const double w[4], const float wf[4], const bool nz[4]) {
                     bool any = false;
                     float e[4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         e[q] = wf[q];
-                        const bool nz = MODE == kPairUnit ? wf[q] != 0.f : w[q] != 0.0;
                         ws[q] += w[q];
-                        any = any || nz;
-                        within += nz;
+                        any = any || nz[q];
+                        within += nz[q];
                     }
                     if (PACK == 1 || (PACK == 2 && g.pack)) {
                         // the four slots carry {hi(w0, w1), lo(w0, w1), hi(w2, w3), lo(w2, w3)}
@@ -1110,7 +1176,7 @@ __device__ __forceinline__ void group_tile_item(const GridArgs &a, const GroupAr
         if ((lane & 7) == 0 && (!(q & 1) || xin) && (!(q >> 1) || yin))
             wsum[pix0 + (q & 1) + (uint64_t)(q >> 1) * g.nx] = W;
     }
-    pc.within += within;
+    pc.add(0, within, 0);
 }
 
 // Exclusive scan of n u32 counts into u64 offsets (out[n] = the total), in

@@ -44,15 +44,15 @@ __global__ void k_noalloc_prep(HpxParams h, uint64_t firstring, uint64_t usedrin
     if (p < npix) prep_item(h, firstring, usedrings, disc, X, Y, prep, stats, p);
 }
 
-template <bool GEN>  // fields whose kernel is not GAUSS1D
-__global__ void __launch_bounds__(kGroupThreads, kGroupCtas) k_noalloc_grid(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+template <int MODE>  // as pair_weights
+__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_noalloc_grid(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
                                                           const float *__restrict__ data, uint32_t cstride,
                                                           float *__restrict__ out, float *__restrict__ wout) {
     __shared__ GroupShared S[kGroupWarps];
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
     const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
-    if (grp < ngroups) grid1_item<GEN>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
+    if (grp < ngroups) grid1_item<MODE>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
     flush_counts(pc, a.stats);
 }
 
@@ -134,12 +134,12 @@ extern "C" hcg_status hcg_grid_noalloc(hcg_context *ctx, const hcg_field *field,
         const GridArgs a = grid_args(field, prep, ctx->d_stats);
         const uint64_t ngroups = (uint64_t)((target->nx + 1) / 2) * ((target->ny + 1) / 2);
         const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
-        if (field->kernel_type == HCG_GAUSS1D)
-            k_noalloc_grid<false><<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride,
-                                                       cube, weights_out);
-        else
-            k_noalloc_grid<true><<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride,
-                                                      cube, weights_out);
+        const int mode = pair_mode1(field, a);
+        auto grid1 = mode == kPairOther ? k_noalloc_grid<kPairOther>
+                     : mode == kPairUnit ? k_noalloc_grid<kPairUnit>
+                                         : k_noalloc_grid<kPairGeneral>;
+        grid1<<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride, cube,
+                                             weights_out);
         cudaEventRecord(ctx->ev1, s);
         if (e == cudaSuccess) e = cudaGetLastError();
     }
