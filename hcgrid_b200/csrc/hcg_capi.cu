@@ -192,9 +192,9 @@ static hcg_status grid_checked(hcg_context *ctx, const hcg_field *field, const h
     cudaError_t e = grid_field(ctx, field, target, dc, layout, dw, engine, why);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "grid", why);
     if (tc || field->nchan > 1) {
-        unsigned long long to = 0;
-        CK(ctx, cudaMemcpyAsync(&to, &ctx->d_stats->timeouts, sizeof(to), cudaMemcpyDeviceToHost, s), "timeouts");
+        CK(ctx, cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, s), "timeouts");
         CK(ctx, cudaStreamSynchronize(s), "grid");
+        const unsigned long long to = ctx->h_stats->timeouts;
         if (to)
             return fail(ctx, HCG_ETIMEOUT, std::to_string(to) + (tc ? " tensor-core" : " FP32 staging") +
                                                 " pipeline waits ran out");
@@ -278,7 +278,8 @@ hcg_status hcg_context_create(int device, void *stream, hcg_context **out) {
         if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
         c->copy_stream = nullptr;
     }
-    if (cudaMalloc(&c->d_stats, sizeof(DevStats)) != cudaSuccess || cudaMemset(c->d_stats, 0, sizeof(DevStats)) ||
+    if (cudaMalloc(&c->d_stats, sizeof(DevStats)) != cudaSuccess ||
+        cudaMallocHost(&c->h_stats, sizeof(DevStats)) != cudaSuccess || cudaMemset(c->d_stats, 0, sizeof(DevStats)) ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaEventCreate(&c->evp[0]) != cudaSuccess || cudaEventCreate(&c->evp[1]) != cudaSuccess ||
         cudaEventCreate(&c->evp[2]) != cudaSuccess || cudaEventCreate(&c->evp[3]) != cudaSuccess) {
@@ -299,6 +300,7 @@ static void ctx_teardown(hcg_context *ctx) {
     ctx->scratch.release(ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->d_stats);
+    cudaFreeHost(ctx->h_stats);
     cudaEventDestroy(ctx->ev0);
     cudaEventDestroy(ctx->ev1);
     for (auto &ev : ctx->evp) cudaEventDestroy(ev);

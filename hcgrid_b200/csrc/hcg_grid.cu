@@ -72,12 +72,9 @@ __global__ void __launch_bounds__(kWeightThreads, MODE == kPairUnit ? kWeightCta
     flush_counts(pc, a.stats);
 }
 
-// Candidate counts of the groups whose tile's ring span exceeds the tile
-// table; a few resident blocks, which return at once when no tile does.
-__global__ void __launch_bounds__(kGroupThreads) k_group_count(GridArgs a, GroupArgs g, uint32_t *__restrict__ cap,
-                                                     const unsigned long long *__restrict__ overflow) {
+// Candidate counts of the groups whose tile's ring span exceeds the tile table.
+__global__ void __launch_bounds__(kGroupThreads) k_group_count(GridArgs a, GroupArgs g, uint32_t *__restrict__ cap) {
     __shared__ GroupShared S[kGroupWarps];
-    if (*overflow == 0) return;
     const int warp = threadIdx.x >> 5;
     for (uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp; grp < g.ngroups; grp += gridDim.x * (uint64_t)kGroupWarps)
         group_count_item(a, g, cap, grp, S[warp]);
@@ -189,7 +186,10 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
     cudaStream_t s = ctx->stream;
     cudaError_t e = cudaSuccess;
     const uint64_t P = (uint64_t)t->nx * t->ny;
-    if ((e = cudaMemsetAsync(&ctx->d_stats->timeouts, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
+    // the counters of this grid pass: overflow, timeouts, tc_macs, ustat, entries
+    if ((e = cudaMemsetAsync(&ctx->d_stats->overflow, 0, sizeof(DevStats) - offsetof(DevStats, overflow), s)) !=
+        cudaSuccess)
+        return e;
     PixPrep *prep = (PixPrep *)ctx->scratch.get(0, P * sizeof(PixPrep), s, e);
     if (e != cudaSuccess) return e;
     cudaEventRecord(ctx->ev0, s);
@@ -237,11 +237,6 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         T.ulo = (uint32_t *)ctx->scratch.get(11, ntiles * kTileMaxRings * sizeof(uint32_t), s, e);
         T.base = (uint32_t *)ctx->scratch.get(12, ntiles * (kTileMaxRings + 1) * sizeof(uint32_t), s, e);
         T.ring_idx = (uint16_t *)ctx->scratch.get(14, ntiles * kTileMaxSpan * sizeof(uint16_t), s, e);
-        unsigned long long *rowoff =
-            (unsigned long long *)ctx->scratch.get(13, (T.nty + 4) * sizeof(unsigned long long), s, e);
-        const uint32_t parts = (uint32_t)std::min<uint64_t>(1024, (g.ngroups + 4095) / 4096 + 1);
-        unsigned long long *psum =
-            (unsigned long long *)ctx->scratch.get(15, (parts + 1) * sizeof(unsigned long long), s, e);
         T.cap = cap;  // the tile pass counts each group's candidates
         {
             // the tile pass keeps each group's windows for the weight pass (up to 4 GiB of them)
@@ -256,56 +251,68 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         T.overflow = &ctx->d_stats->overflow;
         T.pad = tc ? 8 : 1;  // the tensor-core engine loads ring runs as boxes of 8 samples
         T.ustat = ctx->d_stats->ustat;
+        T.off = off;
+        T.entries = &ctx->d_stats->entries;
         if (e != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(T.overflow, 0, 3 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(T.ustat, 0, 2 * sizeof(unsigned long long), s)) != cudaSuccess) return e;
         if (ntiles <= 148 * 4)
             k_tile_rings<8><<<(unsigned)ntiles, 256, 0, s>>>(a, g, T);
         else
             k_tile_rings<4><<<(unsigned)ntiles, 128, 0, s>>>(a, g, T);
-        // groups of tiles whose ring span exceeds the table (cap unknown) are counted here
-        k_group_count<<<std::min(gblocks, 148u * 3), kGroupThreads, 0, s>>>(a, g, cap, T.overflow);
-        k_scan_sums<<<parts, kScanThreads, 0, s>>>(cap, g.ngroups, parts, psum);
-        k_scan_psum<<<1, kScanThreads, 0, s>>>(psum, parts);
-        k_scan_apply<<<parts, kScanThreads, 0, s>>>(cap, g.ngroups, parts, psum, off);
-        // entry offsets at tile-row boundaries: the work is split into runs of
-        // tile rows whose entries fit the context's entry budget
-        const uint64_t groups_per_row = (uint64_t)(kTileY / 2) * g.gx;
-        k_row_offsets<<<(T.nty + 1 + 255) / 256, 256, 0, s>>>(off, g.ngroups, groups_per_row, T.nty, rowoff);
-        if ((e = cudaMemcpyAsync(rowoff + T.nty + 1, T.overflow, sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
-                                 s)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(rowoff + T.nty + 2, T.ustat, 2 * sizeof(unsigned long long),
-                                 cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-            return e;
         cudaEventRecord(ctx->evp[1], s);
-        std::vector<unsigned long long> ro(T.nty + 4);
-        if ((e = cudaMemcpyAsync(ro.data(), rowoff, ro.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                 s)) != cudaSuccess)
+        if ((e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, s)) !=
+                cudaSuccess ||
+            (e = cudaStreamSynchronize(s)) != cudaSuccess)
             return e;
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-        const bool tiled = ro[T.nty + 1] == 0;  // every tile's ring span fits the tile table
+        const DevStats tp = *ctx->h_stats;
+        const unsigned long long budget = ctx->entry_budget / (sizeof(uint32_t) + sizeof(float4));
+        const uint64_t groups_per_row = (uint64_t)(kTileY / 2) * g.gx;
+        // The entries lie in the order the tile pass counted them when they fit
+        // the entry budget; else, and with tiles beyond the ring table (whose
+        // groups are counted now), the groups' counts are scanned and the work is
+        // split into runs of tile rows that fit it.
+        std::vector<unsigned long long> ro(T.nty + 1, 0);
+        ro[T.nty] = tp.entries;
+        const bool whole = tp.overflow == 0 && tp.entries <= budget;
+        if (!whole) {
+            unsigned long long *rowoff =
+                (unsigned long long *)ctx->scratch.get(13, (T.nty + 1) * sizeof(unsigned long long), s, e);
+            const uint32_t parts = (uint32_t)std::min<uint64_t>(1024, (g.ngroups + 4095) / 4096 + 1);
+            unsigned long long *psum =
+                (unsigned long long *)ctx->scratch.get(15, (parts + 1) * sizeof(unsigned long long), s, e);
+            if (e != cudaSuccess) return e;
+            if (tp.overflow) k_group_count<<<std::min(gblocks, 148u * 3), kGroupThreads, 0, s>>>(a, g, cap);
+            k_scan_sums<<<parts, kScanThreads, 0, s>>>(cap, g.ngroups, parts, psum);
+            k_scan_psum<<<1, kScanThreads, 0, s>>>(psum, parts);
+            k_scan_apply<<<parts, kScanThreads, 0, s>>>(cap, g.ngroups, parts, psum, off);
+            k_row_offsets<<<(T.nty + 1 + 255) / 256, 256, 0, s>>>(off, g.ngroups, groups_per_row, T.nty, rowoff);
+            if ((e = cudaMemcpyAsync(ro.data(), rowoff, ro.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                     s)) != cudaSuccess ||
+                (e = cudaStreamSynchronize(s)) != cudaSuccess)
+                return e;
+        }
+        const bool tiled = tp.overflow == 0;  // every tile's ring span fits the tile table
         if (tc && !tiled && !f->d_spec) {
             why = "a tile spans more than " + std::to_string(kTileMaxSpan) + " rings or holds samples in more than " +
                   std::to_string(kTileMaxRings) + ": the FP32 fallback needs the FP32 spectra";
             return cudaErrorInvalidValue;
         }
         const uint32_t ostride = layout == HCG_LAYOUT_CHANNEL_MAJOR ? 0 : f->nchan;  // 0: [channel][pixel]
-        if (tc && tiled && tc_use_weights(ctx, f, ro[T.nty + 2], ro[T.nty], ntiles)) {
+        if (tc && tiled && tc_use_weights(ctx, f, tp.ustat[0], ro[T.nty], ntiles)) {
             // dense tiles: the tensor-core kernel evaluates the weights itself (no entries)
             cudaEventRecord(ctx->evp[2], s);
             if ((e = tc_weights(ctx, f, a, g, T, ntiles, d_cube, ostride, d_wts, why)) != cudaSuccess) return e;
             cudaEventRecord(ctx->ev1, s);
             return cudaGetLastError();
         }
-        const unsigned long long budget = ctx->entry_budget / (sizeof(uint32_t) + sizeof(float4));
         std::vector<std::pair<uint32_t, uint32_t>> chunks;
-        unsigned long long most = 1;
+        unsigned long long most = whole ? std::max(tp.entries, 1ULL) : 1;
         for (uint32_t ra = 0; ra < T.nty;) {
             uint32_t rb = ra + 1;
             // a run fits the entry budget and the 65535 limit of the grid's y dimension
-            while (rb < T.nty && ro[rb + 1] - ro[ra] <= budget && (uint64_t)(rb + 1 - ra) * T.ntx <= 65535) ++rb;
+            while (rb < T.nty && (whole || ro[rb + 1] - ro[ra] <= budget) && (uint64_t)(rb + 1 - ra) * T.ntx <= 65535)
+                ++rb;
             chunks.push_back({ra, rb});
-            most = std::max(most, ro[rb] - ro[ra]);
+            if (!whole) most = std::max(most, ro[rb] - ro[ra]);
             ra = rb;
         }
         uint32_t *e_idx = (uint32_t *)ctx->scratch.get(5, (most + 1) * sizeof(uint32_t), s, e);
@@ -332,7 +339,7 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
             }
             gc.g0 = std::min<uint64_t>((uint64_t)ch.first * groups_per_row, g.ngroups);
             gc.g1 = std::min<uint64_t>((uint64_t)ch.second * groups_per_row, g.ngroups);
-            gc.ebase = ro[ch.first];
+            gc.ebase = whole ? 0 : ro[ch.first];
             if (gc.g1 <= gc.g0) continue;
             unsigned cb = (unsigned)((gc.g1 - gc.g0 + 7) / 8), gb = (ch.second - ch.first) * T.ntx;
             TileArgs tt = T;
@@ -353,7 +360,7 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
                 TileArgs Tc = T;
                 Tc.t0 = (uint64_t)ch.first * T.ntx;
                 e = tc_accum(ctx, f, gc, Tc, (uint64_t)(ch.second - ch.first) * T.ntx, off, cnt, e_idx, e_w, wsum, dst,
-                             ostride, d_wts, ro[T.nty + 3], why);
+                             ostride, d_wts, tp.ustat[1], why);
                 if (e != cudaSuccess) return e;
             } else if (tiled) {
                 TileArgs Tc = T;

@@ -25,6 +25,7 @@ struct DevStats {
     unsigned long long timeouts;  // bounded device waits that ran out (tensor-core engine)
     unsigned long long tc_macs;   // tensor-core multiply-adds issued (tensor-core engine)
     unsigned long long ustat[2];  // staged slots of all tiles and of the largest (tile pass)
+    unsigned long long entries;   // union candidates of the tiles' groups (tile pass)
 };
 
 // One HEALPix ring that holds samples, with the ring half of loc2pix
@@ -136,6 +137,7 @@ struct hcg_context {
     double last_r = -1, last_res = -1;
     hcg::HpxParams hpx = {};
     hcg::DevStats *d_stats = nullptr;
+    hcg::DevStats *h_stats = nullptr;  // page-locked: the counters as a call reads them back
     hcg::Scratch scratch;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t evp[4] = {nullptr, nullptr, nullptr, nullptr};  // phase boundaries inside hcg_grid

@@ -972,6 +972,8 @@ struct TileArgs {
     uint4 *win;                // [tile][kWinSpan][kTileGroups][2]: the group's 4 pixel windows per ring (or null)
     unsigned long long *overflow;  // tiles beyond the ring table (their groups are counted by group_count_item)
     uint32_t pad;  // ring runs take a multiple of `pad` slots (> 1: the tensor-core engine's 8-row boxes)
+    unsigned long long *off;    // entry offset of each group, from the tile pass (or null: scanned later)
+    unsigned long long *entries;  // with off: entries handed out so far
     unsigned long long *ustat;  // [0]: sum, [1]: largest of the tiles' staged slots U (or null)
 };
 
@@ -1388,7 +1390,22 @@ __device__ __forceinline__ void tile_rings_item(const GridArgs &a, const GroupAr
         const uint32_t gxi = (uint32_t)(tile % T.ntx) * (kTileX / 2) + tid % (kTileX / 2);
         const uint32_t gyi = (uint32_t)(tile / T.ntx) * (kTileY / 2) + tid / (kTileX / 2);
         const uint64_t grp = (uint64_t)gyi * g.gx + gxi;
-        if (gxi < g.gx && grp < g.ngroups) T.cap[grp] = known ? s_cnt[tid] : kCapUnknown;
+        const bool in = gxi < g.gx && grp < g.ngroups;
+        if (in) T.cap[grp] = known ? s_cnt[tid] : kCapUnknown;
+        if (T.off && known) {
+            // the tile's place among the entries, in the order the tiles come:
+            // one atomic a tile instead of a scan of all groups (four launches)
+            uint32_t incl = in ? s_cnt[tid] : 0u;
+            const uint32_t mine_n = incl;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            unsigned long long first = 0;
+            if (lane == 31) first = atomicAdd(T.entries, (unsigned long long)incl);
+            first = __shfl_sync(0xffffffffu, first, 31);
+            if (in) T.off[grp] = first + incl - mine_n;
+        }
     };
     // a span beyond the table keeps no windows and no unions; its groups are
     // counted later, its candidate statistic is taken here all the same
