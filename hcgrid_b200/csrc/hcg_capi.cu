@@ -77,8 +77,7 @@ void release_field(hcg_field *f, cudaStream_t s) {
     if (f->d_spec) cudaFreeAsync(f->d_spec, s);
     free_split(f, s);
     if (f->geom_refs && --*f->geom_refs > 0) return;
-    void *ps[] = {f->d_keys, f->d_perm, f->d_inv, f->d_l2,    f->d_b2,
-                  f->d_cb2,  f->d_w,    f->d_half, f->d_lut, f->d_rings, f->d_rwin, f->d_ptab};
+    void *ps[] = {f->d_samples, f->d_ringmem, f->d_ptab};
     for (void *p : ps)
         if (p) cudaFreeAsync(p, s);
     delete f->geom_refs;
@@ -279,7 +278,7 @@ hcg_status hcg_context_create(int device, void *stream, hcg_context **out) {
         c->copy_stream = nullptr;
     }
     if (cudaMalloc(&c->d_stats, sizeof(DevStats)) != cudaSuccess ||
-        cudaMallocHost(&c->h_stats, sizeof(DevStats)) != cudaSuccess || cudaMemset(c->d_stats, 0, sizeof(DevStats)) ||
+        cudaMallocHost(&c->h_stats, kHostBack) != cudaSuccess || cudaMemset(c->d_stats, 0, sizeof(DevStats)) ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaEventCreate(&c->evp[0]) != cudaSuccess || cudaEventCreate(&c->evp[1]) != cudaSuccess ||
         cudaEventCreate(&c->evp[2]) != cudaSuccess || cudaEventCreate(&c->evp[3]) != cudaSuccess) {

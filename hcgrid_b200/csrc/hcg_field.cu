@@ -33,12 +33,12 @@ struct KeyRange {
 // samples) held the kernel at 175 us.
 __global__ void __launch_bounds__(256) k_sample_keys(HpxParams h, uint64_t n, const double *__restrict__ lon,
                                                      const double *__restrict__ lat, uint64_t *__restrict__ keys,
-                                                     KeyRange *range, DevStats *stats) {
+                                                     KeyRange *range, unsigned long long *invalid, DevStats *stats) {
     __shared__ unsigned long long s_nmin[8], s_kmax[8];
     unsigned long long nmin = 0, kmax = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const double lo = lon[i], la = lat[i];
-        if (!isfinite(lo) || !isfinite(la) || fabs(la) > 90.0) atomicAdd(&stats->invalid_input, 1ULL);
+        if (!isfinite(lo) || !isfinite(la) || fabs(la) > 90.0) atomicAdd(invalid, 1ULL);
         const double theta = dsub(kHalfPi, dmul(kDeg2Rad, la));
         const double phi = dmul(kDeg2Rad, lo);
         int hard;
@@ -688,40 +688,69 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     cudaStream_t s = ctx->stream;
     const uint64_t n = f->n;
     cudaError_t e;
-    uint64_t *k0 = nullptr, *k1 = nullptr;
-    uint32_t *v0 = nullptr, *hist = nullptr, *perm = nullptr;
-    // device words read back: the keys' range, then the pixel tables' total and the largest weight
+    uint64_t *k0 = nullptr;  // the samples' keys, then the words read back (one allocation)
+    uint32_t *v0 = nullptr;  // the sort's buffers
+    uint8_t *mem = nullptr;
+    // device words read back: the keys' range and invalid samples, then the pixel tables' total and the largest weight
     struct Back {
         KeyRange range;
-        unsigned long long total, wbits;
+        unsigned long long invalid, total, wbits;
     };
-    Back *back = nullptr;
-    Back hb{};
+    static_assert(sizeof(Back) <= kHostBack, "read back through the context's page-locked buffer");
+    Back *back = nullptr, *hb = reinterpret_cast<Back *>(ctx->h_stats);
     RingAcc *acc = nullptr;
+    // the next `count` elements of an allocation, 256-byte aligned; with a null
+    // `at` only the offset advances
+    size_t used = 0;
+    auto carve = [&](auto *&p, uint64_t count) {
+        using E = std::remove_reference_t<decltype(*p)>;
+        used = (used + 255) & ~(size_t)255;
+        p = reinterpret_cast<E *>(mem + used);
+        used += count * sizeof(E);
+    };
+    auto samples = [&]() {
+        used = 0;
+        carve(f->d_keys, n + 1);
+        carve(f->d_l2, n);
+        carve(f->d_b2, n);
+        carve(f->d_cb2, n);
+        carve(f->d_w, n);
+        carve(f->d_half, 2 * n);
+        carve(f->d_perm, n);
+        carve(f->d_inv, n);
+    };
+    auto ringmem = [&]() {
+        used = 0;
+        carve(f->d_rings, f->usedrings);
+        carve(f->d_rwin, f->usedrings);
+        carve(acc, f->usedrings);
+        carve(f->d_lut, f->usedrings + 1);
+    };
+    const size_t key_bytes = ((n + 1) * sizeof(uint64_t) + 255) & ~(size_t)255;
 #define TRY(x)                         \
     do {                               \
         e = (x);                       \
         if (e != cudaSuccess) goto fail; \
     } while (0)
-    TRY(dalloc(&k0, (n + 1) * sizeof(uint64_t), s, ctx->pool));
-    TRY(dalloc(&k1, (n + 1) * sizeof(uint64_t), s, ctx->pool));
-    TRY(dalloc(&perm, n * sizeof(uint32_t), s, ctx->pool));
-    TRY(dalloc(&back, sizeof(Back), s, ctx->pool));
-    TRY(cudaMemsetAsync(&ctx->d_stats->invalid_input, 0, sizeof(unsigned long long), s));
+    samples();
+    TRY(dalloc(&f->d_samples, used, s, ctx->pool));
+    mem = static_cast<uint8_t *>(f->d_samples);
+    samples();
+    TRY(dalloc(&k0, key_bytes + sizeof(Back), s, ctx->pool));
+    back = reinterpret_cast<Back *>(reinterpret_cast<uint8_t *>(k0) + key_bytes);
     TRY(cudaMemsetAsync(back, 0, sizeof(Back), s));
-    k_sample_keys<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(f->hpx, n, d_lon, d_lat, k0, &back->range, ctx->d_stats);
+    k_sample_keys<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(
+        f->hpx, n, d_lon, d_lat, k0, &back->range, &back->invalid, ctx->d_stats);
     TRY(cudaGetLastError());
     {
-        unsigned long long invalid = 0;
-        TRY(cudaMemcpyAsync(&hb, back, sizeof hb, cudaMemcpyDeviceToHost, s));
-        TRY(cudaMemcpyAsync(&invalid, &ctx->d_stats->invalid_input, sizeof invalid, cudaMemcpyDeviceToHost, s));
+        TRY(cudaMemcpyAsync(hb, back, sizeof *hb, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
-        if (invalid) {
-            why = "non-finite coordinates or |lat| > 90 in " + std::to_string(invalid) + " samples";
+        if (hb->invalid) {
+            why = "non-finite coordinates or |lat| > 90 in " + std::to_string(hb->invalid) + " samples";
             e = cudaErrorInvalidValue;
             goto fail;
         }
-        const uint64_t kmin = ~hb.range.nmin, kmax = hb.range.kmax;
+        const uint64_t kmin = ~hb->range.nmin, kmax = hb->range.kmax;
         f->firstring = pix2ring(f->hpx, kmin);
         f->usedrings = 1 + pix2ring(f->hpx, kmax) - f->firstring;
         const uint64_t span_bits = 64 - (kmax == kmin ? 64 : __builtin_clzll(kmax - kmin));
@@ -729,7 +758,7 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         const bool wide = span_bits > 32;
         if (n <= kSmallSort && !wide) {
             TRY(cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
-            k_sort_small<<<1, kSmallThreads, kSmallSmem, s>>>(k0, k1, perm, (uint32_t)n, passes, kmin);
+            k_sort_small<<<1, kSmallThreads, kSmallSmem, s>>>(k0, f->d_keys, f->d_perm, (uint32_t)n, passes, kmin);
             TRY(cudaGetLastError());
         } else {
             // tiles of 16 x 256 keys write the longest runs; below about two
@@ -737,10 +766,13 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
             const bool small = n < (1u << 20);
             const size_t word = wide ? 8 : 4, tile = kSortThreads * (wide ? 8 : small ? 4 : 16);
             const size_t nblocks = (n + std::min<size_t>(tile, kSortThreads * 8) - 1) / std::min<size_t>(tile, kSortThreads * 8);
-            TRY(dalloc(&v0, 2 * n * (word + 4) + 16, s, ctx->pool));
-            TRY(dalloc(&hist, 256 * nblocks * sizeof(uint32_t) + 8 * 256 * sizeof(unsigned long long), s, ctx->pool));
-            unsigned long long *total = (unsigned long long *)hist;
+            const size_t pairs = (2 * n * (word + 4) + 255) & ~(size_t)255;
+            TRY(dalloc(&v0, pairs + 256 * nblocks * sizeof(uint32_t) + 8 * 256 * sizeof(unsigned long long), s,
+                       ctx->pool));
+            unsigned long long *total = (unsigned long long *)((uint8_t *)v0 + pairs);
             uint32_t *counts = (uint32_t *)(total + 8 * 256), *va = v0 + 2 * n * (word / 4), *vb = va + n;
+            uint64_t *const k1 = f->d_keys;
+            uint32_t *const perm = f->d_perm;
             TRY(cudaMemsetAsync(total, 0, passes * 256 * sizeof(unsigned long long), s));
             if (wide)
                 TRY((sort_passes<uint64_t, 8>(k0, n, passes, kmin, (uint64_t *)v0, (uint64_t *)v0 + n, va, vb, k1,
@@ -751,20 +783,11 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
                 TRY((sort_passes<uint32_t, 16>(k0, n, passes, kmin, v0, v0 + n, va, vb, k1, perm, counts, total, s)));
         }
     }
-    std::swap(k0, k1);
-    f->d_keys = k0;
-    f->d_perm = perm;
-    k0 = nullptr;
-    perm = nullptr;
-    TRY(dalloc(&f->d_lut, (f->usedrings + 1) * sizeof(uint32_t), s, ctx->pool));
-    TRY(dalloc(&f->d_rings, f->usedrings * sizeof(RingRec), s, ctx->pool));
-    TRY(dalloc(&f->d_l2, n * sizeof(double), s, ctx->pool));
-    TRY(dalloc(&f->d_b2, n * sizeof(double), s, ctx->pool));
-    TRY(dalloc(&f->d_cb2, n * sizeof(double), s, ctx->pool));
-    TRY(dalloc(&f->d_half, 2 * n * sizeof(double2), s, ctx->pool));
-    TRY(dalloc(&f->d_w, n * sizeof(double), s, ctx->pool));
-    TRY(dalloc(&f->d_inv, n * sizeof(uint32_t), s, ctx->pool));
-    TRY(dalloc(&acc, f->usedrings * sizeof(RingAcc), s, ctx->pool));
+    mem = nullptr;
+    ringmem();
+    TRY(dalloc(&f->d_ringmem, used, s, ctx->pool));
+    mem = static_cast<uint8_t *>(f->d_ringmem);
+    ringmem();
     TRY(cudaMemsetAsync(acc, 0, f->usedrings * sizeof(RingAcc), s));
     {
         const unsigned rblocks = (unsigned)((f->usedrings + 255) / 256), nblk = (unsigned)((n + 255) / 256);
@@ -775,38 +798,33 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
                                              ctx->d_stats);
         k_ring_offsets<<<1, 1024, 0, s>>>(f->d_rings, f->usedrings, &back->total);
         TRY(cudaGetLastError());
-        TRY(cudaMemcpyAsync(&hb, back, sizeof hb, cudaMemcpyDeviceToHost, s));
+        TRY(cudaMemcpyAsync(hb, back, sizeof *hb, cudaMemcpyDeviceToHost, s));
         TRY(cudaStreamSynchronize(s));
         f->wmax = 1.0;
         f->unit_w = d_w == nullptr;
-        if (d_w) memcpy(&f->wmax, &hb.wbits, sizeof hb.wbits);
+        if (d_w) memcpy(&f->wmax, &hb->wbits, sizeof hb->wbits);
         // Pixel tables: one u32 per HEALPix pixel between the first and last
         // sample of each ring and one more, when they fit in max(2^24, 4n)
         // entries (HCG_RING_TABLE_MAX overrides; 0 keeps the binary searches).
         uint64_t cap = std::max<uint64_t>(1ull << 24, 4 * n);
         if (const char *v = getenv("HCG_RING_TABLE_MAX")) cap = strtoull(v, nullptr, 10);
-        if (hb.total > 0 && hb.total <= cap &&
-            dalloc(&f->d_ptab, hb.total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess) {
+        if (hb->total > 0 && hb->total <= cap &&
+            dalloc(&f->d_ptab, hb->total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess) {
             k_ring_ptab<<<nblk, 256, 0, s>>>(f->hpx, n, f->firstring, f->d_rings, f->d_keys, f->d_ptab);
             if (f->hpx.order <= kQuickOrder) {
-                TRY(dalloc(&f->d_rwin, f->usedrings * sizeof(RingWin), s, ctx->pool));
                 k_ring_windows<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_rings, f->d_rwin);
             }
         } else {
             cudaGetLastError();
             k_ring_no_tables<<<rblocks, 256, 0, s>>>(f->d_rings, f->usedrings);
         }
+        if (!f->d_ptab || f->hpx.order > kQuickOrder) f->d_rwin = nullptr;  // the general windows
         TRY(cudaGetLastError());
-        f->ptab_entries = f->d_ptab ? hb.total : 0;
+        f->ptab_entries = f->d_ptab ? hb->total : 0;
     }
 fail:
-    if (acc) cudaFreeAsync(acc, s);
     if (k0) cudaFreeAsync(k0, s);
-    if (k1) cudaFreeAsync(k1, s);
     if (v0) cudaFreeAsync(v0, s);
-    if (perm) cudaFreeAsync(perm, s);
-    if (hist) cudaFreeAsync(hist, s);
-    if (back) cudaFreeAsync(back, s);
 #undef TRY
     return e;
 }

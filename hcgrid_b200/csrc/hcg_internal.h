@@ -94,6 +94,9 @@ struct PixPrep {
     float icb1;            // >= 1 / cb1 (chord windows)
 };
 
+constexpr size_t kHostBack = 256;
+static_assert(sizeof(DevStats) <= kHostBack, "the read-back buffer holds the counters");
+
 // Stream-ordered allocation from a context's memory pool. The pool keeps
 // freed memory mapped (release threshold: never), so the multi-GB buffers of
 // one call are reused by the next instead of being unmapped at every
@@ -137,7 +140,7 @@ struct hcg_context {
     double last_r = -1, last_res = -1;
     hcg::HpxParams hpx = {};
     hcg::DevStats *d_stats = nullptr;
-    hcg::DevStats *h_stats = nullptr;  // page-locked: the counters as a call reads them back
+    hcg::DevStats *h_stats = nullptr;  // page-locked (kHostBack bytes): what a call reads back
     hcg::Scratch scratch;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t evp[4] = {nullptr, nullptr, nullptr, nullptr};  // phase boundaries inside hcg_grid
@@ -166,6 +169,8 @@ struct hcg_field {
     bool unit_w = true;   // no per-sample weights were given: all 1
     double wbound = 1.0;  // bound of |weight| of an accepted pair: wmax * the kernel's bound
     uint64_t firstring = 0, usedrings = 0;
+    // the geometry below lies in three allocations: per sample, per ring, pixel tables
+    void *d_samples = nullptr, *d_ringmem = nullptr;
     uint64_t *d_keys = nullptr;   // n + 1, sorted, sentinel npix
     uint32_t *d_perm = nullptr;   // sorted position -> input index
     uint32_t *d_inv = nullptr;    // input index -> sorted position
