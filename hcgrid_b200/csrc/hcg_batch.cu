@@ -484,10 +484,7 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
         if (tc) {
             d.T.pad = 8;  // ring runs as boxes of 8 samples
             d.tc_shape = (uint32_t)kb_shape_of(ctx, f);
-            if (!tc_prepare_job(f, (int)kKbNb[d.tc_shape], &B.h_maps[2 * i], d.tc)) {
-                why = "cuTensorMapEncodeTiled";
-                return cudaErrorInvalidValue;
-            }
+            tc_job_fields(f, (int)kKbNb[d.tc_shape], d.tc);  // the maps follow while the geometry runs
             d.g.pack = 1;  // the tensor-core builders take packed hi/lo weights
             d.g.fmt = d.tc.fmt;
             d.g.wscale = d.tc.wscale;
@@ -599,9 +596,6 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
             if (d.tc.nb) {
                 TcJob &c = d.tc;
                 c.map = B.d_maps + 2 * i;
-                c.out_map = tc_out_map(&B.h_maps[2 * i + 1], d.out, d.ostride, d.g.nx, d.g.ny, c.nchan, c.nb)
-                                ? B.d_maps + 2 * i + 1
-                                : nullptr;
                 c.g = d.g;
                 c.T = d.T;
                 c.off = d.off;
@@ -641,11 +635,6 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
         (e = cudaMemsetAsync(B.d_jovf, 0, njobs * sizeof(unsigned long long), s)) != cudaSuccess ||
         (e = cudaMemsetAsync(B.d_jusum, 0, 2 * njobs * sizeof(unsigned long long), s)) != cudaSuccess)
         return e;
-    if (tcn && ((e = cudaMemcpyAsync(B.d_maps, B.h_maps, 2 * njobs * sizeof(CUtensorMap), cudaMemcpyHostToDevice,
-                                     s)) != cudaSuccess ||
-                (e = cudaMemcpyAsync(B.d_tclist, B.h_tclist, tc_off[kKbShapes] * sizeof(uint32_t),
-                                     cudaMemcpyHostToDevice, s)) != cudaSuccess))
-        return e;
     if (!B.exec_geom && (e = capture(ctx, B)) != cudaSuccess) return e;
     // geometry graph, then the entry totals of every job
     cudaEventRecord(ctx->ev0, s);
@@ -658,6 +647,29 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
         (e = cudaMemcpyAsync(B.h_jusum, B.d_jusum, 2 * njobs * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                              s)) != cudaSuccess)
         return e;
+    if (tcn) {
+        // The tensor maps (a driver call each, two a job) are only read by the
+        // sums: encoded while the geometry graph runs
+        bool ok = true;
+        for (uint32_t i = 0; i < njobs && ok; ++i) {
+            TcJob &c = J[i].tc;
+            if (!c.nb) continue;
+            ok = tc_job_map(jobs[i].field, c, &B.h_maps[2 * i]);
+            c.out_map = tc_out_map(&B.h_maps[2 * i + 1], J[i].out, J[i].ostride, J[i].g.nx, J[i].g.ny, c.nchan, c.nb)
+                            ? B.d_maps + 2 * i + 1
+                            : nullptr;
+        }
+        if (!ok) {
+            cudaStreamSynchronize(s);  // nothing queued outlives the call's buffers
+            why = "cuTensorMapEncodeTiled";
+            return cudaErrorInvalidValue;
+        }
+        if ((e = cudaMemcpyAsync(B.d_maps, B.h_maps, 2 * njobs * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s)) !=
+                cudaSuccess ||
+            (e = cudaMemcpyAsync(B.d_tclist, B.h_tclist, tc_off[kKbShapes] * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                                 s)) != cudaSuccess)
+            return e;
+    }
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
     // Routing: jobs whose tiles overflowed the ring table, tensor-core jobs
     // with dense tiles (the single-job kernel evaluates their weights itself)

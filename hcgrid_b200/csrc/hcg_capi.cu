@@ -949,7 +949,7 @@ hcg_status hcg_autotune_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *j
         hcg_batch_tuning t = {};
         t.channel_class = cls;
         t.jobs = (uint32_t)by[cls].size();
-        t.shape = kKbDefaultShape;
+        t.shape = 0;
         for (int sh = 0; sh < kKbShapes; ++sh) {
             {
                 Guard g(ctx);

@@ -215,7 +215,11 @@ constexpr uint64_t kBatchMaxPixels = 1ull << 20;  // larger targets skip hcg_gri
 //   2: 128 x 64 x 3                         3: 64 x 64 x 4
 constexpr int kKbShapes = 4;
 constexpr uint32_t kKbNb[kKbShapes] = {4, 4, 2, 1};
-constexpr int kKbDefaultShape = 0;
+// Default shape by channel class: the narrowest that holds the channels of one
+// or two 64-channel blocks (64 jobs of 10,000 samples on 64 x 64 pixels: 64
+// channels 869 us with shape 3, 936 with 0; 128 channels 911 with shape 2, 961
+// with 0), 256-channel items above (256 channels 1022 with 0, 1194 with 2).
+constexpr int kKbDefaultShape[3] = {3, 2, 0};
 // channel class of a split field: 64-channel blocks 1, 2, 3-4, 5-8, ... -> 0, 1, 2, 3, ...
 inline int tc_class_of(uint32_t cpad) {
     const uint32_t b = cpad / 64;
@@ -235,8 +239,8 @@ inline bool tc_weights_fit(const hcg_field *f) { return f->wbound <= 0x1p100; }
 inline bool fp32_weights_fit(const hcg_field *f) { return f->nchan <= 1 || !(f->wbound > 0x1p100); }
 // the batch engine's tensor-core shape for a split field's channel class
 inline int kb_shape_of(const hcg_context *ctx, const hcg_field *f) {
-    const int c = ctx->kb_shape[tc_class_of(f->xcpad)];
-    return c >= 0 && c < kKbShapes ? c : kKbDefaultShape;
+    const int cls = tc_class_of(f->xcpad), c = ctx->kb_shape[cls];
+    return c >= 0 && c < kKbShapes ? c : kKbDefaultShape[cls < 2 ? cls : 2];
 }
 inline int auto_engine(const hcg_field *f) {
     return (f->xfmt && f->nchan > 1 && f->xnonfinite == 0 && tc_weights_fit(f)) ? f->xfmt : HCG_ENGINE_FP32;

@@ -310,17 +310,24 @@ void tc_entry_format(const hcg_field *f, uint32_t &fmt, float &wscale) {
     wscale = tc_weight_scale(f, fmt != 0);
 }
 
-bool tc_prepare_job(const hcg_field *f, int nb_max, CUtensorMap *map, TcJob &J) {
+void tc_job_fields(const hcg_field *f, int nb_max, TcJob &J) {
     const uint32_t nblk64 = f->xcpad / 64;
     J.nb = nblk64 < (uint32_t)nb_max ? nblk64 : (uint32_t)nb_max;
     J.ncb = (nblk64 + J.nb - 1) / J.nb;
-    if (!make_map(map, f->d_xhi, f->n, f->xcpad, J.nb)) return false;
     J.nchan = f->nchan;
     J.nrows = (uint32_t)f->n;
     J.fmt = f->xfmt == HCG_ENGINE_TC_BF16 ? 1u : 0u;
     J.wscale = tc_weight_scale(f, J.fmt != 0);
     J.inv_scale = f->d_xinv;
-    return true;
+}
+
+bool tc_job_map(const hcg_field *f, const TcJob &J, CUtensorMap *map) {
+    return make_map(map, f->d_xhi, f->n, f->xcpad, J.nb);
+}
+
+bool tc_prepare_job(const hcg_field *f, int nb_max, CUtensorMap *map, TcJob &J) {
+    tc_job_fields(f, nb_max, J);
+    return tc_job_map(f, J, map);
 }
 
 cudaError_t tc_set_smem(const void *kernel, uint32_t bytes) {

@@ -157,7 +157,9 @@ struct TcShared {
 // hcg_tc.cu: the tensor maps and format fields of a field with split
 // spectra (false: the maps could not be encoded); the shared-memory opt-in of
 // a kernel built on tc_item.
-bool tc_prepare_job(const hcg_field *f, int nb_max, CUtensorMap *map, TcJob &J);
+void tc_job_fields(const hcg_field *f, int nb_max, TcJob &J);  // all but the maps
+bool tc_job_map(const hcg_field *f, const TcJob &J, CUtensorMap *map);
+bool tc_prepare_job(const hcg_field *f, int nb_max, CUtensorMap *map, TcJob &J);  // both
 bool tc_out_map(CUtensorMap *m, float *out, uint32_t ostride, uint32_t nx, uint32_t ny, uint32_t nchan, uint32_t nb);
 cudaError_t tc_set_smem(const void *kernel, uint32_t bytes);
 int tc_pick(const hcg_context *ctx, const hcg_field *f);
