@@ -505,6 +505,7 @@ hcg_status hcg_field_share(const hcg_field *src, hcg_field **out) {
     hcg_field *f = new (std::nothrow) hcg_field(*src);
     if (!f) return fail(ctx, HCG_ENOMEM, "host allocation");
     f->d_spec = nullptr;
+    f->amax_set = false;
     f->nchan = f->cstride = 0;
     f->d_xhi = f->d_xlo = nullptr;
     f->d_xinv = nullptr;
@@ -705,6 +706,7 @@ hcg_status hcg_grid_planes(hcg_context *ctx, const hcg_field *geometry, const hc
             fb[b] = new (std::nothrow) hcg_field(*geometry);
             if (!fb[b]) return fail(ctx, HCG_ENOMEM, "host allocation");
             fb[b]->d_spec = nullptr;
+            fb[b]->amax_set = false;
             fb[b]->nchan = fb[b]->cstride = 0;
             fb[b]->d_xhi = fb[b]->d_xlo = nullptr;
             fb[b]->d_xinv = nullptr;

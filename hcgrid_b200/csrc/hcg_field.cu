@@ -618,13 +618,66 @@ inline uint32_t row_threads(uint32_t cstride) {
     return t;
 }
 
-// out[j][0..cstride) = in[perm[j]][0..nchan), zero padded.
+// out[j][0..cstride) = in[perm[j]][0..nchan), zero padded, and the channels'
+// largest finite magnitudes and the count of non-finite values on the way (the
+// split needs them; a pass of its own reads the spectra once more, 90 us for
+// 500,000 x 256). Block (x, y) takes `rows` rows of channels [128 y, 128 y +
+// 128); a thread keeps one channel quad, so its maxima stay in registers and a
+// channel costs one atomic a block.
 __global__ void __launch_bounds__(256) k_permute_rows(uint64_t n, uint32_t nchan, uint32_t cstride, uint32_t tpr,
+                                                      uint32_t rows,
                                                       const uint32_t *__restrict__ perm, const float *__restrict__ in,
-                                                      float *__restrict__ out) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, j = i / tpr;
-    if (j >= n) return;
-    copy_row(in + (uint64_t)__ldg(perm + j) * nchan, out + j * cstride, nchan, cstride, (uint32_t)(i % tpr), tpr);
+                                                      float *__restrict__ out, unsigned int *__restrict__ amax,
+                                                      unsigned long long *__restrict__ nonfinite) {
+    __shared__ uint4 s_m[256];
+    const uint32_t c = blockIdx.y * 128 + 4 * (threadIdx.x % tpr), step = 256 / tpr;
+    const bool vec = (nchan & 3) == 0 && ((uintptr_t)in & 15) == 0;
+    uint32_t m[4] = {0, 0, 0, 0}, bad = 0;
+    if (c < cstride) {
+        const uint64_t j0 = blockIdx.x * (uint64_t)rows, j1 = min(n, j0 + rows);
+        auto row = [&](uint64_t j) {
+            const float *src = in + (uint64_t)__ldg(perm + j) * nchan + c;
+            if (vec) return __ldg(reinterpret_cast<const float4 *>(src));
+            return make_float4(__ldg(src), c + 1 < nchan ? __ldg(src + 1) : 0.f, c + 2 < nchan ? __ldg(src + 2) : 0.f,
+                               c + 3 < nchan ? __ldg(src + 3) : 0.f);
+        };
+        auto put = [&](uint64_t j, const float4 &v) {
+            *reinterpret_cast<float4 *>(out + j * cstride + c) = v;
+            const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t u = __float_as_uint(x[i]) & 0x7fffffffu;
+                const bool fin = u < 0x7f800000u;
+                m[i] = max(m[i], fin ? u : 0u);
+                bad += !fin;
+            }
+        };
+        uint64_t j = j0 + threadIdx.x / tpr;
+        for (; j + 3 * step < j1; j += 4 * step) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = row(j + u * step);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) put(j + u * step, v[u]);
+        }
+        for (; j < j1; j += step) put(j, row(j));
+    }
+    if (nchan == 1) return;  // a single channel is not split
+    s_m[threadIdx.x] = make_uint4(m[0], m[1], m[2], m[3]);
+    if (bad) atomicAdd(nonfinite, (unsigned long long)bad);
+    __syncthreads();
+    if (threadIdx.x < tpr && c < cstride) {
+        for (uint32_t t = threadIdx.x + tpr; t < 256; t += tpr) {
+            const uint4 o = s_m[t];
+            m[0] = max(m[0], o.x);
+            m[1] = max(m[1], o.y);
+            m[2] = max(m[2], o.z);
+            m[3] = max(m[3], o.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (c + i < nchan && m[i]) atomicMax(amax + c + i, m[i]);
+    }
 }
 
 // out[j][c] = in[c][perm[j]]: 32x32 tiles through shared memory.
@@ -842,10 +895,11 @@ cudaError_t upload_spectra(hcg_context *ctx, hcg_field *f, const float *h_in, ui
         f->d_spec = nullptr;
     }
     cudaError_t e = cudaSuccess;
-    if (!f->d_spec) e = dalloc(&f->d_spec, f->n * cstride * sizeof(float), s, ctx->pool);
+    if (!f->d_spec) e = dalloc(&f->d_spec, spec_bytes(f->n, cstride), s, ctx->pool);
     if (e != cudaSuccess) return e;
     f->nchan = nchan;
     f->cstride = cstride;
+    f->amax_set = false;
     const uint64_t n = f->n;
     // chunk geometry: whole input rows (sample-major) or whole planes (channel-major)
     const uint64_t unit = layout == HCG_LAYOUT_SAMPLE_MAJOR ? (uint64_t)nchan * 4 : n * 4;
@@ -899,9 +953,10 @@ cudaError_t upload_plane_block(hcg_context *ctx, hcg_field *f, const float *h_pl
         cudaFreeAsync(f->d_spec, us);
         f->d_spec = nullptr;
     }
-    if (!f->d_spec && (e = dalloc(&f->d_spec, n * cstride * sizeof(float), us, ctx->pool)) != cudaSuccess) return e;
+    if (!f->d_spec && (e = dalloc(&f->d_spec, spec_bytes(n, cstride), us, ctx->pool)) != cudaSuccess) return e;
     f->nchan = nb;
     f->cstride = cstride;
+    f->amax_set = false;
     if (n == 0) return cudaSuccess;
     const uint64_t per = std::max<uint64_t>(1, stage_bytes / (n * 4));
     for (uint64_t u0 = 0; u0 < nb; u0 += per, ++chunks) {
@@ -930,14 +985,23 @@ cudaError_t permute_spectra(hcg_context *ctx, hcg_field *f, const float *d_in, u
         f->d_spec = nullptr;
     }
     cudaError_t e = cudaSuccess;
-    if (!f->d_spec) e = dalloc(&f->d_spec, f->n * cstride * sizeof(float), s, ctx->pool);
+    if (!f->d_spec) e = dalloc(&f->d_spec, spec_bytes(f->n, cstride), s, ctx->pool);
     if (e != cudaSuccess) return e;
     f->nchan = nchan;
     f->cstride = cstride;
+    f->amax_set = false;
     if (layout == HCG_LAYOUT_SAMPLE_MAJOR) {
-        const uint32_t tpr = row_threads(cstride);
-        k_permute_rows<<<(unsigned)((f->n * tpr + 255) / 256), 256, 0, s>>>(f->n, nchan, cstride, tpr, f->d_perm, d_in,
-                                                                            f->d_spec);
+        const SpecMax mx(f->d_spec, f->n, cstride);
+        if (nchan > 1)
+            e = cudaMemsetAsync(mx.amax, 0, cstride * sizeof(float) + 2 * sizeof(unsigned long long), s);
+        if (e != cudaSuccess) return e;
+        // a row a thread up to eight blocks an SM, then longer blocks up to 1024 rows
+        const uint32_t tpr = row_threads(cstride), cblk = (cstride + 127) / 128;
+        const uint32_t rows =
+            (uint32_t)std::max<uint64_t>(256 / tpr, std::min<uint64_t>(1024, f->n * cblk / (148 * 8)));
+        k_permute_rows<<<dim3((unsigned)((f->n + rows - 1) / rows), cblk), 256, 0, s>>>(
+            f->n, nchan, cstride, tpr, rows, f->d_perm, d_in, f->d_spec, mx.amax, mx.bad);
+        f->amax_set = nchan > 1;
     } else {
         dim3 grid((unsigned)((f->n + 31) / 32), (cstride + 31) / 32);
         k_permute_cols<<<grid, dim3(32, 8), 0, s>>>(f->n, nchan, cstride, f->d_perm, d_in, f->d_spec);

@@ -184,7 +184,8 @@ struct hcg_field {
     uint64_t ptab_entries = 0;
     hcg::RingRec *d_rings = nullptr;
     hcg::RingWin *d_rwin = nullptr;  // the rings' window records, or none (no tables, nside > 2^26)
-    float *d_spec = nullptr;      // [n][cstride], sorted
+    float *d_spec = nullptr;      // [n][cstride], sorted (spec_bytes: followed by the channel maxima's words)
+    bool amax_set = false;        // those hold the present spectra's maxima and non-finite count (SpecMax)
     uint32_t nchan = 0, cstride = 0;
     // 16-bit hi/lo split of the sorted spectra for the tensor-core engine
     uint16_t *d_xhi = nullptr, *d_xlo = nullptr;  // [n][xcpad]
@@ -203,6 +204,18 @@ struct hcg_target {
 
 // Launchers (hcg_field.cu, hcg_grid.cu). All return cudaGetLastError().
 namespace hcg {
+// A field's spectra allocation: the rows, then per channel the bits of the
+// largest finite magnitude and the count of non-finite values.
+inline size_t spec_bytes(uint64_t n, uint32_t cstride) {
+    return ((size_t)n + 1) * cstride * sizeof(float) + 2 * sizeof(unsigned long long);
+}
+struct SpecMax {
+    unsigned int *amax;
+    unsigned long long *bad;
+    SpecMax(float *spec, uint64_t n, uint32_t cstride)
+        : amax(reinterpret_cast<unsigned int *>(spec + (size_t)n * cstride)),
+          bad(reinterpret_cast<unsigned long long *>(amax + cstride)) {}
+};
 constexpr int kTcClasses = 8;
 constexpr int kTcConfigCount = 6;  // tensor-core pipeline shapes (hcg_tc_set_config)
 constexpr int kTcDefaultPrefetch = 0;  // chunks the producer prefetches into L2 ahead of its loads (0: none)

@@ -227,46 +227,42 @@ cudaError_t split_spectra(hcg_context *ctx, hcg_field *f, int fmt_engine, std::s
     const uint32_t cpad = (f->nchan + 63) / 64 * 64;
     const uint64_t n = f->n;
     uint16_t *hi = nullptr, *lo = nullptr;
-    float *scale = nullptr, *inv = nullptr;
-    unsigned int *amax = nullptr;
-    unsigned long long *bad = nullptr;
+    float *inv = nullptr;  // [cpad] inverse scales (kept), then [cpad] scales
     const size_t nb = (size_t)n * cpad * sizeof(uint16_t);
     if ((e = dalloc(&hi, nb ? 2 * nb : 16, s, ctx->pool)) != cudaSuccess ||
-        (e = dalloc(&scale, cpad * sizeof(float), s, ctx->pool)) != cudaSuccess ||
-        (e = dalloc(&inv, cpad * sizeof(float), s, ctx->pool)) != cudaSuccess ||
-        (e = dalloc(&amax, cpad * sizeof(unsigned int) + sizeof(unsigned long long), s, ctx->pool)) != cudaSuccess) {
+        (e = dalloc(&inv, 2 * cpad * sizeof(float), s, ctx->pool)) != cudaSuccess) {
         why = "split spectra of " + std::to_string(2 * nb) + " bytes";
         if (hi) cudaFreeAsync(hi, s);
-        if (scale) cudaFreeAsync(scale, s);
-        if (inv) cudaFreeAsync(inv, s);
         return e;
     }
+    float *const scale = inv + cpad;
     lo = hi + (size_t)n * cpad;  // [2][cpad / 64][n][64]: the lo half follows the hi half
-    bad = (unsigned long long *)(amax + cpad);  // cpad is a multiple of 64: 8-byte aligned
-    cudaMemsetAsync(amax, 0, cpad * sizeof(unsigned int) + sizeof(unsigned long long), s);
     const float wscale = tc_weight_scale(f, fmt != 0);
-    if (n > 0) {
+    const SpecMax mx(f->d_spec, n, f->cstride);
+    if (!f->amax_set) {  // spectra that did not come as device rows
+        cudaMemsetAsync(mx.amax, 0, f->cstride * sizeof(float) + 2 * sizeof(unsigned long long), s);
         uint32_t quads = 1;  // channel quads of a block's row: a power of two up to 256
         while (quads < kAmaxThreads && 4 * quads < f->cstride) quads *= 2;
         const uint32_t cblk = (f->cstride + 4 * quads - 1) / (4 * quads), rows = kAmaxThreads / quads;
         // about eight resident blocks an SM in all, at least four rows a thread
         const uint64_t want = (148 * 8 + cblk - 1) / cblk, most = (n + 4 * rows - 1) / (4 * rows);
-        k_split_amax<<<dim3(cblk, (unsigned)std::min<uint64_t>(want, most)), kAmaxThreads, 0, s>>>(
-            f->d_spec, n, f->nchan, f->cstride, quads, amax, bad);
+        if (n > 0)
+            k_split_amax<<<dim3(cblk, (unsigned)std::min<uint64_t>(want, most)), kAmaxThreads, 0, s>>>(
+                f->d_spec, n, f->nchan, f->cstride, quads, mx.amax, mx.bad);
+        f->amax_set = true;
     }
-    k_split_scales<<<(cpad + 255) / 256, 256, 0, s>>>(amax, f->nchan, cpad, fmt, wscale, scale, inv);
+    k_split_scales<<<(cpad + 255) / 256, 256, 0, s>>>(mx.amax, f->nchan, cpad, fmt, wscale, scale, inv);
     if (n > 0)
         k_split<<<(unsigned)((n + kSplitRows - 1) / kSplitRows), 256, 0, s>>>(f->d_spec, n, f->nchan, f->cstride,
                                                                               cpad, fmt, scale, hi, lo);
-    unsigned long long nonfinite = 0;
-    cudaMemcpyAsync(&nonfinite, bad, sizeof(nonfinite), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(amax, s);
-    cudaFreeAsync(scale, s);
+    unsigned long long *const back = reinterpret_cast<unsigned long long *>(ctx->h_stats);
+    cudaMemcpyAsync(back, mx.bad, sizeof *back, cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess) {
         cudaFreeAsync(hi, s);
         cudaFreeAsync(inv, s);
         return e;
     }
+    const unsigned long long nonfinite = *back;
     free_split(f, s);
     f->d_xhi = hi;
     f->d_xlo = lo;
