@@ -861,9 +861,13 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const C
 // geometry, so no entries are written or read and no FP64 weight pass runs
 // before. Twelve builder warps (latency hiding for the FP64 chains): thread
 // bt owns operand row m = bt % 128 (pixel (m % 16, m / 16) of the tile) and
-// the 8-slot pieces p = bt / 128 (mod 3) of each 64-slot chunk. Per chunk
-// the first 64 builders load the chunk's sample geometry into shared memory
-// (cp.async, one chunk ahead); then, for each slot whose sample lies in its
+// a third of the 8-slot pieces of each 64-slot chunk, the third changing from
+// chunk to chunk (eight pieces make 3, 3 and 2). Per chunk 64 builders, of each
+// third in turn, load the next chunk's sample geometry into shared memory
+// (cp.async on the buffer's mbarrier); builders meet at these barriers alone, so
+// that a warp may run up to two chunks ahead of another (a barrier of all
+// builders per chunk left a fifth of their time waiting: 9.4 against 8.1 ms).
+// For each slot whose sample lies in its
 // pixel's window of the slot's ring (ring_window_mc, the windows the tile pass
 // unioned), a builder evaluates the FP64 distance, cutoff and FP32 Gaussian
 // (pair_weights' arithmetic; UNIT: its kPairUnit form), accumulates the FP64
@@ -871,13 +875,14 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const C
 // stores). The next ring's window is loaded when a ring begins. What bounds it:
 // issue, about 45 instructions a (pixel, slot) pair at three builder warps a
 // scheduler (eight builder warps with more registers, or samples read through
-// L1 without the chunk barriers, were slower: 10.5 and 12.4 against 9.3 ms on
+// L1, were slower: 10.5 and 12.4 against 9.3 ms, as are sixteen at 80 registers,
+// 9.2 against 8.1 ms, on
 // 150,000 samples x 64 channels, 768 x 768 pixels, beam 54 pixels wide; 13.5 ms
 // with FP64 cutoff tests, weights converted to and from FP64, and the window
 // fetched at each ring). The epilogue adds
 // the three partial weight sums of a row from shared memory.
 constexpr int kTcGeo = 64;          // slots per chunk of the direct builders
-constexpr int kTcGeoBufs = 2;       // geometry buffers: loads run one chunk ahead
+constexpr int kTcGeoBufs = 3;       // geometry buffers: loads run one chunk ahead of a builder, builders drift by one
 constexpr int kTcDRow = 3;          // direct builders per operand row
 constexpr int kTcDBuilders = kTcDRow * kTcM;
 constexpr int kTcDThreads = 64 + kTcDBuilders + kTcBuilders;  // producer, MMA, builders, epilogue
@@ -885,6 +890,7 @@ constexpr int kTcDThreads = 64 + kTcDBuilders + kTcBuilders;  // producer, MMA, 
 struct TcDShared {
     uint64_t full_a[kTcMaxStages], full_b[kTcMaxStages], empty[kTcMaxStages];
     uint64_t acc_full[2], acc_empty[2], ws_full[2], ws_empty[2];
+    uint64_t geo_full[kTcGeoBufs], geo_empty[kTcGeoBufs];
     uint32_t tmem;
     volatile int abort;
     uint32_t ulo[kTileMaxRings], base[kTileMaxRings + 1];    // the producer's current item
@@ -949,10 +955,21 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
     const float x2scale = a.x2scale;
     const float wscale = J.wscale;
     const uint32_t fmt = J.fmt;
-    // geometry of chunk kk into buffer kk % kTcGeoBufs (threads 0..63, one slot each)
+    double wsum = 0.0;
+    uint32_t within = 0;
+    bool failed = false;
+    // geometry of chunk kk (chunk g = gk + kk of this CTA) into buffer g %
+    // kTcGeoBufs: the first 64 builders of operand row part g % kTcDRow, one
+    // slot each; the copies' arrivals complete the buffer's barrier
     auto load = [&](uint32_t kk) {
-        if (bt < kTcGeo && kk < nchunks) {
-            const uint32_t slot = kk * KC + bt;
+        const uint32_t g = gk + kk, b = g % kTcGeoBufs;
+        if (kk < nchunks && qb == g % kTcDRow && m < (uint32_t)kTcGeo && !failed && !S.abort) {
+            if (g >= kTcGeoBufs && !mbar_wait(&S.geo_empty[b], (g / kTcGeoBufs - 1) & 1, kTcWaitNs)) {
+                tc_give_up(S, timeouts);
+                failed = true;
+                return;
+            }
+            const uint32_t slot = kk * KC + m;
             uint32_t idx = nrows - 1;
             if (slot < U) {
                 int lo = 0, hi = nrt;
@@ -962,12 +979,11 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
                 }
                 idx = min(S.bulo[lo] + (slot - S.bbase[lo]), nrows - 1);
             }
-            const uint32_t b = kk % kTcGeoBufs;
-            cp_async16(&S.g_half[b][bt], a.half + idx, true);
-            cp_async16(reinterpret_cast<uint8_t *>(&S.g_half[b][bt]) + 16, a.half + a.n + idx, true);
-            if (!UNIT) cp_async8(&S.g_w[b][bt], a.w + idx);
+            cp_async16(&S.g_half[b][m], a.half + idx, true);
+            cp_async16(reinterpret_cast<uint8_t *>(&S.g_half[b][m]) + 16, a.half + a.n + idx, true);
+            if (!UNIT) cp_async8(&S.g_w[b][m], a.w + idx);
+            cp_async_arrive(&S.geo_full[b]);
         }
-        cp_async_commit();
     };
     load(0);
     // ring cursor: compacted ring c of the current slot and this pixel's window
@@ -988,26 +1004,20 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
         }
         return w;
     };
-    double wsum = 0.0;
-    uint32_t within = 0;
-    bool failed = false;
     for (uint32_t k = 0; k < nchunks; ++k) {
-        const uint32_t g = gk + k, s = g % ST;
-        named_barrier(4, kTcDBuilders);  // every builder is done with chunk k - 1's geometry
+        const uint32_t g = gk + k, s = g % ST, b = g % kTcGeoBufs;
         load(k + 1);
-        cp_async_wait<1>();  // this thread's copies of chunk k have landed
-        bool bad = S.abort;
-        if (!bad && g >= ST && !mbar_wait(&S.empty[s], ((g / ST) - 1) & 1, kTcWaitNs)) {
+        if (!failed && !S.abort &&
+            ((g >= ST && !mbar_wait(&S.empty[s], ((g / ST) - 1) & 1, kTcWaitNs)) ||
+             !mbar_wait(&S.geo_full[b], (g / kTcGeoBufs) & 1, kTcWaitNs))) {
             tc_give_up(S, timeouts);
-            bad = true;
-        }
-        if (named_barrier_or(4, kTcDBuilders, bad)) {  // chunk k's geometry visible; the same exit in every builder
             failed = true;
-            break;
         }
-        const uint32_t b = k % kTcGeoBufs;
+        failed = __any_sync(0xffffffffu, failed || S.abort);  // the same exit in every lane
+        if (failed) break;
         uint8_t *ah = st.A_hi(s), *al = st.A_lo(s);
-        for (uint32_t s8 = qb; s8 < KC / 8; s8 += kTcDRow) {
+        // eight pieces over three parts: the parts with three change from chunk to chunk
+        for (uint32_t s8 = (qb + g) % kTcDRow; s8 < KC / 8; s8 += kTcDRow) {
             // ring runs take multiples of 8 slots: one ring per 8-slot piece
             const uint32_t slot0 = k * KC + s8 * 8;
             if (slot0 < U && (slot0 >= cnext || c < 0)) {
@@ -1101,8 +1111,10 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
         }
         fence_proxy_async_smem();
         mbar_arrive(&S.full_a[s]);
+        __syncwarp();
+        if ((bt & 31) == 0) mbar_arrive(&S.geo_empty[b]);
     }
-    cp_async_wait<0>();  // no geometry copy outlives the item
+    cp_async_wait_all();  // no geometry copy outlives the item
     // the pixel's FP64 weight sum for the epilogue (after it has read the sum two items back)
     if (!failed && il >= 2 && !mbar_wait(&S.ws_empty[a2], ((il >> 1) - 1) & 1, kTcWaitNs)) tc_give_up(S, timeouts);
     S.wsum[a2][qb][m] = valid ? wsum : 0.0;
@@ -1132,6 +1144,10 @@ __device__ __forceinline__ void tc_persist_weights(TcDShared &S, const TcJob &J,
             mbar_init(&S.acc_empty[a], kTcBuilders);
             mbar_init(&S.ws_full[a], kTcDBuilders);
             mbar_init(&S.ws_empty[a], kTcBuilders);
+        }
+        for (int b = 0; b < kTcGeoBufs; ++b) {
+            mbar_init(&S.geo_full[b], kTcGeo);
+            mbar_init(&S.geo_empty[b], kTcDBuilders / 32);
         }
         S.abort = 0;
         mbar_fence_init();
