@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kWeightThreads, 4) kb_group(BatchHdr *H, const
             if (over) atomicAdd(&H->pool_overflow, 1ULL);
             continue;
         }
-        if (J.a.unit_w && J.a.series32)
+        if (J.a.unit_w && J.a.w32ok)
             group_tile_item<kPairUnit>(J.a, J.g, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, true, tile, 0, 1, S, pc);
         else
             group_tile_item<kPairGeneral>(J.a, J.g, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, true, tile, 0, 1, S, pc);

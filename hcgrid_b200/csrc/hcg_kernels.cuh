@@ -187,7 +187,7 @@ struct GridArgs {
     double hlo, hhi;      // haversine thresholds bracketing sphere_radius (see grid_args)
     int series;           // d^2 from the arcsine-squared series (small sphere_radius)
     double hpolar;        // haversine bound of every accepted pair (chord windows)
-    float x2scale;        // 4 R2D^2 p0 log2(e): the FP32 Gaussian's exponent per unit of the series
+    float x2c[3];         // -4 R2D^2 p0 log2(e) times 1, 1/3, 8/45: the FP32 Gaussian's exponent by powers of h
     int series32;         // series && GAUSS1D: accepted pairs below the band take gauss_series_f32
     uint32_t ktype;       // HCG_GAUSS1D, HCG_GAUSS2D or HCG_TAPERED_SINC
     int ktaper;           // TAPERED_SINC with HCG_TAPER_FIX
@@ -199,6 +199,7 @@ struct GridArgs {
     float hlo32, hhi32;   // <= hlo, >= hhi: the brackets an FP32 haversine decides
     double e2scale;       // -4 R2D^2 p0 log2(e): GAUSS1D's base-2 exponent per unit of the series
     int exp2ok;           // series, GAUSS1D, and no accepted pair's weight is below 2^-1000 (exp2_small)
+    int w32ok;            // the same for 2^-120: no accepted pair's FP32 weight is zero
     uint64_t n;           // samples
     double spa, cpa;      // GAUSS2D: sine and cosine of the position angle
 };
@@ -219,7 +220,6 @@ inline GridArgs grid_args(const hcg_field *f, const PixPrep *prep, DevStats *sta
     a.hhi = hstar * (1.0 + 1e-9);
     a.series = hstar < 1e-3;
     a.hpolar = hstar * (1.0 + 1e-6);
-    a.x2scale = (float)(4.0 * kRad2Deg * kRad2Deg * f->kparam0 * 1.4426950408889634);
     a.ktype = f->kernel_type;
     a.series32 = a.series && f->kernel_type == HCG_GAUSS1D;
     a.ktaper = f->taper_fix;
@@ -230,6 +230,10 @@ inline GridArgs grid_args(const hcg_field *f, const PixPrep *prep, DevStats *sta
     a.hpolar32 = (float)(hstar * (1.0 + 2e-6));
     a.unit_w = f->unit_w;
     a.e2scale = -4.0 * kRad2Deg * kRad2Deg * f->kparam0 * 1.4426950408889634;
+    a.x2c[0] = (float)a.e2scale;
+    a.x2c[1] = (float)(a.e2scale / 3.0);
+    a.x2c[2] = (float)(a.e2scale * (8.0 / 45.0));
+    a.w32ok = a.series32 && a.e2scale <= 0.0 && a.e2scale * hstar * 1.01 > -120.0;
     a.exp2ok = a.series32 && a.e2scale <= 0.0 && a.e2scale * hstar * 1.01 > -1000.0;
     a.hlo32 = (float)(a.hlo * (1.0 - 2e-7));
     a.hhi32 = (float)(a.hhi * (1.0 + 2e-7));
@@ -470,13 +474,13 @@ __device__ __forceinline__ float gauss_f32(double x) {
     return r;
 }
 
-// The same for an accepted pair whose cutoff FP64 has decided, from its
-// haversine h < 1e-3: the arcsine-squared series (four terms) in FP32. The
-// exponent's relative error stays below 3e-7, the weight's below 1.6e-6 at
-// d = 3 sigma (x2scale = 4 R2D^2 p0 log2 e).
-__device__ __forceinline__ float gauss_series_f32(double h, float x2scale) {
-    const float hf = (float)h;
-    const float t = -(hf * (1.f + hf * (1.f / 3.f + hf * (8.f / 45.f + hf * (4.f / 35.f))))) * x2scale;
+// The same for an accepted pair whose cutoff is decided, from its haversine h <
+// 1e-3 rounded to FP32: the arcsine-squared series h (1 + h / 3 + 8 h^2 / 45)
+// (the next term is 2e-10 of it) with the scale folded into its coefficients.
+// The exponent's relative error stays below 3e-7, the weight's below 1.6e-6 at
+// d = 3 sigma.
+__device__ __forceinline__ float gauss_series_f32(float hf, const float (&c)[3]) {
+    const float t = hf * (c[0] + hf * (c[1] + hf * c[2]));
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
     return r;
@@ -587,7 +591,7 @@ __device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t 
     const PairHav v = pair_hav(Q.h, sl2, sb2);
     if (v.h > a.hhi) return 0.0;
     if (v.h < a.hlo) {
-        if (F32 && !GEN && a.series32) return win * (double)gauss_series_f32(v.h, a.x2scale);
+        if (F32 && !GEN && a.series32) return win * (double)gauss_series_f32((float)v.h, a.x2c);
         return kernel_at<F32, GEN>(a, Q.h, Q.cb1, v, sl2, sb2, win, pair_d2(a, v.h));
     }
     const double d = dist_deg(Q.l1, Q.b1, Q.cb1, __ldg(a.l2 + idx), __ldg(a.b2 + idx),
@@ -625,9 +629,9 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
         if (F32) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                wf[i] = acc[i] ? gauss_series_f32(v[i].h, a.x2scale) : 0.f;
+                wf[i] = acc[i] ? gauss_series_f32((float)v[i].h, a.x2c) : 0.f;
                 w[i] = (double)wf[i];
-                nz[i] = wf[i] != 0.f;
+                nz[i] = acc[i];
             }
         } else {
             double t[4];
@@ -652,7 +656,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
         if (F32 && !GEN && a.series32) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const float gs = gauss_series_f32(v[i].h, a.x2scale);
+                const float gs = gauss_series_f32((float)v[i].h, a.x2c);
                 w[i] = acc[i] ? win * (double)gs : 0.0;
             }
         } else {
@@ -688,7 +692,7 @@ inline int pair_mode1(const hcg_field *f, const GridArgs &a) {
     return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.exp2ok ? kPairUnit : kPairGeneral;
 }
 inline int pair_mode(const hcg_field *f, const GridArgs &a) {
-    return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.series32 ? kPairUnit : kPairGeneral;
+    return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.w32ok ? kPairUnit : kPairGeneral;
 }
 
 // Sums of four values over a warp's lanes: lanes 8q .. 8q + 7 return value q's
@@ -743,17 +747,21 @@ __device__ __forceinline__ void group_load(GroupShared &S, const PixPrep *__rest
 }
 
 // One block of up to 32 rings (lane = ring) of a group: every union candidate,
-// 32 at a time, tested against the four pixels; `body(idx, slot, w, wf, nz)`
-// gets the candidate's weights. Warp-collective. What bounds it: instruction
-// issue (about 40 a pair) with the FP64 pipe next. The ring of a candidate is
-// found from one reduction of the ring ends that fall into the round (a bit
-// each) instead of a search by shuffles, its record read from shared memory
-// instead of sixteen shuffles, and a candidate's geometry is loaded once for
-// four pixels.
+// 32 at a time, tested against the four pixels; `body(x, slot, w, wf, nz)` gets
+// the candidate's spectrum value (single channel: `data`, rows of `cstride`) and
+// weights. Warp-collective. What bounds it: instruction issue (about 40 a pair)
+// with the FP64 pipe next. The ring of a candidate is found from one reduction of
+// the ring ends that fall into the round (a bit each) instead of a search by
+// shuffles, its record read from shared memory instead of sixteen shuffles, and a
+// candidate's geometry is loaded once for four pixels, a round ahead (4,000,000
+// samples on 1200 x 1200 pixels: 1524 -> 1424 us single channel, 945 -> 898 us
+// for the entries; copies through shared memory or ring ends kept as bits there
+// cost as many instructions as they saved).
 template <bool F32, int MODE, typename BODY>
 __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s_h, const double *s_cb1,
                                              GroupRecords &S, uint64_t pix0, uint32_t nx, const uint32_t lo[4],
-                                             const uint32_t hi[4], uint32_t shift, BODY body) {
+                                             const uint32_t hi[4], uint32_t shift, const float *__restrict__ data,
+                                             uint32_t cstride, BODY body) {
     const int lane = threadIdx.x & 31;
     uint32_t glo = 0xffffffffu, ghi = 0;
 #pragma unroll
@@ -780,6 +788,22 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
         S.rc[c] = make_uint2(lo[3], n(3));
     }
     __syncwarp();
+    // the round's samples, fetched while the round before is worked on
+    int r = 0;
+    double2 nsl, nsb;
+    float nx1 = 0.f;
+    auto fetch = [&](uint32_t tb) {
+        const unsigned ends = __reduce_or_sync(0xffffffffu, len && incl > tb && incl - tb < 32 ? 1u << (incl - tb) : 0u);
+        const int c0 = __popc(__ballot_sync(0xffffffffu, len && incl <= tb));
+        const bool act = tb + lane < total;
+        r = act ? c0 + __popc(ends & (0xffffffffu >> (31 - lane))) : c0;
+        // a lane past the last candidate repeats the round's first one, outside every window
+        const uint32_t idx = S.ra[r].x + (act ? tb + lane : tb);
+        nsl = __ldg(a.half + idx);
+        nsb = __ldg(a.half + a.n + idx);
+        if (!F32) nx1 = __ldg(data + (uint64_t)idx * cstride);
+    };
+    if (total) fetch(0);
     for (uint32_t tb = 0; tb < total; tb += 32) {
         // the pixels' constants are read anew each round (the barrier keeps the
         // compiler from holding their 40 registers, which cost a third of the warps)
@@ -791,16 +815,13 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
             ph[q] = s_h[q];
             cb1[q] = MODE == kPairOther ? s_cb1[q] : 0.0;  // only the other kernels take it
         }
-        const uint32_t t = tb + lane;
-        const unsigned ends = __reduce_or_sync(0xffffffffu, len && incl > tb && incl - tb < 32 ? 1u << (incl - tb) : 0u);
-        const int c0 = __popc(__ballot_sync(0xffffffffu, len && incl <= tb));
-        const bool act = t < total;
-        const int r = act ? c0 + __popc(ends & (0xffffffffu >> (31 - lane))) : c0;
+        const bool act = tb + lane < total;
         const uint4 ra = S.ra[r], rb = S.rb[r];
         const uint2 rc = S.rc[r];
-        // a lane past the last candidate repeats the round's first one, outside every window
-        const uint32_t idx = ra.x + (act ? t : tb);
-        const double2 sl2 = __ldg(a.half + idx), sb2 = __ldg(a.half + a.n + idx);
+        const uint32_t idx = ra.x + (act ? tb + lane : tb);
+        const double2 sl2 = nsl, sb2 = nsb;
+        const float x = nx1;
+        if (tb + 32 < total) fetch(tb + 32);
         const double win = MODE == kPairUnit || a.unit_w ? 1.0 : __ldg(a.w + idx);
         const bool in[4] = {act && idx - ra.z < ra.w, act && idx - rb.x < rb.y, act && idx - rb.z < rb.w,
                             act && idx - rc.x < rc.y};
@@ -808,7 +829,7 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
         float wf[4];
         bool nz[4];
         pair_weights<F32, MODE>(a, a.prep + pix0, nx, ph, cb1, sl2, sb2, win, idx, in, w, wf, nz);
-        body(idx, idx + ra.y, w, wf, nz);
+        body(x, idx + ra.y, w, wf, nz);
     }
 }
 
@@ -878,9 +899,9 @@ __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint3
             nr = G.r1 - G.r0 + 1;
             group_lane_windows(a, G, G.r0 + rb + lane, pix0, nx, lo, hi, ref, skips);
         }
-        group_rounds<false, MODE>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u,
-                                  [&](uint32_t idx, uint32_t, const double w[4], const float[4], const bool nz[4]) {
-            const double x = (double)__ldg(data + (uint64_t)idx * cstride);
+        group_rounds<false, MODE>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u, data, cstride,
+                                  [&](float v, uint32_t, const double w[4], const float[4], const bool nz[4]) {
+            const double x = (double)v;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 if (nz[q]) {
@@ -1142,8 +1163,8 @@ __device__ __forceinline__ void group_tile_item(const GridArgs &a, const GroupAr
                 }
             }
             group_rounds<true, MODE>(
-                a, S.px[gl].h, S.px[gl].cb1, S.rec[warp], pix0, g.nx, lo, hi, shift,
-                [&](uint32_t, uint32_t slot, const double w[4], const float wf[4], const bool nz[4]) {
+                a, S.px[gl].h, S.px[gl].cb1, S.rec[warp], pix0, g.nx, lo, hi, shift, nullptr, 0u,
+                [&](float, uint32_t slot, const double w[4], const float wf[4], const bool nz[4]) {
                     bool any = false;
                     float e[4];
 #pragma unroll

@@ -439,7 +439,7 @@ cudaError_t tc_weights(hcg_context *ctx, const hcg_field *f, const GridArgs &a, 
     J.wout = wout;
     tc_pipeline(ctx, f, J);
     const uint32_t b = f->xcpad / 64;
-    const bool unit = a.unit_w && a.series32;
+    const bool unit = a.unit_w && a.w32ok;
     if (b >= 4)
         return unit ? launch_tc_weights<TcCfgN4S2, true>(ctx, f, J, T, ntiles, why)
                     : launch_tc_weights<TcCfgN4S2, false>(ctx, f, J, T, ntiles, why);

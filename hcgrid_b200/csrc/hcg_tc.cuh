@@ -952,7 +952,6 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
     const double hlo = a.hlo, hhi = a.hhi, p0 = a.p0;
     const float hlo32 = a.hlo32, hhi32 = a.hhi32;
     const bool series = a.series != 0;
-    const float x2scale = a.x2scale;
     const float wscale = J.wscale;
     const uint32_t fmt = J.fmt;
     double wsum = 0.0;
@@ -1071,14 +1070,14 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
                         const float hf = (float)h;
                         const bool acc = inw && hf < hlo32;
                         if (inw && !acc && hf <= hhi32) band |= 1u << e;
-                        wv[e] = acc ? gauss_series_f32(h, x2scale) : 0.f;
+                        wv[e] = acc ? gauss_series_f32(hf, a.x2c) : 0.f;
                         wsum += (double)wv[e];
-                        within += wv[e] != 0.f;
+                        within += acc;
                     } else {
                         // the Gaussian of an accepted pair, as pair_weights evaluates it
                         float ex;
                         if (series) {
-                            ex = gauss_series_f32(h, x2scale);
+                            ex = gauss_series_f32((float)h, a.x2c);
                         } else {
                             const double d = 2.0 * asin(sqrt(h)) * kRad2Deg;
                             ex = gauss_f32(d * d * p0);
