@@ -197,7 +197,7 @@ struct GridArgs {
     float hpolar32;       // >= hpolar
     int unit_w;           // every sample weight is 1
     float hlo32, hhi32;   // <= hlo, >= hhi: the brackets an FP32 haversine decides
-    double e2scale;       // -4 R2D^2 p0 log2(e): GAUSS1D's base-2 exponent per unit of the series
+    double e2c[5];        // -4 R2D^2 p0 log2(e) times 1, 1/3, 8/45, 4/35, 128/1575: GAUSS1D's base-2 exponent by powers of h
     int exp2ok;           // series, GAUSS1D, and no accepted pair's weight is below 2^-1000 (exp2_small)
     int w32ok;            // the same for 2^-120: no accepted pair's FP32 weight is zero
     uint64_t n;           // samples
@@ -229,12 +229,12 @@ inline GridArgs grid_args(const hcg_field *f, const PixPrep *prep, DevStats *sta
     a.firstring = f->firstring;
     a.hpolar32 = (float)(hstar * (1.0 + 2e-6));
     a.unit_w = f->unit_w;
-    a.e2scale = -4.0 * kRad2Deg * kRad2Deg * f->kparam0 * 1.4426950408889634;
-    a.x2c[0] = (float)a.e2scale;
-    a.x2c[1] = (float)(a.e2scale / 3.0);
-    a.x2c[2] = (float)(a.e2scale * (8.0 / 45.0));
-    a.w32ok = a.series32 && a.e2scale <= 0.0 && a.e2scale * hstar * 1.01 > -120.0;
-    a.exp2ok = a.series32 && a.e2scale <= 0.0 && a.e2scale * hstar * 1.01 > -1000.0;
+    const double e2scale = -4.0 * kRad2Deg * kRad2Deg * f->kparam0 * 1.4426950408889634;
+    const double series[5] = {1.0, 1.0 / 3.0, 8.0 / 45.0, 4.0 / 35.0, 128.0 / 1575.0};
+    for (int i = 0; i < 5; ++i) a.e2c[i] = e2scale * series[i];
+    for (int i = 0; i < 3; ++i) a.x2c[i] = (float)a.e2c[i];
+    a.w32ok = a.series32 && e2scale <= 0.0 && e2scale * hstar * 1.01 > -120.0;
+    a.exp2ok = a.series32 && e2scale <= 0.0 && e2scale * hstar * 1.01 > -1000.0;
     a.hlo32 = (float)(a.hlo * (1.0 - 2e-7));
     a.hhi32 = (float)(a.hhi * (1.0 + 2e-7));
     a.n = f->n;
@@ -513,25 +513,23 @@ __device__ __forceinline__ double pair_d2(const GridArgs &a, double h) {
 }
 
 // 2^t for -1000 < t <= 0: the nearest integer by adding and subtracting
-// 1.5 * 2^52, the Taylor series of 2^f = exp(f ln 2) on |f| <= 1/2 (degree 13,
-// remainder below 5e-18), and the integer into the exponent. The range is known,
-// so nothing is tested; within 2 ulp.
+// 1.5 * 2^52, 2^f on |f| <= 1/2 by its interpolant of degree 11 in the Chebyshev
+// points (4e-18 of it, 2e-17 with the coefficients rounded), and the integer into
+// the exponent. The range is known, so nothing is tested; within 2 ulp.
 __device__ __forceinline__ double exp2_small(double t) {
-    const double big = 6755399441055744.0, k = t + big, f = t - (k - big), x = f * 0.6931471805599453;
-    double p = 1.0 / 6227020800.0;
-    p = fma(p, x, 1.0 / 479001600.0);
-    p = fma(p, x, 1.0 / 39916800.0);
-    p = fma(p, x, 1.0 / 3628800.0);
-    p = fma(p, x, 1.0 / 362880.0);
-    p = fma(p, x, 1.0 / 40320.0);
-    p = fma(p, x, 1.0 / 5040.0);
-    p = fma(p, x, 1.0 / 720.0);
-    p = fma(p, x, 1.0 / 120.0);
-    p = fma(p, x, 1.0 / 24.0);
-    p = fma(p, x, 1.0 / 6.0);
-    p = fma(p, x, 0.5);
-    p = fma(p, x, 1.0);
-    p = fma(p, x, 1.0);
+    const double big = 6755399441055744.0, k = t + big, f = t - (k - big);
+    double p = 4.4558179083360645e-10;
+    p = fma(p, f, 7.074194297288521e-09);
+    p = fma(p, f, 1.0178057087733941e-07);
+    p = fma(p, f, 1.3215432535912375e-06);
+    p = fma(p, f, 1.5252733841556773e-05);
+    p = fma(p, f, 0.00015403530463724353);
+    p = fma(p, f, 0.001333355814640647);
+    p = fma(p, f, 0.009618129107587256);
+    p = fma(p, f, 0.055504108664821625);
+    p = fma(p, f, 0.24022650695910158);
+    p = fma(p, f, 0.6931471805599453);
+    p = fma(p, f, 1.0);
     return __hiloint2double(__double2hiint(p) + (__double2loint(k) << 20), __double2loint(p));
 }
 
@@ -638,8 +636,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const double h = v[i].h;
-                t[i] = (h * a.e2scale) *
-                       (1.0 + h * (1.0 / 3.0 + h * (8.0 / 45.0 + h * (4.0 / 35.0 + h * (128.0 / 1575.0)))));
+                t[i] = h * (a.e2c[0] + h * (a.e2c[1] + h * (a.e2c[2] + h * (a.e2c[3] + h * a.e2c[4]))));
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
