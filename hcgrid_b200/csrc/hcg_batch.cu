@@ -106,6 +106,30 @@ __device__ __forceinline__ unsigned long long block_fetch(BatchHdr *H, int q) {
     return s_item;
 }
 
+// A block's copy of the geometry part of its present job's descriptor: read at
+// every pair test and ring, and from global memory each read is an L1 access that
+// stores in between make the compiler repeat.
+struct JobGeo {
+    GridArgs a;
+    GroupArgs g;
+    TileArgs T;
+};
+struct JobGeoShared {
+    alignas(16) uint32_t w[sizeof(JobGeo) / 4];
+    // Block-collective, after a barrier that ends the previous item.
+    __device__ __forceinline__ const JobGeo &load(const JobDesc &J, int j, int &cur) {
+        static_assert(offsetof(JobDesc, g) == offsetof(JobGeo, g) && offsetof(JobDesc, T) == offsetof(JobGeo, T),
+                      "a descriptor begins with its geometry part");
+        if (j != cur) {
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(&J);
+            for (uint32_t i = threadIdx.x; i < sizeof(JobGeo) / 4; i += blockDim.x) w[i] = __ldg(src + i);
+            cur = j;
+            __syncthreads();
+        }
+        return *reinterpret_cast<const JobGeo *>(w);
+    }
+};
+
 __device__ __forceinline__ unsigned long long warp_fetch(BatchHdr *H, int q) {
     unsigned long long v = 0;
     if ((threadIdx.x & 31) == 0) v = atomicAdd(&H->head[q], 1ULL);
@@ -113,12 +137,14 @@ __device__ __forceinline__ unsigned long long warp_fetch(BatchHdr *H, int q) {
 }
 
 __global__ void __launch_bounds__(128, kRingCtas) kb_tile_rings(BatchHdr *H, const JobDesc *__restrict__ jobs) {
+    __shared__ JobGeoShared S;
+    int cur = -1;
     for (;;) {
         unsigned long long it = block_fetch(H, Q_TILE);
         if (it >= H->tot_tile) return;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.tile_base; });
-        const JobDesc &J = jobs[j];
-        tile_rings_item<4>(J.a, J.g, J.T, it - J.tile_base);
+        const JobGeo &J = S.load(jobs[j], j, cur);
+        tile_rings_item<4>(J.a, J.g, J.T, it - jobs[j].tile_base);
     }
 }
 
@@ -140,33 +166,38 @@ __global__ void __launch_bounds__(256) kb_group_count(BatchHdr *H, const JobDesc
 }
 
 // The weight pass, a tile per item. The pool must hold the tile's entries;
-// otherwise its groups are skipped and reported (no entries recorded: the pass
-// is replayed once the pool has grown).
+// otherwise its groups are skipped and reported (no entries recorded: the pass is
+// replayed once the pool has grown). 64 observations of 10,000 samples: 177 us,
+// 213 us with descriptors read from global memory (the tile pass 118 and 150 us);
+// halves or quarters of tiles for an even last round repeat the tile's loads, 220 us.
 __global__ void __launch_bounds__(kWeightThreads, 4) kb_group(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
     __shared__ TileGroupShared S;
+    __shared__ JobGeoShared SJ;
     PairCounts pc;
+    int cur = -1;
     for (;;) {
         unsigned long long it = block_fetch(H, Q_GEOM);
         if (it >= H->tot_tile) break;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.tile_base; });
-        const JobDesc &J = jobs[j];
-        if (J.skip) continue;
-        const uint64_t tile = it - J.tile_base;
+        const JobDesc &D = jobs[j];
+        if (D.skip) continue;
+        const JobGeo &J = SJ.load(D, j, cur);
+        const uint64_t tile = it - D.tile_base;
         bool over = false;
         if (threadIdx.x < kTileGroups) {
             const uint32_t gxi = (uint32_t)(tile % J.T.ntx) * (kTileX / 2) + threadIdx.x % (kTileX / 2);
             const uint32_t gyi = (uint32_t)(tile / J.T.ntx) * (kTileY / 2) + threadIdx.x / (kTileX / 2);
             const uint64_t grp = (uint64_t)gyi * J.g.gx + gxi;
-            if (gxi < J.g.gx && grp < J.g.ngroups && J.off[grp] + J.cap[grp] > H->entry_cap) over = true;
+            if (gxi < J.g.gx && grp < J.g.ngroups && D.off[grp] + D.cap[grp] > H->entry_cap) over = true;
         }
         if (__syncthreads_or(over)) {
             if (over) atomicAdd(&H->pool_overflow, 1ULL);
             continue;
         }
         if (J.a.unit_w && J.a.w32ok)
-            group_tile_item<kPairUnit>(J.a, J.g, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, true, tile, 0, 1, S, pc);
+            group_tile_item<kPairUnit>(J.a, J.g, D.off, H->e_idx, H->e_w, D.cnt, D.wsum, J.T, true, tile, 0, 1, S, pc);
         else
-            group_tile_item<kPairGeneral>(J.a, J.g, J.off, H->e_idx, H->e_w, J.cnt, J.wsum, J.T, true, tile, 0, 1, S, pc);
+            group_tile_item<kPairGeneral>(J.a, J.g, D.off, H->e_idx, H->e_w, D.cnt, D.wsum, J.T, true, tile, 0, 1, S, pc);
     }
     flush_counts(pc, stats);
 }
