@@ -53,7 +53,7 @@ class BatchTuning(C.Structure):
                 ("spread", C.c_float)]
 
 
-BATCH_SHAPES = 4  # hcg_batch_set_shape: 0: 256 ch x 32 slots x 4 stages, 1: 256 x 64 x 2, 2: 128 x 64 x 3, 3: 64 x 64 x 4
+BATCH_SHAPES = 4  # hcg_batch_set_shape: 0: 256 ch x 32 slots x 4 stages, 1: 256 x 64 x 2, 2: 128 x 32 x 2, 3: 64 x 32 x 3
 
 TUNE_PREFETCH = (0, 2, 4, 6, 8)
 TUNE_STRIP = (0, 4, 8, 16, 32)

@@ -241,58 +241,46 @@ __global__ void __launch_bounds__(kTileThreads) kb_accum(BatchHdr *H, const JobD
     }
 }
 
-// Tensor-core channel sums: one CTA per SM takes (job, channel block, tile)
-// items from the queue of its pipeline shape SH (the jobs whose channel
-// class the context assigns that shape); barrier phases and TMEM persist
-// across items. One launch per shape, in sequence; a shape without items
-// returns at once.
+// Tensor-core channel sums: persistent CTAs (tc_persist: the epilogue of an item
+// runs beside the next item's MMAs), one an SM or two for the shapes of up to 128
+// channels, take every gridDim-th (job, channel block, tile) item of their
+// pipeline shape SH (the jobs whose channel class the context assigns that
+// shape). One launch per shape, in sequence; a shape without items returns at
+// once. What bounds it: the builders' scattered operand stores and the short K of
+// a small job's tile (a few chunks), so that two CTAs with half the stages beat
+// one. 64 observations of 10,000 samples, 64 channels: 204 us; 252 with one CTA of
+// 64-slot chunks x 4 stages; 279 with an item's roles in turn (builders storing the
+// tile themselves, the rings loaded between items).
 template <int SH>
 struct KbShape;
 template <> struct KbShape<0> { using Cfg = TcCfgN4K32; };
 template <> struct KbShape<1> { using Cfg = TcCfgN4S2; };
-template <> struct KbShape<2> { using Cfg = TcCfgN2S3; };
-template <> struct KbShape<3> { using Cfg = TcCfgN1S4; };
+template <> struct KbShape<2> { using Cfg = TcCfgN2K32; };
+template <> struct KbShape<3> { using Cfg = TcCfgN1K32; };
 static_assert(kKbShapes == 4, "one KbShape per batch tensor-core shape");
 
 template <int SH>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kTcPersistThreads, SH >= 2 ? 2 : 1)
     kb_tc(BatchHdr *H, const JobDesc *__restrict__ jobs, unsigned long long *timeouts,
           unsigned long long *macs) {
     using KbTcCfg = typename KbShape<SH>::Cfg;
     static_assert(KbTcCfg::kNb == kKbNb[SH], "shape table and configurations agree");
-    __shared__ TcShared S;
+    __shared__ TcPShared S;
     // entries incomplete (this pass is replayed after the pool grows), or no items of this shape
     if (H->pool_overflow || H->tot_tc[SH] == 0) return;
-    tc_setup<KbTcCfg>(S);
-    uint32_t gk = 0, itn = 0;
     const uint32_t *list = H->tc_list + H->tc_off[SH];
     const int nlist = (int)(H->tc_off[SH + 1] - H->tc_off[SH]);
-    for (;;) {
-        if (threadIdx.x == 0) S.item = S.abort ? ~0ULL : atomicAdd(&H->head[Q_TC + SH], 1ULL);
-        __syncthreads();
-        const unsigned long long it = S.item;
-        if (it >= H->tot_tc[SH]) break;
+    tc_persist<KbTcCfg>(S, H->tot_tc[SH], [&](uint64_t it) {
         int lo = 0, hi = nlist;  // the shape's last job whose base is <= it
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (jobs[list[mid]].tc_base <= it) lo = mid; else hi = mid;
         }
-        const int j = (int)list[lo];
-        if (jobs[j].skip) {
-            __syncthreads();  // every thread has read S.item
-            continue;
-        }
-        const TcJob &J = jobs[j].tc;
-        const unsigned long long local = it - jobs[j].tc_base;
-        const uint64_t ntiles = (uint64_t)J.T.ntx * J.T.nty;
-        const uint64_t tile = local % ntiles;  // tiles fastest: neighbours share staged samples in L2
-        tc_load_rings(S, J.T, tile);
-        __syncthreads();
-        tc_item<KbTcCfg>(S, J, J.map, J.out_map, tile, (uint32_t)(local / ntiles), gk, itn, timeouts, macs);
-        ++itn;
-        __syncthreads();  // every role is done with the item's ring table and accumulator
-    }
-    tc_teardown<KbTcCfg>(S, gk, timeouts);
+        const JobDesc &D = jobs[list[lo]];
+        const uint64_t local = it - D.tc_base, ntiles = (uint64_t)D.tc.T.ntx * D.tc.T.nty;
+        // tiles fastest: neighbours share staged samples in L2
+        return TcItem{D.skip ? nullptr : &D.tc, D.tc.map, local % ntiles, (uint32_t)(local / ntiles)};
+    }, timeouts, macs);
 }
 
 __global__ void __launch_bounds__(kGroupThreads, 4) kb_1chan(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
@@ -339,7 +327,7 @@ struct BatchState {
     int nsm = 0;
     void *scratch[11] = {};
     size_t scratch_size[11] = {};
-    CUtensorMap *d_maps = nullptr, *h_maps = nullptr;  // two per job: spectra (hi and lo halves), cube
+    CUtensorMap *d_maps = nullptr, *h_maps = nullptr;  // one per job: the spectra's hi and lo halves
     unsigned long long *d_jovf = nullptr, *h_jovf = nullptr;  // per job: tiles beyond the ring table
     unsigned long long *d_jent = nullptr, *h_jent = nullptr;  // per job: entries
     unsigned long long *d_jusum = nullptr, *h_jusum = nullptr;  // per job: staged slots of its tiles (sum, largest)
@@ -393,10 +381,10 @@ static cudaError_t capture(hcg_context *ctx, BatchState &B) {
             kb_group<<<n * 4, kWeightThreads, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
             kb_accum<<<n, kTileThreads, smem, s>>>(B.d_hdr, B.d_jobs, &ctx->d_stats->timeouts);
             unsigned long long *to = &ctx->d_stats->timeouts, *macs = &ctx->d_stats->tc_macs;
-            kb_tc<0><<<n, kTcThreads, KbShape<0>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
-            kb_tc<1><<<n, kTcThreads, KbShape<1>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
-            kb_tc<2><<<n, kTcThreads, KbShape<2>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
-            kb_tc<3><<<n, kTcThreads, KbShape<3>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
+            kb_tc<0><<<n, kTcPersistThreads, KbShape<0>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
+            kb_tc<1><<<n, kTcPersistThreads, KbShape<1>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
+            kb_tc<2><<<2 * n, kTcPersistThreads, KbShape<2>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
+            kb_tc<3><<<2 * n, kTcPersistThreads, KbShape<3>::Cfg::kSmem, s>>>(B.d_hdr, B.d_jobs, to, macs);
             kb_1chan<<<n * 4, kGroupThreads, 0, s>>>(B.d_hdr, B.d_jobs, ctx->d_stats);
         }
         cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -483,10 +471,10 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
         if ((e = dalloc(&B.d_tclist, B.job_cap * sizeof(uint32_t), s, ctx->pool)) != cudaSuccess) return e;
         if ((e = cudaMallocHost(&B.h_tclist, B.job_cap * sizeof(uint32_t))) != cudaSuccess) return e;
     }
-    if (2 * njobs > B.map_cap) {
+    if (njobs > B.map_cap) {
         if (B.d_maps) cudaFreeAsync(B.d_maps, s);
         if (B.h_maps) cudaFreeHost(B.h_maps);
-        B.map_cap = std::max<uint32_t>(2 * njobs, 128);
+        B.map_cap = std::max<uint32_t>(njobs, 64);
         if ((e = dalloc(&B.d_maps, B.map_cap * sizeof(CUtensorMap), s, ctx->pool)) != cudaSuccess) return e;
         if ((e = cudaMallocHost(&B.h_maps, B.map_cap * sizeof(CUtensorMap))) != cudaSuccess) return e;
     }
@@ -626,7 +614,7 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
             d.wout = jobs[i].weights;
             if (d.tc.nb) {
                 TcJob &c = d.tc;
-                c.map = B.d_maps + 2 * i;
+                c.map = B.d_maps + i;
                 c.g = d.g;
                 c.T = d.T;
                 c.off = d.off;
@@ -679,23 +667,20 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
                              s)) != cudaSuccess)
         return e;
     if (tcn) {
-        // The tensor maps (a driver call each, two a job) are only read by the
+        // The tensor maps (a driver call each) are only read by the
         // sums: encoded while the geometry graph runs
         bool ok = true;
         for (uint32_t i = 0; i < njobs && ok; ++i) {
             TcJob &c = J[i].tc;
             if (!c.nb) continue;
-            ok = tc_job_map(jobs[i].field, c, &B.h_maps[2 * i]);
-            c.out_map = tc_out_map(&B.h_maps[2 * i + 1], J[i].out, J[i].ostride, J[i].g.nx, J[i].g.ny, c.nchan, c.nb)
-                            ? B.d_maps + 2 * i + 1
-                            : nullptr;
+            ok = tc_job_map(jobs[i].field, c, &B.h_maps[i]);
         }
         if (!ok) {
             cudaStreamSynchronize(s);  // nothing queued outlives the call's buffers
             why = "cuTensorMapEncodeTiled";
             return cudaErrorInvalidValue;
         }
-        if ((e = cudaMemcpyAsync(B.d_maps, B.h_maps, 2 * njobs * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s)) !=
+        if ((e = cudaMemcpyAsync(B.d_maps, B.h_maps, njobs * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s)) !=
                 cudaSuccess ||
             (e = cudaMemcpyAsync(B.d_tclist, B.h_tclist, tc_off[kKbShapes] * sizeof(uint32_t), cudaMemcpyHostToDevice,
                                  s)) != cudaSuccess)

@@ -225,14 +225,15 @@ constexpr uint64_t kBatchMaxPixels = 1ull << 20;  // larger targets skip hcg_gri
 // per channel class (hcg_batch_set_shape, hcg_autotune_batch): 64-channel
 // blocks per item (the MMA's N / 64), K slots per chunk and stages.
 //   0: 256 channels x 32 slots x 4 stages   1: 256 x 64 x 2
-//   2: 128 x 64 x 3                         3: 64 x 64 x 4
+//   2: 128 x 32 x 2, two CTAs an SM         3: 64 x 32 x 3, two CTAs an SM
 constexpr int kKbShapes = 4;
 constexpr uint32_t kKbNb[kKbShapes] = {4, 4, 2, 1};
 // Default shape by channel class: the narrowest that holds the channels of one
-// or two 64-channel blocks (64 jobs of 10,000 samples on 64 x 64 pixels: 64
-// channels 869 us with shape 3, 936 with 0; 128 channels 911 with shape 2, 961
-// with 0), 256-channel items above (256 channels 1022 with 0, 1194 with 2).
-constexpr int kKbDefaultShape[3] = {3, 2, 0};
+// or two 64-channel blocks, 256-channel items above (64 jobs of 10,000 samples on
+// 64 x 64 pixels, us with shapes 0 / 1 / 2 / 3: 64 channels 845 / 777 / 733 / 725,
+// 128 channels 864 / 799 / 761 / 906, 192 channels 887 / 831 / 952 / 1077, 512
+// channels 1238 / 1176 / 1383 / 1944; one CTA of 128 x 64 x 3 795 at 128).
+constexpr int kKbDefaultShape[3] = {3, 2, 1};
 // channel class of a split field: 64-channel blocks 1, 2, 3-4, 5-8, ... -> 0, 1, 2, 3, ...
 inline int tc_class_of(uint32_t cpad) {
     const uint32_t b = cpad / 64;

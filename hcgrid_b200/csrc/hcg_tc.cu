@@ -40,7 +40,9 @@ __global__ void __launch_bounds__(kTcPersistThreads, 1)
                       unsigned long long *timeouts, unsigned long long *macs) {
     __shared__ TcPShared S;
     if (threadIdx.x == 0) sm100::prefetch_tensormap(&tm);
-    tc_persist<Cfg>(S, J, &tm, nitems, ntiles, timeouts, macs);
+    tc_persist<Cfg>(S, nitems, [&](uint64_t it) {
+        return TcItem{&J, &tm, J.T.t0 + tc_walk(it / J.ncb, ntiles, J.T.ntx, J.strip), (uint32_t)(it % J.ncb)};
+    }, timeouts, macs);
 }
 
 template <class Cfg, bool UNIT>  // UNIT: unit sample weights, FP32 series Gaussian (pair_weights' kPairUnit)

@@ -92,6 +92,8 @@ using TcCfgN4S2 = TcCfg<4, 2, 64>;  // 256 channels per item, 64-slot chunks, 2 
 using TcCfgN2S3 = TcCfg<2, 3, 64>;  // 128 channels, 64-slot chunks, 3 stages
 using TcCfgN1S4 = TcCfg<1, 4, 64>;  // 64 channels, 64-slot chunks, 4 stages
 using TcCfgN4K32 = TcCfg<4, 4, 32>;  // 256 channels, 32-slot chunks, 4 stages
+using TcCfgN2K32 = TcCfg<2, 2, 32>;  // 128 channels, 32-slot chunks, 2 stages: two CTAs an SM
+using TcCfgN1K32 = TcCfg<1, 3, 32>;  // 64 channels, 32-slot chunks, 3 stages: two CTAs an SM
 // 4, 5: shapes 0 and 3 in the persistent kernel (one CTA per SM, epilogue
 // overlapped with the next item)
 static_assert(kTcConfigCount == 6, "hcg_tc_set_config numbers the shapes 0-3 above and 4-5 persistent");
@@ -118,7 +120,6 @@ struct TcJob {
     float *out;
     uint32_t ostride;   // 0: [channel][pixel]; else [pixel][ostride]
     float *wout;
-    const CUtensorMap *out_map;  // 3-D map of the cube (null: direct stores); box = one item
     GridArgs a;                  // geometry of the direct-weight builders (tc_build_weights)
     uint32_t pf;                 // the producer prefetches chunk k + pf into L2 (pf <= stages: k + stages)
     uint32_t strip;              // persistent kernels' tile walk: strips of `strip` tile columns (0: rows)
@@ -394,7 +395,7 @@ __device__ __forceinline__ void tc_mma_seg(SH &S, const TcJob &J, uint32_t nchun
             ok = false;
         }
         tc_fence_after();
-        const uint32_t d_tmem = S.tmem + a * 256u;
+        const uint32_t d_tmem = S.tmem + a * (uint32_t)Cfg::kTmemCols;
         const uint32_t kend = q + 1 == nseg ? nchunks : (q + 1) * (kTcSegSlots / KC);
         uint32_t acc = 0;
         for (; k < kend && ok && !S.abort; ++k) {
@@ -668,7 +669,7 @@ struct TcPShared {
 // Epilogue warps (128 threads, index eb), one item from accumulator `a`:
 // normalise and store straight from registers (16-byte stores along channels
 // for [pixel][channel] cubes; along pixels for [channel][pixel] cubes).
-template <uint32_t KC, class SH, bool WSMEM = false>
+template <class Cfg, class SH, bool WSMEM = false>
 __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64_t tile, uint32_t cblk,
                                                    uint32_t nchunks, uint32_t il, uint32_t &gse, int eb,
                                                    unsigned long long *timeouts) {
@@ -689,7 +690,7 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
     const uint64_t P = (uint64_t)G.nx * G.ny;
     const uint64_t p = (uint64_t)yy * G.nx + xx;
     const float *sc = S.inv_scale[ia];
-    const uint32_t nseg = tc_segments<KC>(nchunks);
+    const uint32_t nseg = tc_segments<Cfg::kK>(nchunks);
     bool store = false;
     float inv = 0.f;
     for (uint32_t q = 0; q < nseg; ++q, ++gse) {
@@ -718,7 +719,7 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
         for (uint32_t cb = 0; cb < 2 * J.nb; ++cb) {
             uint32_t r[32];
             if (nchunks > 0) {
-                tmem_ld_32x32b_x32(S.tmem + a * 256u + ((q4 * 32u) << 16) + cb * 32u, r);
+                tmem_ld_32x32b_x32(S.tmem + a * (uint32_t)Cfg::kTmemCols + ((q4 * 32u) << 16) + cb * 32u, r);
                 tmem_wait_ld();
             } else {
 #pragma unroll
@@ -786,9 +787,18 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
     }
 }
 
-template <class Cfg>
-__device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const CUtensorMap *map, uint64_t nitems, uint64_t ntiles,
-                                           unsigned long long *timeouts, unsigned long long *macs) {
+// One item of a persistent kernel: a tile's channel block of a job (none: skip).
+struct TcItem {
+    const TcJob *J;
+    const CUtensorMap *map;
+    uint64_t tile;
+    uint32_t cblk;
+};
+
+// `item(it)`: the same in every thread.
+template <class Cfg, class ITEM>
+__device__ __forceinline__ void tc_persist(TcPShared &S, uint64_t nitems, ITEM item, unsigned long long *timeouts,
+                                           unsigned long long *macs) {
     using namespace sm100;
     constexpr uint32_t ST = Cfg::kStages, KC = Cfg::kK;
     static_assert(Cfg::kTmemCols <= 256, "two accumulators fit the 512 TMEM columns");
@@ -807,16 +817,19 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const C
         mbar_fence_init();
     }
     if (warp == 1) {
-        tmem_alloc(&S.tmem, 512);
+        tmem_alloc(&S.tmem, 2 * Cfg::kTmemCols);
         tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     uint32_t gk = 0, il = 0, gs = 0, gse = 0;  // chunks, items, MMA and epilogue segments
-    for (uint64_t it = blockIdx.x; it < nitems; it += gridDim.x, ++il) {
-        const uint64_t tile = J.T.t0 + tc_walk(it / J.ncb, ntiles, J.T.ntx, J.strip);
-        const uint32_t cblk = (uint32_t)(it % J.ncb);
+    for (uint64_t it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const TcItem W = item(it);
+        if (!W.J) continue;
+        const TcJob &J = *W.J;
+        const uint64_t tile = W.tile;
+        const uint32_t cblk = W.cblk;
         const uint32_t U = J.T.U[tile];
         const uint32_t nchunks = (U + KC - 1) / KC;
         if (warp == 0) {
@@ -826,15 +839,16 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const C
             for (int j = lane; j < nrt; j += 32) S.ulo[j] = J.T.ulo[tile * kTileMaxRings + j];
             for (int j = lane; j <= nrt; j += 32) S.base[j] = J.T.base[tile * (kTileMaxRings + 1) + j];
             __syncwarp();
-            tc_produce<Cfg>(S, J, map, cblk, U, nchunks, gk, nrt, timeouts);
+            tc_produce<Cfg>(S, J, W.map, cblk, U, nchunks, gk, nrt, timeouts);
         } else if (warp == 1) {
             if (lane == 0) tc_mma_seg<Cfg, true>(S, J, nchunks, gk, gs, timeouts, macs);
         } else if (warp < 6) {
             tc_build<Cfg>(S, J, tile, nchunks, gk, tid - 64, timeouts);
         } else {
-            tc_epilogue_direct<KC>(S, J, tile, cblk, nchunks, il, gse, tid - 192, timeouts);
+            tc_epilogue_direct<Cfg>(S, J, tile, cblk, nchunks, il, gse, tid - 192, timeouts);
         }
         gk += nchunks;
+        ++il;
     }
     // the copies of the last chunks land before the shared memory is given back
     if (tid == 0) {
@@ -850,7 +864,7 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, const TcJob &J, const C
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(S.tmem, 512);
+        tmem_dealloc(S.tmem, 2 * Cfg::kTmemCols);
     }
 }
 
@@ -1176,7 +1190,7 @@ __device__ __forceinline__ void tc_persist_weights(TcDShared &S, const TcJob &J,
         } else if (tid < 64 + kTcDBuilders) {
             tc_build_weights<Cfg, UNIT>(S, J, tile, cblk, U, nchunks, gk, il, tid - 64, timeouts);
         } else {
-            tc_epilogue_direct<KC, TcDShared, true>(S, J, tile, cblk, nchunks, il, gse, tid - (64 + kTcDBuilders),
+            tc_epilogue_direct<Cfg, TcDShared, true>(S, J, tile, cblk, nchunks, il, gse, tid - (64 + kTcDBuilders),
                                                 timeouts);
         }
         gk += nchunks;

@@ -299,11 +299,11 @@ hcg_status hcg_grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs)
 
 /* Pipeline shape of the batch pass's tensor-core kernel, per channel class
  * (the tensor-core classes of hcg_tc_set_pipeline; -1: every class; shape -1
- * restores the default: 3 up to 64 channels, 2 up to 128, 0 above). Every shape
+ * restores the default: 3 up to 64 channels, 2 up to 128, 1 above). Every shape
  * takes 16 x 8-pixel tiles (128 pixels per item, the MMA's M); they differ in channels per item (the MMA's N),
  * sample slots per pipeline chunk and pipeline depth:
  *   0: 256 channels x 32 slots x 4 stages   1: 256 x 64 x 2
- *   2: 128 x 64 x 3                         3: 64 x 64 x 4
+ *   2: 128 x 32 x 2 (two CTAs an SM)        3: 64 x 32 x 3 (two CTAs an SM)
  * The cubes do not depend on the shape. No reference counterpart (HCGrid
  * grids one job per call). */
 #define HCG_BATCH_SHAPES 4
