@@ -462,7 +462,6 @@ hcg_status hcg_field_set_spectra(hcg_field *field, uint32_t nchan, const float *
         CK(ctx, cudaMemcpyAsync(tmp, values, nb, cudaMemcpyHostToDevice, s), "spectra upload");
         dv = tmp;
     }
-    free_split(field, s);  // the split, if any, described the previous spectra
     cudaError_t e = permute_spectra(ctx, field, dv, nchan, layout);
     if (tmp) cudaFreeAsync(tmp, s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "spectra permute");
