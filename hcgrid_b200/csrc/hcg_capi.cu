@@ -278,7 +278,7 @@ hcg_status hcg_context_create(int device, void *stream, hcg_context **out) {
         c->copy_stream = nullptr;
     }
     if (cudaMalloc(&c->d_stats, sizeof(DevStats)) != cudaSuccess ||
-        cudaMallocHost(&c->h_stats, kHostBack) != cudaSuccess || cudaMemset(c->d_stats, 0, sizeof(DevStats)) ||
+        !(c->h_stats = static_cast<DevStats *>(calloc(1, kHostBack))) || cudaMemset(c->d_stats, 0, sizeof(DevStats)) ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         cudaEventCreate(&c->evp[0]) != cudaSuccess || cudaEventCreate(&c->evp[1]) != cudaSuccess ||
         cudaEventCreate(&c->evp[2]) != cudaSuccess || cudaEventCreate(&c->evp[3]) != cudaSuccess) {
@@ -299,7 +299,7 @@ static void ctx_teardown(hcg_context *ctx) {
     ctx->scratch.release(ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->d_stats);
-    cudaFreeHost(ctx->h_stats);
+    free(ctx->h_stats);
     cudaEventDestroy(ctx->ev0);
     cudaEventDestroy(ctx->ev1);
     for (auto &ev : ctx->evp) cudaEventDestroy(ev);

@@ -749,7 +749,7 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         KeyRange range;
         unsigned long long invalid, total, wbits;
     };
-    static_assert(sizeof(Back) <= kHostBack, "read back through the context's page-locked buffer");
+    static_assert(sizeof(Back) <= kHostBack, "read back through the context's host words");
     Back *back = nullptr, *hb = reinterpret_cast<Back *>(ctx->h_stats);
     RingAcc *acc = nullptr;
     // the next `count` elements of an allocation, 256-byte aligned; with a null

@@ -140,7 +140,8 @@ struct hcg_context {
     double last_r = -1, last_res = -1;
     hcg::HpxParams hpx = {};
     hcg::DevStats *d_stats = nullptr;
-    hcg::DevStats *h_stats = nullptr;  // page-locked (kHostBack bytes): what a call reads back
+    hcg::DevStats *h_stats = nullptr;  // host words (kHostBack bytes) that a call reads back; ordinary memory:
+                                   // page-locked, a read-back is 3 us faster and a context 1 to 3 ms slower
     hcg::Scratch scratch;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t evp[4] = {nullptr, nullptr, nullptr, nullptr};  // phase boundaries inside hcg_grid
