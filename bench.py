@@ -948,8 +948,8 @@ def main():
     cube = torch.empty((job.nchan, P) if LAY == api.CHANNEL_MAJOR else (P, job.nchan), dtype=torch.float32,
                        device=dev)
     wts = torch.empty(P, dtype=torch.float32, device=dev)
-    # prep, tile rings, count of overflowed tiles, 3-pass scan, row offsets, weights, sums
-    launches_per_step = 2 if job.nchan == 1 else 9
+    # prep, tile rings (with the entry offsets), weights, sums; prep and the grid kernel
+    launches_per_step = 2 if job.nchan == 1 else 4
 
     tune = None
     if engine != api.ENGINE_FP32 and job.nchan > 1:
@@ -1045,9 +1045,9 @@ def main():
 
     # dominant kernel and its roofline
     tc = engine != api.ENGINE_FP32 and job.nchan > 1
-    phase_names = ["pixel setup", "candidate count+scan", "FP64 weights (k_group)",
+    phase_names = ["pixel setup", "tile tables and candidate counts", "FP64 weights (k_group)",
                    "channel sums (k_tile_tc)" if tc else "channel sums (k_tile_accum)"]
-    kernels = ["k_pixel_prep", "k_group<true>+k_scan_offsets", "k_group<false>", "k_tile_tc" if tc else "k_tile_accum"]
+    kernels = ["k_pixel_prep", "k_tile_rings", "k_group", "k_tile_tc" if tc else "k_tile_accum"]
     if job.nchan == 1:
         phase_names[3] = "single-channel gridding (k_grid_1chan)"
         kernels[3] = "k_grid_1chan"
