@@ -3,7 +3,8 @@
 // Every phase is one persistent launch over the work of all jobs: a fixed
 // number of CTAs per SM pull work items (pixels, 2x2 groups, tiles, tile x
 // channel-slice pairs) from a device-side queue (an atomic head per phase)
-// and look the item's job up in a device job table. Launch shapes do not
+// and look the item's job up in a device job table (the tensor-core launches
+// take every gridDim-th item). Launch shapes do not
 // depend on the batch, and all per-batch state (job table, queue heads,
 // totals, scratch pointers) lives in device memory, so the phases are
 // captured once into two CUDA graphs and replayed for every batch:
@@ -55,7 +56,7 @@ struct JobDesc {
     uint32_t skip;  // routed to the single-job path: no entries, no sums here
 };
 
-enum { Q_TILE = 0, Q_GEOM, Q_ACC, Q_C1, Q_TC, Q_N = Q_TC + kKbShapes };
+enum { Q_TILE = 0, Q_GEOM, Q_ACC, Q_C1, Q_N };
 
 struct BatchHdr {
     uint32_t njobs;

@@ -1097,6 +1097,12 @@ hcg_status hcg_set_coarsening_factor(hcg_context *ctx, uint32_t factor) {
 hcg_status hcg_context_trim(hcg_context *ctx) {
     if (!ctx) return HCG_EINVAL;
     Guard g(ctx);
+    for (int slot : {kScratchKeys, kScratchSort}) {  // the sort's buffers: nothing holds on to them
+        if (slot >= (int)ctx->scratch.ptr.size() || !ctx->scratch.ptr[slot]) continue;
+        cudaFreeAsync(ctx->scratch.ptr[slot], ctx->stream);
+        ctx->scratch.ptr[slot] = nullptr;
+        ctx->scratch.size[slot] = 0;
+    }
     CK(ctx, cudaStreamSynchronize(ctx->stream), "trim");
     if (ctx->pool) CK(ctx, cudaMemPoolTrimTo(ctx->pool, 0), "trim");
     return HCG_OK;

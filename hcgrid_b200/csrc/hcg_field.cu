@@ -800,7 +800,7 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
     TRY(dalloc(&f->d_samples, used, s, ctx->pool));
     mem = static_cast<uint8_t *>(f->d_samples);
     samples();
-    TRY(temp(k0, 25, key_bytes + sizeof(Back)));
+    TRY(temp(k0, kScratchKeys, key_bytes + sizeof(Back)));
     back = reinterpret_cast<Back *>(reinterpret_cast<uint8_t *>(k0) + key_bytes);
     TRY(cudaMemsetAsync(back, 0, sizeof(Back), s));
     k_sample_keys<<<(unsigned)std::min<uint64_t>((n + 255) / 256, 148 * 8), 256, 0, s>>>(
@@ -831,7 +831,7 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
             const size_t word = wide ? 8 : 4, tile = kSortThreads * (wide ? 8 : small ? 4 : 16);
             const size_t nblocks = (n + std::min<size_t>(tile, kSortThreads * 8) - 1) / std::min<size_t>(tile, kSortThreads * 8);
             const size_t pairs = (2 * n * (word + 4) + 255) & ~(size_t)255;
-            TRY(temp(v0, 26, pairs + 256 * nblocks * sizeof(uint32_t) + 8 * 256 * sizeof(unsigned long long)));
+            TRY(temp(v0, kScratchSort, pairs + 256 * nblocks * sizeof(uint32_t) + 8 * 256 * sizeof(unsigned long long)));
             unsigned long long *total = (unsigned long long *)((uint8_t *)v0 + pairs);
             uint32_t *counts = (uint32_t *)(total + 8 * 256), *va = v0 + 2 * n * (word / 4), *vb = va + n;
             uint64_t *const k1 = f->d_keys;

@@ -109,6 +109,7 @@ inline cudaError_t dalloc(T **p, size_t bytes, cudaStream_t s, cudaMemPool_t poo
     return dalloc(reinterpret_cast<void **>(p), bytes, s, pool);
 }
 
+constexpr int kScratchKeys = 25, kScratchSort = 26;  // scratch slots of a field's sort
 // Grow-only device scratch buffers, stream-ordered.
 struct Scratch {
     cudaMemPool_t pool = nullptr;

@@ -148,7 +148,6 @@ struct TcShared {
     uint64_t full_a[kTcMaxStages], full_b[kTcMaxStages], empty[kTcMaxStages], acc_full;
     uint32_t tmem;
     volatile int abort;
-    unsigned long long item;
     uint32_t ulo[kTileMaxRings], base[kTileMaxRings + 1];
     float inv_scale[kTcMaxN];              // the item's channels: 1 / (channel scale * weight scale)
     float4 ring_w[kTcRing * kTcBuilders];  // builders' entry rings, [position][thread]
@@ -882,18 +881,17 @@ __device__ __forceinline__ void tc_persist(TcPShared &S, uint64_t nitems, ITEM i
 // that a warp may run up to two chunks ahead of another (a barrier of all
 // builders per chunk left a fifth of their time waiting: 9.4 against 8.1 ms).
 // For each slot whose sample lies in its
-// pixel's window of the slot's ring (ring_window_mc, the windows the tile pass
+// pixel's window of the slot's ring (the windows the tile pass
 // unioned), a builder evaluates the FP64 distance, cutoff and FP32 Gaussian
 // (pair_weights' arithmetic; UNIT: its kPairUnit form), accumulates the FP64
 // weight sum and writes its hi/lo pieces of the K-major operand row (16-byte
 // stores). The next ring's window is loaded when a ring begins. What bounds it:
 // issue, about 45 instructions a (pixel, slot) pair at three builder warps a
-// scheduler (eight builder warps with more registers, or samples read through
-// L1, were slower: 10.5 and 12.4 against 9.3 ms, as are sixteen at 80 registers,
-// 9.2 against 8.1 ms, on
-// 150,000 samples x 64 channels, 768 x 768 pixels, beam 54 pixels wide; 13.5 ms
-// with FP64 cutoff tests, weights converted to and from FP64, and the window
-// fetched at each ring). The epilogue adds
+// scheduler. 150,000 samples x 64 channels, 768 x 768 pixels, beam 54 pixels
+// wide: 8.1 ms; 9.2 with sixteen builder warps at 80 registers; with the barrier
+// a chunk 9.4, and then 10.5 with eight builder warps and more registers, 12.4
+// with samples read through L1, 13.5 with FP64 cutoff tests, weights converted to
+// and from FP64, and the window fetched at each ring. The epilogue adds
 // the three partial weight sums of a row from shared memory.
 constexpr int kTcGeo = 64;          // slots per chunk of the direct builders
 constexpr int kTcGeoBufs = 3;       // geometry buffers: loads run one chunk ahead of a builder, builders drift by one
