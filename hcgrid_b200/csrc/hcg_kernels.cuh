@@ -50,7 +50,9 @@ __device__ __forceinline__ void prep_item(HpxParams h, uint64_t firstring, uint6
     if (!isfinite(x) || !isfinite(y)) {
         P.ur = 0; P.nr = 0; P.polar = 0;
         for (int e = 0; e < 2; ++e) P.tt[e] = 0.0;
-        P.h = PixHalf{0.0, 1.0, 0.0, 1.0};
+        // a blank pixel accepts no pair, also where coarsening gives it its run's
+        // windows: its haversine is infinite
+        P.h = PixHalf{0.0, 0.0, __longlong_as_double(0x7ff0000000000000ll), 0.0};
         out[p] = P;
         return;
     }
