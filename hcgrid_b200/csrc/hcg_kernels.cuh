@@ -79,6 +79,9 @@ __device__ __forceinline__ void prep_item(HpxParams h, uint64_t firstring, uint6
     P.h.sl *= rc;
     P.h.cl *= rc;
     sincos(P.b1 * 0.5, &P.h.sb, &P.h.cb);
+    // A pixel past a pole (|lat| > 90, cos(lat) < 0) has no such operands: its
+    // haversines are NaN, and pair_band takes each of its pairs by the full formula
+    if (P.cb1 < 0.0) P.h.sl = P.h.cl = __longlong_as_double(0x7ff8000000000000ll);
     out[p] = P;
 }
 
@@ -267,7 +270,7 @@ __device__ __forceinline__ bool ring_window_mc(const GridArgs &a, const RingRec 
     ref_len = 0;
     if (!ring_window(a.h, R, P, a.keys, a.ptab, lo, hi)) return false;
     ref_len = hi > lo ? hi - lo : 0;
-    if (R.lut_lo == 0 || hi <= lo) return true;
+    if (R.lut_lo == 0 || hi <= lo || !(P.cb1 >= 0.0)) return true;  // past a pole the bound does not hold
     // hav(db) >= y^2 (1 - y^2 / 3) with y = db / 2 (sin y >= y - y^3 / 6)
     const double y = 0.5 * fmax(0.0, fmax(R.bmin - P.b1, P.b1 - R.bmax));
     const double hb = y < 1.0 ? y * y * (1.0 - y * y * (1.0 / 3.0)) : 0.0;
@@ -348,9 +351,10 @@ __device__ __forceinline__ GroupGeo group_geo(GET get) {
         const double lp = P->l1 - 2.0 * kPi * floor(P->l1 * (0.5 / kPi));
         G.lmin = fmin(G.lmin, lp);
         G.lmax = fmax(G.lmax, lp);
-        G.bmin = fmin(G.bmin, P->b1);
-        G.bmax = fmax(G.bmax, P->b1);
-        G.icb = P->icb1 >= 0.f ? fmaxf(G.icb, P->icb1) : __int_as_float(0x7f800000);
+        const bool past = !(P->icb1 >= 0.f);  // past a pole: no bound, in latitude neither
+        G.bmin = fmin(G.bmin, past ? -1e300 : P->b1);
+        G.bmax = fmax(G.bmax, past ? 1e300 : P->b1);
+        G.icb = past ? __int_as_float(0x7f800000) : fmaxf(G.icb, P->icb1);
     }
     if (G.lmax - G.lmin > kPi) G.icb = __int_as_float(0x7f800000);  // the group straddles phi = 0
     return G;
@@ -550,6 +554,12 @@ __device__ __forceinline__ double exp2_small(double t) {
     return __hiloint2double(__double2hiint(p) + (__double2loint(k) << 20), __double2loint(p));
 }
 
+__device__ __forceinline__ double ellipse_xy(const GridArgs &a, double x, double y, double &n2) {
+    const double ys = y * a.cpa - x * a.spa, xc = x * a.cpa + y * a.spa;
+    n2 = x * x + y * y;
+    return (a.p0 * a.p0) * (ys * ys) + (a.kp1 * a.kp1) * (xc * xc);
+}
+
 // GAUSS2D's ellipse term of a pair, as a quotient: (sigma_maj sin)^2 +
 // (sigma_min cos)^2 of (bearing - PA), times n2, which is returned beside it
 // (kernel_other derives the bearing's tangent y / x).
@@ -559,9 +569,7 @@ __device__ __forceinline__ double ellipse(const GridArgs &a, const PixHalf &q, d
     const double cb = q.cb * sb2.y + q.sb * sb2.x;  // cos((b1 - b2) / 2)
     const double y = -2.0 * (v.sl * cl);
     const double x = 2.0 * (2.0 * (q.sb * q.cb) * (v.sl * v.sl) - cb1 * v.sb * cb);
-    const double ys = y * a.cpa - x * a.spa, xc = x * a.cpa + y * a.spa;
-    n2 = x * x + y * y;
-    return (a.p0 * a.p0) * (ys * ys) + (a.kp1 * a.kp1) * (xc * xc);
+    return ellipse_xy(a, x, y, n2);
 }
 
 // 1 / x, x >= 1e-300: the hardware's approximation (20 bits) and three
@@ -573,6 +581,13 @@ __device__ __forceinline__ double reciprocal(double x) {
 #pragma unroll
     for (int i = 0; i < 3; ++i) r = fma(r, fma(-x, r, 1.0), r);
     return r;
+}
+
+// GAUSS2D from its ellipse term.
+__device__ __forceinline__ double gauss2d(const GridArgs &a, double num, double n2, double d2) {
+    const double ell = n2 > 0.0 ? num / n2 : 0.0;
+    const double pp = a.p0 * a.kp1;
+    return exp(-0.5 * d2 * ell / (pp * pp));
 }
 
 // The grid kernels other than GAUSS1D (gridding.cu:242-256), FP64, for an
@@ -592,9 +607,7 @@ __device__ __forceinline__ double kernel_other(const GridArgs &a, const PixHalf 
     if (a.ktype == HCG_GAUSS2D) {
         double n2;
         const double num = ellipse(a, q, cb1, v, sl2, sb2, n2);
-        const double ell = n2 > 0.0 ? num / n2 : 0.0;
-        const double pp = p0 * p1;
-        return exp(-0.5 * d2 * ell / (pp * pp));
+        return gauss2d(a, num, n2, d2);
     }
     const double arg = kPi * sqrt(d2) / p0;
     const double x = arg / p2;
@@ -617,7 +630,8 @@ __device__ __forceinline__ double kernel_at(const GridArgs &a, const PixHalf &q,
 }
 
 // A pair near the cutoff (rare): inside the band [hlo, hhi] the reference's
-// full formula decides. Out of line, by value and from memory again, so that the
+// full formula decides, and for pixels past a pole (NaN haversine) it decides
+// every pair. Out of line, by value and from memory again, so that the
 // loop around it keeps nothing for it.
 template <bool F32, bool GEN>
 __device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t idx) {
@@ -630,9 +644,15 @@ __device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t 
         if (F32 && !GEN && a.series32) return win * (double)gauss_series_f32((float)v.h, a.x2c);
         return kernel_at<F32, GEN>(a, Q.h, Q.cb1, v, sl2, sb2, win, pair_d2(a, v.h));
     }
-    const double d = dist_deg(Q.l1, Q.b1, Q.cb1, __ldg(a.l2 + idx), __ldg(a.b2 + idx),
-                              __ldg(a.cb2 + idx));
+    const double l2 = __ldg(a.l2 + idx), b2 = __ldg(a.b2 + idx), cb2 = __ldg(a.cb2 + idx);
+    const double d = dist_deg(Q.l1, Q.b1, Q.cb1, l2, b2, cb2);
     if (!(d < a.sphere_radius)) return 0.0;
+    if (GEN && a.ktype == HCG_GAUSS2D) {  // the bearing from the positions as well
+        double n2;
+        const double num = ellipse_xy(a, Q.cb1 * sin(b2) - sin(Q.b1) * cb2 * cos(l2 - Q.l1), cb2 * sin(l2 - Q.l1), n2);
+        const double k = gauss2d(a, num, n2, d * d);
+        return win * (F32 ? (double)(float)k : k);
+    }
     return kernel_at<F32, GEN>(a, Q.h, Q.cb1, v, sl2, sb2, win, d * d);
 }
 
@@ -660,7 +680,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
         for (int i = 0; i < 4; ++i) {
             const float hf = (float)v[i].h;
             acc[i] = in[i] && hf < a.hlo32;
-            if (in[i] && !acc[i] && hf <= a.hhi32) band |= 1u << i;
+            if (in[i] && !acc[i] && !(hf > a.hhi32)) band |= 1u << i;
         }
         if (F32) {
 #pragma unroll
@@ -683,7 +703,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             acc[i] = in[i] && v[i].h < a.hlo;
-            if (in[i] && !acc[i] && v[i].h <= a.hhi) band |= 1u << i;
+            if (in[i] && !acc[i] && !(v[i].h > a.hhi)) band |= 1u << i;
         }
         if (F32 && !GEN && a.series32) {
 #pragma unroll

@@ -1081,7 +1081,7 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
                         // as pair_weights with kPairUnit
                         const float hf = (float)h;
                         const bool acc = inw && hf < hlo32;
-                        if (inw && !acc && hf <= hhi32) band |= 1u << e;
+                        if (inw && !acc && !(hf > hhi32)) band |= 1u << e;
                         wv[e] = acc ? gauss_series_f32(hf, a.x2c) : 0.f;
                         wsum += (double)wv[e];
                         within += acc;
@@ -1095,7 +1095,7 @@ __device__ __forceinline__ void tc_build_weights(TcDShared &S, const TcJob &J, u
                             ex = gauss_f32(d * d * p0);
                         }
                         const bool acc = inw && h < hlo;
-                        if (inw && h >= hlo && h <= hhi) band |= 1u << e;
+                        if (inw && !acc && !(h > hhi)) band |= 1u << e;
                         const double wt = acc ? S.g_w[b][s8 * 8 + half * 4 + e] * (double)ex : 0.0;
                         wv[e] = (float)wt;
                         wsum += wt;
