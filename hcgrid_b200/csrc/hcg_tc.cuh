@@ -52,6 +52,7 @@
 #include <cuda_fp16.h>
 
 #include "hcg_kernels.cuh"
+#include "hcg_segments.h"
 #include "hcg_sm100.cuh"
 
 namespace hcg {
@@ -351,27 +352,6 @@ __device__ __forceinline__ bool tc_mma(SH &S, const TcJob &J, uint32_t nchunks, 
     return ok;
 }
 
-// Accumulation segments of the persistent kernels: the tensor cores' FP32
-// accumulation drops low bits of the products it adds (the sums come out low
-// by up to ~2^-24 of the running sum per MMA), so long K loops drift. An
-// item's chunks are accumulated in segments of kTcSegSlots staged slots (the
-// last one also takes a remainder of up to half a segment), each in a fresh
-// accumulator (the two TMEM halves in turn), and the epilogue adds the
-// segments with round-to-nearest FP32 adds (in the cube buffer) before it
-// normalises them.
-constexpr uint32_t kTcSegSlots = 1024;
-// The one-item kernels (k_tile_tc, the batch kernel) accumulate an item in one
-// segment: they take tiles of at most this many staged slots (longer ones go to
-// the persistent kernels).
-constexpr uint32_t kTcOneSegmentSlots = 1536;
-
-// segments of an item of `nchunks` chunks of KC slots
-template <uint32_t KC>
-__host__ __device__ constexpr uint32_t tc_segments(uint32_t nchunks) {
-    constexpr uint32_t seg = kTcSegSlots / KC;  // chunks per segment
-    return nchunks > seg + seg / 2 ? (nchunks + seg / 2 - 1) / seg : 1;
-}
-
 // MMA issue (one thread) of one item in segments; `gs` counts the CTA's
 // segments (accumulator gs & 1, barriers acc_full / acc_empty by parity).
 // AMN: the weight operand is MN-major (the entries builders, tc_build), else
@@ -384,7 +364,7 @@ __device__ __forceinline__ void tc_mma_seg(SH &S, const TcJob &J, uint32_t nchun
     const TcStage<Cfg> st{tc_smem_base()};
     const uint32_t idesc =
         AMN ? idesc_f16_mnmaj_a_mnmaj_b(J.fmt, kTcM, 64 * J.nb) : idesc_f16_kmaj_a_mnmaj_b(J.fmt, kTcM, 64 * J.nb);
-    const uint32_t nseg = tc_segments<KC>(nchunks);
+    const uint32_t nseg = tc_segments(KC, nchunks);
     bool ok = true;
     uint32_t k = 0, issued = 0;
     for (uint32_t q = 0; q < nseg; ++q, ++gs) {
@@ -395,7 +375,7 @@ __device__ __forceinline__ void tc_mma_seg(SH &S, const TcJob &J, uint32_t nchun
         }
         tc_fence_after();
         const uint32_t d_tmem = S.tmem + a * (uint32_t)Cfg::kTmemCols;
-        const uint32_t kend = q + 1 == nseg ? nchunks : (q + 1) * (kTcSegSlots / KC);
+        const uint32_t kend = tc_segment_end(nchunks, nseg, q);
         uint32_t acc = 0;
         for (; k < kend && ok && !S.abort; ++k) {
             const uint32_t g = gk + k, s = g % ST, ph = (g / ST) & 1;
@@ -689,7 +669,7 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
     const uint64_t P = (uint64_t)G.nx * G.ny;
     const uint64_t p = (uint64_t)yy * G.nx + xx;
     const float *sc = S.inv_scale[ia];
-    const uint32_t nseg = tc_segments<Cfg::kK>(nchunks);
+    const uint32_t nseg = tc_segments(Cfg::kK, nchunks);
     bool store = false;
     float inv = 0.f;
     for (uint32_t q = 0; q < nseg; ++q, ++gse) {
