@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(128, kRingCtas) kb_tile_rings(BatchHdr *H, con
         if (it >= H->tot_tile) return;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.tile_base; });
         const JobGeo &J = S.load(jobs[j], j, cur);
-        tile_rings_item<4>(J.a, J.g, J.T, it - jobs[j].tile_base);
+        tile_rings_item<4, false>(J.a, J.g, J.T, it - jobs[j].tile_base);
     }
 }
 
@@ -295,9 +295,9 @@ __global__ void __launch_bounds__(kGroupThreads, 4) kb_1chan(BatchHdr *H, const 
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.c1_base; });
         const JobDesc &J = jobs[j];
         if (J.a.unit_w && J.a.exp2ok)  // GAUSS1D jobs only
-            grid1_item<kPairUnit>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp], pc);
+            grid1_item<kPairUnit, false>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp], pc);
         else
-            grid1_item<kPairGeneral>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp], pc);
+            grid1_item<kPairGeneral, false>(J.a, J.g.nx, J.g.ny, J.spec, J.cstride, J.out, J.wout, it - J.c1_base, S[warp], pc);
     }
     flush_counts(pc, stats);
 }

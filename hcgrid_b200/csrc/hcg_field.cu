@@ -464,9 +464,9 @@ __global__ void k_ring_no_tables(RingRec *__restrict__ rings, uint64_t usedrings
     if (k < usedrings) rings[k].span = 0, rings[k].tbl = 0;
 }
 
-// The rings' window records.
+// The rings' window records (before k_ring_no_tables).
 __global__ void k_ring_windows(HpxParams h, uint64_t firstring, uint64_t usedrings, const RingRec *__restrict__ rings,
-                               RingWin *__restrict__ out) {
+                               bool tables, RingWin *__restrict__ out) {
     const uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (k >= usedrings) return;
     const RingRec R = rings[k];
@@ -483,7 +483,7 @@ __global__ void k_ring_windows(HpxParams h, uint64_t firstring, uint64_t usedrin
     w.pmin = R.pmin;
     w.span = R.span;
     const bool centred = r >= h.nside && r <= 3 * h.nside && ((r + h.nside) & 1);
-    w.tbl = R.tbl | (R.eq ? kRingEq : 0) | (centred ? 0 : kRingHalf);
+    w.tbl = (tables ? R.tbl : (uint32_t)R.startpix) | (R.eq ? kRingEq : 0) | (centred ? 0 : kRingHalf);
     out[k] = w;
 }
 
@@ -871,17 +871,18 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         // entries (HCG_RING_TABLE_MAX overrides; 0 keeps the binary searches).
         uint64_t cap = std::max<uint64_t>(1ull << 24, 4 * n);
         if (const char *v = getenv("HCG_RING_TABLE_MAX")) cap = strtoull(v, nullptr, 10);
-        if (hb->total > 0 && hb->total <= cap &&
-            dalloc(&f->d_ptab, hb->total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess) {
+        const bool tables = hb->total > 0 && hb->total <= cap &&
+                            dalloc(&f->d_ptab, hb->total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess;
+        if (f->hpx.order <= kQuickOrder)
+            k_ring_windows<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_rings, tables, f->d_rwin);
+        else
+            f->d_rwin = nullptr;  // the general windows
+        if (tables) {
             k_ring_ptab<<<nblk, 256, 0, s>>>(f->hpx, n, f->firstring, f->d_rings, f->d_keys, f->d_ptab);
-            if (f->hpx.order <= kQuickOrder) {
-                k_ring_windows<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_rings, f->d_rwin);
-            }
         } else {
             cudaGetLastError();
             k_ring_no_tables<<<rblocks, 256, 0, s>>>(f->d_rings, f->usedrings);
         }
-        if (!f->d_ptab || f->hpx.order > kQuickOrder) f->d_rwin = nullptr;  // the general windows
         TRY(cudaGetLastError());
         f->ptab_entries = f->d_ptab ? hb->total : 0;
     }

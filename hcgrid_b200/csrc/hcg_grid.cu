@@ -46,15 +46,15 @@ __global__ void k_pixel_prep(HpxParams h, uint64_t firstring, uint64_t usedrings
     if (p < npixmap) prep_item(h, firstring, usedrings, disc, X, Y, out, stats, p);
 }
 
-template <int MODE>  // as pair_weights
-__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_grid_1chan(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+template <int MODE, bool TABLES>  // as pair_weights, group_windows_any
+__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_grid_1chan(const __grid_constant__ GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
                                                         const float *__restrict__ data, uint32_t cstride,
                                                         float *__restrict__ out, float *__restrict__ wout) {
     __shared__ GroupShared S[kGroupWarps];
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
     const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
-    if (grp < ngroups) grid1_item<MODE>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
+    if (grp < ngroups) grid1_item<MODE, TABLES>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
     flush_counts(pc, a.stats);
 }
 
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroup
 // weights (0)
 template <int MODE, int PACK>
 __global__ void __launch_bounds__(kWeightThreads, MODE == kPairUnit ? kWeightCtas : 4)
-    k_group(GridArgs a, GroupArgs g, const unsigned long long *__restrict__ off, uint32_t *__restrict__ e_idx,
+    k_group(const __grid_constant__ GridArgs a, GroupArgs g, const unsigned long long *__restrict__ off, uint32_t *__restrict__ e_idx,
             float4 *__restrict__ e_w, uint32_t *__restrict__ cnt, double *__restrict__ wsum, TileArgs tiles, bool tiled) {
     __shared__ TileGroupShared S;
     PairCounts pc;
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(kWeightThreads, MODE == kPairUnit ? kWeightCta
 }
 
 // Candidate counts of the groups whose tile's ring span exceeds the tile table.
-__global__ void __launch_bounds__(kGroupThreads) k_group_count(GridArgs a, GroupArgs g, uint32_t *__restrict__ cap) {
+__global__ void __launch_bounds__(kGroupThreads) k_group_count(const __grid_constant__ GridArgs a, GroupArgs g, uint32_t *__restrict__ cap) {
     __shared__ GroupShared S[kGroupWarps];
     const int warp = threadIdx.x >> 5;
     for (uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp; grp < g.ngroups; grp += gridDim.x * (uint64_t)kGroupWarps)
@@ -92,9 +92,9 @@ __global__ void __launch_bounds__(256) k_group_accum(GroupArgs g, const unsigned
         group_accum_item(g, off, cnt, e_idx, e_w, wsum, spec, nchan, cstride, out, ostride, wout, grp);
 }
 
-template <int W>
-__global__ void __launch_bounds__(32 * W, W == 4 ? kRingCtas : 2) k_tile_rings(GridArgs a, GroupArgs g, TileArgs T) {
-    tile_rings_item<W>(a, g, T, T.t0 + blockIdx.x);
+template <int W, bool TABLES>
+__global__ void __launch_bounds__(32 * W, W == 4 ? kRingCtas : 2) k_tile_rings(const __grid_constant__ GridArgs a, GroupArgs g, TileArgs T) {
+    tile_rings_item<W, TABLES>(a, g, T, T.t0 + blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kTileThreads, 1) k_tile_accum(GroupArgs g, TileArgs T,
@@ -204,9 +204,10 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         const uint64_t ngroups = (uint64_t)((t->nx + 1) / 2) * ((t->ny + 1) / 2);
         const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
         const int mode = pair_mode1(f, a);
-        auto grid1 = mode == kPairOther ? k_grid_1chan<kPairOther>
-                     : mode == kPairUnit ? k_grid_1chan<kPairUnit>
-                                         : k_grid_1chan<kPairGeneral>;
+        const bool tab = table_windows(a);
+        auto grid1 = mode == kPairOther  ? (tab ? k_grid_1chan<kPairOther, true> : k_grid_1chan<kPairOther, false>)
+                     : mode == kPairUnit ? (tab ? k_grid_1chan<kPairUnit, true> : k_grid_1chan<kPairUnit, false>)
+                                         : (tab ? k_grid_1chan<kPairGeneral, true> : k_grid_1chan<kPairGeneral, false>);
         grid1<<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else {
@@ -255,9 +256,9 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         T.entries = &ctx->d_stats->entries;
         if (e != cudaSuccess) return e;
         if (ntiles <= 148 * 4)
-            k_tile_rings<8><<<(unsigned)ntiles, 256, 0, s>>>(a, g, T);
+            (table_windows(a) ? k_tile_rings<8, true> : k_tile_rings<8, false>)<<<(unsigned)ntiles, 256, 0, s>>>(a, g, T);
         else
-            k_tile_rings<4><<<(unsigned)ntiles, 128, 0, s>>>(a, g, T);
+            (table_windows(a) ? k_tile_rings<4, true> : k_tile_rings<4, false>)<<<(unsigned)ntiles, 128, 0, s>>>(a, g, T);
         cudaEventRecord(ctx->evp[1], s);
         if ((e = cudaMemcpyAsync(ctx->h_stats, ctx->d_stats, sizeof(DevStats), cudaMemcpyDeviceToHost, s)) !=
                 cudaSuccess ||

@@ -55,8 +55,8 @@ struct RingRec {
     double bmin, bmax;
 };
 
-// What the windows of a ring with a pixel table need, in one 64-byte record
-// (RingRec, 104 bytes, serves the general form): the doubles as RingRec has
+// What the windows of a ring need, in one 64-byte record (RingRec, 104 bytes,
+// serves the general form): the doubles as RingRec has
 // them, the chord bounds rounded outwards to floats, and ring-local 32-bit
 // pixel numbers. nside <= 2^26 (kQuickOrder).
 struct __align__(16) RingWin {
@@ -65,9 +65,9 @@ struct __align__(16) RingWin {
     double inv_dp;           // pixels per radian of phi
     float icb;               // >= 1 / cbmin
     float dphi;              // >= RingRec::dphi + 2e-9
-    uint32_t lut_lo, lut_hi;
+    uint32_t lut_lo, lut_hi; // the ring's samples (read where the field has no tables)
     uint32_t pmin, span;     // span 0: no window of the ring holds samples
-    uint64_t tbl;            // table offset | kRingEq | kRingHalf
+    uint64_t tbl;            // table offset, or without tables the ring's first pixel mod 2^32; | kRingEq | kRingHalf
 };
 constexpr uint64_t kRingEq = 1ull << 63;    // equatorial form of the window edges
 constexpr uint64_t kRingHalf = 1ull << 62;  // first pixel centre half a pixel from phi 0
@@ -185,7 +185,7 @@ struct hcg_field {
     uint32_t *d_ptab = nullptr;   // per-ring pixel tables (RingRec::tbl), or none when too large
     uint64_t ptab_entries = 0;
     hcg::RingRec *d_rings = nullptr;
-    hcg::RingWin *d_rwin = nullptr;  // the rings' window records, or none (no tables, nside > 2^26)
+    hcg::RingWin *d_rwin = nullptr;  // the rings' window records, or none (nside > 2^26)
     float *d_spec = nullptr;      // [n][cstride], sorted (spec_bytes: followed by the channel maxima's words)
     bool amax_set = false;        // those hold the present spectra's maxima and non-finite count (SpecMax)
     uint32_t nchan = 0, cstride = 0;

@@ -188,7 +188,7 @@ struct GridArgs {
     double sphere_radius, p0;
     DevStats *stats;
     const double2 *half;  // sorted samples' pair operands (hcg_field::d_half)
-    const uint32_t *ptab; // per-ring pixel tables (RingRec::tbl)
+    const uint32_t *ptab; // per-ring pixel tables (RingRec::tbl), or null: too large for the field
     double hlo, hhi;      // haversine thresholds bracketing sphere_radius (see grid_args)
     int series;           // d^2 from the arcsine-squared series (small sphere_radius)
     double hpolar;        // haversine bound of every accepted pair (chord windows)
@@ -197,7 +197,7 @@ struct GridArgs {
     uint32_t ktype;       // HCG_GAUSS1D, HCG_GAUSS2D or HCG_TAPERED_SINC
     int ktaper;           // TAPERED_SINC with HCG_TAPER_FIX
     double kp1, kp2;      // second and third kernel parameters (p0 is the first)
-    const RingWin *rwin;  // the rings' window records (null: ring_window_mc's general form only)
+    const RingWin *rwin;  // the rings' window records (null: nside > 2^26, the general form only)
     uint64_t firstring;
     float hpolar32;       // >= hpolar
     int unit_w;           // every sample weight is 1
@@ -293,13 +293,12 @@ __device__ __forceinline__ bool ring_window_mc(const GridArgs &a, const RingRec 
     return true;
 }
 
-// Out of line and by value, so that only a thread that comes here stores its
-// arguments.
+// Out of line: the loops around it keep nothing for it.
 struct RingWindow {
     uint32_t lo, hi, ref_len;
     bool ok;
 };
-__device__ __noinline__ RingWindow ring_window_call(GridArgs a, PixPrep P, int k) {
+__device__ __noinline__ RingWindow ring_window_call(const GridArgs &a, const PixPrep &P, int k) {
     RingWindow w;
     w.ok = ring_window_mc(a, a.rings[k], P, w.lo, w.hi, w.ref_len);
     return w;
@@ -361,7 +360,7 @@ __device__ __forceinline__ GroupGeo group_geo(GET get) {
 }
 
 // The windows of a group's four pixels in the field's ring k in the general
-// form, for fields without window records and stray edges.
+// form, for fields without window records (nside > 2^26) and stray edges.
 __device__ __forceinline__ void group_windows_general(const GridArgs &a, int k, const GroupGeo &G, uint64_t pix0,
                                                       uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
                                                       uint32_t &skips) {
@@ -379,6 +378,28 @@ __device__ __forceinline__ void group_windows_general(const GridArgs &a, int k, 
     }
 }
 
+// First sample of a ring ([first, last), pixels from `start` on) at or after each of
+// N ring-local pixels: N binary searches in step, so that their loads are in flight
+// together.
+template <int N>
+__device__ __forceinline__ void lower_bounds(const uint64_t *__restrict__ keys, uint32_t first, uint32_t last,
+                                             uint32_t start, const uint32_t (&pix)[N], uint32_t (&at)[N]) {
+    // ring-local pixels are at most 2^28: the keys' low words decide
+    const uint32_t *key = reinterpret_cast<const uint32_t *>(keys);
+#pragma unroll
+    for (int i = 0; i < N; ++i) at[i] = first;
+    uint32_t n = last - first;
+    for (; n > 1; n -= n / 2) {
+        uint32_t v[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = __ldg(key + 2 * (uint64_t)(at[i] + n / 2 - 1)) - start;
+#pragma unroll
+        for (int i = 0; i < N; ++i) at[i] += v[i] < pix[i] ? n / 2 : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) at[i] += n && __ldg(key + 2 * (uint64_t)at[i]) - start < pix[i] ? 1 : 0;
+}
+
 // The windows of a group's four pixels in the field's ring k from its 64-byte
 // record: the reference window of each pixel (ring_window's integers, from the
 // same rounded operations on ring-local 32-bit pixel numbers; an edge that
@@ -390,6 +411,12 @@ __device__ __forceinline__ void group_windows_general(const GridArgs &a, int k, 
 // windows' lengths, `skips` such rings. What bounds it: instruction issue; a
 // general window takes about 600 instructions (four FP64 divisions, a root,
 // 64-bit pixel numbers, a 104-byte record), a group's four here about 300.
+// TABLE: the first sample at or after a pixel from the ring's pixel table, else
+// (fields too sparse for tables, or with rings that span the circle) by the group's
+// ten binary searches in step. 2,000,000 samples on 1200 x 1200 pixels, 10 a beam,
+// a pass with one channel / 16 channels on the FP32 engine: 2.78 / 5.66 ms; 5.66 /
+// 8.73 with a general window for each pixel in turn, 4.56 / 6.03 with one a thread.
+template <bool TABLE>
 __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &R, int k, const GroupGeo &G,
                                               uint64_t pix0, uint32_t nx, uint32_t lo[4], uint32_t hi[4],
                                               uint32_t &ref, uint32_t &skips) {
@@ -398,9 +425,10 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
     const bool eq = (R.tbl & kRingEq) != 0;
     const int i4 = eq ? 4 * ns : 4 * min(ring, 4 * ns - ring);  // pixels of the ring
     const int span = (int)R.span, pmin = (int)R.pmin;
-    const uint32_t *t = a.ptab + (R.tbl & kRingTbl);
+    const uint32_t *t = a.ptab + (TABLE ? R.tbl & kRingTbl : 0);
     auto first_of = [&](int pix) { return __ldg(t + max(0, min(pix - pmin, span))); };  // first sample at or after pix
     uint32_t clo = 0, chi = 0xffffffffu;
+    int cl = 0, ch = i4;  // !TABLE: the chord's first pixel and the one after its last
     if (span) {
         const float y = 0.5f * (float)fmax(0.0, fmax(R.bmin - G.bmax, G.bmin - R.bmax));
         const float hb = y < 1.f ? y * y * (1.f - y * y * (1.f / 3.f)) * (1.f - 1e-6f) : 0.f;
@@ -413,8 +441,13 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
             const double w = (double)W * R.inv_dp + 1e-4, s = (R.tbl & kRingHalf) ? 0.5 : 0.0;
             const int jl = __double2int_ru(G.lmin * R.inv_dp - s - w), jh = __double2int_rd(G.lmax * R.inv_dp - s + w);
             if (jl >= 0 && jh < i4 && jh - jl + 1 < i4) {  // else: wraps, the reference windows stay
-                clo = first_of(jl);
-                chi = first_of(jh + 1);
+                if (TABLE) {
+                    clo = first_of(jl);
+                    chi = first_of(jh + 1);
+                } else {
+                    cl = jl;
+                    ch = jh + 1;
+                }
             }
         }
     }
@@ -458,7 +491,25 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
         return;
     }
     uint32_t rl[4] = {0, 0, 0, 0}, rh[4] = {0, 0, 0, 0};
-    if (span) {  // else no samples, or the first used ring (the reference's search returns "none")
+    if (!TABLE && span) {
+        uint32_t pix[10], at[10];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool whole = G.polar >> q & 1u;
+            pix[q] = whole ? 0u : (uint32_t)e0[q];
+            pix[4 + q] = whole ? (uint32_t)i4 : (uint32_t)(e1[q] + 1);
+        }
+        pix[8] = (uint32_t)cl;
+        pix[9] = (uint32_t)max(ch, 0);
+        lower_bounds(a.keys, R.lut_lo, R.lut_hi, (uint32_t)R.tbl, pix, at);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            rl[q] = at[q];
+            rh[q] = at[4 + q];
+        }
+        clo = at[8];
+        chi = min(chi, at[9]);
+    } else if (span) {  // else no samples, or the first used ring (the reference's search returns "none")
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const bool whole = G.polar >> q & 1u;
@@ -473,6 +524,39 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
         ref += act ? h - rl[q] : 0u;
         lo[q] = act ? max(rl[q], clo) : 0u;
         hi[q] = act ? max(lo[q], min(h, chi)) : 0u;
+    }
+}
+
+// The form for the field, or TABLES: the table's (the call of the others costs a
+// kernel registers: 4,000,000 samples on 1200 x 1200 pixels, single channel, 1982
+// against 1967 us). The searches are out of line.
+struct GroupWin {
+    uint32_t lo[4], hi[4], ref, skips;
+};
+__device__ __noinline__ GroupWin group_windows_search(const GridArgs &a, GroupGeo G, int k, uint64_t pix0,
+                                                      uint32_t nx) {
+    GroupWin w;
+    w.ref = w.skips = 0;
+    group_windows<false>(a, a.rwin[k], k, G, pix0, nx, w.lo, w.hi, w.ref, w.skips);
+    return w;
+}
+template <bool TABLES>
+__device__ __forceinline__ void group_windows_any(const GridArgs &a, int k, const GroupGeo &G, uint64_t pix0,
+                                                  uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
+                                                  uint32_t &skips) {
+    if (TABLES || (a.ptab && a.rwin)) {
+        group_windows<true>(a, a.rwin[k], k, G, pix0, nx, lo, hi, ref, skips);
+    } else if (a.rwin) {
+        const GroupWin w = group_windows_search(a, G, k, pix0, nx);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            lo[q] = w.lo[q];
+            hi[q] = w.hi[q];
+        }
+        ref += w.ref;
+        skips += w.skips;
+    } else {
+        group_windows_general(a, k, G, pix0, nx, lo, hi, ref, skips);
     }
 }
 
@@ -634,7 +718,7 @@ __device__ __forceinline__ double kernel_at(const GridArgs &a, const PixHalf &q,
 // every pair. Out of line, by value and from memory again, so that the
 // loop around it keeps nothing for it.
 template <bool F32, bool GEN>
-__device__ __noinline__ double pair_band(GridArgs a, const PixPrep *P, uint32_t idx) {
+__device__ __noinline__ double pair_band(const GridArgs &a, const PixPrep *P, uint32_t idx) {
     const PixPrep Q = *P;
     const double2 sl2 = __ldg(a.half + idx), sb2 = __ldg(a.half + a.n + idx);
     const double win = __ldg(a.w + idx);
@@ -764,6 +848,8 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
     }
 }
 
+// The windows of the field's rings are those of pixel tables.
+inline bool table_windows(const GridArgs &a) { return a.ptab && a.rwin; }
 // The single-channel and the multi-channel pair mode of a field.
 inline int pair_mode1(const hcg_field *f, const GridArgs &a) {
     return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.exp2ok ? kPairUnit : kPairGeneral;
@@ -912,16 +998,15 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
 
 // Windows of this lane's ring k of a group computed from the pixels in the
 // warp's shared memory.
+template <bool TABLES>
 __device__ __forceinline__ void group_lane_windows(const GridArgs &a, const GroupGeo &G, int k, uint64_t pix0,
                                                    uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
                                                    uint32_t &skips) {
     if (k > G.r1) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) lo[q] = hi[q] = 0;
-    } else if (a.rwin) {
-        group_windows(a, a.rwin[k], k, G, pix0, nx, lo, hi, ref, skips);
     } else {
-        group_windows_general(a, k, G, pix0, nx, lo, hi, ref, skips);
+        group_windows_any<TABLES>(a, k, G, pix0, nx, lo, hi, ref, skips);
     }
 }
 
@@ -958,7 +1043,7 @@ __device__ __forceinline__ void flush_counts(const PairCounts &c, DevStats *stat
 // Single channel: one warp per 2x2 group of pixels, FP64 throughout: the
 // windows (a ring per lane, four pixels each), every union candidate against
 // the four pixels, normalise. Warp-collective.
-template <int MODE>
+template <int MODE, bool TABLES>
 __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint32_t ny,
                                            const float *__restrict__ data, uint32_t cstride, float *__restrict__ out,
                                            float *__restrict__ wout, uint64_t grp, GroupShared &S, PairCounts &pc) {
@@ -974,7 +1059,7 @@ __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint3
         {  // the group's extent is not kept across the pair tests (registers)
             const GroupGeo G = group_geo([&](int q) { return &S.prep[q]; });
             nr = G.r1 - G.r0 + 1;
-            group_lane_windows(a, G, G.r0 + rb + lane, pix0, nx, lo, hi, ref, skips);
+            group_lane_windows<TABLES>(a, G, G.r0 + rb + lane, pix0, nx, lo, hi, ref, skips);
         }
         group_rounds<false, MODE>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u, data, cstride,
                                   [&](float v, uint32_t, const double w[4], const float[4], const bool nz[4]) {
@@ -1106,7 +1191,7 @@ __device__ __forceinline__ void group_count_item(const GridArgs &a, const GroupA
     unsigned long long count = 0;
     for (int rb = G.r0; rb <= G.r1; rb += 32) {
         uint32_t lo[4], hi[4], ref = 0, skips = 0, glo = 0xffffffffu, ghi = 0;
-        group_lane_windows(a, G, rb + lane, pix0, g.nx, lo, hi, ref, skips);
+        group_lane_windows<false>(a, G, rb + lane, pix0, g.nx, lo, hi, ref, skips);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             if (hi[q] > lo[q]) {
@@ -1236,7 +1321,7 @@ __device__ __forceinline__ void group_tile_item(const GridArgs &a, const GroupAr
                         return (!(q & 1) || xin) && (!(q >> 1) || yin) ? a.prep + pix0 + (q & 1) + (uint64_t)(q >> 1) * g.nx
                                                                        : nullptr;
                     });
-                    group_lane_windows(a, G, k, pix0, g.nx, lo, hi, ref, skips);
+                    group_lane_windows<false>(a, G, k, pix0, g.nx, lo, hi, ref, skips);
                 }
             }
             group_rounds<true, MODE>(
@@ -1454,7 +1539,7 @@ __device__ __forceinline__ void group_accum_item(const GroupArgs &g, const unsig
 // W: four warps a tile where the tiles fill the GPU (96 registers, 20 warps an
 // SM), eight where they do not and the latency of one tile is what counts.
 constexpr int kRingCtas = 5;
-template <int W>
+template <int W, bool TABLES>
 __device__ __forceinline__ void tile_rings_item(const GridArgs &a, const GroupArgs &g, const TileArgs &T,
                                                 uint64_t tile) {
     __shared__ uint32_t s_lo[kTileMaxSpan], s_hi[kTileMaxSpan];
@@ -1513,10 +1598,7 @@ __device__ __forceinline__ void tile_rings_item(const GridArgs &a, const GroupAr
     for (int j = warp; j < nrt; j += W) {
         const int k = r0 + j;
         uint32_t lo[4], hi[4], ref = 0;
-        if (a.rwin)
-            group_windows(a, a.rwin[k], k, G, pix0, g.nx, lo, hi, ref, skips);
-        else
-            group_windows_general(a, k, G, pix0, g.nx, lo, hi, ref, skips);
+        group_windows_any<TABLES>(a, k, G, pix0, g.nx, lo, hi, ref, skips);
         cand += ref;
         if (!known) continue;
         if (T.win && j < kWinSpan) {

@@ -44,15 +44,15 @@ __global__ void k_noalloc_prep(HpxParams h, uint64_t firstring, uint64_t usedrin
     if (p < npix) prep_item(h, firstring, usedrings, disc, X, Y, prep, stats, p);
 }
 
-template <int MODE>  // as pair_weights
-__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_noalloc_grid(GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+template <int MODE, bool TABLES>  // as pair_weights, group_windows_any
+__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_noalloc_grid(const __grid_constant__ GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
                                                           const float *__restrict__ data, uint32_t cstride,
                                                           float *__restrict__ out, float *__restrict__ wout) {
     __shared__ GroupShared S[kGroupWarps];
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
     const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
-    if (grp < ngroups) grid1_item<MODE>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
+    if (grp < ngroups) grid1_item<MODE, TABLES>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
     flush_counts(pc, a.stats);
 }
 
@@ -135,9 +135,10 @@ extern "C" hcg_status hcg_grid_noalloc(hcg_context *ctx, const hcg_field *field,
         const uint64_t ngroups = (uint64_t)((target->nx + 1) / 2) * ((target->ny + 1) / 2);
         const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
         const int mode = pair_mode1(field, a);
-        auto grid1 = mode == kPairOther ? k_noalloc_grid<kPairOther>
-                     : mode == kPairUnit ? k_noalloc_grid<kPairUnit>
-                                         : k_noalloc_grid<kPairGeneral>;
+        const bool tab = table_windows(a);
+        auto grid1 = mode == kPairOther  ? (tab ? k_noalloc_grid<kPairOther, true> : k_noalloc_grid<kPairOther, false>)
+                     : mode == kPairUnit ? (tab ? k_noalloc_grid<kPairUnit, true> : k_noalloc_grid<kPairUnit, false>)
+                                         : (tab ? k_noalloc_grid<kPairGeneral, true> : k_noalloc_grid<kPairGeneral, false>);
         grid1<<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride, cube,
                                              weights_out);
         cudaEventRecord(ctx->ev1, s);
