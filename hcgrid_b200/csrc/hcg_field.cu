@@ -871,12 +871,9 @@ cudaError_t build_field(hcg_context *ctx, hcg_field *f, const double *d_lon, con
         // entries (HCG_RING_TABLE_MAX overrides; 0 keeps the binary searches).
         uint64_t cap = std::max<uint64_t>(1ull << 24, 4 * n);
         if (const char *v = getenv("HCG_RING_TABLE_MAX")) cap = strtoull(v, nullptr, 10);
-        const bool tables = hb->total > 0 && hb->total <= cap &&
+        const bool tables = f->hpx.order <= kQuickOrder && hb->total > 0 && hb->total <= cap &&
                             dalloc(&f->d_ptab, hb->total * sizeof(uint32_t), s, ctx->pool) == cudaSuccess;
-        if (f->hpx.order <= kQuickOrder)
-            k_ring_windows<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_rings, tables, f->d_rwin);
-        else
-            f->d_rwin = nullptr;  // the general windows
+        k_ring_windows<<<rblocks, 256, 0, s>>>(f->hpx, f->firstring, f->usedrings, f->d_rings, tables, f->d_rwin);
         if (tables) {
             k_ring_ptab<<<nblk, 256, 0, s>>>(f->hpx, n, f->firstring, f->d_rings, f->d_keys, f->d_ptab);
         } else {

@@ -58,7 +58,7 @@ struct RingRec {
 // What the windows of a ring need, in one 64-byte record (RingRec, 104 bytes,
 // serves the general form): the doubles as RingRec has
 // them, the chord bounds rounded outwards to floats, and ring-local 32-bit
-// pixel numbers. nside <= 2^26 (kQuickOrder).
+// pixel numbers. Pixel tables: nside <= 2^26 (kQuickOrder).
 struct __align__(16) RingWin {
     double t2;
     double bmin, bmax;
@@ -185,7 +185,7 @@ struct hcg_field {
     uint32_t *d_ptab = nullptr;   // per-ring pixel tables (RingRec::tbl), or none when too large
     uint64_t ptab_entries = 0;
     hcg::RingRec *d_rings = nullptr;
-    hcg::RingWin *d_rwin = nullptr;  // the rings' window records, or none (nside > 2^26)
+    hcg::RingWin *d_rwin = nullptr;  // the rings' window records
     float *d_spec = nullptr;      // [n][cstride], sorted (spec_bytes: followed by the channel maxima's words)
     bool amax_set = false;        // those hold the present spectra's maxima and non-finite count (SpecMax)
     uint32_t nchan = 0, cstride = 0;

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "hcg_internal.h"
 #include "hcg_sm100.cuh"
@@ -188,7 +189,7 @@ struct GridArgs {
     double sphere_radius, p0;
     DevStats *stats;
     const double2 *half;  // sorted samples' pair operands (hcg_field::d_half)
-    const uint32_t *ptab; // per-ring pixel tables (RingRec::tbl), or null: too large for the field
+    const uint32_t *ptab; // per-ring pixel tables (RingRec::tbl), or null
     double hlo, hhi;      // haversine thresholds bracketing sphere_radius (see grid_args)
     int series;           // d^2 from the arcsine-squared series (small sphere_radius)
     double hpolar;        // haversine bound of every accepted pair (chord windows)
@@ -197,7 +198,7 @@ struct GridArgs {
     uint32_t ktype;       // HCG_GAUSS1D, HCG_GAUSS2D or HCG_TAPERED_SINC
     int ktaper;           // TAPERED_SINC with HCG_TAPER_FIX
     double kp1, kp2;      // second and third kernel parameters (p0 is the first)
-    const RingWin *rwin;  // the rings' window records (null: nside > 2^26, the general form only)
+    const RingWin *rwin;  // the rings' window records
     uint64_t firstring;
     float hpolar32;       // >= hpolar
     int unit_w;           // every sample weight is 1
@@ -360,7 +361,7 @@ __device__ __forceinline__ GroupGeo group_geo(GET get) {
 }
 
 // The windows of a group's four pixels in the field's ring k in the general
-// form, for fields without window records (nside > 2^26) and stray edges.
+// form, for stray edges.
 __device__ __forceinline__ void group_windows_general(const GridArgs &a, int k, const GroupGeo &G, uint64_t pix0,
                                                       uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
                                                       uint32_t &skips) {
@@ -384,7 +385,7 @@ __device__ __forceinline__ void group_windows_general(const GridArgs &a, int k, 
 template <int N>
 __device__ __forceinline__ void lower_bounds(const uint64_t *__restrict__ keys, uint32_t first, uint32_t last,
                                              uint32_t start, const uint32_t (&pix)[N], uint32_t (&at)[N]) {
-    // ring-local pixels are at most 2^28: the keys' low words decide
+    // ring-local pixels are at most 2^31: the keys' low words decide
     const uint32_t *key = reinterpret_cast<const uint32_t *>(keys);
 #pragma unroll
     for (int i = 0; i < N; ++i) at[i] = first;
@@ -412,23 +413,25 @@ __device__ __forceinline__ void lower_bounds(const uint64_t *__restrict__ keys, 
 // general window takes about 600 instructions (four FP64 divisions, a root,
 // 64-bit pixel numbers, a 104-byte record), a group's four here about 300.
 // TABLE: the first sample at or after a pixel from the ring's pixel table, else
-// (fields too sparse for tables, or with rings that span the circle) by the group's
-// ten binary searches in step. 2,000,000 samples on 1200 x 1200 pixels, 10 a beam,
+// (fields too sparse for tables, or with rings that span the circle, or nside above
+// 2^26) by the group's ten binary searches in step. 2,000,000 samples on 1200 x 1200 pixels, 10 a beam,
 // a pass with one channel / 16 channels on the FP32 engine: 2.78 / 5.66 ms; 5.66 /
 // 8.73 with a general window for each pixel in turn, 4.56 / 6.03 with one a thread.
 template <bool TABLE>
 __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &R, int k, const GroupGeo &G,
                                               uint64_t pix0, uint32_t nx, uint32_t lo[4], uint32_t hi[4],
                                               uint32_t &ref, uint32_t &skips) {
-    const int ns = (int)a.h.nside, ring = (int)(a.firstring + (uint64_t)k);
+    using I = typename std::conditional<TABLE, int, long long>::type;  // tables: nside <= 2^26 (kQuickOrder)
+    auto trunc_u = [](double x) { return TABLE ? (I)__double2uint_rz(x) : (I)__double2ull_rz(x); };
+    const I ns = (I)a.h.nside, ring = (I)(a.firstring + (uint64_t)k);
     const double nsd = (double)ns;
     const bool eq = (R.tbl & kRingEq) != 0;
-    const int i4 = eq ? 4 * ns : 4 * min(ring, 4 * ns - ring);  // pixels of the ring
-    const int span = (int)R.span, pmin = (int)R.pmin;
+    const I i4 = eq ? 4 * ns : 4 * min(ring, (I)(4 * ns - ring));  // pixels of the ring
+    const I span = (I)R.span, pmin = (I)R.pmin;
     const uint32_t *t = a.ptab + (TABLE ? R.tbl & kRingTbl : 0);
-    auto first_of = [&](int pix) { return __ldg(t + max(0, min(pix - pmin, span))); };  // first sample at or after pix
+    auto first_of = [&](I pix) { return __ldg(t + max((I)0, min((I)(pix - pmin), span))); };  // first sample at or after pix
     uint32_t clo = 0, chi = 0xffffffffu;
-    int cl = 0, ch = i4;  // !TABLE: the chord's first pixel and the one after its last
+    I cl = 0, ch = i4;  // !TABLE: the chord's first pixel and the one after its last
     if (span) {
         const float y = 0.5f * (float)fmax(0.0, fmax(R.bmin - G.bmax, G.bmin - R.bmax));
         const float hb = y < 1.f ? y * y * (1.f - y * y * (1.f / 3.f)) * (1.f - 1e-6f) : 0.f;
@@ -439,7 +442,9 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
             // |dphi| <= 2 asin(sqrt(H)) <= 2 sqrt(H / (1 - H)), and a sample lies within dphi of its pixel centre
             const float W = 2.f * sqrtf(__fdividef(H, 1.f - H)) * (1.f + 4e-6f) + R.dphi;
             const double w = (double)W * R.inv_dp + 1e-4, s = (R.tbl & kRingHalf) ? 0.5 : 0.0;
-            const int jl = __double2int_ru(G.lmin * R.inv_dp - s - w), jh = __double2int_rd(G.lmax * R.inv_dp - s + w);
+            const double xl = G.lmin * R.inv_dp - s - w, xh = G.lmax * R.inv_dp - s + w;
+            const I jl = TABLE ? (I)__double2int_ru(xl) : (I)__double2ll_ru(xl);
+            const I jh = TABLE ? (I)__double2int_rd(xh) : (I)__double2ll_rd(xh);
             if (jl >= 0 && jh < i4 && jh - jl + 1 < i4) {  // else: wraps, the reference windows stay
                 if (TABLE) {
                     clo = first_of(jl);
@@ -453,13 +458,13 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
     }
     // straight-line code over the four pixels: the lookups of all of them are
     // in flight together
-    int e0[4], e1[4];
+    I e0[4], e1[4];
     bool stray = false;
     if (eq) {
-        const int c = ((ring - ns) & 1) + 1 + 7 * ns, want = ring - 2 * ns;
+        const I c = ((ring - ns) & 1) + 1 + 7 * ns, want = ring - 2 * ns;
         auto edge = [&](double tt, bool &same) {
             const double t1 = dmul(nsd, dadd(0.5, tt));
-            const int jp = (int)__double2uint_rz(dsub(t1, R.t2)), jm = (int)__double2uint_rz(dadd(t1, R.t2));
+            const I jp = trunc_u(dsub(t1, R.t2)), jm = trunc_u(dadd(t1, R.t2));
             same = same && jp - jm == want;
             return ((jp + jm + c) >> 1) & (i4 - 1);
         };
@@ -473,8 +478,8 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
     } else {
         auto edge = [&](double tt, bool &same) {
             const double tp = dsub(tt, floor(tt));
-            const int ir = (int)__double2uint_rz(dmul(tp, R.t2)) + (int)__double2uint_rz(dmul(dsub(1.0, tp), R.t2)) + 1;
-            const int ip = (int)__double2uint_rz(dmul(tt, (double)ir));
+            const I ir = trunc_u(dmul(tp, R.t2)) + trunc_u(dmul(dsub(1.0, tp), R.t2)) + 1;
+            const I ip = trunc_u(dmul(tt, (double)ir));
             same = same && 4 * ir == i4 && ip < i4;
             return ip;
         };
@@ -500,7 +505,7 @@ __device__ __forceinline__ void group_windows(const GridArgs &a, const RingWin &
             pix[4 + q] = whole ? (uint32_t)i4 : (uint32_t)(e1[q] + 1);
         }
         pix[8] = (uint32_t)cl;
-        pix[9] = (uint32_t)max(ch, 0);
+        pix[9] = (uint32_t)max(ch, (I)0);
         lower_bounds(a.keys, R.lut_lo, R.lut_hi, (uint32_t)R.tbl, pix, at);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -544,9 +549,9 @@ template <bool TABLES>
 __device__ __forceinline__ void group_windows_any(const GridArgs &a, int k, const GroupGeo &G, uint64_t pix0,
                                                   uint32_t nx, uint32_t lo[4], uint32_t hi[4], uint32_t &ref,
                                                   uint32_t &skips) {
-    if (TABLES || (a.ptab && a.rwin)) {
+    if (TABLES || a.ptab) {
         group_windows<true>(a, a.rwin[k], k, G, pix0, nx, lo, hi, ref, skips);
-    } else if (a.rwin) {
+    } else {
         const GroupWin w = group_windows_search(a, G, k, pix0, nx);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -555,8 +560,6 @@ __device__ __forceinline__ void group_windows_any(const GridArgs &a, int k, cons
         }
         ref += w.ref;
         skips += w.skips;
-    } else {
-        group_windows_general(a, k, G, pix0, nx, lo, hi, ref, skips);
     }
 }
 
@@ -849,7 +852,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
 }
 
 // The windows of the field's rings are those of pixel tables.
-inline bool table_windows(const GridArgs &a) { return a.ptab && a.rwin; }
+inline bool table_windows(const GridArgs &a) { return a.ptab != nullptr; }
 // The single-channel and the multi-channel pair mode of a field.
 inline int pair_mode1(const hcg_field *f, const GridArgs &a) {
     return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.exp2ok ? kPairUnit : kPairGeneral;

@@ -1,5 +1,5 @@
-"""Windows of fields without pixel tables: by searches of the sorted samples
-(nside up to 2^26), and in the general form beyond. Pair counts equal to the FP64
+"""Windows of fields without pixel tables: by searches of the sorted samples, in
+32-bit and (nside above 2^26) wider pixel numbers. Pair counts equal to the FP64
 oracle's, cubes and weights within the bounds of the other kernel tests, over caps
 and equator, whole rings, phi = 0, few and many samples a ring, odd and tiny maps."""
 import numpy as np
@@ -24,8 +24,9 @@ CASES = {
     "one_sample": (75.0, -12.0, 1.0, 9, 7, 1800.0, 1),
     "one_pixel": (60.0, 30.0, 0.3, 1, 1, 180.0, 6000),
     "wide_beam": (60.0, 10.0, 30.0, 21, 13, 12000.0, 6000),
-    "general": (75.0, -12.0, 2.5e-5, 21, 19, 0.01, 3000),
-    "general_cap": (300.0, 55.0, 2.5e-5, 21, 19, 0.01, 3000),
+    "fine": (75.0, -12.0, 2.5e-5, 21, 19, 0.01, 3000),
+    "finest": (220.0, -35.0, 1.2e-5, 15, 17, 0.005, 3000),
+    "fine_cap": (300.0, 55.0, 2.5e-5, 21, 19, 0.01, 3000),
 }
 
 
@@ -39,7 +40,7 @@ def test_fields_without_tables(monkeypatch, name, nchan):
     vals = rng.normal(1.0, 0.3, (n, nchan)).astype(np.float32)
     s = fwhm / 3600.0 * synth.FWHM_TO_SIGMA
     g = O.prepare_grid_kernel(s, 3 * s, s / 2)
-    assert (g.hpx.nside > 1 << 26) == name.startswith("general")
+    assert (g.hpx.nside > 1 << 26) == name.startswith("fine")
     ctx = api.Context(0)
     ctx.prepare_grid_kernel(api.GAUSS1D, np.array([s, 0.0, 0.0]), 3 * s, s / 2)
     f = ctx.field(lon, lat)
