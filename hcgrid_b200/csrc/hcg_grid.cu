@@ -47,13 +47,14 @@ __global__ void k_pixel_prep(HpxParams h, uint64_t firstring, uint64_t usedrings
 }
 
 template <int MODE, bool TABLES>  // as pair_weights, group_windows_any
-__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_grid_1chan(const __grid_constant__ GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+__global__ void __launch_bounds__(kGroupThreads, MODE >= kPairEllipse ? 4 : kGroupCtas) k_grid_1chan(const __grid_constant__ GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
                                                         const float *__restrict__ data, uint32_t cstride,
                                                         float *__restrict__ out, float *__restrict__ wout) {
     __shared__ GroupShared S[kGroupWarps];
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
-    const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
+    constexpr int kGroups = kGroupWarps / kGrid1Parts<MODE>;  // of a block
+    const uint64_t grp = blockIdx.x * (uint64_t)kGroups + warp % kGroups;
     if (grp < ngroups) grid1_item<MODE, TABLES>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
     flush_counts(pc, a.stats);
 }
@@ -202,12 +203,15 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
         cudaEventRecord(ctx->evp[1], s);
         cudaEventRecord(ctx->evp[2], s);
         const uint64_t ngroups = (uint64_t)((t->nx + 1) / 2) * ((t->ny + 1) / 2);
-        const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
         const int mode = pair_mode1(f, a);
+        const unsigned nblk = (unsigned)(mode == kPairSlow ? ngroups : (ngroups + kGroupWarps - 1) / kGroupWarps);
         const bool tab = table_windows(a);
-        auto grid1 = mode == kPairOther  ? (tab ? k_grid_1chan<kPairOther, true> : k_grid_1chan<kPairOther, false>)
-                     : mode == kPairUnit ? (tab ? k_grid_1chan<kPairUnit, true> : k_grid_1chan<kPairUnit, false>)
-                                         : (tab ? k_grid_1chan<kPairGeneral, true> : k_grid_1chan<kPairGeneral, false>);
+        auto pick = [&](auto table, auto any) { return tab ? table : any; };
+        auto grid1 = mode == kPairSlow      ? k_grid_1chan<kPairSlow, false>
+                     : mode == kPairEllipse ? pick(k_grid_1chan<kPairEllipse, true>, k_grid_1chan<kPairEllipse, false>)
+                     : mode == kPairSinc    ? pick(k_grid_1chan<kPairSinc, true>, k_grid_1chan<kPairSinc, false>)
+                     : mode == kPairUnit    ? pick(k_grid_1chan<kPairUnit, true>, k_grid_1chan<kPairUnit, false>)
+                                            : pick(k_grid_1chan<kPairGeneral, true>, k_grid_1chan<kPairGeneral, false>);
         grid1<<<nblk, kGroupThreads, 0, s>>>(a, t->nx, t->ny, ngroups, f->d_spec, f->cstride, d_cube, d_wts);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else {
@@ -346,12 +350,12 @@ cudaError_t grid_field(hcg_context *ctx, const hcg_field *f, const hcg_target *t
             TileArgs tt = T;
             tt.t0 = (uint64_t)ch.first * T.ntx;
             const int mode = pair_mode(f, a);
-            auto weights = gc.pack ? (mode == kPairOther  ? k_group<kPairOther, 1>
-                                      : mode == kPairUnit ? k_group<kPairUnit, 1>
-                                                          : k_group<kPairGeneral, 1>)
-                                   : (mode == kPairOther  ? k_group<kPairOther, 0>
-                                      : mode == kPairUnit ? k_group<kPairUnit, 0>
-                                                          : k_group<kPairGeneral, 0>);
+            auto pick = [&](auto packed, auto fp32) { return gc.pack ? packed : fp32; };
+            auto weights = mode == kPairSlow      ? pick(k_group<kPairSlow, 1>, k_group<kPairSlow, 0>)
+                           : mode == kPairEllipse ? pick(k_group<kPairEllipse, 1>, k_group<kPairEllipse, 0>)
+                           : mode == kPairSinc    ? pick(k_group<kPairSinc, 1>, k_group<kPairSinc, 0>)
+                           : mode == kPairUnit    ? pick(k_group<kPairUnit, 1>, k_group<kPairUnit, 0>)
+                                                  : pick(k_group<kPairGeneral, 1>, k_group<kPairGeneral, 0>);
             // two waves of blocks or more: a tile's groups are shared by up to four blocks
             const unsigned parts = gb >= 148 * kWeightCtas * 2 ? 1 : gb >= 148 * kWeightCtas ? 2 : 4;
             weights<<<dim3(gb, parts), kWeightThreads, 0, s>>>(a, gc, off, e_idx, e_w, cnt, wsum, tt, tiled);

@@ -210,6 +210,8 @@ struct GridArgs {
     int w32ok;            // the same for 2^-120: no accepted pair's FP32 weight is zero
     uint64_t n;           // samples
     double spa, cpa;      // GAUSS2D: sine and cosine of the position angle
+    double tsx, tsr, tse; // TAPERED_SINC: the sinc's argument over pi per degree, 1 / (pi tsx), the taper's base-2 exponent per d^2
+    int tsok;             // series, TAPERED_SINC, and the taper stays within 2^-1000 and 2^1000 (exp2_small)
 };
 
 namespace {
@@ -248,6 +250,12 @@ inline GridArgs grid_args(const hcg_field *f, const PixPrep *prep, DevStats *sta
     a.g2scale = -0.5 * 1.4426950408889634 / (s0 * s1);
     a.g2ok = f->kernel_type == HCG_GAUSS2D && a.series &&
              -a.g2scale * f->sphere_radius * f->sphere_radius * std::max(s0, s1) * 1.01 < 1000.0;
+    a.tsx = 1.0 / std::fabs(f->kparam0 * f->kparams[2]);
+    a.tsr = 1.0 / (kPi * a.tsx);
+    const double tp = kPi / (f->kparam0 * f->kparams[1]);
+    a.tse = (f->taper_fix ? -1.4426950408889634 : 1.4426950408889634) * tp * tp;
+    a.tsok = f->kernel_type == HCG_TAPERED_SINC && a.series && a.tsx > 1e-100 && a.tsx < 1e100 &&
+             std::fabs(a.tse) * f->sphere_radius * f->sphere_radius * 1.01 < 1000.0;
     a.hlo32 = (float)(a.hlo * (1.0 - 2e-7));
     a.hhi32 = (float)(a.hhi * (1.0 + 2e-7));
     a.n = f->n;
@@ -750,13 +758,17 @@ __device__ __noinline__ double pair_band(const GridArgs &a, const PixPrep *P, ui
 // that is not accepted costs a select, not a branch. MODE kPairUnit: GAUSS1D
 // with unit-weight samples (F32: the FP32 Gaussian of the series; else
 // exp2_small), where the haversine rounded to FP32 decides all but the pairs
-// within 2e-7 of the cutoff, relative.
-enum { kPairGeneral = 0, kPairUnit = 1, kPairOther = 2 };  // kPairOther: kernels other than GAUSS1D
+// within 2e-7 of the cutoff, relative. kPairEllipse, kPairSinc: GAUSS2D and
+// TAPERED_SINC on small radii and with weights in range; kPairSlow: those kernels
+// beyond, TAPERED_SINC's accepted pairs one by one out of line (pair_band; in line
+// for all four pixels, accepted or not, a single-channel map of 200 x 120 pixels
+// under a beam of 3.3 degrees took 2.85 ms, 1.96 ms so).
+enum { kPairGeneral = 0, kPairUnit = 1, kPairEllipse = 2, kPairSinc = 3, kPairSlow = 4 };
 template <bool F32, int MODE>
 __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P, uint32_t nx, const PixHalf q[4],
                                              const double cb1[4], const double2 &sl2, const double2 &sb2, double win,
                                              uint32_t idx, const bool in[4], double w[4], float wf[4], bool nz[4]) {
-    constexpr bool GEN = MODE == kPairOther;
+    constexpr bool GEN = MODE >= kPairEllipse;
     PairHav v[4];
     bool acc[4];
     unsigned band = 0;
@@ -798,7 +810,22 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
                 const float gs = gauss_series_f32((float)v[i].h, a.x2c);
                 w[i] = acc[i] ? win * (double)gs : 0.0;
             }
-        } else if (GEN && a.g2ok) {
+        } else if (MODE == kPairSlow && a.ktype == HCG_GAUSS2D) {
+            double d2[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d2[i] = pair_d2(a, acc[i] ? v[i].h : 0.0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                double n2;
+                const double num = ellipse(a, q[i], cb1[i], v[i], sl2, sb2, n2), k = gauss2d(a, num, n2, d2[i]);
+                w[i] = acc[i] ? win * (F32 ? (double)(float)k : k) : 0.0;
+            }
+        } else if (MODE == kPairSlow) {
+            for (int i = 0; i < 4; ++i) {
+                if (acc[i]) band |= 1u << i;
+                w[i] = 0.0;
+            }
+        } else if (MODE == kPairEllipse) {
             // GAUSS2D, its weights in range: the four pixels' chains side by side
             // (through kernel_other, a division and a call of exp a pixel in turn,
             // the weight pass of 150,001 samples on 251 x 203 pixels took 148 us;
@@ -817,7 +844,26 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
                 const double k = exp2_small(t[i]);  // of a pair beyond the cutoff: not used
                 w[i] = acc[i] ? win * (F32 ? (double)(float)k : k) : 0.0;
             }
-        } else if (!F32 && !GEN && a.exp2ok) {
+        } else if (MODE == kPairSinc) {
+            // TAPERED_SINC, its taper in range: sin(x) / x with x = pi y, and the
+            // taper from d^2, so that a pair takes one root's reciprocal and no
+            // division (256,456 samples on 85 x 75 pixels, one channel: 300 us; 908
+            // with four divisions, a sine and an exponential through kernel_at)
+            double y[4], ry[4], t[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double d2 = series_d2(v[i].h), r = rsqrt(d2);
+                y[i] = d2 * r * a.tsx;
+                ry[i] = r * a.tsr;
+                t[i] = d2 * a.tse;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double sinc = y[i] * kPi >= 1e-10 ? sinpi(y[i]) * ry[i] : 1.0;
+                const double k = sinc * exp2_small(t[i]);  // of a pair beyond the cutoff: not used
+                w[i] = acc[i] ? win * (F32 ? (double)(float)k : k) : 0.0;
+            }
+        } else if (!F32 && a.exp2ok) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const double k = exp2_small(exponent2(a, v[i].h));
@@ -829,7 +875,7 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
             for (int i = 0; i < 4; ++i) d2[i] = pair_d2(a, acc[i] ? v[i].h : 0.0);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const double k = kernel_at<F32, GEN>(a, q[i], GEN ? cb1[i] : 0.0, v[i], sl2, sb2, win, d2[i]);
+                const double k = kernel_at<F32, false>(a, q[i], 0.0, v[i], sl2, sb2, win, d2[i]);
                 w[i] = acc[i] ? k : 0.0;
             }
         }
@@ -855,10 +901,12 @@ __device__ __forceinline__ void pair_weights(const GridArgs &a, const PixPrep *P
 inline bool table_windows(const GridArgs &a) { return a.ptab != nullptr; }
 // The single-channel and the multi-channel pair mode of a field.
 inline int pair_mode1(const hcg_field *f, const GridArgs &a) {
-    return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.exp2ok ? kPairUnit : kPairGeneral;
+    if (f->kernel_type != HCG_GAUSS1D) return a.g2ok ? kPairEllipse : a.tsok ? kPairSinc : kPairSlow;
+    return a.unit_w && a.exp2ok ? kPairUnit : kPairGeneral;
 }
 inline int pair_mode(const hcg_field *f, const GridArgs &a) {
-    return f->kernel_type != HCG_GAUSS1D ? kPairOther : a.unit_w && a.w32ok ? kPairUnit : kPairGeneral;
+    if (f->kernel_type != HCG_GAUSS1D) return a.g2ok ? kPairEllipse : a.tsok ? kPairSinc : kPairSlow;
+    return a.unit_w && a.w32ok ? kPairUnit : kPairGeneral;
 }
 
 // Sums of four values over a warp's lanes: lanes 8q .. 8q + 7 return value q's
@@ -923,11 +971,11 @@ __device__ __forceinline__ void group_load(GroupShared &S, const PixPrep *__rest
 // samples on 1200 x 1200 pixels: 1524 -> 1424 us single channel, 945 -> 898 us
 // for the entries; copies through shared memory or ring ends kept as bits there
 // cost as many instructions as they saved).
-template <bool F32, int MODE, typename BODY>
+template <bool F32, int MODE, int PARTS = 1, typename BODY>
 __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s_h, const double *s_cb1,
                                              GroupRecords &S, uint64_t pix0, uint32_t nx, const uint32_t lo[4],
                                              const uint32_t hi[4], uint32_t shift, const float *__restrict__ data,
-                                             uint32_t cstride, BODY body) {
+                                             uint32_t cstride, BODY body, uint32_t part = 0) {
     const int lane = threadIdx.x & 31;
     uint32_t glo = 0xffffffffu, ghi = 0;
 #pragma unroll
@@ -969,8 +1017,9 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
         nsb = __ldg(a.half + a.n + idx);
         if (!F32) nx1 = __ldg(data + (uint64_t)idx * cstride);
     };
-    if (total) fetch(0);
-    for (uint32_t tb = 0; tb < total; tb += 32) {
+    const uint32_t tb0 = PARTS > 1 ? 32 * part : 0;
+    if (total > tb0) fetch(tb0);
+    for (uint32_t tb = tb0; tb < total; tb += 32 * PARTS) {
         // the pixels' constants are read anew each round (the barrier keeps the
         // compiler from holding their 40 registers, which cost a third of the warps)
         __syncwarp();
@@ -979,7 +1028,7 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             ph[q] = s_h[q];
-            cb1[q] = MODE == kPairOther ? s_cb1[q] : 0.0;  // only the other kernels take it
+            cb1[q] = MODE == kPairEllipse || MODE == kPairSlow ? s_cb1[q] : 0.0;  // only the ellipse takes it
         }
         const bool act = tb + lane < total;
         const uint4 ra = S.ra[r], rb = S.rb[r];
@@ -987,7 +1036,7 @@ __device__ __forceinline__ void group_rounds(const GridArgs &a, const PixHalf *s
         const uint32_t idx = ra.x + (act ? tb + lane : tb);
         const double2 sl2 = nsl, sb2 = nsb;
         const float x = nx1;
-        if (tb + 32 < total) fetch(tb + 32);
+        if (tb + 32 * PARTS < total) fetch(tb + 32 * PARTS);
         const double win = MODE == kPairUnit || a.unit_w ? 1.0 : __ldg(a.w + idx);
         const bool in[4] = {act && idx - ra.z < ra.w, act && idx - rb.x < rb.y, act && idx - rb.z < rb.w,
                             act && idx - rc.x < rc.y};
@@ -1045,12 +1094,18 @@ __device__ __forceinline__ void flush_counts(const PairCounts &c, DevStats *stat
 
 // Single channel: one warp per 2x2 group of pixels, FP64 throughout: the
 // windows (a ring per lane, four pixels each), every union candidate against
-// the four pixels, normalise. Warp-collective.
+// the four pixels, normalise. Warp-collective. kPairSlow: the block's warps share
+// one group, every kGroupWarps-th round of candidates each (a pair's evaluation
+// is long, so that few pixels leave most of the GPU idle, and the windows formed
+// by each warp cost little beside it); block-collective.
+template <int MODE>
+constexpr int kGrid1Parts = MODE == kPairSlow ? kGroupWarps : 1;
 template <int MODE, bool TABLES>
 __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint32_t ny,
                                            const float *__restrict__ data, uint32_t cstride, float *__restrict__ out,
                                            float *__restrict__ wout, uint64_t grp, GroupShared &S, PairCounts &pc) {
-    const int lane = threadIdx.x & 31;
+    constexpr int PARTS = kGrid1Parts<MODE>;
+    const int lane = threadIdx.x & 31, part = PARTS > 1 ? threadIdx.x >> 5 : 0;
     const uint32_t gx = (nx + 1) / 2, gyi = (uint32_t)(grp / gx), gxi = (uint32_t)(grp % gx);
     const bool xin = 2 * gxi + 1 < nx, yin = 2 * gyi + 1 < ny;
     const uint64_t pix0 = (uint64_t)(2 * gyi) * nx + 2 * gxi;
@@ -1064,7 +1119,7 @@ __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint3
             nr = G.r1 - G.r0 + 1;
             group_lane_windows<TABLES>(a, G, G.r0 + rb + lane, pix0, nx, lo, hi, ref, skips);
         }
-        group_rounds<false, MODE>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u, data, cstride,
+        group_rounds<false, MODE, PARTS>(a, S.h, S.cb1, S.rec, pix0, nx, lo, hi, 0u, data, cstride,
                                   [&](float v, uint32_t, const double w[4], const float[4], const bool nz[4]) {
             const double x = (double)v;
 #pragma unroll
@@ -1075,11 +1130,25 @@ __device__ __forceinline__ void grid1_item(const GridArgs &a, uint32_t nx, uint3
                     ++within;
                 }
             }
-        });
+        }, part);
     }
-    pc.add(ref, within, skips);
-    const double A = warp_sum4(acc), W = warp_sum4(ws);
+    pc.add(part == 0 ? ref : 0, within, part == 0 ? skips : 0);
+    double A = warp_sum4(acc), W = warp_sum4(ws);
     const int q = lane >> 3;
+    if (PARTS > 1) {
+        __shared__ double s_sum[PARTS][8];
+        if ((lane & 7) == 0) {
+            s_sum[part][q] = A;
+            s_sum[part][4 + q] = W;
+        }
+        __syncthreads();
+        if (part != 0) return;
+        A = W = 0.0;
+        for (int p = 0; p < PARTS; ++p) {
+            A += s_sum[p][q];
+            W += s_sum[p][4 + q];
+        }
+    }
     if ((lane & 7) == 0 && (!(q & 1) || xin) && (!(q >> 1) || yin)) {
         const uint64_t p = pix0 + (q & 1) + (uint64_t)(q >> 1) * nx;
         out[p] = (float)(A / W);

@@ -45,13 +45,14 @@ __global__ void k_noalloc_prep(HpxParams h, uint64_t firstring, uint64_t usedrin
 }
 
 template <int MODE, bool TABLES>  // as pair_weights, group_windows_any
-__global__ void __launch_bounds__(kGroupThreads, MODE == kPairOther ? 4 : kGroupCtas) k_noalloc_grid(const __grid_constant__ GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
+__global__ void __launch_bounds__(kGroupThreads, MODE >= kPairEllipse ? 4 : kGroupCtas) k_noalloc_grid(const __grid_constant__ GridArgs a, uint32_t nx, uint32_t ny, uint64_t ngroups,
                                                           const float *__restrict__ data, uint32_t cstride,
                                                           float *__restrict__ out, float *__restrict__ wout) {
     __shared__ GroupShared S[kGroupWarps];
     PairCounts pc;
     const int warp = threadIdx.x >> 5;
-    const uint64_t grp = blockIdx.x * (uint64_t)kGroupWarps + warp;
+    constexpr int kGroups = kGroupWarps / kGrid1Parts<MODE>;  // of a block
+    const uint64_t grp = blockIdx.x * (uint64_t)kGroups + warp % kGroups;
     if (grp < ngroups) grid1_item<MODE, TABLES>(a, nx, ny, data, cstride, out, wout, grp, S[warp], pc);
     flush_counts(pc, a.stats);
 }
@@ -133,12 +134,15 @@ extern "C" hcg_status hcg_grid_noalloc(hcg_context *ctx, const hcg_field *field,
         for (auto &ev : ctx->evp) cudaEventRecord(ev, s);
         const GridArgs a = grid_args(field, prep, ctx->d_stats);
         const uint64_t ngroups = (uint64_t)((target->nx + 1) / 2) * ((target->ny + 1) / 2);
-        const unsigned nblk = (unsigned)((ngroups + kGroupWarps - 1) / kGroupWarps);
         const int mode = pair_mode1(field, a);
+        const unsigned nblk = (unsigned)(mode == kPairSlow ? ngroups : (ngroups + kGroupWarps - 1) / kGroupWarps);
         const bool tab = table_windows(a);
-        auto grid1 = mode == kPairOther  ? (tab ? k_noalloc_grid<kPairOther, true> : k_noalloc_grid<kPairOther, false>)
-                     : mode == kPairUnit ? (tab ? k_noalloc_grid<kPairUnit, true> : k_noalloc_grid<kPairUnit, false>)
-                                         : (tab ? k_noalloc_grid<kPairGeneral, true> : k_noalloc_grid<kPairGeneral, false>);
+        auto pick = [&](auto table, auto any) { return tab ? table : any; };
+        auto grid1 = mode == kPairSlow      ? k_noalloc_grid<kPairSlow, false>
+                     : mode == kPairEllipse ? pick(k_noalloc_grid<kPairEllipse, true>, k_noalloc_grid<kPairEllipse, false>)
+                     : mode == kPairSinc    ? pick(k_noalloc_grid<kPairSinc, true>, k_noalloc_grid<kPairSinc, false>)
+                     : mode == kPairUnit    ? pick(k_noalloc_grid<kPairUnit, true>, k_noalloc_grid<kPairUnit, false>)
+                                            : pick(k_noalloc_grid<kPairGeneral, true>, k_noalloc_grid<kPairGeneral, false>);
         grid1<<<nblk, kGroupThreads, 0, s>>>(a, target->nx, target->ny, ngroups, field->d_spec, field->cstride, cube,
                                              weights_out);
         cudaEventRecord(ctx->ev1, s);
