@@ -710,54 +710,53 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
             float v[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * sc[cb * 32 + i];
-            if (J.ostride == 0) {
+            // The sums of the segments before come back sixteen at a time: a
+            // load behind each store was a round trip to L2 a channel (256
+            // channels, three segments: 90 us a segment, half of it so).
+            float *const row = J.out + p * J.ostride + c0;
+            const bool v8 = J.ostride && (J.ostride & 7) == 0 && c0 + 32 <= J.nchan && (((uintptr_t)J.out) & 31) == 0;
+            const bool v4 = J.ostride && (J.ostride & 3) == 0 && c0 + 32 <= J.nchan && (((uintptr_t)J.out) & 15) == 0;
 #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    if (c0 + i < J.nchan) {
-                        float *d = J.out + (uint64_t)(c0 + i) * P + p;
-                        *d = (q ? *d + v[i] : v[i]) * f;
-                    }
-            } else {
-                float *dst = J.out + p * J.ostride + c0;
-                if ((J.ostride & 7) == 0 && c0 + 32 <= J.nchan && (((uintptr_t)J.out) & 31) == 0) {
-                    // 32-byte accesses: each store fills whole sectors of the pixel's row
+            for (int h = 0; h < 32; h += 16) {
+                float *const at = J.ostride ? row + h : J.out + (uint64_t)(c0 + h) * P + p;
+                const uint64_t step = J.ostride ? 1 : P;
+                float o[16];
+                auto eight = [&](int i) -> float (&)[8] { return *reinterpret_cast<float (*)[8]>(o + 8 * i); };
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float o[8];
+                for (int i = 0; i < 16; ++i) o[i] = 0.f;
+                if (q) {
+                    if (v8) {  // 32-byte accesses: each store fills whole sectors of the pixel's row
+                        ld_global_v8(at, eight(0));
+                        ld_global_v8(at + 8, eight(1));
+                    } else if (v4) {
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) o[u] = v[8 * i + u];
-                        if (q) {
-                            float b[8];
-                            ld_global_v8(dst + 8 * i, b);
-#pragma unroll
-                            for (int u = 0; u < 8; ++u) o[u] += b[u];
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 t = reinterpret_cast<const float4 *>(at)[i];
+                            o[4 * i] = t.x;
+                            o[4 * i + 1] = t.y;
+                            o[4 * i + 2] = t.z;
+                            o[4 * i + 3] = t.w;
                         }
+                    } else {
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) o[u] *= f;
-                        st_global_v8(dst + 8 * i, o);
+                        for (int i = 0; i < 16; ++i)
+                            if (c0 + h + i < J.nchan) o[i] = at[i * step];
                     }
-                } else if ((J.ostride & 3) == 0 && c0 + 32 <= J.nchan && (((uintptr_t)J.out) & 15) == 0) {
-                    float4 *d4 = reinterpret_cast<float4 *>(dst);
+                }
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float4 o = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                        if (q) {
-                            const float4 b = d4[i];
-                            o.x += b.x;
-                            o.y += b.y;
-                            o.z += b.z;
-                            o.w += b.w;
-                        }
-                        o.x *= f;
-                        o.y *= f;
-                        o.z *= f;
-                        o.w *= f;
-                        d4[i] = o;
-                    }
+                for (int i = 0; i < 16; ++i) o[i] = (q ? o[i] + v[h + i] : v[h + i]) * f;
+                if (v8) {
+                    st_global_v8(at, eight(0));
+                    st_global_v8(at + 8, eight(1));
+                } else if (v4) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        reinterpret_cast<float4 *>(at)[i] =
+                            make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        if (c0 + i < J.nchan) dst[i] = (q ? dst[i] + v[i] : v[i]) * f;
+                    for (int i = 0; i < 16; ++i)
+                        if (c0 + h + i < J.nchan) at[i * step] = o[i];
                 }
             }
         }
