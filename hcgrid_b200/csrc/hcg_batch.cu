@@ -60,6 +60,7 @@ enum { Q_TILE = 0, Q_GEOM, Q_ACC, Q_C1, Q_N };
 
 struct BatchHdr {
     uint32_t njobs;
+    uint32_t wparts;  // blocks that share a tile in the weight pass
     unsigned long long tot_pix, tot_grp, tot_tile, tot_acc, tot_c1;
     unsigned long long tot_tc[kKbShapes];  // items of each tensor-core shape
     const uint32_t *tc_list;               // jobs of shape k: tc_list[tc_off[k] .. tc_off[k + 1])
@@ -76,6 +77,14 @@ struct BatchHdr {
 };
 
 constexpr int kPersistPerSM = 8;
+
+// Blocks that share a tile's groups in the weight pass, by the batch's tiles (4 x
+// 148 blocks are resident; each repeats the tile's loads). Whole passes on the FP32
+// engine with 1 / 2 / 4 / 8 blocks a tile: 120 tiles of 4,000 samples a beam 1863 /
+// 1458 / 1239 / 1192 us, 288 of 1,000 855 / 738 / 744 / 745, 1,024 of 1,000 2069 /
+// 2040 / 2032 / 2048; on the tensor cores 748 tiles 457 / 441 / 435 / 455, 2,048
+// tiles 729 / 733 / 768 / 835.
+inline uint32_t weight_parts(uint64_t tiles) { return tiles >= 8 * 148 ? 1 : tiles >= 4 * 148 ? 2 : tiles >= 148 ? 4 : 8; }
 
 // Job owning item `it` of a phase: last job whose base is <= it.
 template <typename F>
@@ -169,8 +178,9 @@ __global__ void __launch_bounds__(256) kb_group_count(BatchHdr *H, const JobDesc
 // The weight pass, a tile per item. The pool must hold the tile's entries;
 // otherwise its groups are skipped and reported (no entries recorded: the pass is
 // replayed once the pool has grown). 64 observations of 10,000 samples: 177 us,
-// 213 us with descriptors read from global memory (the tile pass 118 and 150 us);
-// halves or quarters of tiles for an even last round repeat the tile's loads, 220 us.
+// 213 us with descriptors read from global memory (the tile pass 118 and 150 us).
+// Where the batch's tiles are fewer than the resident blocks, several blocks share
+// a tile (weight_parts).
 __global__ void __launch_bounds__(kWeightThreads, 4) kb_group(BatchHdr *H, const JobDesc *__restrict__ jobs, DevStats *stats) {
     __shared__ TileGroupShared S;
     __shared__ JobGeoShared SJ;
@@ -178,6 +188,8 @@ __global__ void __launch_bounds__(kWeightThreads, 4) kb_group(BatchHdr *H, const
     int cur = -1;
     for (;;) {
         unsigned long long it = block_fetch(H, Q_GEOM);
+        const uint32_t parts = H->wparts, part = (uint32_t)(it % parts);
+        it /= parts;
         if (it >= H->tot_tile) break;
         int j = find_job(jobs, H->njobs, it, [](const JobDesc &d) { return d.tile_base; });
         const JobDesc &D = jobs[j];
@@ -196,9 +208,9 @@ __global__ void __launch_bounds__(kWeightThreads, 4) kb_group(BatchHdr *H, const
             continue;
         }
         if (J.a.unit_w && J.a.w32ok)
-            group_tile_item<kPairUnit>(J.a, J.g, D.off, H->e_idx, H->e_w, D.cnt, D.wsum, J.T, true, tile, 0, 1, S, pc);
+            group_tile_item<kPairUnit>(J.a, J.g, D.off, H->e_idx, H->e_w, D.cnt, D.wsum, J.T, true, tile, part, parts, S, pc);
         else
-            group_tile_item<kPairGeneral>(J.a, J.g, D.off, H->e_idx, H->e_w, D.cnt, D.wsum, J.T, true, tile, 0, 1, S, pc);
+            group_tile_item<kPairGeneral>(J.a, J.g, D.off, H->e_idx, H->e_w, D.cnt, D.wsum, J.T, true, tile, part, parts, S, pc);
     }
     flush_counts(pc, stats);
 }
@@ -632,6 +644,7 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
         BatchHdr &h = *B.h_hdr;
         memset(&h, 0, sizeof h);
         h.njobs = njobs;
+        h.wparts = weight_parts(tile);
         h.tot_pix = pix;
         h.tot_grp = grp;
         h.tot_tile = tile;
