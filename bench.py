@@ -816,7 +816,7 @@ def config4_run(args):
            "launch_bound_blocks": tiny_out,
            "batch_tuning": {"classes": tuning, "how": "hcg_autotune_batch on the first window: per channel class, "
                             "each of the 4 shapes (0: 256 ch x 32 slots x 4 stages, 1: 256 x 64 x 2, "
-                            "2: 128 x 64 x 3, 3: 64 x 64 x 4) timed as one hcg_grid_batch of the class's "
+                            "2: 128 x 32 x 2, 3: 64 x 32 x 3) timed as one hcg_grid_batch of the class's "
                             "blocks, best of %d runs after a warm-up" % args.tune_reps},
            "gpu_launches": None, "e2e": None, "cpu_baseline": None}
     ctx.close()

@@ -703,8 +703,8 @@ cudaError_t grid_batch(hcg_context *ctx, uint32_t njobs, const hcg_job *jobs, st
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
     // Routing: jobs whose tiles overflowed the ring table, tensor-core jobs
     // with dense tiles (the single-job kernel evaluates their weights itself)
-    // or with tiles longer than one accumulation segment (the single-job
-    // kernels accumulate in segments), then the jobs with the most entries
+    // or with tiles of more than kTcOneSegmentSlots staged slots (kb_tc's narrow
+    // chunks are for short tiles; where the line would lie best is not measured), then the jobs with the most entries
     // until the rest fit the context's entry budget.
     fallback.assign(njobs, 0);
     unsigned long long total = 0;

@@ -18,8 +18,11 @@
 //   k_pixel_prep     per pixel: ring range and the phi half of loc2pix
 //   k_grid_1chan     one warp per 2x2 pixel group, candidates spread over
 //                    lanes, FP64
-//   k_group          one warp per 2x2 pixel group: FP64 weights written as
-//                    compact (sample, w[4]) entries
+//   k_tile_rings     one block per 16x8-pixel tile: windows, the tile's union,
+//                    candidate counts and entry offsets
+//   k_group          one block (or a half, a quarter) per tile, a warp per 2x2
+//                    group in turn: FP64 weights written as compact
+//                    (sample, w[4]) entries
 //   k_group_accum    one warp per group: FP32 channel accumulation from the
 //                    entries, 4 channels per lane, normalised on store
 #include <cuda_runtime.h>

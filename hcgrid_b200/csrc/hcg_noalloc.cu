@@ -12,7 +12,7 @@
 //
 // The scratch is the per-pixel setup (ring range and the phi half of the
 // window arithmetic, 88 bytes a pixel) in a file-scope __device__ array of
-// kNoAllocMaxPixels entries: 131072 pixels, 12 MiB, held by every GPU that
+// kNoAllocMaxPixels entries: 131072 pixels, 11 MiB, held by every GPU that
 // loads the library until the process exits. Host code may not pass the
 // array's name to a kernel (on the host it names a stand-in, not device
 // memory), so its device address is looked up once per device with
@@ -34,6 +34,8 @@ namespace hcg {
 namespace {
 
 constexpr uint64_t kNoAllocMaxPixels = 131072;
+
+static_assert(sizeof(PixPrep) * kNoAllocMaxPixels == 11u << 20, "the size the documentation states");
 
 static __device__ __align__(256) PixPrep g_noalloc_prep[kNoAllocMaxPixels];
 

@@ -19,7 +19,8 @@ namespace hcg {
 constexpr uint32_t kTcSegSlots = 896;
 // The one-item kernel (k_tile_tc) accumulates an item in one segment: it takes
 // tiles of at most this many staged slots (longer ones go to the persistent
-// kernels, and jobs that hold one leave a batch).
+// kernels, and jobs that hold one leave a batch, whose kernel could take them in
+// segments as well).
 constexpr uint32_t kTcOneSegmentSlots = 1536;
 
 // segments of an item of `nchunks` chunks of `kc` slots, and the end of segment q

@@ -630,8 +630,9 @@ __device__ __forceinline__ void tc_item(TcShared &S, const TcJob &J, const CUten
 // role walks the sequence on its own, coupled to the others only through
 // mbarriers: the producer runs ahead into the next item while the MMAs of the
 // current one run, and four epilogue warps (6-9) drain item i's accumulator
-// while the MMAs of item i+1 fill the other one (two TMEM accumulators of 256
-// columns).
+// while the MMAs of item i+1 fill the other one (two TMEM accumulators of
+// kTmemCols columns: the shapes of up to 128 channels fit two CTAs an SM, which the
+// batch kernel runs).
 constexpr int kTcPersistThreads = 320;
 
 struct TcPShared {

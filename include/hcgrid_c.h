@@ -376,7 +376,7 @@ hcg_status hcg_synchronize(hcg_context *ctx);
  * stall of cudaMalloc/cudaFree; or a host application whose own allocator
  * already holds the GPU's memory and lends the library only the inputs and
  * outputs. Its per-pixel scratch is a fixed array inside the library of
- * 131072 pixels (12 MiB, held on every GPU that loads the library until the
+ * 131072 pixels (11 MiB, held on every GPU that loads the library until the
  * process exits): larger targets are rejected with HCG_EINVAL. cube and
  * weights_out (optional) are device buffers of nx*ny floats on the
  * context's device, and field and target must belong to a context on that
