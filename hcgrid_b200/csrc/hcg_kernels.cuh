@@ -354,7 +354,9 @@ __device__ __forceinline__ GroupGeo group_geo(GET get) {
         const double lp = P->l1 - 2.0 * kPi * floor(P->l1 * (0.5 / kPi));
         G.lmin = fmin(G.lmin, lp);
         G.lmax = fmax(G.lmax, lp);
-        const bool past = !(P->icb1 >= 0.f);  // past a pole: no bound, in latitude neither
+        // past a pole: no bound, in latitude neither; a blank pixel (NaN) accepts
+        // nothing and leaves the others theirs
+        const bool past = P->icb1 < 0.f;
         G.bmin = fmin(G.bmin, past ? -1e300 : P->b1);
         G.bmax = fmax(G.bmax, past ? 1e300 : P->b1);
         G.icb = past ? __int_as_float(0x7f800000) : fmaxf(G.icb, P->icb1);
