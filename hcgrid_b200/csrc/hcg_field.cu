@@ -1040,10 +1040,16 @@ cudaError_t permute_spectra(hcg_context *ctx, hcg_field *f, const float *d_in, u
         if (nchan > 1)
             e = cudaMemsetAsync(mx.amax, 0, cstride * sizeof(float) + 2 * sizeof(unsigned long long), s);
         if (e != cudaSuccess) return e;
-        // a row a thread up to eight blocks an SM, then longer blocks up to 1024 rows
+        // Two to eight blocks an SM, by 160 KB of spectra a block (the blocks of a
+        // channel take turns at its maximum), up to 1024 rows. 200,000 samples, a
+        // call with eight an SM / by this rule / without maxima: 2 channels 32.5 /
+        // 25 / 30 us, 64 channels 51 / 41 / 45, 128 channels 65 / 58 / 55; 500,000 x
+        // 256 channels 193 / 193 / 166 (a pass of its own for the maxima: 90).
         const uint32_t tpr = row_threads(cstride), cblk = (cstride + 127) / 128;
+        const uint64_t blocks = std::max<uint64_t>(
+            148 * 2, std::min<uint64_t>(148 * 8, f->n * cstride * sizeof(float) / 160000));
         const uint32_t rows =
-            (uint32_t)std::max<uint64_t>(256 / tpr, std::min<uint64_t>(1024, f->n * cblk / (148 * 8)));
+            (uint32_t)std::max<uint64_t>(256 / tpr, std::min<uint64_t>(1024, f->n * cblk / blocks));
         k_permute_rows<<<dim3((unsigned)((f->n + rows - 1) / rows), cblk), 256, 0, s>>>(
             f->n, nchan, cstride, tpr, rows, f->d_perm, d_in, f->d_spec, mx.amax, mx.bad);
         f->amax_set = nchan > 1;
