@@ -711,6 +711,13 @@ __device__ __forceinline__ void tc_epilogue_direct(SH &S, const TcJob &J, uint64
             float v[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * sc[cb * 32 + i];
+            if (J.ostride == 0 && q == 0) {  // planes, nothing to add: one address a channel, no order to keep
+                float *d = J.out + (uint64_t)c0 * P + p;
+#pragma unroll
+                for (int i = 0; i < 32; ++i, d += P)
+                    if (c0 + i < J.nchan) *d = v[i] * f;
+                continue;
+            }
             // The sums of the segments before come back sixteen at a time: a
             // load behind each store was a round trip to L2 a channel (256
             // channels, three segments: 90 us a segment, half of it so).
