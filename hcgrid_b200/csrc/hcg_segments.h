@@ -2,8 +2,8 @@
 //
 // The tensor cores' FP32 accumulation drops low bits of the products it adds
 // (the sums come out low by up to ~2^-24 of the running sum per MMA), so long K
-// loops drift. An item of more than one and a half times kTcSegSlots staged slots
-// is accumulated in equal segments of at most kTcSegSlots, each in a fresh
+// loops drift. An item of more than kTcWholeSlots staged slots is accumulated in
+// equal segments of kTcSegSlots at most (up to a chunk), each in a fresh
 // accumulator (the two TMEM halves in turn), and the epilogue adds the segments
 // with round-to-nearest FP32 adds (in the cube buffer) before it normalises them.
 // What drifts is the slots with weight: the closer the staged list fits the beam,
@@ -16,7 +16,7 @@
 
 namespace hcg {
 
-constexpr uint32_t kTcSegSlots = 896;
+constexpr uint32_t kTcSegSlots = 992, kTcWholeSlots = 1344;
 // The one-item kernel (k_tile_tc) accumulates an item in one segment: it takes
 // tiles of at most this many staged slots (longer ones go to the persistent
 // kernels, and jobs that hold one leave a batch, whose kernel could take them in
@@ -25,8 +25,8 @@ constexpr uint32_t kTcOneSegmentSlots = 1536;
 
 // segments of an item of `nchunks` chunks of `kc` slots, and the end of segment q
 HCG_HD uint32_t tc_segments(uint32_t kc, uint32_t nchunks) {
-    const uint32_t seg = kTcSegSlots / kc;  // chunks per segment
-    return nchunks > seg + seg / 2 ? (nchunks + seg - 1) / seg : 1;
+    const uint64_t slots = (uint64_t)nchunks * kc;
+    return slots > kTcWholeSlots ? (uint32_t)((slots + kTcSegSlots - 1) / kTcSegSlots) : 1;
 }
 HCG_HD uint32_t tc_segment_end(uint32_t nchunks, uint32_t nseg, uint32_t q) {
     return (uint32_t)((uint64_t)nchunks * (q + 1) / nseg);

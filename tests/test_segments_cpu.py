@@ -1,6 +1,6 @@
 """The accumulation segments of the tensor-core kernels: an item is either whole,
-of at most 1,344 staged slots, or falls into segments of at most 896, none empty,
-whose lengths differ by a chunk at most and which cover it."""
+of at most 1,344 staged slots, or falls into segments of at most 992, rounded up to
+a chunk, none empty, whose lengths differ by a chunk at most and which cover it."""
 import ctypes as C
 import os
 import subprocess
@@ -32,5 +32,5 @@ def test_segments_are_short_and_equal(lib, kc):
         for q in qs:
             begin = lib.hs_end(n, nseg, q - 1) if q else 0
             size.append(lib.hs_end(n, nseg, q) - begin)
-        assert nseg == 1 or (min(size) >= 1 and max(size) - min(size) <= 1 and max(size) * kc <= 896)
+        assert nseg == 1 or (min(size) >= 1 and max(size) - min(size) <= 1 and (max(size) - 1) * kc < 992)
         assert lib.hs_end(n, nseg, nseg - 1) == n
