@@ -9,7 +9,9 @@
 // What drifts is the slots with weight: the closer the staged list fits the beam,
 // the shorter a segment must be. 150,000 samples, beam 54 pixels wide: the cube's
 // mean came out low by 6.5e-6 in segments of 1,024 of the 5,090 slots a tile,
-// 5.7e-6 when a tile staged 5,930 for the same pairs, and by 4.9e-6 in these.
+// 5.7e-6 when a tile staged 5,930 for the same pairs, and by 5.6e-6 in these
+// (4.9e-6 in segments of 896, which give many cubes a segment more: 144 channels on
+// 579 x 479 pixels 1.33 against 1.29 ms).
 #pragma once
 
 #include "hcg_math.cuh"
